@@ -342,10 +342,10 @@ __device__ __forceinline__ void clear_bits_range(uint32_t* bits, int64_t nwords,
 
 
 // Wavefront ray tracing of one ray set, three kernel kinds:
-//  * k_cand: one warp per batch of 32 patches, whose records the lanes load together; then, patch
+//  * k_cand: one warp per batch of 4 to 32 patches, whose records the lanes load together; then, patch
 //    by patch, one lane per pixel row of the patch's pixel window (the reference's CELL_CULLING
 //    window, k_windows): each row's rays that pass the bounding-box and equatorial-disc test form
-//    an interval, found by binary search with the exact test.  One atomic per list and batch
+//    an interval, found by moving a predicted end with the exact test.  One atomic per list and batch
 //    reserves the slots; the (ray, patch) pairs follow in row-major order, in the sphere list
 //    (atoms and probes) or the torus list; a patch's candidates stay contiguous, so the
 //    intersection kernels read its record once per warp;
@@ -355,7 +355,7 @@ __device__ __forceinline__ void clear_bits_range(uint32_t* bits, int64_t nwords,
 //    through a per-ray atomic counter;
 //  * k_fill: one CTA per 32x4 ray tile loads each ray's hits, sorts them and performs the
 //    interval fill.
-// A k_cand batch of 32 patches, staged in shared memory (structure of arrays, one entry per lane
+// A k_cand batch of up to 32 patches, staged in shared memory (structure of arrays, one entry per lane
 // of the warp that loaded it): the operands of candidate() rounded as there, the pixel window
 // and where the patch's rays start.
 struct CandBatch {
@@ -372,8 +372,10 @@ struct CandBatch {
 //   Low(m)  = pa(m) >= lo_fd && (dx < 0 || disc(dx))   holds on an upper set of m,
 //   High(m) = pa(m) <= hi_fd && (dx > 0 || disc(dx))   holds on a lower set of m,
 // and candidate() (box in both axes, then disc) passes exactly when the row's box test holds and
-// Low(m) && High(m).  The row's candidates are the interval [first Low, last High] of the
-// window, found by two binary searches with the exact double-precision tests.
+// Low(m) && High(m).  The row's candidates are the interval [first Low, last High] of the window.
+// Both ends start at the pixel that an FP32 half chord predicts and are moved with the exact
+// double-precision tests until the test flips there, which the monotone tests make the same pixel
+// that a search of the whole window finds, in 4 tests instead of 2 log2(window).
 __device__ __forceinline__ int cand_row(const CandBatch& q, int p, int row, int* a) {
   *a = 0;
   const double pld = (q.mn_ld[p] + (double)(q.n0[p] + row) * q.side[p]) + q.delta[p];
@@ -384,26 +386,34 @@ __device__ __forceinline__ int cand_row(const CandBatch& q, int p, int row, int*
   const double dy2 = dy * dy;
   // skin cells other than Del0 have no equatorial-disc test (src/SkinSurface.cpp:3578-3587)
   const bool disc = q.disc[p];
-  int lo = q.m0[p], hi = q.m1[p] + 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    const double pa = (mn + (double)mid * side) + delta;
-    const double dx = cf - pa;
-    const bool low = !(pa < lo_fd) && (!disc || dx < 0. || !(dx * dx + dy2 > r2));
-    if (low) hi = mid;
-    else lo = mid + 1;
+  const int m0 = q.m0[p], m1 = q.m1[p];
+  double from = lo_fd, to = hi_fd;
+  if (disc) {
+    if (dy2 > r2 && cf == cf) return 0;  // no pixel of the row passes the disc test
+    const double h = (double)sqrtf((float)(r2 - dy2));
+    from = fmax(from, cf - h);
+    to = fmin(to, cf + h);
   }
+  const double inv = (double)(1.0f / (float)side), org = mn + delta;
+  const auto low = [&](int m) {
+    const double pa = (mn + (double)m * side) + delta;
+    const double dx = cf - pa;
+    return !(pa < lo_fd) && (!disc || dx < 0. || !(dx * dx + dy2 > r2));
+  };
+  const auto high = [&](int m) {
+    const double pa = (mn + (double)m * side) + delta;
+    const double dx = cf - pa;
+    return !(pa > hi_fd) && (!disc || dx > 0. || !(dx * dx + dy2 > r2));
+  };
+  // the predictions are clamped as doubles: a box far outside the grid does not fit an int
+  int lo = (int)fmin(fmax(ceil((from - org) * inv), (double)m0), (double)m1 + 1.);
+  while (lo > m0 && low(lo - 1)) lo--;
+  while (lo <= m1 && !low(lo)) lo++;
+  int hi = (int)fmin(fmax(floor((to - org) * inv) + 1., (double)lo), (double)m1 + 1.);
+  while (hi > lo && !high(hi - 1)) hi--;
+  while (hi <= m1 && high(hi)) hi++;
   *a = lo;
-  hi = q.m1[p] + 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    const double pa = (mn + (double)mid * side) + delta;
-    const double dx = cf - pa;
-    const bool high = !(pa > hi_fd) && (!disc || dx > 0. || !(dx * dx + dy2 > r2));
-    if (!high) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo - *a;
+  return hi - lo;
 }
 
 // Smallest lane whose inclusive prefix v exceeds k (k below the warp total).
@@ -417,20 +427,33 @@ __device__ __forceinline__ int owner_lane(int v, int k) {
   return rr;
 }
 
-__global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co) {
+// Rows of a batch whose interval stays in shared memory between the counting and the writing pass
+// (first pixel relative to the window and count, 16 bits each); the others are found again.
+constexpr int kCandRows = 320;
+constexpr uint32_t kCandRowAgain = 0xffffffffu;
+
+// ppw: patches of a warp's batch (launch_trace picks it so that small patch sets fill the GPU).
+// Latency-bound (dependent double-precision tests, 5-step shuffles per row group), 12 % of the warps
+// resident with 32 patches per warp on a 20,000-atom cast: what counts is warps in flight.  Per
+// launch, 32 patches per warp and binary searches in both passes -> as it is here: 26 -> 5.7 us
+// (327 atoms, scale 2), 46 -> 8.8 us (2,000, scale 3), 77 -> 25 us (20,000, scale 4), 194 -> 179 us
+// (64 conformers, 580,000 patches, whose warps filled the GPU before).
+__global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co, int ppw) {
   __shared__ CandBatch s_batch[8];
+  __shared__ uint32_t s_row[8][kCandRows];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   CandBatch& q = s_batch[wib];
+  uint32_t* const rows = s_row[wib];
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t base = (blockIdx.x * (int64_t)(blockDim.x >> 5) + wib) * 32; base < C.P.n; base += warps * 32) {
-    // 1. the batch's 32 patches, one per lane
+  for (int64_t base = (blockIdx.x * (int64_t)(blockDim.x >> 5) + wib) * ppw; base < C.P.n; base += warps * ppw) {
+    // 1. the batch's patches, one per lane
     int H = 0;
     {
       const int64_t pid = base + lane;
       q.ty[lane] = 0;
       q.pid[lane] = (int)pid;
       const int32_t* w = C.P.win + 6 * pid;
-      if (pid < C.P.n && w[0] >= 0) {
+      if (lane < ppw && pid < C.P.n && w[0] >= 0) {
         const StructDev& S = C.B.s[C.B.patch_struct[pid]];
         const GridDev& g = S.g;
         const RaySet rs = make_ray_set(C.set, g);
@@ -484,7 +507,11 @@ __global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co) {
       const int row = kk - __shfl_sync(0xffffffffu, hexcl, p);
       const int hp = __shfl_sync(0xffffffffu, H, p);
       int a, cnt = 0;
-      if (k < R) cnt = cand_row(q, p, row, &a);
+      if (k < R) {
+        cnt = cand_row(q, p, row, &a);
+        const int rel = a - q.m0[p];
+        if (k < kCandRows) rows[k] = (cnt == 0) ? 0u : ((rel | cnt) >> 16 ? kCandRowAgain : (uint32_t)(rel << 16 | cnt));
+      }
       int cincl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -531,7 +558,15 @@ __global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co) {
       const int p = owner_lane(hincl, kk);
       const int row = kk - __shfl_sync(0xffffffffu, hexcl, p);
       int a = 0, cnt = 0;
-      if (k < R) cnt = cand_row(q, p, row, &a);
+      if (k < R) {
+        const uint32_t kept = k < kCandRows ? rows[k] : kCandRowAgain;
+        if (kept == kCandRowAgain) {
+          cnt = cand_row(q, p, row, &a);
+        } else {
+          a = q.m0[p] + (int)(kept >> 16);
+          cnt = (int)(kept & 0xffffu);
+        }
+      }
       int cincl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1153,9 +1188,15 @@ cudaError_t launch_trace(const PatchDev& P, const BatchDev& B, int set, int64_t 
   if (ev) cudaEventRecord(ev[0], s);
   if (P.n > 0) {
     const int wpb = tp.cand_threads / 32;
-    int64_t blocks = (P.n + 32 * wpb - 1) / (32 * wpb);
+    // patches per warp: 32 where the set fills 16 warps per SM that way, fewer (down to 4) below
+    // patches per warp: 32 where the set gives 64 warps per SM (a full SM) that way, fewer below,
+    // but no fewer than 4, whose rows fill the 32 lanes (skin, 97,000 patches: 238 us with 32, 213
+    // with 16 warps per SM as the line, 172 with 64)
+    const int64_t per = P.n / ((int64_t)sm_count() * 64);
+    const int ppw = per < 4 ? 4 : (per > 32 ? 32 : (int)per);
+    int64_t blocks = (P.n + ppw * wpb - 1) / (ppw * wpb);
     if (blocks > (int64_t)sm_count() * 64) blocks = (int64_t)sm_count() * 64;
-    k_cand<<<(unsigned)blocks, tp.cand_threads, 0, s>>>(C, co);
+    k_cand<<<(unsigned)blocks, tp.cand_threads, 0, s>>>(C, co, ppw);
   }
   if (ev) cudaEventRecord(ev[1], s);
   if (panel == 0) launch_isect<0>(C, co, hs, precision, tp, s);
