@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -64,6 +65,61 @@ struct DevBuf {
   }
 };
 
+// Pinned host blocks for the small reads and writes of a call, kept for the next context when one is
+// destroyed (pinning takes longer than a small call); at most kPinKept bytes are kept.  Portable
+// memory, so a block serves any device; shared by all threads.
+constexpr size_t kPinKept = (size_t)32 << 20;
+struct PinPool {
+  std::mutex mu;
+  std::vector<std::pair<void*, size_t>> kept;
+  size_t bytes = 0;
+};
+PinPool& pin_pool() {
+  static PinPool* pool = new PinPool;  // lives to the process's end: contexts may outlive static objects
+  return *pool;
+}
+
+struct PinBuf {
+  void* p = nullptr;
+  size_t cap = 0;
+  cudaError_t ensure(size_t bytes) {
+    if (bytes <= cap) return cudaSuccess;
+    release();
+    PinPool& pool = pin_pool();
+    {
+      std::lock_guard<std::mutex> g(pool.mu);
+      for (size_t q = 0; q < pool.kept.size(); q++)
+        if (pool.kept[q].second >= bytes) {
+          p = pool.kept[q].first;
+          cap = pool.kept[q].second;
+          pool.bytes -= cap;
+          pool.kept.erase(pool.kept.begin() + q);
+          return cudaSuccess;
+        }
+    }
+    const size_t want = std::max<size_t>((bytes + 4095) & ~(size_t)4095, 16384);
+    cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocPortable);
+    if (e == cudaSuccess) cap = want;
+    else p = nullptr;
+    return e;
+  }
+  template <class T>
+  T* as() const { return (T*)p; }
+  void release() {
+    if (!p) return;
+    PinPool& pool = pin_pool();
+    std::lock_guard<std::mutex> g(pool.mu);
+    if (pool.bytes + cap <= kPinKept) {
+      pool.kept.emplace_back(p, cap);
+      pool.bytes += cap;
+    } else {
+      cudaFreeHost(p);
+    }
+    p = nullptr;
+    cap = 0;
+  }
+};
+
 }  // namespace
 
 struct nsg_ctx {
@@ -76,27 +132,27 @@ struct nsg_ctx {
   int32_t nstruct = 0;
   std::vector<NsGrid> grids;
   std::vector<nsg::StructDev> sd;
-  DevBuf d_sd, d_patch_struct, d_tile_struct[3], d_ray_base[nsg::kRaySets], d_mc_base, d_row_base, d_row_chunks;
-  int64_t nchunks = 0;
-  int64_t tiles_tot[3] = {0, 0, 0}, rays_tot[nsg::kRaySets] = {0, 0, 0, 0, 0, 0}, mc_tot = 0, rows_tot = 0, words_tot = 0, awords_tot = 0;
+  DevBuf d_layout, d_patch_struct;
+  PinBuf h_layout;  // host side of d_layout
+  PinBuf h_read;    // counts and sums that a call reads back
+  int64_t tiles_tot[3] = {0, 0, 0}, rays_tot[nsg::kRaySets] = {0, 0, 0, 0, 0, 0}, mc_tot = 0, words_tot = 0, awords_tot = 0;
   int32_t patch_nstruct = 0;  // structures the uploaded patches belong to
   bool patch_struct_valid = false;
   std::vector<double> volumes, areas;
-  DevBuf vol_struct, area_struct, seg_part;
+  DevBuf seg_part;
   // patches
   int64_t np = 0, npool = 0;
   double probe = 1.4;
-  DevBuf f64, i32, pool, flag, win, pool32, quad32, quadl, kind_mask_d;
+  DevBuf f64, i32, pool, flag, win, pool32, quad32, quadl;
   bool pool32_valid = false;
-  int kind_mask = 0;  // patch kinds present (bit per kind), valid when kind_mask_valid
-  bool kind_mask_valid = false;
+  int kind_mask = 0;  // patch kinds present (bit per kind), of the last ray cast
   const double* ext_f64 = nullptr;  // device-resident patch arrays bound by the caller
   const int32_t* ext_i32 = nullptr;
   const double* ext_pool = nullptr;
   const int8_t* ext_flag = nullptr;
   bool has_patches = false;
   // binning per panel
-  DevBuf tile_cnt[3], tile_off[3], tile_list[3], bin_area;
+  DevBuf tile_cnt[3], tile_off[3], tile_list[3], win_sums;
   int64_t win_area[3] = {0, 0, 0};
   // wavefront tracing: candidate lists and the slot-major hit store
   // per ray set (slot s when the ray sets run on their own streams, slot 0 otherwise)
@@ -119,7 +175,7 @@ struct nsg_ctx {
   DevBuf status, bits, vol_ray[nsg::kRaySets], epsmap;
   DevBuf pairs, ray_pair_off, ray_pair_cnt, cursors, ovf_rays[nsg::kRaySets], ovf_scratch, err;
   DevBuf hits, ray_hit_off[nsg::kRaySets], ray_hit_cnt[nsg::kRaySets];
-  int64_t pair_cap = 0, hit_cap = 0;
+  int64_t pair_cap = 0, hit_cap = 0, n_pairs = 0;
   int flags = 0;
   int precision = 0;
   double volume = 0;
@@ -129,6 +185,8 @@ struct nsg_ctx {
   DevBuf sruns, srun_off, srun_cnt, fr_cnt, fr_off, fruns, frow;
   int64_t srun_cap = 0, n_fruns = 0;
   bool status_dense = false;
+  bool runs_ready = false;     // the free runs of the last cast (or difference) are built
+  bool cav_labels = false;     // cc_label_of holds the region labels of the last detection
   bool have_eps = false;     // the last ray cast built the epsilon maps
   bool eps_filled = false;   // cavity filling has been applied to them
   // ideb map and boundary grid points (node index, ibgp, type, projection, projection flag), the
@@ -137,7 +195,8 @@ struct nsg_ctx {
   int64_t n_bgp = 0, n_bgp_ext = 0;
   bool have_bgp = false, bgp_projected = false;
   // cavities
-  DevBuf labels, is_root, roots, cc_count, cc_desc, cc_label_of, cc_fill_of, nroots_d;
+  DevBuf labels, is_root, roots, cc_label_of, cc_fill_of, cc_block;
+  int64_t cc_cap = 4096;       // regions that cc_block holds
   int ncav = 0;
   std::vector<double> cav_size;
   std::vector<int32_t> cav_filled;
@@ -152,10 +211,11 @@ struct nsg_ctx {
   std::vector<int32_t> cav_atom_off, cav_atom_list;
   DevBuf ca_atoms, ca_cell_off, ca_cell_atoms, ca_pairs, ca_alt, ca_count;
   // mesh
-  DevBuf amap, cube_vl, vstruct, chunk_off;
+  DevBuf amap, cube_vl, vstruct, mc_block;
+  // capacities of a triangulation per vertex of the cast's pairs, raised when one did not suffice
+  double vert_ratio = 1.0625, cube_ratio = 1.125, tri_ratio = 2.25;
   nsg::TuneParams tune;
-  DevBuf surv_cnt, surv_off, vpos, vkey, row_act_cnt, row_mid_cnt, row_act_off, row_mid_off, act_rec, act_mid,
-      tri_cnt, tri_off, tris, cube_area, red_out, bnd_list, bnd_cursor;
+  DevBuf vpos, vkey, act_rec, tri_cnt, tris, cube_area, red_out, bnd_list;
   int64_t n_vert = 0, n_analytic = 0, n_tri = 0, n_active = 0;
   double area = 0;
   DevBuf temp;  // cub temporary storage
@@ -208,15 +268,26 @@ nsg::GridDev grid_dev(const NsGrid& g) {
   return d;
 }
 
+// The per-structure tables of a batch, one after another in d_layout: the descriptors, then arrays of
+// n + 1 bases (the last is the total) of the ray sets, the MC ray ordinals, the map words and the
+// panels' tiles.
+constexpr int kLayoutArrays = nsg::kRaySets + 2 + 3;
+size_t layout_bytes(int32_t n) {
+  return (size_t)n * sizeof(nsg::StructDev) + (size_t)kLayoutArrays * (n + 1) * sizeof(int64_t);
+}
+
 nsg::BatchDev batch_dev(nsg_ctx* c) {
+  static_assert(sizeof(nsg::StructDev) % sizeof(int64_t) == 0, "the base arrays follow the descriptors");
   nsg::BatchDev B{};
   B.n = c->nstruct;
-  B.s = c->d_sd.as<nsg::StructDev>();
+  B.s = c->d_layout.as<nsg::StructDev>();
   B.patch_struct = c->d_patch_struct.as<int32_t>();
-  for (int i = 0; i < 3; i++) B.tile_struct[i] = c->d_tile_struct[i].as<int32_t>();
-  for (int i = 0; i < nsg::kRaySets; i++) B.ray_base[i] = c->d_ray_base[i].as<int64_t>();
-  B.mc_base = c->d_mc_base.as<int64_t>();
-  B.row_base = c->d_row_base.as<int64_t>();
+  const int64_t* base = (const int64_t*)(B.s + B.n);
+  const int64_t step = B.n + 1;
+  for (int i = 0; i < nsg::kRaySets; i++) B.ray_base[i] = base + i * step;
+  B.mc_base = base + nsg::kRaySets * step;
+  B.aword_base = base + (nsg::kRaySets + 1) * step;
+  for (int i = 0; i < 3; i++) B.tile_base[i] = base + (nsg::kRaySets + 2 + i) * step;
   return B;
 }
 
@@ -227,20 +298,28 @@ cudaError_t upload_vec(DevBuf& d, const std::vector<T>& h, cudaStream_t s) {
   return cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
-// Host and device layout of the batch: per-structure bases of tiles, rays, MC ray ordinals, cube
-// rows and bit words, and the reverse maps tile -> structure.
+// Host and device layout of the batch: per-structure bases of tiles, rays, MC ray ordinals, map
+// words and bit words, filled in one pinned block and sent in one copy.
 int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
-  std::vector<nsg::StructDev> sd(n);
-  std::vector<int64_t> rb[nsg::kRaySets], mcb(n + 1), rowb(n + 1);
-  std::vector<int32_t> ts[3];
-  std::vector<int4> chunks;  // marching-cubes row chunks: structure, first row, row count
-  constexpr int32_t kRowChunk = 32;  // cube rows per chunk: one warp, one row per lane
-  for (int i = 0; i < nsg::kRaySets; i++) rb[i].resize(n + 1);
-  int64_t tiles[3] = {0, 0, 0}, rays[nsg::kRaySets] = {0, 0, 0, 0, 0, 0}, mc = 0, rows = 0, words = 0, awords = 0;
   for (int32_t b = 0; b < n; b++) {
     const NsGrid& G = grids[b];
     if (G.nx < 3 || G.ny < 3 || G.nz < 3) return fail(NSG_ERR_ARG, "grid must have at least 3 nodes per axis");
     if (G.nx * G.ny * G.nz >= (int64_t)1 << 31) return fail(NSG_ERR_ARG, "grid larger than 2^31 nodes");
+  }
+  // an earlier layout may still be on its way out of the pinned block
+  CK(cudaStreamSynchronize(c->stream));
+  CK(c->h_layout.ensure(layout_bytes(n)));
+  CK(c->d_layout.ensure(layout_bytes(n)));
+  nsg::StructDev* sd = c->h_layout.as<nsg::StructDev>();
+  int64_t* base = (int64_t*)(sd + n);
+  int64_t *rb[nsg::kRaySets], *tb[3];
+  for (int i = 0; i < nsg::kRaySets; i++) rb[i] = base + i * (int64_t)(n + 1);
+  int64_t* mcb = base + nsg::kRaySets * (int64_t)(n + 1);
+  int64_t* awb = base + (nsg::kRaySets + 1) * (int64_t)(n + 1);
+  for (int i = 0; i < 3; i++) tb[i] = base + (nsg::kRaySets + 2 + i) * (int64_t)(n + 1);
+  int64_t tiles[3] = {0, 0, 0}, rays[nsg::kRaySets] = {0, 0, 0, 0, 0, 0}, mc = 0, words = 0, awords = 0;
+  for (int32_t b = 0; b < n; b++) {
+    const NsGrid& G = grids[b];
     nsg::StructDev& S = sd[b];
     S.g = grid_dev(G);
     S.A = G.A;
@@ -249,10 +328,8 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
     words += S.nwords;
     for (int panel = 0; panel < 3; panel++) {
       nsg::RaySet rs = nsg::make_ray_set(panel == 0 ? 0 : panel + 1, S.g);
-      int64_t nt = ((rs.nb + nsg::kTileM - 1) / nsg::kTileM) * ((rs.na + nsg::kTileN - 1) / nsg::kTileN);
-      S.tile_base[panel] = tiles[panel];
-      ts[panel].insert(ts[panel].end(), nt, b);
-      tiles[panel] += nt;
+      S.tile_base[panel] = tb[panel][b] = tiles[panel];
+      tiles[panel] += ((rs.nb + nsg::kTileM - 1) / nsg::kTileM) * ((rs.na + nsg::kTileN - 1) / nsg::kTileN);
     }
     for (int set = 0; set < nsg::kRaySets; set++) {
       nsg::RaySet rs = nsg::make_ray_set(set, S.g);
@@ -261,13 +338,8 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
     }
     S.mc_base = mcb[b] = mc;
     mc += G.nz * G.ny + G.ny * G.nx + G.nz * G.nx;
-    S.row_base = rowb[b] = rows;
-    S.aword_base = awords;
+    S.aword_base = awb[b] = awords;
     awords += ((G.nx - 2 + 31) / 32) * (G.ny - 2) * (G.nz - 2);
-    const int64_t srows = (G.ny - 2) * (G.nz - 2);
-    for (int64_t r = 0; r < srows; r += kRowChunk)
-      chunks.push_back(make_int4(b, (int32_t)r, (int32_t)std::min<int64_t>(kRowChunk, srows - r), 0));
-    rows += srows;
     for (int d = 0; d < 3; d++) {
       S.ray_dir[d] = (S.g.mn[d] + (double)(S.g.n[d] - 1) * S.g.side) - (S.g.mn[d] + 0.0 * S.g.side);
       S.inv_dir[d] = 1.0 / S.ray_dir[d];
@@ -279,23 +351,16 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
     if (rays[i] >= (int64_t)1 << 31) return fail(NSG_ERR_CAPACITY, "more than 2^31 rays in one ray set of a batch");
   }
   mcb[n] = mc;
-  rowb[n] = rows;
-  CK(upload_vec(c->d_sd, sd, c->stream));
-  for (int i = 0; i < 3; i++) CK(upload_vec(c->d_tile_struct[i], ts[i], c->stream));
-  for (int i = 0; i < nsg::kRaySets; i++) CK(upload_vec(c->d_ray_base[i], rb[i], c->stream));
-  CK(upload_vec(c->d_mc_base, mcb, c->stream));
-  CK(upload_vec(c->d_row_base, rowb, c->stream));
-  CK(upload_vec(c->d_row_chunks, chunks, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  c->nchunks = (int64_t)chunks.size();
+  awb[n] = awords;
+  for (int i = 0; i < 3; i++) tb[i][n] = tiles[i];
+  CK(cudaMemcpyAsync(c->d_layout.p, sd, layout_bytes(n), cudaMemcpyHostToDevice, c->stream));
   c->nstruct = n;
   c->grids.assign(grids, grids + n);
-  c->sd = sd;
+  c->sd.assign(sd, sd + n);
   c->grid = grids[0];
   for (int i = 0; i < 3; i++) c->tiles_tot[i] = tiles[i];
   for (int i = 0; i < nsg::kRaySets; i++) c->rays_tot[i] = rays[i];
   c->mc_tot = mc;
-  c->rows_tot = rows;
   c->words_tot = words;
   c->awords_tot = awords;
   c->has_grid = true;
@@ -353,34 +418,13 @@ int scan_counts(nsg_ctx* c, const In* in, int64_t n, int64_t* out, int64_t* tota
   tb = c->temp.cap;
   CK(cub::DeviceScan::ExclusiveScan(c->temp.p, tb, in, out, cub::Sum(), (int64_t)0, n, c->stream));
   if (total) {
-    int64_t last_off = 0;
-    In last_cnt = 0;
-    if (n > 0) {
-      CK(cudaMemcpyAsync(&last_off, out + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-      CK(cudaMemcpyAsync(&last_cnt, in + n - 1, sizeof(In), cudaMemcpyDeviceToHost, c->stream));
-    }
+    // the total is formed on the device, behind the offsets, and read back once
+    CK(c->h_read.ensure(sizeof(int64_t)));
+    LAUNCH(nsg::launch_scan_total(in, n, out, c->stream));
+    CK(cudaMemcpyAsync(c->h_read.p, out + n, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    *total = last_off + (int64_t)last_cnt;
-    CK(cudaMemcpyAsync(out + n, total, sizeof(int64_t), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    *total = *c->h_read.as<int64_t>();
   }
-  return NSG_OK;
-}
-
-
-// Window-area sum of a panel (the bound of its candidate count).
-int panel_area(nsg_ctx* c, int panel) {
-  const int set = panel == 0 ? 0 : panel + 1;
-  const nsg::BatchDev B = batch_dev(c);
-  nsg::PatchDev P = patch_dev(c);
-  CK(c->bin_area.ensure(3 * sizeof(unsigned long long)));
-  unsigned long long* area = c->bin_area.as<unsigned long long>() + panel;
-  CK(cudaMemsetAsync(area, 0, sizeof(unsigned long long), c->stream));
-  LAUNCH(nsg::launch_bin_count(P, B, set, nullptr, area, c->stream));
-  unsigned long long a_host = 0;
-  CK(cudaMemcpyAsync(&a_host, area, sizeof(a_host), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  c->win_area[panel] = (int64_t)a_host;
   return NSG_OK;
 }
 
@@ -393,7 +437,7 @@ int bin_panel(nsg_ctx* c, int panel) {
   CK(c->tile_off[panel].ensure((ntiles + 1) * sizeof(int64_t)));
   CK(cudaMemsetAsync(c->tile_cnt[panel].p, 0, (ntiles + 1) * sizeof(int32_t), c->stream));
   nsg::PatchDev P = patch_dev(c);
-  LAUNCH(nsg::launch_bin_count(P, B, set, c->tile_cnt[panel].as<int32_t>(), nullptr, c->stream));
+  LAUNCH(nsg::launch_bin_count(P, B, set, c->tile_cnt[panel].as<int32_t>(), c->stream));
   int64_t total = 0;
   int rc = scan_counts(c, c->tile_cnt[panel].as<int32_t>(), ntiles, c->tile_off[panel].as<int64_t>(), &total);
   if (rc) return rc;
@@ -421,8 +465,10 @@ nsg::RunArgs run_args(nsg_ctx* c) {
   return A;
 }
 
-// Free runs of every status row (complement of the inside runs).
-int build_free_runs(nsg_ctx* c) {
+// Free runs of every status row (complement of the inside runs), built when the first call after a
+// cast asks for the status map, the cavities or the ideb map.
+int ensure_free_runs(nsg_ctx* c) {
+  if (c->runs_ready) return NSG_OK;
   const int64_t nrows = c->grid.ny * c->grid.nz;
   CK(c->fr_cnt.ensure(nrows * sizeof(int32_t)));
   CK(c->fr_off.ensure((nrows + 1) * sizeof(int64_t)));
@@ -436,11 +482,17 @@ int build_free_runs(nsg_ctx* c) {
   c->n_fruns = n;
   A = run_args(c);
   LAUNCH(nsg::launch_free_runs(A, 1, c->stream));
+  c->runs_ready = true;
   return NSG_OK;
 }
 
-// Dense status map from the runs (labels when cavity detection ran).
-int materialize_status(nsg_ctx* c, const int32_t* label_of_dev) {
+// Dense status map from the runs (with the region labels when cavity detection ran), unless it is
+// there already: written for the calls that read it, not by every cast or detection.
+int ensure_dense_status(nsg_ctx* c) {
+  if (c->status_dense) return NSG_OK;
+  int rc = ensure_free_runs(c);
+  if (rc) return rc;
+  const int32_t* label_of_dev = c->cav_labels ? c->cc_label_of.as<int32_t>() : nullptr;
   const NsGrid& g = c->grid;
   CK(c->status.ensure(g.nx * g.ny * g.nz * sizeof(int32_t)));
   nsg::RunArgs A = run_args(c);
@@ -469,8 +521,6 @@ int nsg_ctx_create(int device, nsg_ctx** out) {
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return fail(NSG_ERR_CUDA, "cudaStreamCreate", e); }
   c->own_stream = true;
-  e = nsg::mc_init_tables();
-  if (e != cudaSuccess) { cudaStreamDestroy(c->stream); delete c; return fail(NSG_ERR_CUDA, "mc tables", e); }
   *out = c;
   return NSG_OK;
 }
@@ -479,26 +529,22 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   if (!c) return NSG_ERR_ARG;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->kind_mask_d, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield, &c->b_gatoms, &c->counters, &c->bin_area,
+  DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield, &c->b_gatoms, &c->counters, &c->win_sums,
                     &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_node, &c->bgp_ibgp, &c->bgp_type,
                     &c->bgp_pos, &c->bgp_nor, &c->bgp_flag, &c->bgp_n, &c->aux_cnt, &c->aux_off, &c->aux_list, &c->pairs,
                     &c->ray_pair_off, &c->ray_pair_cnt, &c->cursors, &c->ovf_scratch, &c->err, &c->hits,
                     &c->pair_pid, &c->ovf_pscratch, &c->gvol, &c->garea, &c->vpid, &c->vgrad,
-                    &c->d_atoms, &c->d_patch_atoms, &c->d_gatoms_vol, &c->d_gatoms_area, &c->d_bad, &c->amap, &c->cube_vl, &c->vstruct, &c->chunk_off, &c->ca_atoms, &c->ca_cell_off, &c->ca_cell_atoms, &c->ca_pairs, &c->ca_alt, &c->ca_count,
+                    &c->d_atoms, &c->d_patch_atoms, &c->d_gatoms_vol, &c->d_gatoms_area, &c->d_bad, &c->amap, &c->cube_vl, &c->vstruct, &c->mc_block, &c->ca_atoms, &c->ca_cell_off, &c->ca_cell_atoms, &c->ca_pairs, &c->ca_alt, &c->ca_count,
                     &c->d_patch_off, &c->d_pool_off, &c->d_atom_off,
                     &c->labels, &c->is_root, &c->sruns, &c->srun_off, &c->srun_cnt, &c->fr_cnt, &c->fr_off,
-                    &c->fruns, &c->frow, &c->roots, &c->cc_count, &c->cc_desc, &c->cc_label_of,
-                    &c->cc_fill_of, &c->nroots_d, &c->surv_cnt, &c->surv_off, &c->vpos, &c->vkey,
-                    &c->row_act_cnt, &c->row_mid_cnt, &c->row_act_off, &c->row_mid_off, &c->act_rec,
-                    &c->act_mid, &c->tri_cnt, &c->tri_off, &c->tris, &c->cube_area, &c->red_out, &c->bnd_list,
-                    &c->bnd_cursor, &c->temp};
+                    &c->fruns, &c->frow, &c->roots, &c->cc_block, &c->cc_label_of,
+                    &c->cc_fill_of, &c->cav_label, &c->sh_support, &c->sh_removed[0], &c->sh_removed[1],
+                    &c->sh_later, &c->sh_filled, &c->sh_nrem, &c->sh_changed, &c->vpos, &c->vkey, &c->act_rec,
+                    &c->tri_cnt, &c->tris, &c->cube_area, &c->red_out, &c->bnd_list, &c->temp};
   for (DevBuf* b : bufs) b->release();
   for (int i = 0; i < 3; i++) { c->tile_cnt[i].release(); c->tile_off[i].release(); c->tile_list[i].release(); }
-  c->d_sd.release(); c->d_patch_struct.release(); c->d_mc_base.release(); c->d_row_base.release();
-  c->d_row_chunks.release();
-  c->vol_struct.release(); c->area_struct.release(); c->seg_part.release();
-  for (int i = 0; i < 3; i++) c->d_tile_struct[i].release();
-  for (int i = 0; i < nsg::kRaySets; i++) c->d_ray_base[i].release();
+  c->d_layout.release(); c->d_patch_struct.release(); c->seg_part.release();
+  c->h_layout.release(); c->h_read.release();
   for (int i = 0; i < nsg::kRaySets; i++) {
     c->vol_ray[i].release(); c->ovf_rays[i].release(); c->ray_hit_off[i].release(); c->ray_hit_cnt[i].release();
     c->cand_sph[i].release(); c->cand_tor[i].release(); c->def_sph[i].release(); c->def_tor[i].release();
@@ -514,6 +560,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   for (int i = 0; i < nsg::kRaySets; i++)
     for (int q = 0; q < 4; q++)
       if (c->sub_ev[i][q]) cudaEventDestroy(c->sub_ev[i][q]);
+  if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return NSG_OK;
@@ -550,7 +597,6 @@ static int upload_common(nsg_ctx* c, int64_t n, int64_t npool, double probe) {
   CK(c->win.ensure(std::max<int64_t>(n, 1) * 6 * sizeof(int32_t)));
   c->has_patches = true;
   c->pool32_valid = false;
-  c->kind_mask_valid = false;
   c->b_valid = false;
   c->patch_nstruct = 1;
   c->patch_struct_valid = false;
@@ -999,15 +1045,24 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   const bool pids = grad || (flags & 64);
   // the marching-cubes vertices carry their patch index in 29 bits (vpid_pack, mc.cu)
   if (pids && c->np >= ((int64_t)1 << 29)) return fail(NSG_ERR_CAPACITY, "more than 2^29 patches with patch ids");
-  if (!c->kind_mask_valid) {
-    // which patch kinds are present (SES and / or skin cells) selects the intersection kernels
-    CK(c->kind_mask_d.ensure(sizeof(int)));
-    CK(cudaMemsetAsync(c->kind_mask_d.p, 0, sizeof(int), c->stream));
+  // patch windows, the panels' window areas (the bound of their candidate counts) and the patch kinds
+  // (which select the intersection kernels), in one launch and one read
+  {
     nsg::PatchDev P0 = patch_dev(c);
-    LAUNCH(nsg::launch_kind_mask(P0, c->kind_mask_d.as<int>(), c->stream));
-    CK(cudaMemcpyAsync(&c->kind_mask, c->kind_mask_d.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(c->win_sums.ensure(4 * sizeof(unsigned long long)));
+    CK(c->h_read.ensure(4 * sizeof(unsigned long long)));
+    stage_begin(c, kStageBin);
+    CK(cudaMemsetAsync(c->win_sums.p, 0, 4 * sizeof(unsigned long long), c->stream));
+    LAUNCH(nsg::launch_windows(P0, c->win.as<int32_t>(), B, c->win_sums.as<unsigned long long>(), c->stream));
+    stage_end(c, kStageBin);
+    CK(cudaMemcpyAsync(c->h_read.p, c->win_sums.p, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    c->kind_mask_valid = true;
+    const unsigned long long* sums = c->h_read.as<unsigned long long>();
+    for (int panel = 0; panel < 3; panel++) {
+      const bool used = panel == 0 ? (do_status || do_eps || do_mc) : (do_mc || do_eps);
+      c->win_area[panel] = used ? (int64_t)sums[panel] : 0;
+    }
+    c->kind_mask = (int)sums[3];
   }
   if (grad && (c->kind_mask & nsg::kSkinKinds))
     return fail(NSG_ERR_STATE, "gradients are provided for SES and mesh patch sets, not for skin cells");
@@ -1028,15 +1083,6 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     c->pool32_valid = true;
   }
   nsg::PatchDev P = patch_dev(c);
-  stage_begin(c, kStageBin);
-  LAUNCH(nsg::launch_windows(P, c->win.as<int32_t>(), B, c->stream));
-  for (int panel = 0; panel < 3; panel++) {
-    if (panel == 0 && !(do_status || do_eps || do_mc)) continue;
-    if (panel > 0 && !(do_mc || do_eps)) continue;
-    int rc = panel_area(c, panel);
-    if (rc) return rc;
-  }
-  stage_end(c, kStageBin);
   const int64_t nwords = c->words_tot;
   const int64_t nrays_mc = c->mc_tot;
   const int64_t nrows = c->rays_tot[0];
@@ -1047,13 +1093,16 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   }
   if (do_mc) {
     CK(c->bits.ensure(nwords * sizeof(uint32_t)));
-    CK(cudaMemsetAsync(c->bits.p, 0xff, nwords * sizeof(uint32_t), c->stream));
     CK(c->ray_pair_off.ensure(nrays_mc * sizeof(int64_t)));
-    CK(c->ray_pair_cnt.ensure(nrays_mc * sizeof(int32_t)));
-    CK(cudaMemsetAsync(c->ray_pair_cnt.p, 0, nrays_mc * sizeof(int32_t), c->stream));
+    CK(c->ray_pair_cnt.ensure(nrays_mc * sizeof(int32_t)));  // every ray's count is written by the fill
     if (c->pair_cap == 0) c->pair_cap = std::max<int64_t>(4 * nrays_mc, 1 << 16);
   }
-  CK(c->cursors.ensure(64 * sizeof(unsigned long long)));
+  // the cursors (64 words, the error flag in the last) and, behind them, the structures' volume sums:
+  // one clear before and one read after the cast
+  const int32_t nb = c->nstruct;
+  const size_t read_bytes = (64 + (size_t)nb) * sizeof(unsigned long long);
+  CK(c->cursors.ensure(read_bytes));
+  CK(c->h_read.ensure(read_bytes));
   // the ray sets run on their own streams (each with its own candidate lists and hit store) so
   // that the double-precision intersection launches of one set overlap the integer-bound candidate
   // and fill launches of another; or, with concurrent_sets off, one after another on the context's
@@ -1085,9 +1134,12 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       }
     }
   }
-  CK(c->err.ensure(sizeof(int32_t)));
+  CK(c->seg_part.ensure((size_t)nsg::kMaxSegArrays * nb * nsg::kSegParts * sizeof(double)));
   const int ovf_cap = 1 << 16;
-  for (int attempt = 0; attempt < 4; attempt++) {
+  const double* const vsum = (const double*)(c->h_read.as<unsigned long long>() + 64);
+  int nvol = 0;
+  bool done = false;
+  for (int attempt = 0; attempt < 12 && !done; attempt++) {
     if (do_mc) CK(c->pairs.ensure(c->pair_cap * 2 * sizeof(double)));
     if (do_mc && pids) CK(c->pair_pid.ensure(c->pair_cap * sizeof(int2)));
     if (grad)
@@ -1109,7 +1161,6 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     }
     if (do_status || do_eps) {
       CK(c->sruns.ensure(c->srun_cap * sizeof(int2)));
-      CK(cudaMemsetAsync(c->srun_cnt.p, 0, nrows * sizeof(int32_t), c->stream));
     }
     if (keep_hits) {
       if (c->hit_cap == 0)
@@ -1118,11 +1169,10 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       CK(c->hits.ensure(c->hit_cap * sizeof(double)));
     }
     CK(cudaMemsetAsync(c->cursors.p, 0, 64 * sizeof(unsigned long long), c->stream));
-    CK(cudaMemsetAsync(c->err.p, 0, sizeof(int32_t), c->stream));
     if (do_mc) CK(cudaMemsetAsync(c->bits.p, 0xff, nwords * sizeof(uint32_t), c->stream));
     // cursors: 0 pairs, 1 kept hits, 2 status runs, 4..6 the overflow counts of the six ray sets
     // (int32), 8 + 2 s the candidate counts of set s (spheres, tori), 20 + 2 s its deferred counts,
-    // 32 + 4 s its split torus counts (at +1 and +3)
+    // 32 + 4 s its split torus counts (at +1 and +3), 63 the error flag
     unsigned long long* cur = c->cursors.as<unsigned long long>();
     int32_t* ovf_count = (int32_t*)(cur + 4);
     int sets[nsg::kRaySets], nsets = 0;
@@ -1167,7 +1217,7 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       o.ovf_rays = c->ovf_rays[s].as<int32_t>();
       o.ovf_cap = ovf_cap;
       o.ovf_count = ovf_count + s;
-      o.error_flag = c->err.as<int32_t>();
+      o.error_flag = (int32_t*)(cur + 63);
       o.counters = c->profile ? c->counters.as<unsigned long long>() : nullptr;
       if (do_eps && (s == 0 || s >= 4)) {
         o.epsmap = c->epsmap.as<int32_t>();
@@ -1222,9 +1272,29 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
         }
       }
     }
-    int32_t novf[nsg::kRaySets] = {0, 0, 0, 0, 0, 0};
-    CK(cudaMemcpyAsync(novf, ovf_count, nsg::kRaySets * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    // volume: A * sum of interval lengths over the ray sets / number of ray sets, per structure; the
+    // per-structure sums run in an order fixed by the structure alone, so a structure's volume does
+    // not depend on the batch it is part of
+    const auto sum_and_read = [&]() -> int {
+      nsg::SegArrays seg{};
+      nvol = 0;
+      for (int si = 0; si < nsets; si++) {
+        seg.v[nvol] = c->vol_ray[sets[si]].as<double>();
+        seg.base[nvol++] = B.ray_base[sets[si]];
+      }
+      LAUNCH(nsg::launch_segment_sums(seg, nvol, nb, INT64_MAX, (double*)(cur + 64), c->seg_part.as<double>(),
+                                      c->stream));
+      CK(cudaMemcpyAsync(c->h_read.p, cur, read_bytes, cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      return NSG_OK;
+    };
+    {
+      int rc = sum_and_read();
+      if (rc) return rc;
+    }
+    const unsigned long long* const used = c->h_read.as<unsigned long long>();
+    int32_t novf[nsg::kRaySets];
+    memcpy(novf, used + 4, sizeof novf);
     int64_t tot_ovf = 0;
     bool tiles_built[3] = {false, false, false};
     stage_begin(c, kStageOverflow);
@@ -1248,12 +1318,14 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     }
     stage_end(c, kStageOverflow);
     c->last_overflow_rays = tot_ovf;
+    if (tot_ovf) {
+      int rc = sum_and_read();  // the overflow rays' lengths and pairs are in now
+      if (rc) return rc;
+    }
     if (c->profile) {
       CK(cudaMemcpyAsync(c->counter_host, c->counters.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                          c->stream));
-      unsigned long long cand[2 * nsg::kRaySets];
-      CK(cudaMemcpyAsync(cand, cur + 8, 2 * nsg::kRaySets * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                         c->stream));
+      const unsigned long long* cand = used + 8;
       CK(cudaStreamSynchronize(c->stream));
       // candidate pairs (spheres + tori) and torus pairs of all ray sets
       c->counter_host[nsg::kCntCandidates] = 0;
@@ -1263,12 +1335,12 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
         c->counter_host[nsg::kCntTorus] += cand[2 * sets[si] + 1];
       }
     }
-    int32_t errflag = 0;
-    unsigned long long used[3] = {0, 0, 0};
-    CK(cudaMemcpyAsync(&errflag, c->err.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(used, cur, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (errflag == 0) break;
+    const int32_t errflag = (int32_t)(used[63] & 0xffffffffu);
+    if (errflag == 0) {
+      c->n_pairs = do_mc ? (int64_t)used[0] : 0;
+      done = true;
+      continue;
+    }
     if (errflag == 3) { c->pair_cap = std::max<int64_t>(2 * c->pair_cap, (int64_t)used[0] + 1024); continue; }
     if (errflag == 2) { c->hit_cap = std::max<int64_t>(2 * c->hit_cap, (int64_t)used[1] + 1024); continue; }
     if (errflag == 5) { c->srun_cap = std::max<int64_t>(2 * c->srun_cap, (int64_t)used[2] + 1024); continue; }
@@ -1276,31 +1348,12 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     if (errflag == 7) { c->def_cap *= 2; continue; }
     return fail(NSG_ERR_CAPACITY, errflag == 1 ? "too many overflow rays" : "ray hit capacity exceeded");
   }
-  // volume: A * sum of interval lengths over the ray sets / number of ray sets, per structure; the
-  // per-structure sums run in an order fixed by the structure alone, so a structure's volume does
-  // not depend on the batch it is part of
-  const int32_t nb = c->nstruct;
-  std::vector<double> vsum(nb, 0.0);
-  int flag_sum = 0;
-  CK(c->vol_struct.ensure(nb * sizeof(double)));
-  CK(c->seg_part.ensure((size_t)nb * nsg::kSegParts * sizeof(double)));
-  for (int s = 0; s < nsg::kRaySets; s++) {
-    if (!cast(s)) continue;
-    LAUNCH(nsg::launch_segment_sums(c->vol_ray[s].as<double>(), B.ray_base[s], nullptr, nb,
-                                    c->vol_struct.as<double>(), c->seg_part.as<double>(), flag_sum > 0, c->stream));
-    flag_sum++;
-  }
-  if (flag_sum) {
-    CK(cudaMemcpyAsync(vsum.data(), c->vol_struct.p, nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-  }
-  for (int32_t b = 0; b < nb; b++) c->volumes[b] = flag_sum ? c->grids[b].A * vsum[b] / flag_sum : 0.0;
+  if (!done) return fail(NSG_ERR_CAPACITY, "ray cast capacities did not settle");
+  for (int32_t b = 0; b < nb; b++) c->volumes[b] = nvol ? c->grids[b].A * vsum[b] / nvol : 0.0;
   c->volume = c->volumes[0];
   if (volume) *volume = c->volume;
-  if ((do_status || do_eps) && nb == 1) {
-    int rc = build_free_runs(c);
-    if (rc) return rc;
-  }
+  c->runs_ready = false;
+  c->cav_labels = false;
   c->status_dense = false;
   c->cav_detected = c->have_cav_atoms = false;
   c->shape_filtered = c->ideb_ready = false;
@@ -1352,7 +1405,13 @@ namespace {
 // difference map is labelled), else the first region found is the outside.
 int detect_cavities(nsg_ctx* c, double cav_vol, bool pockets, int* ncav_out) {
   const NsGrid& g = c->grid;
+  {
+    int rc = ensure_free_runs(c);
+    if (rc) return rc;
+  }
   const int64_t nr = c->n_fruns;
+  c->cav_labels = false;
+  c->status_dense = false;
   c->cav_size.clear();
   c->cav_filled.clear();
   c->cav_count.clear();
@@ -1363,44 +1422,50 @@ int detect_cavities(nsg_ctx* c, double cav_vol, bool pockets, int* ncav_out) {
   CK(c->labels.ensure(std::max<int64_t>(nr, 1) * sizeof(int32_t)));
   CK(c->is_root.ensure(std::max<int64_t>(nr, 1)));
   CK(c->roots.ensure(std::max<int64_t>(nr, 1) * sizeof(int32_t)));
-  CK(c->nroots_d.ensure(sizeof(int32_t)));
   nsg::RunArgs A = run_args(c);
   c->launches += 3;
   CK(nsg::run_label(A, c->is_root.as<uint8_t>(), c->stream));
+  // the regions' roots, then their sizes and first descending nodes: the count of regions, the sizes
+  // and the nodes lie in one block that is read once (again when there are more regions than it holds)
   int32_t nroots = 0;
+  const unsigned long long* cnt = nullptr;
+  const unsigned int* desc = nullptr;
   if (nr > 0) {
     size_t tb = 0;
     CK(nsg::run_select_roots(c->is_root.as<uint8_t>(), nr, nullptr, nullptr, nullptr, &tb, c->stream));
     CK(c->temp.ensure(tb));
-    tb = c->temp.cap;
-    CK(nsg::run_select_roots(c->is_root.as<uint8_t>(), nr, c->roots.as<int32_t>(), c->nroots_d.as<int32_t>(),
-                             c->temp.p, &tb, c->stream));
-    CK(cudaMemcpyAsync(&nroots, c->nroots_d.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    for (int pass = 0; pass < 2; pass++) {
+      const int64_t cap = c->cc_cap;
+      const size_t bytes = (1 + (size_t)cap) * sizeof(unsigned long long) + (size_t)cap * sizeof(unsigned int);
+      CK(c->cc_block.ensure(bytes));
+      CK(c->h_read.ensure(bytes));
+      unsigned long long* blk = c->cc_block.as<unsigned long long>();
+      unsigned int* desc_d = (unsigned int*)(blk + 1 + cap);
+      CK(cudaMemsetAsync(blk, 0, (1 + (size_t)cap) * sizeof(unsigned long long), c->stream));
+      CK(cudaMemsetAsync(desc_d, 0xff, (size_t)cap * sizeof(unsigned int), c->stream));
+      tb = c->temp.cap;
+      CK(nsg::run_select_roots(c->is_root.as<uint8_t>(), nr, c->roots.as<int32_t>(), (int32_t*)blk, c->temp.p, &tb,
+                               c->stream));
+      LAUNCH(nsg::run_stats(A, c->roots.as<int32_t>(), (const int32_t*)blk, (int32_t)cap, blk + 1, desc_d, c->stream));
+      CK(cudaMemcpyAsync(c->h_read.p, blk, bytes, cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      nroots = *c->h_read.as<int32_t>();
+      cnt = c->h_read.as<unsigned long long>() + 1;
+      desc = (const unsigned int*)(cnt + cap);
+      if (nroots <= cap) break;
+      c->cc_cap = nroots;  // the statistics pass did nothing
+    }
   }
   if (nroots == 0) {
     c->ncav = 0;
-    int rc = materialize_status(c, nullptr);
-    if (rc) return rc;
     stage_end(c, kStageCavity);
     c->cav_detected = true;
     if (ncav_out) *ncav_out = 0;
     return NSG_OK;
   }
-  CK(c->cc_count.ensure(nroots * sizeof(unsigned long long)));
-  CK(c->cc_desc.ensure(nroots * sizeof(unsigned int)));
-  CK(cudaMemsetAsync(c->cc_count.p, 0, nroots * sizeof(unsigned long long), c->stream));
-  CK(cudaMemsetAsync(c->cc_desc.p, 0xff, nroots * sizeof(unsigned int), c->stream));
-  LAUNCH(nsg::run_stats(A, c->roots.as<int32_t>(), nroots, c->cc_count.as<unsigned long long>(),
-                        c->cc_desc.as<unsigned int>(), c->stream));
-  std::vector<unsigned long long> cnt(nroots);
-  std::vector<unsigned int> desc(nroots);
-  CK(cudaMemcpyAsync(cnt.data(), c->cc_count.p, nroots * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(desc.data(), c->cc_desc.p, nroots * sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   std::vector<int32_t> label_of(nroots, 0);
   std::vector<uint8_t> fill_of(nroots, 0);
-  nsg_cavity_order(nroots, desc.data(), label_of.data());
+  nsg_cavity_order(nroots, desc, label_of.data());
   if (pockets)
     for (auto& l : label_of) l++;
   const int32_t id = NS_STATUS_TEMPORARY_OUT + nroots + (pockets ? 1 : 0);
@@ -1432,10 +1497,8 @@ int detect_cavities(nsg_ctx* c, double cav_vol, bool pockets, int* ncav_out) {
     c->eps_filled = true;
     c->have_bgp = false;
   }
-  int rc = materialize_status(c, c->cc_label_of.as<int32_t>());
-  if (rc) return rc;
+  c->cav_labels = true;  // the dense map is written, with these labels, when a call reads it
   stage_end(c, kStageCavity);
-  CK(cudaStreamSynchronize(c->stream));
   c->cav_detected = true;
   if (ncav_out) *ncav_out = c->ncav;
   c->n_vert = c->n_tri = 0;
@@ -1465,14 +1528,10 @@ int nsg_pocket_difference(nsg_ctx* c, nsg_ctx* small, double fill_volume, int* n
   if (g.nx != h.nx || g.ny != h.ny || g.nz != h.nz) return fail(NSG_ERR_ARG, "the two grids differ");
   CK(cudaSetDevice(c->device));
   const int64_t nn = g.nx * g.ny * g.nz;
-  if (!c->status_dense) {
-    int rc = materialize_status(c, nullptr);
-    if (rc) return rc;
-  }
-  if (!small->status_dense) {
-    int rc = materialize_status(small, nullptr);
-    if (rc) return rc;
-  }
+  int rc = ensure_dense_status(c);
+  if (rc) return rc;
+  rc = ensure_dense_status(small);
+  if (rc) return rc;
   CK(cudaStreamSynchronize(small->stream));
   stage_begin(c, kStageCavity);
   CK(c->ca_count.ensure(2 * sizeof(unsigned long long)));
@@ -1492,7 +1551,8 @@ int nsg_pocket_difference(nsg_ctx* c, nsg_ctx* small, double fill_volume, int* n
   c->status_dense = c->cav_detected = true;
   c->shape_filtered = c->have_cav_atoms = false;
   c->eps_filled = false;
-  int rc = ndiff ? nsg_filter_cavities(c, 1.4, 1, nullptr) : NSG_OK;
+  c->cav_labels = false;
+  rc = ndiff ? nsg_filter_cavities(c, 1.4, 1, nullptr) : NSG_OK;
   if (rc) return rc;
   if (ndiff) LAUNCH(nsg::pocket_cav2out(c->status.as<int32_t>(), c->cav_label.as<int32_t>(), nn, c->stream));
   // the filtered map's free runs replace the cast's, then the regions are labelled as pockets
@@ -1509,18 +1569,23 @@ int nsg_pocket_difference(nsg_ctx* c, nsg_ctx* small, double fill_volume, int* n
   c->n_fruns = nr;
   A = run_args(c);
   LAUNCH(nsg::dense_free_runs(A, c->status.as<int32_t>(), 1, c->stream));
+  c->runs_ready = true;
   stage_end(c, kStageCavity);
   return detect_cavities(c, fill_volume, true, n_pockets);
 }
 
 int nsg_filter_cavities(nsg_ctx* c, double probe_radius, int modify_status, int64_t* n_removed) {
   if (!c || !(probe_radius > 0)) return NSG_ERR_ARG;
-  if (!c->cav_detected || !c->status_dense || c->nstruct != 1)
+  if (!c->cav_detected || c->nstruct != 1)
     return fail(NSG_ERR_STATE, "the shape filter needs nsg_cavities after the cast");
   if (c->shape_filtered) return fail(NSG_ERR_STATE, "the shape filter runs once per cavity detection");
   if (n_removed) *n_removed = 0;
   if (c->ncav == 0) return NSG_OK;
   CK(cudaSetDevice(c->device));
+  {
+    int rc = ensure_dense_status(c);
+    if (rc) return rc;
+  }
   const NsGrid& g = c->grid;
   const int64_t nn = g.nx * g.ny * g.nz;
   const int ncav = c->ncav;
@@ -1605,194 +1670,172 @@ int nsg_triangulate(nsg_ctx* c, double* area_out, int64_t* nverts, int64_t* ntri
   if (!c || !c->have_bits) return fail(NSG_ERR_STATE, "triangulation needs the accurate-triangulation rays");
   CK(cudaSetDevice(c->device));
   const nsg::BatchDev B = batch_dev(c);
-  const int64_t nrays = c->mc_tot;
-  CK(c->surv_cnt.ensure(nrays * sizeof(int32_t)));
-  CK(c->surv_off.ensure((nrays + 1) * sizeof(int64_t)));
-  nsg::VertArgs V{};
-  V.B = B;
-  V.nrays = nrays;
-  V.ray_pair_off = c->ray_pair_off.as<int64_t>();
-  V.ray_pair_cnt = c->ray_pair_cnt.as<int32_t>();
-  V.pairs = c->pairs.as<double>();
-  V.bits = c->bits.as<uint32_t>();
-  V.surv_cnt = c->surv_cnt.as<int32_t>();
-  V.surv_off = c->surv_off.as<int64_t>();
-  stage_begin(c, kStageVertex);
-  LAUNCH(nsg::launch_vert(V, 0, c->stream));
-  int64_t n_an = 0;
-  int rc = scan_counts(c, c->surv_cnt.as<int32_t>(), nrays, c->surv_off.as<int64_t>(), &n_an);
-  if (rc) return rc;
-  // rows of cubes
-  const int64_t nrows = c->rows_tot;
-  CK(c->row_act_cnt.ensure((nrows + 1) * sizeof(int64_t)));
-  CK(c->row_act_off.ensure((nrows + 1) * sizeof(int64_t)));
-  nsg::MCArgs M{};
-  M.B = B;
-  M.row_chunks = c->d_row_chunks.as<int4>();
-  M.nchunks = c->nchunks;
-  M.bits = c->bits.as<uint32_t>();
-  M.surv_cnt = c->surv_cnt.as<int32_t>();
-  M.surv_off = c->surv_off.as<int64_t>();
-  M.n_analytic = n_an;
-  M.nrows = nrows;
-  M.row_act_cnt = c->row_act_cnt.as<int64_t>();
-  stage_end(c, kStageVertex, false);
-  stage_begin(c, kStageMC);
-  // active cubes, their map and vertex slots (the vertex pass writes into the slots)
-  LAUNCH(nsg::launch_mc_rows(M, 0, c->stream));
-  int64_t n_act = 0, n_mid = 0;
-  rc = scan_counts(c, c->row_act_cnt.as<int64_t>(), nrows, c->row_act_off.as<int64_t>(), &n_act);
-  if (rc) return rc;
-  if (n_act >= ((int64_t)1 << 31) / 12) return fail(NSG_ERR_CAPACITY, "too many active cubes in one batch");
-  M.row_act_off = c->row_act_off.as<int64_t>();
-  CK(c->act_rec.ensure(std::max<int64_t>(n_act, 1) * sizeof(int4)));
-  CK(c->act_mid.ensure(std::max<int64_t>(n_act, 1) * sizeof(int32_t)));
-  CK(c->row_mid_cnt.ensure(std::max<int64_t>(n_act, 1) * sizeof(int32_t)));
-  CK(c->row_mid_off.ensure((n_act + 1) * sizeof(int64_t)));
-  M.act_rec = c->act_rec.as<int4>();
-  M.act_mid = c->act_mid.as<int32_t>();
-  M.mid_cnt = c->row_mid_cnt.as<int32_t>();
-  M.mid_off = c->row_mid_off.as<int64_t>();
-  M.n_active = n_act;
-  // the active-cube map (per 32 cubes of a row: their active bits and the first one's index) and
-  // 12 vertex slots per active cube, all -1 until the vertices are written into them
-  CK(c->amap.ensure(std::max<int64_t>(c->awords_tot, 1) * sizeof(int2)));
-  CK(c->cube_vl.ensure(std::max<int64_t>(n_act, 1) * 12 * sizeof(int32_t)));
-  M.amap = c->amap.as<int2>();
-  M.cube_vl = c->cube_vl.as<int32_t>();
-  // triangle counts per active cube: the case table's for interior cubes (written by the
-  // classification), a count over the vertex slots for the listed low-face cubes
-  CK(c->tri_cnt.ensure(std::max<int64_t>(n_act, 1) * sizeof(int32_t)));
-  CK(c->bnd_list.ensure(std::max<int64_t>(n_act, 1) * sizeof(int32_t)));
-  CK(c->bnd_cursor.ensure(sizeof(unsigned long long)));
-  CK(cudaMemsetAsync(c->bnd_cursor.p, 0, sizeof(unsigned long long), c->stream));
-  M.tri_cnt = c->tri_cnt.as<int32_t>();
-  M.bnd_list = c->bnd_list.as<int32_t>();
-  M.bnd_cursor = c->bnd_cursor.as<unsigned long long>();
-  LAUNCH(nsg::launch_mc_rows(M, 1, c->stream));
-  stage_end(c, kStageMC, false);
-  // analytic vertices, then each first vertex of an edge into the slots of the edge's cubes
-  stage_begin(c, kStageVertex);
-  CK(c->vkey.ensure(std::max<int64_t>(n_an, 1) * sizeof(int4)));
-  CK(c->vpos.ensure(std::max<int64_t>(n_an, 1) * 3 * sizeof(double)));
-  V.vpos = c->vpos.as<double>();
-  V.vkey = c->vkey.as<int4>();
-  CK(c->vstruct.ensure(std::max<int64_t>(n_an, 1) * sizeof(int32_t)));
-  V.vstruct = c->vstruct.as<int32_t>();
+  const int32_t nb = c->nstruct;
   const bool grad = c->grad_mode && c->have_gvol;
-  if (c->have_pids) {
-    CK(c->vpid.ensure(std::max<int64_t>(n_an, 1) * sizeof(int32_t)));
-    V.pair_pid = c->pair_pid.as<int2>();
-    V.vpid = c->vpid.as<int32_t>();
-  }
-  LAUNCH(nsg::launch_vert(V, 1, c->stream));
-  stage_end(c, kStageVertex);
-  stage_begin(c, kStageMC);
-  M.vpos = c->vpos.as<double>();
-  M.vkey = c->vkey.as<int4>();
-  M.vstruct = c->vstruct.as<int32_t>();
-  {
+  // Every pass places its items by look-back and leaves its count on the device, where the next
+  // passes read it: the host reads the counts and the areas once, at the end.  The capacities come
+  // from the pairs of the cast (two vertices each, and about as many active cubes); a pass that
+  // exceeds one is seen in the counts, and the triangulation runs again with larger arrays.
+  const int64_t pair_verts = 2 * c->n_pairs;
+  int64_t cap_vert = (int64_t)(c->vert_ratio * (double)pair_verts) + 4096;
+  int64_t cap_active = (int64_t)(c->cube_ratio * (double)pair_verts) + 4096;
+  int64_t cap_tri = (int64_t)(c->tri_ratio * (double)pair_verts) + 8192;
+  int64_t counts[nsg::kMcCounts] = {0};
+  for (int attempt = 0;; attempt++) {
+    cap_active = std::min<int64_t>(cap_active, ((int64_t)1 << 31) / 12 - 1);
+    // counts, areas, error flag, tickets | look-back words of the four passes | per-structure offsets
+    const nsg::McTickets tk = nsg::mc_tickets(c->mc_tot, c->awords_tot, cap_active);
+    const int64_t head = nsg::kMcCounts + nb + 4;
+    const int64_t offs = head + tk.vert + tk.rows + tk.mid + tk.tris;
+    const int64_t zeroed = offs + 2 * ((int64_t)nb + 1);
+    CK(c->mc_block.ensure(zeroed * sizeof(int64_t)));
+    CK(c->h_read.ensure(head * sizeof(int64_t)));
+    int64_t* blk = c->mc_block.as<int64_t>();
+    double* areas_d = (double*)(blk + nsg::kMcCounts);
+    int32_t* err_d = (int32_t*)(blk + nsg::kMcCounts + nb);
+    unsigned int* tickets = (unsigned int*)(blk + nsg::kMcCounts + nb + 1);
+    unsigned long long* look = (unsigned long long*)(blk + head);
+    int64_t* voff = blk + offs;
+    int64_t* aoff = voff + nb + 1;
+    stage_begin(c, kStageVertex);
+    CK(cudaMemsetAsync(blk, 0, zeroed * sizeof(int64_t), c->stream));
+    CK(c->vkey.ensure(cap_vert * sizeof(int4)));
+    CK(c->vpos.ensure(cap_vert * 3 * sizeof(double)));
+    CK(c->vstruct.ensure(cap_vert * sizeof(int32_t)));
+    CK(c->act_rec.ensure(cap_active * sizeof(int4)));
+    // the active-cube map (per 32 cubes of a row: their active bits and the first one's index) and
+    // 12 vertex slots per active cube, all -1 until the vertices are written into them
+    CK(c->amap.ensure(std::max<int64_t>(c->awords_tot, 1) * sizeof(int2)));
+    CK(c->cube_vl.ensure(cap_active * 12 * sizeof(int32_t)));
+    CK(c->tri_cnt.ensure(cap_active * sizeof(int32_t)));
+    CK(c->bnd_list.ensure(cap_active * sizeof(int32_t)));
+    CK(c->cube_area.ensure(cap_active * sizeof(double)));
+    CK(c->tris.ensure(cap_tri * 3 * sizeof(int32_t)));
+    nsg::VertArgs V{};
+    V.B = B;
+    V.nrays = c->mc_tot;
+    V.ray_pair_off = c->ray_pair_off.as<int64_t>();
+    V.ray_pair_cnt = c->ray_pair_cnt.as<int32_t>();
+    V.pairs = c->pairs.as<double>();
+    V.bits = c->bits.as<uint32_t>();
+    V.vpos = c->vpos.as<double>();
+    V.vkey = c->vkey.as<int4>();
+    V.vstruct = c->vstruct.as<int32_t>();
+    V.cap = cap_vert;
+    if (c->have_pids) {
+      CK(c->vpid.ensure(cap_vert * sizeof(int32_t)));
+      V.pair_pid = c->pair_pid.as<int2>();
+      V.vpid = c->vpid.as<int32_t>();
+    }
+    V.voff = voff;
+    V.counts = blk;
+    V.lb = nsg::LookBack{look, tickets, err_d};
+    nsg::MCArgs M{};
+    M.B = B;
+    M.bits = c->bits.as<uint32_t>();
+    M.vpos = V.vpos;
+    M.vkey = V.vkey;
+    M.vstruct = V.vstruct;
+    M.cap_vert = cap_vert;
+    M.cap_active = cap_active;
+    M.cap_tri = cap_tri;
+    M.nwords_map = c->awords_tot;
+    M.act_rec = c->act_rec.as<int4>();
+    M.tri_cnt = c->tri_cnt.as<int32_t>();
+    M.bnd_list = c->bnd_list.as<int32_t>();
+    M.amap = c->amap.as<int2>();
+    M.cube_vl = c->cube_vl.as<int32_t>();
+    M.tris = c->tris.as<int32_t>();
+    M.cube_area = c->cube_area.as<double>();
+    M.voff = voff;
+    M.aoff = aoff;
+    M.counts = blk;
+    M.lb_rows = nsg::LookBack{look + tk.vert, tickets + 1, err_d};
+    M.lb_mid = nsg::LookBack{look + tk.vert + tk.rows, tickets + 2, err_d};
+    M.lb_tris = nsg::LookBack{look + tk.vert + tk.rows + tk.mid, tickets + 3, err_d};
+    LAUNCH(nsg::launch_vert(V, c->stream));
+    stage_end(c, kStageVertex);
+    stage_begin(c, kStageMC);
     // The slots are cleared to -1 and the analytic vertices written into them structure chunk by
     // structure chunk, each chunk's slots small enough to stay in L2 between the two: the push's
-    // 4-byte stores then complete sectors in L2 instead of making DRAM read every sector back.
-    const int32_t nb = c->nstruct;
-    CK(c->chunk_off.ensure(2 * (size_t)(nb + 1) * sizeof(int64_t)));
-    int64_t* d_off = c->chunk_off.as<int64_t>();
-    LAUNCH(nsg::launch_gather_i64(c->surv_off.as<int64_t>(), B.mc_base, nb + 1, d_off, c->stream));
-    LAUNCH(nsg::launch_gather_i64(c->row_act_off.as<int64_t>(), B.row_base, nb + 1, d_off + nb + 1, c->stream));
-    std::vector<int64_t> off(2 * (size_t)(nb + 1));
-    CK(cudaMemcpyAsync(off.data(), d_off, off.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    const int64_t* voff = off.data();
-    const int64_t* aoff = off.data() + nb + 1;
+    // 4-byte stores then complete sectors in L2 instead of making DRAM read every sector back.  A
+    // structure's share of the cubes is taken from its share of the patches: the chunk lines only
+    // steer the cache.  Where all slots take a tenth of L2 the classification clears them itself
+    // (one launch less); at 1.1 M cubes in one structure that would cost the push 60 us instead of 34.
     constexpr int64_t kChunkCubes = (int64_t)1 << 20;  // 48 MB of slots
+    M.clear_slots = pair_verts <= kChunkCubes / 4;
+    LAUNCH(nsg::launch_mc_rows(M, c->stream));
+    const auto share = [&](int32_t b0, int32_t b1) -> int64_t {
+      const double np = (double)std::max<int64_t>(c->patch_off[nb], 1);
+      return (int64_t)((double)pair_verts * ((double)(c->patch_off[b1] - c->patch_off[b0]) / np)) + 1;
+    };
     for (int32_t b0 = 0; b0 < nb;) {
-      int32_t b1 = b0 + 1;
-      while (b1 < nb && aoff[b1 + 1] - aoff[b0] <= kChunkCubes) b1++;
-      const int64_t a0 = aoff[b0], a1 = aoff[b1];
-      if (a1 > a0) CK(cudaMemsetAsync(c->cube_vl.as<int32_t>() + 12 * a0, 0xff, (a1 - a0) * 12 * sizeof(int32_t),
-                                      c->stream));
-      LAUNCH(nsg::launch_mc_push(M, voff[b0], voff[b1], c->stream));
+      int32_t b1 = M.clear_slots ? nb : b0 + 1;
+      while (b1 < nb && share(b0, b1 + 1) <= kChunkCubes) b1++;
+      const int64_t n = share(b0, b1);
+      if (!M.clear_slots) LAUNCH(nsg::launch_mc_clear(M, b0, b1, n, c->stream));
+      LAUNCH(nsg::launch_mc_push(M, b0, b1, n, c->stream));
       b0 = b1;
     }
-  }
-  // midpoint vertices of cut edges without an analytic vertex
-  LAUNCH(nsg::launch_mc_mid(M, 0, c->stream));
-  rc = scan_counts(c, c->row_mid_cnt.as<int32_t>(), n_act, c->row_mid_off.as<int64_t>(), &n_mid);
-  if (rc) return rc;
-  const int64_t n_v = n_an + n_mid;
-  if ((size_t)n_v * sizeof(int4) > c->vkey.cap || (size_t)n_v * 3 * sizeof(double) > c->vpos.cap) {
-    DevBuf nk, np_;
-    CK(nk.ensure(n_v * sizeof(int4)));
-    CK(np_.ensure(n_v * 3 * sizeof(double)));
-    if (n_an) {
-      CK(cudaMemcpyAsync(nk.p, c->vkey.p, n_an * sizeof(int4), cudaMemcpyDeviceToDevice, c->stream));
-      CK(cudaMemcpyAsync(np_.p, c->vpos.p, n_an * 3 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    // midpoint vertices of cut edges without an analytic vertex
+    LAUNCH(nsg::launch_mc_mid(M, c->stream));
+    if (grad) {
+      const nsg::PatchDev P = patch_dev(c);
+      const int64_t nv = std::max<int64_t>(pair_verts, 1);
+      CK(c->vgrad.ensure(nv * sizeof(double)));
+      CK(c->garea.ensure(std::max<int64_t>(c->np, 1) * NS_GRAD_PER_PATCH * sizeof(double)));
+      CK(cudaMemsetAsync(c->vgrad.p, 0, nv * sizeof(double), c->stream));
+      CK(cudaMemsetAsync(c->garea.p, 0, std::max<int64_t>(c->np, 1) * NS_GRAD_PER_PATCH * sizeof(double), c->stream));
+      M.vpid = c->vpid.as<int32_t>();
+      M.vgrad = c->vgrad.as<double>();
+      M.garea = c->garea.as<double>();
+      M.f64 = P.f64;
+      M.i32 = P.i32;
+      M.probe = P.probe;
     }
+    LAUNCH(nsg::launch_mc_tris_bnd(M, c->stream));
+    LAUNCH(nsg::launch_mc_tris(M, c->tune.mc_tris_bpsm, c->stream));
+    if (grad) LAUNCH(nsg::launch_grad_vert(M, pair_verts, c->stream));
+    // per-structure areas in an order fixed by the structure alone (independent of the batch)
+    CK(c->seg_part.ensure((size_t)nb * nsg::kSegParts * sizeof(double)));
+    nsg::SegArrays seg{};
+    seg.v[0] = M.cube_area;
+    seg.base[0] = aoff;
+    LAUNCH(nsg::launch_segment_sums(seg, 1, nb, cap_active, areas_d, c->seg_part.as<double>(), c->stream));
+    CK(cudaMemcpyAsync(c->h_read.p, blk, head * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    c->vkey.release();
-    c->vpos.release();
-    c->vkey = nk;
-    c->vpos = np_;
+    stage_end(c, kStageMC);
+    const int64_t* got = c->h_read.as<int64_t>();
+    memcpy(counts, got, sizeof counts);
+    if (*(const int32_t*)(got + nsg::kMcCounts + nb) != 0)
+      return fail(NSG_ERR_TIMEOUT, "a look-back wait of the triangulation ran out");
+    const int64_t n_act = counts[nsg::kMcActive];
+    const int64_t n_v = counts[nsg::kMcAnalytic] + counts[nsg::kMcMidpoint];
+    if (n_act >= ((int64_t)1 << 31) / 12) return fail(NSG_ERR_CAPACITY, "too many active cubes in one batch");
+    if (n_act <= cap_active && n_v <= cap_vert && counts[nsg::kMcTriangle] <= cap_tri) {
+      memcpy(c->areas.data(), got + nsg::kMcCounts, nb * sizeof(double));
+      break;
+    }
+    // the counts past a dropped pass are not known yet: room for them is found in the next run
+    if (attempt >= 4) return fail(NSG_ERR_CAPACITY, "triangulation capacities did not settle");
+    cap_active = std::max(cap_active, n_act + n_act / 16);
+    cap_vert = std::max(cap_vert, n_v + n_v / 16);
+    cap_tri = std::max(cap_tri, std::max(counts[nsg::kMcTriangle], 2 * n_act) + n_act / 8);
+    // the next triangulations of this context start from these ratios
+    const double pv = (double)std::max<int64_t>(pair_verts, 4096);
+    c->cube_ratio = std::min(std::max(c->cube_ratio, (double)cap_active / pv), 16.0);
+    c->vert_ratio = std::min(std::max(c->vert_ratio, (double)cap_vert / pv), 16.0);
+    c->tri_ratio = std::min(std::max(c->tri_ratio, (double)cap_tri / pv), 32.0);
   }
-  if ((size_t)n_v * sizeof(int32_t) > c->vstruct.cap) {
-    DevBuf ns;
-    CK(ns.ensure(n_v * sizeof(int32_t)));
-    if (n_an) CK(cudaMemcpyAsync(ns.p, c->vstruct.p, n_an * sizeof(int32_t), cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    c->vstruct.release();
-    c->vstruct = ns;
-  }
-  M.vpos = c->vpos.as<double>();
-  M.vkey = c->vkey.as<int4>();
-  M.vstruct = c->vstruct.as<int32_t>();
-  LAUNCH(nsg::launch_mc_mid(M, 1, c->stream));
-  M.n_active = n_act;
-  CK(c->tri_off.ensure((n_act + 1) * sizeof(int64_t)));
-  CK(c->cube_area.ensure(std::max<int64_t>(n_act, 1) * sizeof(double)));
-  M.tri_cnt = c->tri_cnt.as<int32_t>();
-  M.cube_area = c->cube_area.as<double>();
-  if (grad) {
-    const nsg::PatchDev P = patch_dev(c);
-    CK(c->vgrad.ensure(std::max<int64_t>(n_an, 1) * sizeof(double)));
-    CK(c->garea.ensure(std::max<int64_t>(c->np, 1) * NS_GRAD_PER_PATCH * sizeof(double)));
-    CK(cudaMemsetAsync(c->vgrad.p, 0, std::max<int64_t>(n_an, 1) * sizeof(double), c->stream));
-    CK(cudaMemsetAsync(c->garea.p, 0, std::max<int64_t>(c->np, 1) * NS_GRAD_PER_PATCH * sizeof(double), c->stream));
-    M.vpid = c->vpid.as<int32_t>();
-    M.vgrad = c->vgrad.as<double>();
-    M.garea = c->garea.as<double>();
-    M.f64 = P.f64;
-    M.i32 = P.i32;
-    M.probe = P.probe;
-  }
-  LAUNCH(nsg::launch_mc_tris_bnd(M, c->stream));
-  int64_t n_tri = 0;
-  rc = scan_counts(c, c->tri_cnt.as<int32_t>(), n_act, c->tri_off.as<int64_t>(), &n_tri);
-  if (rc) return rc;
-  CK(c->tris.ensure(std::max<int64_t>(n_tri, 1) * 3 * sizeof(int32_t)));
-  M.tri_off = c->tri_off.as<int64_t>();
-  M.tris = c->tris.as<int32_t>();
-  LAUNCH(nsg::launch_mc_tris(M, c->tune.mc_tris_bpsm, c->stream));
-  if (grad) LAUNCH(nsg::launch_grad_vert(M, c->stream));
   c->have_garea = grad;
-  // per-structure areas in an order fixed by the structure alone (independent of the batch)
-  CK(c->area_struct.ensure(c->nstruct * sizeof(double)));
-  CK(c->seg_part.ensure((size_t)c->nstruct * nsg::kSegParts * sizeof(double)));
-  LAUNCH(nsg::launch_segment_sums(c->cube_area.as<double>(), c->row_act_off.as<int64_t>(), B.row_base, c->nstruct,
-                                  c->area_struct.as<double>(), c->seg_part.as<double>(), false, c->stream));
-  CK(cudaMemcpyAsync(c->areas.data(), c->area_struct.p, c->nstruct * sizeof(double), cudaMemcpyDeviceToHost,
-                     c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  const double area = c->areas[0];
-  stage_end(c, kStageMC);
-  c->n_analytic = n_an;
-  c->n_vert = n_v;
-  c->n_tri = n_tri;
-  c->n_active = n_act;
-  c->area = area;
-  if (area_out) *area_out = area;
-  if (nverts) *nverts = n_v;
-  if (ntris) *ntris = n_tri;
+  c->n_analytic = counts[nsg::kMcAnalytic];
+  c->n_vert = c->n_analytic + counts[nsg::kMcMidpoint];
+  c->n_tri = counts[nsg::kMcTriangle];
+  c->n_active = counts[nsg::kMcActive];
+  c->area = c->areas[0];
+  if (area_out) *area_out = c->area;
+  if (nverts) *nverts = c->n_vert;
+  if (ntris) *ntris = c->n_tri;
   return NSG_OK;
 }
 
@@ -1827,10 +1870,8 @@ int nsg_download_status(nsg_ctx* c, int32_t* dst) {
   if (!c || !dst || !c->have_status) return NSG_ERR_STATE;
   if (c->nstruct != 1) return fail(NSG_ERR_STATE, "the dense status map is kept for a single structure");
   CK(cudaSetDevice(c->device));
-  if (!c->status_dense) {
-    int rc = materialize_status(c, nullptr);
-    if (rc) return rc;
-  }
+  int rc = ensure_dense_status(c);
+  if (rc) return rc;
   const NsGrid& g = c->grid;
   CK(cudaMemcpyAsync(dst, c->status.p, g.nx * g.ny * g.nz * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1866,10 +1907,14 @@ int nsg_download_cavities(nsg_ctx* c, double* sizes, int32_t* filled) {
 int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int32_t* offsets, int32_t* atoms,
                      int64_t* n_total) {
   if (!c || (n_atoms > 0 && !atoms_xyzr) || n_atoms < 0 || (atoms && !offsets)) return NSG_ERR_ARG;
-  if (!c->cav_detected || !c->status_dense || c->nstruct != 1)
+  if (!c->cav_detected || c->nstruct != 1)
     return fail(NSG_ERR_STATE, "cavity atoms need nsg_cavities after the cast");
   if (!c->have_cav_atoms) {
     CK(cudaSetDevice(c->device));
+    {
+      int rc = ensure_dense_status(c);
+      if (rc) return rc;
+    }
     const NsGrid& g = c->grid;
     c->cav_atom_off.assign(c->ncav + 1, 0);
     c->cav_atom_list.clear();
@@ -1924,6 +1969,7 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
         CK(cudaMemcpyAsync(c->ca_cell_atoms.p, cell_atoms.data(), n_atoms * sizeof(int32_t), cudaMemcpyHostToDevice,
                            c->stream));
       CK(cudaMemsetAsync(c->ca_count.p, 0, 2 * sizeof(unsigned long long), c->stream));
+      CK(c->err.ensure(sizeof(int32_t)));
       CK(cudaMemsetAsync(c->err.p, 0, sizeof(int32_t), c->stream));
       nsg::CavAtomArgs A{};
       A.status = c->status.as<int32_t>();
@@ -2014,6 +2060,8 @@ int nsg_download_idebmap(nsg_ctx* c, uint8_t* dst) {
   const size_t nn = (size_t)g.nx * g.ny * g.nz;
   if (!c->ideb_ready) {
     CK(c->ideb.ensure(nn));
+    int rc = ensure_free_runs(c);
+    if (rc) return rc;
     nsg::RunArgs A = run_args(c);
     LAUNCH(nsg::ideb_write(A, c->eps_filled ? c->cc_fill_of.as<uint8_t>() : nullptr, c->ideb.as<uint8_t>(),
                            c->stream));

@@ -111,8 +111,10 @@ __global__ void k_run_compress(int32_t* L, int64_t n, uint8_t* is_root) {
 // Region index of every run (binary search in the sorted roots), region node counts and first
 // node in descending-z scan order.  Lanes of a warp in the same region are combined before the
 // atomics.
-__global__ void k_run_stats(RunArgs A, const int32_t* __restrict__ roots, int32_t nroots, unsigned long long* count,
-                            unsigned int* desc_key) {
+__global__ void k_run_stats(RunArgs A, const int32_t* __restrict__ roots, const int32_t* __restrict__ nroots_d,
+                            int32_t cap, unsigned long long* count, unsigned int* desc_key) {
+  const int32_t nroots = *nroots_d;
+  if (nroots > cap) return;  // the caller makes room and calls again; L is untouched
   const int64_t plane = A.nx * A.ny;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < A.nruns; u += (int64_t)gridDim.x * blockDim.x) {
     unsigned act = __activemask();
@@ -478,10 +480,10 @@ cudaError_t run_select_roots(const uint8_t* is_root, int64_t n, int32_t* roots, 
   return cub::DeviceSelect::Flagged(temp, *temp_bytes, it, is_root, roots, nroots, n, s);
 }
 
-cudaError_t run_stats(const RunArgs& A, const int32_t* roots, int32_t nroots, unsigned long long* count,
-                      unsigned int* desc_key, cudaStream_t s) {
-  if (A.nruns <= 0 || nroots <= 0) return cudaSuccess;
-  k_run_stats<<<grid_for(A.nruns), 256, 0, s>>>(A, roots, nroots, count, desc_key);
+cudaError_t run_stats(const RunArgs& A, const int32_t* roots, const int32_t* nroots, int32_t cap,
+                      unsigned long long* count, unsigned int* desc_key, cudaStream_t s) {
+  if (A.nruns <= 0) return cudaSuccess;
+  k_run_stats<<<grid_for(A.nruns), 256, 0, s>>>(A, roots, nroots, cap, count, desc_key);
   return cudaGetLastError();
 }
 

@@ -30,8 +30,9 @@ cudaError_t run_label(const RunArgs& A, uint8_t* is_root, cudaStream_t s);
 cudaError_t run_select_roots(const uint8_t* is_root, int64_t n, int32_t* roots, int32_t* nroots, void* temp,
                              size_t* temp_bytes, cudaStream_t s);
 // Region sizes (nodes) and first nodes in descending-z scan order; L becomes the region index.
-cudaError_t run_stats(const RunArgs& A, const int32_t* roots, int32_t nroots, unsigned long long* count,
-                      unsigned int* desc_key, cudaStream_t s);
+// nroots is the device count of run_select_roots; with more regions than cap nothing is done.
+cudaError_t run_stats(const RunArgs& A, const int32_t* roots, const int32_t* nroots, int32_t cap,
+                      unsigned long long* count, unsigned int* desc_key, cudaStream_t s);
 // Cavity filling on the insideness bits.
 cudaError_t run_fill(const RunArgs& A, const uint8_t* fill_of, uint32_t* bits, int64_t nwords, cudaStream_t s);
 // Dense status map from the runs; label_of == nullptr writes TEMPORARY_OUT for free nodes.

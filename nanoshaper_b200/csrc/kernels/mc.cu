@@ -22,19 +22,14 @@
 // areas; here |cross product| / 2, the same quantity) (triangulationKernel :9075-9318,
 // getTriangles :14559-14780).  Triangles with an edge without a vertex are skipped, as the
 // reference does.
-#include <cub/cub.cuh>
-
-#include "../mc_cases.h"
 #include "grad.cuh"
+#include "lookback.cuh"
 #include "mc.h"
+#include "mc_tables.cuh"
 
 namespace nsg {
 
 namespace {
-
-__constant__ int8_t c_tri[256][16];  // triangle edge lists, -1 terminated
-__constant__ uint16_t c_emask[256];  // cut-edge mask per case
-__constant__ uint8_t c_ntri[256];    // case-table triangles per case
 
 // Node coordinate, and the grid edge a point on a ray along axis d lies on: the nearest node after
 // the half-side shift, floor((p - min) * scale + 0.5).  Each operation is rounded on its own (the
@@ -55,14 +50,54 @@ struct RayId {
   int64_t m, n;
 };
 
+// Local ray ordinal r of a structure; a panel has fewer than 2^31 rays, so its divisions run in
+// 32 bits.
 __device__ __forceinline__ RayId ray_of(const GridDev& g, int64_t r) {
   const int64_t NX = g.n[0], NY = g.n[1], NZ = g.n[2];
   RayId id;
-  int64_t R0 = NZ * NY, R1 = NY * NX;
-  if (r < R0) { id.panel = 0; id.n = r / NY; id.m = r - id.n * NY; }
-  else if (r < R0 + R1) { int64_t q = r - R0; id.panel = 1; id.n = q / NX; id.m = q - id.n * NX; }
-  else { int64_t q = r - R0 - R1; id.panel = 2; id.n = q / NX; id.m = q - id.n * NX; }
+  const int64_t R0 = NZ * NY, R1 = NY * NX;
+  unsigned w = (unsigned)NX, q;
+  if (r < R0) { id.panel = 0; q = (unsigned)r; w = (unsigned)NY; }
+  else if (r < R0 + R1) { id.panel = 1; q = (unsigned)(r - R0); }
+  else { id.panel = 2; q = (unsigned)(r - R0 - R1); }
+  const unsigned n = q / w;
+  id.n = n;
+  id.m = q - n * w;
   return id;
+}
+
+// Structure of ascending items of a batch: one search for the warp's first item, then a step per
+// structure boundary, so that a pass over several items per lane searches once.
+struct StructWalk {
+  const int64_t* base;
+  int n, b;
+  int64_t next;  // first item of the structure after b
+  __device__ __forceinline__ StructWalk(const int64_t* __restrict__ base_, int n_, int64_t warp_first)
+      : base(base_), n(n_), b(0) {
+    if (n > 1) b = find_struct(base, n, warp_first);
+    next = base[b + 1];
+  }
+  __device__ __forceinline__ int at(int64_t x) {
+    while (x >= next && b + 1 < n) next = base[++b + 1];
+    return b;
+  }
+};
+
+// Position of set bit k (from the lowest, k < popc(m)) of m.
+__device__ __forceinline__ int nth_bit(unsigned m, int k) {
+  int pos = 0;
+#pragma unroll
+  for (int step = 16; step; step >>= 1) {
+    const int c = __popc(m & ((1u << step) - 1u));
+    if (k >= c) {
+      k -= c;
+      m >>= step;
+      pos += step;
+    } else {
+      m &= (1u << step) - 1u;
+    }
+  }
+  return pos;
 }
 
 // Edge key (ix, iy, iz, dir) of the vertex at ray position index a.
@@ -124,54 +159,139 @@ __device__ __forceinline__ void push_vertex(const int2* __restrict__ amap, int32
   }
 }
 
-template <bool emit>
-__global__ void k_vert(VertArgs A) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < A.nrays; r += (int64_t)gridDim.x * blockDim.x) {
-    int np = A.ray_pair_cnt[r];
-    if (!emit) {
-      int cnt = 0;
-      if (np > 0) {
-        const StructDev& S = A.B.s[find_struct(A.B.mc_base, A.B.n, r)];
-        const GridDev& g = S.g;
-        const uint32_t* bits = A.bits + S.word_base;
-        RayId id = ray_of(g, r - S.mc_base);
-        int vc = id.panel == 0 ? 0 : (id.panel == 1 ? 2 : 1);
-        const double* pr = A.pairs + 2 * A.ray_pair_off[r];
-        for (int q = 0; q < 2 * np; q++)
-          if (keeps(g, bits, S.nwords, edge_key(id, edge_index(g, vc, pr[q])))) cnt++;
-      }
-      A.surv_cnt[r] = cnt;
+constexpr int kPassThreads = 256;
+
+// Whether the passes before left complete arrays: no look-back wait ran out and their items fit.
+__device__ __forceinline__ bool cubes_ok(const MCArgs& A) {
+  return *A.lb_rows.err == 0 && A.counts[kMcActive] <= A.cap_active && A.counts[kMcAnalytic] <= A.cap_vert;
+}
+
+// Items (rays, map words, cubes) per thread of a one-pass kernel.  A block waits for the blocks
+// before it about as long as it counts, so a large input wants tickets with more work: 4 items per
+// thread where that leaves four blocks per SM, 8 (for the passes that have them) where it leaves 16;
+// a small input is spread over more blocks.  Triangles of 64 conformers, 8.4 M cubes: 1,053 us
+// with 1 item (and a 32-ticket look-back), 639 with 4, 579 with 8; of one 20,000-atom molecule,
+// 1.1 M cubes: 123, 84, 90.  Vertices of the conformers: 520, 381, 462.
+int pass_items(int64_t items, int most) {
+  const int64_t per_sm = (int64_t)sm_count() * kPassThreads;
+  if (most >= 8 && items >= per_sm * 8 * 16) return 8;
+  return items >= per_sm * 4 * 4 ? 4 : 1;
+}
+constexpr int kVertItems = 4, kRowsItems = 8, kMidItems = 4, kTrisItems = 8;
+
+// Vertices in one pass, one thread per ray, a ticket of consecutive rays per block (lookback.cuh): the
+// thread keeps a mask of its pair ends whose edge is cut, the block places its vertices behind
+// those of the tickets before it, and the warp writes them with a vertex per lane (coalesced; the
+// surviving ends of a ray per lane leave half the lanes idle).  Latency-bound (bit and pair
+// gathers).  Count pass, scan and write pass before -> this: 64 conformers (4.3 M rays, 8.4 M
+// vertices) 466 + 30 -> 381 us; 20,000 atoms, where 1.2 M rays hold few hits, 64 + 8 -> 75 us and no
+// host round trip between the passes.
+template <int kItems>
+__global__ void __launch_bounds__(kPassThreads) k_vert(VertArgs A) {
+  __shared__ unsigned int s_ticket;
+  const unsigned t = take_ticket(A.lb, &s_ticket);
+  const int lane = threadIdx.x & 31;
+  const int64_t r0 = (int64_t)t * (kPassThreads * kItems) + (threadIdx.x >> 5) * (32 * kItems) + lane;
+  unsigned mask[kItems];  // kept ends among the first 32
+  int cnt[kItems], sum = 0;
+  const StructWalk start(A.B.mc_base, A.B.n, r0 - lane);
+  StructWalk walk = start;
+#pragma unroll
+  for (int x = 0; x < kItems; x++) {
+    const int64_t r = r0 + 32 * x;
+    const bool valid = r < A.nrays;
+    mask[x] = 0;
+    cnt[x] = 0;
+    const int b = walk.at(r);
+    const int np = valid ? A.ray_pair_cnt[r] : 0;
+    if (np > 0) {
+      const StructDev& S = A.B.s[b];
+      const RayId id = ray_of(S.g, r - S.mc_base);
+      const int vc = id.panel == 0 ? 0 : (id.panel == 1 ? 2 : 1);
+      const double* pr = A.pairs + 2 * A.ray_pair_off[r];
+      for (int q = 0; q < 2 * np; q++)
+        if (keeps(S.g, A.bits + S.word_base, S.nwords, edge_key(id, edge_index(S.g, vc, pr[q])))) {
+          cnt[x]++;
+          if (q < 32) mask[x] |= 1u << q;
+        }
+    }
+    sum += cnt[x];
+  }
+  int64_t off = warp_offset<kPassThreads>(A.lb, t, warp_total(sum));
+  if (off < 0) return;
+  walk = start;
+  const auto emit = [&](int b, const RayId& id, int64_t po, int q, int64_t o) {
+    if (o >= A.cap) return;
+    const GridDev& g = A.B.s[b].g;
+    const double delta = NS_DELTA - g.hside;
+    const int vc = id.panel == 0 ? 0 : (id.panel == 1 ? 2 : 1);
+    const double x = A.pairs[2 * po + q];
+    const int4 e = edge_key(id, edge_index(g, vc, x));
+    double p0, p1, p2;
+    if (id.panel == 0) { p0 = x; p1 = gcoord(g, 1, id.m) + delta; p2 = gcoord(g, 2, id.n) + delta; }
+    else if (id.panel == 1) { p0 = gcoord(g, 0, id.m) + delta; p1 = gcoord(g, 1, id.n) + delta; p2 = x; }
+    else { p0 = gcoord(g, 0, id.m) + delta; p1 = x; p2 = gcoord(g, 2, id.n) + delta; }
+    A.vpos[3 * o + 0] = p0;
+    A.vpos[3 * o + 1] = p1;
+    A.vpos[3 * o + 2] = p2;
+    A.vkey[o] = e;
+    A.vstruct[o] = b;
+    if (A.vpid) {
+      const int2 pp = A.pair_pid[po + (q >> 1)];
+      A.vpid[o] = vpid_pack((q & 1) ? pp.y : pp.x, e.w);
+    }
+  };
+#pragma unroll 1
+  for (int x = 0; x < kItems; x++) {
+    const int64_t r = r0 + 32 * x;
+    const bool valid = r < A.nrays;
+    int c = cnt[0];
+    unsigned m = mask[0];
+#pragma unroll
+    for (int y = 1; y < kItems; y++)
+      if (x == y) { c = cnt[y]; m = mask[y]; }
+    const int b = walk.at(r);
+    const StructDev& S = A.B.s[b];
+    const int incl = warp_incl(c);
+    const int T = __shfl_sync(0xffffffffu, incl, 31);
+    if (valid && r == S.mc_base) A.voff[b] = off + incl - c;
+    if (r == A.nrays - 1) A.voff[A.B.n] = A.counts[kMcAnalytic] = off + incl;
+    if (T == 0) continue;
+    RayId id{0, 0, 0};
+    int64_t po = 0;
+    if (c > 0) {
+      id = ray_of(S.g, r - S.mc_base);
+      po = A.ray_pair_off[r];
+    }
+    if (__any_sync(0xffffffffu, c > 0 && A.ray_pair_cnt[r] > 16)) {
+      // a ray of the overflow path (more ends than the mask holds): each lane writes its own
+      // vertices
+      int64_t o = off + incl - c;
+      const int vc = id.panel == 0 ? 0 : (id.panel == 1 ? 2 : 1);
+      const int ends = c > 0 ? 2 * A.ray_pair_cnt[r] : 0;
+      for (int q = 0; q < ends; q++)
+        if (q < 32 ? (m >> q) & 1u
+                   : keeps(S.g, A.bits + S.word_base, S.nwords,
+                           edge_key(id, edge_index(S.g, vc, A.pairs[2 * po + q]))))
+          emit(b, id, po, q, o++);
+      off += T;
       continue;
     }
-    if (np == 0 || A.surv_cnt[r] == 0) continue;
-    const StructDev& S = A.B.s[find_struct(A.B.mc_base, A.B.n, r)];
-    const GridDev& g = S.g;
-    const uint32_t* bits = A.bits + S.word_base;
-    RayId id = ray_of(g, r - S.mc_base);
-    int vc = id.panel == 0 ? 0 : (id.panel == 1 ? 2 : 1);
-    const double* pr = A.pairs + 2 * A.ray_pair_off[r];
-    const double delta = NS_DELTA - g.hside;
-    double base[3];
-    if (id.panel == 0) { base[1] = gcoord(g, 1, id.m) + delta; base[2] = gcoord(g, 2, id.n) + delta; }
-    else if (id.panel == 1) { base[0] = gcoord(g, 0, id.m) + delta; base[1] = gcoord(g, 1, id.n) + delta; }
-    else { base[0] = gcoord(g, 0, id.m) + delta; base[2] = gcoord(g, 2, id.n) + delta; }
-    int64_t o = A.surv_off[r];
-    for (int q = 0; q < 2 * np; q++) {
-      int4 e = edge_key(id, edge_index(g, vc, pr[q]));
-      if (!keeps(g, bits, S.nwords, e)) continue;
-      double p[3] = {base[0], base[1], base[2]};
-      p[vc] = pr[q];
-      A.vpos[3 * o + 0] = p[0];
-      A.vpos[3 * o + 1] = p[1];
-      A.vpos[3 * o + 2] = p[2];
-      A.vkey[o] = e;
-      A.vstruct[o] = (int32_t)(&S - A.B.s);
-      if (A.vpid) {
-        const int2 pp = A.pair_pid[A.ray_pair_off[r] + (q >> 1)];
-        A.vpid[o] = vpid_pack((q & 1) ? pp.y : pp.x, e.w);
-      }
-      o++;
+    const int im = (int)id.m, in = (int)id.n;
+    for (int j0 = 0; j0 < T; j0 += 32) {
+      const int j = j0 + lane;
+      const int l = owner_lane(incl, j < T ? j : T - 1);
+      const int k = j - __shfl_sync(0xffffffffu, incl - c, l);
+      const unsigned ml = __shfl_sync(0xffffffffu, m, l);
+      const int64_t pol = __shfl_sync(0xffffffffu, po, l);
+      RayId il;
+      il.panel = __shfl_sync(0xffffffffu, id.panel, l);
+      il.m = __shfl_sync(0xffffffffu, im, l);
+      il.n = __shfl_sync(0xffffffffu, in, l);
+      const int bl = __shfl_sync(0xffffffffu, b, l);
+      if (j < T) emit(bl, il, pol, nth_bit(ml, k), off + j);
     }
+    off += T;
   }
 }
 
@@ -189,128 +309,215 @@ __device__ __forceinline__ uint32_t bits32_pair(const uint32_t* __restrict__ bit
   return x;
 }
 
-// Cube rows (j, k), one thread per row; a warp takes a chunk of consecutive rows of one structure.
-// The thread walks its row 32 cubes at a time: the cubes' corners come from the four bit rows
-// they touch (corner inside = bit 0), one pair of words per bit row, and a cube is active unless
-// its 8 corners agree.  Pass 0 counts the active cubes of the row; pass 1 writes them in i order
-// at the row's offset and the row's words of the active-cube map.
-template <bool emit>
-__global__ void k_mc_rows(MCArgs A) {
-  __shared__ uint8_t s_ntri[256];
-  for (int t = threadIdx.x; t < 256; t += blockDim.x) s_ntri[t] = c_ntri[t];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t ch = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); ch < A.nchunks; ch += warps) {
-    const int4 C = A.row_chunks[ch];  // structure, first local row, row count
-    const StructDev& S = A.B.s[C.x];
-    const int NX = (int)S.g.n[0], NY = (int)S.g.n[1];
-    const uint32_t* bits = A.bits + S.word_base;
-    const int32_t nwords = (int32_t)S.nwords;
-    const int W = (NX - 2 + 31) >> 5;
-    for (int rr = lane; rr < C.z; rr += 32) {
-      const int lr = C.y + rr;
-      const int j = 1 + lr % (NY - 2), k = 1 + lr / (NY - 2);
-      const int64_t grow = S.row_base + lr;
-      const int32_t b00 = (k * NY + j) * NX, b10 = b00 + NX, b01 = b00 + NX * NY, b11 = b01 + NX;
-      int64_t slot = emit ? A.row_act_off[grow] : 0;
-      int32_t run = 0;
-      for (int word = 0; word < W; word++) {
-        const int32_t ic = 1 + 32 * word;
-        const int32_t nvalid = NX - 1 - ic;
-        const uint32_t vm = nvalid >= 32 ? 0xffffffffu : ((1u << nvalid) - 1u);
-        // corners i and i + 1 of each of the four bit rows from one pair of words per row
-        uint32_t c[8], n0, n1, n2, n3;
-        c[0] = ~bits32_pair(bits, nwords, b00 + ic, &n0);
-        c[1] = ~n0;
-        c[3] = ~bits32_pair(bits, nwords, b10 + ic, &n1);
-        c[2] = ~n1;
-        c[4] = ~bits32_pair(bits, nwords, b01 + ic, &n2);
-        c[5] = ~n2;
-        c[7] = ~bits32_pair(bits, nwords, b11 + ic, &n3);
-        c[6] = ~n3;
-        uint32_t d = 0;
+// The 32 cubes of a map word: row (j, k), first cube ic, and in c the inside bits of the cubes' 8
+// corners (corner inside = bit 0 of the grid), one pair of words per bit row; returns the active
+// cubes, those whose corners do not agree.
+__device__ __forceinline__ uint32_t word_cubes(const MCArgs& A, const StructDev& S, int64_t idx, int* ic, int* j, int* k,
+                                               uint32_t* c) {
+  const int NX = (int)S.g.n[0], NY = (int)S.g.n[1];
+  const uint32_t* bits = A.bits + S.word_base;
+  const int32_t nwords = (int32_t)S.nwords;
+  const unsigned W = (unsigned)(NX - 2 + 31) >> 5;
+  const unsigned local = (unsigned)(idx - S.aword_base);
+  const unsigned lr = local / W;
+  *ic = 1 + 32 * (int)(local - lr * W);
+  const unsigned kk = lr / (unsigned)(NY - 2);
+  *j = 1 + (int)(lr - kk * (unsigned)(NY - 2));
+  *k = 1 + (int)kk;
+  const int32_t b00 = (*k * NY + *j) * NX, b10 = b00 + NX, b01 = b00 + NX * NY, b11 = b01 + NX;
+  const int32_t nvalid = NX - 1 - *ic;
+  const uint32_t vm = nvalid >= 32 ? 0xffffffffu : ((1u << nvalid) - 1u);
+  uint32_t n0, n1, n2, n3;
+  c[0] = ~bits32_pair(bits, nwords, b00 + *ic, &n0);
+  c[1] = ~n0;
+  c[3] = ~bits32_pair(bits, nwords, b10 + *ic, &n1);
+  c[2] = ~n1;
+  c[4] = ~bits32_pair(bits, nwords, b01 + *ic, &n2);
+  c[5] = ~n2;
+  c[7] = ~bits32_pair(bits, nwords, b11 + *ic, &n3);
+  c[6] = ~n3;
+  uint32_t d = 0;
 #pragma unroll
-        for (int q = 1; q < 8; q++) d |= c[0] ^ c[q];
-        const uint32_t act = d & vm;
-        if (!emit) {
-          run += __popc(act);
-          continue;
-        }
-        A.amap[S.aword_base + (int64_t)lr * W + word] = make_int2((int)act, (int)slot);
-        for (uint32_t m = act; m; m &= m - 1) {
-          const int bit = __ffs(m) - 1;
-          int cs = 0;
+  for (int q = 1; q < 8; q++) d |= c[0] ^ c[q];
+  return d & vm;
+}
+
+// Cube classification in one pass, one thread per 32 cubes of a cube row (a word of the active-cube
+// map), a ticket of consecutive words per block: the block places its active cubes behind those of
+// the tickets before it (words in (k, j, i) order), and each warp writes the records, slots and
+// triangle counts of its words with a cube per lane.  Consecutive lanes read consecutive words of
+// the bit rows; the words that hold active cubes are read a second time, from L1.
+// Row per thread in a count and a write pass before -> this: 64 conformers (300 M cubes) 255 + 30 ->
+// 289 us; 20,000 atoms (236 M cubes) 156 + 8 -> 149 us; 2,000 atoms 15 + 5 -> 24 us, without the
+// host round trip (about 20 us).
+template <int kItems>
+__global__ void __launch_bounds__(kPassThreads) k_mc_rows(MCArgs A) {
+  __shared__ unsigned int s_ticket;
+  __shared__ uint32_t s_corner[kPassThreads / 32][8][32];
+  const unsigned t = take_ticket(A.lb_rows, &s_ticket);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i0 = (int64_t)t * (kPassThreads * kItems) + w * (32 * kItems) + lane;
+  uint32_t act[kItems];
+  int sum = 0;
+  const StructWalk start(A.B.aword_base, A.B.n, i0 - lane);
+  StructWalk walk = start;
 #pragma unroll
-          for (int q = 0; q < 8; q++) cs |= ((c[q] >> bit) & 1u) << q;
-          // every cut edge of a cube with i, j, k >= 2 has a vertex (an analytic one, or the
-          // midpoint its owner cube adds), so its triangles are the case table's; a cube on the
-          // low faces of the cube range may lack vertices on edges whose owner lies outside the
-          // range, and is counted after the midpoint vertices are in place (k_mc_tris_bnd)
-          if (ic + bit >= 2 && j >= 2 && k >= 2) {
-            A.tri_cnt[slot] = s_ntri[cs];
-          } else {
-            A.tri_cnt[slot] = 0;
-            const unsigned long long q = atomicAdd(A.bnd_cursor, 1ull);
-            A.bnd_list[q] = (int32_t)slot;
-          }
-          A.act_rec[slot++] = make_int4(ic + bit, j, k, cs | (C.x << 11));
-        }
-      }
-      if (!emit) A.row_act_cnt[grow] = run;
+  for (int x = 0; x < kItems; x++) {
+    const int64_t idx = i0 + 32 * x;
+    const bool valid = idx < A.nwords_map;
+    const int b = walk.at(idx);
+    act[x] = 0;
+    if (valid) {
+      int ic, j, k;
+      uint32_t c[8];
+      act[x] = word_cubes(A, A.B.s[b], idx, &ic, &j, &k, c);
     }
+    sum += __popc(act[x]);
+  }
+  int64_t off = warp_offset<kPassThreads>(A.lb_rows, t, warp_total(sum));
+  if (off < 0) return;
+  walk = start;
+#pragma unroll 1
+  for (int x = 0; x < kItems; x++) {
+    const int64_t idx = i0 + 32 * x;
+    const bool valid = idx < A.nwords_map;
+    const int b = walk.at(idx);
+    const StructDev& S = A.B.s[b];
+    uint32_t a = act[0];
+#pragma unroll
+    for (int y = 1; y < kItems; y++)
+      if (x == y) a = act[y];
+    const int cnt = __popc(a);
+    const int incl = warp_incl(cnt);
+    const int T = __shfl_sync(0xffffffffu, incl, 31);
+    if (valid) {
+      const int64_t first = off + incl - cnt;
+      A.amap[idx] = make_int2((int)a, (int)first);
+      if (idx == S.aword_base) A.aoff[b] = first;
+      if (idx == A.nwords_map - 1) A.aoff[A.B.n] = A.counts[kMcActive] = first + cnt;
+    }
+    if (T == 0) continue;
+    int ic = 0, j = 0, k = 0;
+    uint32_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (a) word_cubes(A, S, idx, &ic, &j, &k, c);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; q++) s_corner[w][q][lane] = c[q];
+    __syncwarp();
+    for (int j0 = 0; j0 < T; j0 += 32) {
+      const int y = j0 + lane;
+      const int l = owner_lane(incl, y < T ? y : T - 1);
+      const int first = __shfl_sync(0xffffffffu, incl - cnt, l);
+      const unsigned al = __shfl_sync(0xffffffffu, a, l);
+      const int il = __shfl_sync(0xffffffffu, ic, l), jl = __shfl_sync(0xffffffffu, j, l),
+                kl = __shfl_sync(0xffffffffu, k, l), bl = __shfl_sync(0xffffffffu, b, l);
+      const int64_t slot = off + y;
+      if (y >= T || slot >= A.cap_active) continue;
+      const int bit = nth_bit(al, y - first);
+      int cs = 0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) cs |= ((s_corner[w][q][l] >> bit) & 1u) << q;
+      const int i = il + bit;
+      // every cut edge of a cube with i, j, k >= 2 has a vertex (an analytic one, or the midpoint
+      // its owner cube adds), so its triangles are the case table's; a cube on the low faces of the
+      // cube range may lack vertices on edges whose owner lies outside the range, and is counted
+      // after the midpoint vertices are in place (k_mc_tris_bnd)
+      int ntri = d_mc.ntri[cs];
+      if (i < 2 || jl < 2 || kl < 2) {
+        ntri = 0;
+        const unsigned long long q = atomicAdd((unsigned long long*)(A.counts + kMcLowFace), 1ull);
+        A.bnd_list[q] = (int32_t)slot;
+      }
+      A.tri_cnt[slot] = ntri;
+      A.act_rec[slot] = make_int4(i, jl, kl, cs | (bl << 11));
+      if (A.clear_slots) {
+        int4* v = reinterpret_cast<int4*>(A.cube_vl + 12 * slot);
+        const int4 none = make_int4(-1, -1, -1, -1);
+        v[0] = none;
+        v[1] = none;
+        v[2] = none;
+      }
+    }
+    off += T;
   }
 }
 
-// One thread per active cube.  Pass 0: which of the cube's own edges 5, 6, 10 need a midpoint
-// vertex (cut edge without an analytic vertex); the mask goes to bits 8..10 of the record and the
-// count to mid_cnt.  Pass 1: writes those vertices at their final indices (act_mid) and into the
-// slots of the cubes that share their edges.
-template <bool emit>
-__global__ void k_mc_mid(MCArgs A) {
-  // case tables in shared memory: a constant-bank read with a different index per lane is
-  // serialised across the warp
-  __shared__ uint16_t s_emask[256];
-  for (int t = threadIdx.x; t < 256; t += blockDim.x) s_emask[t] = c_emask[t];
-  __syncthreads();
-  for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < A.n_active; a += (int64_t)gridDim.x * blockDim.x) {
-    int4 rec = A.act_rec[a];
+// Vertex slots of the active cubes of structures [b0, b1) to -1.
+__global__ void k_mc_clear(MCArgs A, int b0, int b1) {
+  if (!cubes_ok(A)) return;
+  int4* v = reinterpret_cast<int4*>(A.cube_vl);
+  const int4 none = make_int4(-1, -1, -1, -1);
+  for (int64_t q = 3 * A.aoff[b0] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < 3 * A.aoff[b1];
+       q += (int64_t)gridDim.x * blockDim.x)
+    v[q] = none;
+}
+
+// Midpoint vertices in one pass, one thread per active cube, a ticket of consecutive cubes per
+// block: which of the cube's own edges 5 (y at (i+1, j, k+1)), 6 (x at (i, j+1, k+1)), 10 (z at
+// (i+1, j+1, k)) are cut and carry no analytic vertex (their slots are still empty after the
+// analytic push); the vertices follow the analytic ones in (k, j, i, edge) order and go into the
+// slots of the cubes that share their edges.  An edge is slot 5, 6 or 10 of its owner alone, so no
+// cube's test reads a slot that another cube's midpoint is written to.  Bound by the slot reads.
+template <int kItems>
+__global__ void __launch_bounds__(kPassThreads) k_mc_mid(MCArgs A) {
+  __shared__ unsigned int s_ticket;
+  const int64_t n_act = A.counts[kMcActive], n_an = A.counts[kMcAnalytic];
+  if (!cubes_ok(A)) return;
+  const unsigned t = take_ticket(A.lb_mid, &s_ticket);
+  if ((int64_t)t * (kPassThreads * kItems) >= n_act) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t a0 = (int64_t)t * (kPassThreads * kItems) + (threadIdx.x >> 5) * (32 * kItems) + lane;
+  int mm[kItems], s5[kItems], s6[kItems], s10[kItems], sum = 0;
+#pragma unroll
+  for (int x = 0; x < kItems; x++) {
+    const int64_t a = a0 + 32 * x < n_act ? a0 + 32 * x : n_act - 1;
+    mm[x] = A.act_rec[a].w & 255;
+    s5[x] = A.cube_vl[12 * a + 5];
+    s6[x] = A.cube_vl[12 * a + 6];
+    s10[x] = A.cube_vl[12 * a + 10];
+  }
+#pragma unroll
+  for (int x = 0; x < kItems; x++) {
+    // edges 5, 6 and 10 join corners 5-6, 6-7 and 2-6
+    const int cs = mm[x], c6 = (cs >> 6) & 1;
+    mm[x] = 0;
+    if (((cs >> 5) & 1) != c6 && s5[x] < 0) mm[x] |= 1;
+    if (((cs >> 7) & 1) != c6 && s6[x] < 0) mm[x] |= 2;
+    if (((cs >> 2) & 1) != c6 && s10[x] < 0) mm[x] |= 4;
+    if (a0 + 32 * x >= n_act) mm[x] = 0;
+    sum += __popc(mm[x]);
+  }
+  int64_t off = warp_offset<kPassThreads>(A.lb_mid, t, warp_total(sum));
+  if (off < 0) return;
+#pragma unroll
+  for (int x = 0; x < kItems; x++) {
+    const int64_t a = a0 + 32 * x;
+    const int m = mm[x], cnt = __popc(m);
+    const int incl = warp_incl(cnt);
+    if (a == n_act - 1) A.counts[kMcMidpoint] = off + incl;
+    int64_t v = n_an + off + incl - cnt;
+    off += __shfl_sync(0xffffffffu, incl, 31);
+    if (!m || v + cnt > A.cap_vert) continue;
+    const int4 rec = A.act_rec[a];
     const int i = rec.x, j = rec.y, k = rec.z;
     const StructDev& S = A.B.s[rec_struct(rec.w)];
     const GridDev& g = S.g;
-    if (!emit) {
-      // own edges 5 (y at (i+1, j, k+1)), 6 (x at (i, j+1, k+1)), 10 (z at (i+1, j+1, k)) that are
-      // cut and carry no analytic vertex: their slots are still empty after the analytic push
-      const int em = s_emask[rec.w & 255];
-      const int4 s47 = reinterpret_cast<const int4*>(A.cube_vl + 12 * a)[1];
-      const int s10 = A.cube_vl[12 * a + 10];
-      int mm = 0;
-      if ((em & 32) && s47.y < 0) mm |= 1;
-      if ((em & 64) && s47.z < 0) mm |= 2;
-      if ((em & 1024) && s10 < 0) mm |= 4;
-      A.act_rec[a].w = (rec.w & ~(7 << 8)) | (mm << 8);
-      A.mid_cnt[a] = __popc(mm);
-      continue;
-    }
-    int mm = (rec.w >> 8) & 7;
-    int64_t v = A.n_analytic + A.mid_off[a];
-    A.act_mid[a] = (int32_t)v;
-    for (int q = 0; q < __popc(mm); q++) A.vstruct[v + q] = rec_struct(rec.w);
-    if (mm & 1) {
+    for (int q = 0; q < cnt; q++) A.vstruct[v + q] = rec_struct(rec.w);
+    if (m & 1) {
       A.vpos[3 * v] = gcoord(g, 0, i + 1) - g.hside; A.vpos[3 * v + 1] = gcoord(g, 1, j);
       A.vpos[3 * v + 2] = gcoord(g, 2, k + 1) - g.hside;
       A.vkey[v] = make_int4(i + 1, j, k + 1, NS_Y_DIR);
       push_vertex(A.amap, A.cube_vl, S, NS_Y_DIR, i + 1, j, k + 1, (int32_t)v);
       v++;
     }
-    if (mm & 2) {
+    if (m & 2) {
       A.vpos[3 * v] = gcoord(g, 0, i); A.vpos[3 * v + 1] = gcoord(g, 1, j + 1) - g.hside;
       A.vpos[3 * v + 2] = gcoord(g, 2, k + 1) - g.hside;
       A.vkey[v] = make_int4(i, j + 1, k + 1, NS_X_DIR);
       push_vertex(A.amap, A.cube_vl, S, NS_X_DIR, i, j + 1, k + 1, (int32_t)v);
       v++;
     }
-    if (mm & 4) {
+    if (m & 4) {
       A.vpos[3 * v] = gcoord(g, 0, i + 1) - g.hside; A.vpos[3 * v + 1] = gcoord(g, 1, j + 1) - g.hside;
       A.vpos[3 * v + 2] = gcoord(g, 2, k);
       A.vkey[v] = make_int4(i + 1, j + 1, k, NS_Z_DIR);
@@ -323,7 +530,9 @@ __global__ void k_mc_mid(MCArgs A) {
 // edge's cubes.  A ray's vertices are sorted along it and an edge's vertices all lie on one ray,
 // so they have consecutive ids: vertex v is the first of its edge unless vertex v - 1 has the same
 // edge key in the same structure.  Each slot is written once, with a plain store.
-__global__ void k_mc_push(MCArgs A, int64_t v0, int64_t v1) {
+__global__ void k_mc_push(MCArgs A, int b0, int b1) {
+  if (!cubes_ok(A)) return;
+  const int64_t v0 = A.voff[b0], v1 = A.voff[b1];
   for (int64_t v = v0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < v1; v += (int64_t)gridDim.x * blockDim.x) {
     const int4 e = A.vkey[v];
     const int32_t sv = A.vstruct[v];
@@ -335,24 +544,18 @@ __global__ void k_mc_push(MCArgs A, int64_t v0, int64_t v1) {
   }
 }
 
-// dst[q] = src[idx[q]]: per-structure offsets out of batch-wide prefix sums.
-__global__ void k_gather_i64(const int64_t* __restrict__ src, const int64_t* __restrict__ idx, int64_t n,
-                             int64_t* dst) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q < n) dst[q] = src[idx[q]];
-}
-
 // Triangle counts of the active cubes on the low faces of the cube range (listed by k_mc_rows): the
 // case-table triangles whose three edges have vertices.
 __global__ void k_mc_tris_bnd(MCArgs A) {
-  const int64_t n = (int64_t)*A.bnd_cursor;
+  if (!cubes_ok(A)) return;
+  const int64_t n = A.counts[kMcLowFace];
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
     const int32_t a = A.bnd_list[q];
     const int c = A.act_rec[a].w & 255;
     const int32_t* cv = A.cube_vl + 12 * (int64_t)a;
     int cnt = 0;
-    for (int t = 0; t < 16 && c_tri[c][t] >= 0; t += 3)
-      if (cv[c_tri[c][t]] >= 0 && cv[c_tri[c][t + 1]] >= 0 && cv[c_tri[c][t + 2]] >= 0) cnt++;
+    for (int t = 0; t < 16 && d_mc.tri[c][t] >= 0; t += 3)
+      if (cv[d_mc.tri[c][t]] >= 0 && cv[d_mc.tri[c][t + 1]] >= 0 && cv[d_mc.tri[c][t + 2]] >= 0) cnt++;
     A.tri_cnt[a] = cnt;
   }
 }
@@ -361,27 +564,45 @@ constexpr int kTrisThreads = 256;
 constexpr int kTrisWarps = kTrisThreads / 32;
 constexpr int kMaxCubeTris = 5;  // the most triangles of a case
 
-// Triangles, 32 active cubes per warp: the lanes load their cubes' 12 vertex slots into shared
-// memory, then the warp's triangles (tri_cnt per cube, at tri_off) are spread over the lanes, one
-// per lane, whatever the cubes' cases.  Each writes its triangle with reversed winding (coalesced
-// across the warp) and its area (and, in gradient mode, the area's derivatives with respect to its
-// analytic vertices); each cube's area is the sum of its triangles' in case-table order.
-template <int kMinBlocks>
+// Triangles, 32 active cubes per warp at a time, a ticket of consecutive cubes per block: the block
+// places its triangles (tri_cnt per cube) behind those of the tickets before it; then the lanes
+// load their cubes' 12 vertex slots into shared memory and the warp's triangles are spread over its
+// lanes, one per lane, whatever the cubes' cases.  Each writes its triangle with reversed winding
+// (coalesced across the warp) and its area (and, in gradient mode, the area's derivatives with
+// respect to its analytic vertices); each cube's area is the sum of its triangles' in case-table
+// order.  Bound by the vertex gathers.  Scan of the counts, then triangles -> this: 64
+// conformers 30 + 582 -> 579 us, 20,000 atoms 8 + 145 -> 83 us (most of it the case table, which
+// every block read from the constant bank), 2,000 atoms 5 + 28 -> 22 us.
+template <int kMinBlocks, int kItems>
 __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) {
-  __shared__ int8_t s_tri[256][16];
-  __shared__ uint8_t s_ntri[256];
+  __shared__ unsigned int s_ticket;
+  __shared__ alignas(16) int8_t s_tri[256][16];
+  __shared__ alignas(16) uint8_t s_ntri[256];
   // per warp: each cube's vertex slots ([slot][lane]) and the areas of the warp's triangles
   __shared__ int32_t s_vid[kTrisWarps][12][32];
   __shared__ double s_area[kTrisWarps][kMaxCubeTris * 32];
-  for (int t = threadIdx.x; t < 256 * 16; t += blockDim.x) (&s_tri[0][0])[t] = (&c_tri[0][0])[t];
-  for (int t = threadIdx.x; t < 256; t += blockDim.x) s_ntri[t] = c_ntri[t];
-  __syncthreads();
+  const int64_t n_act = A.counts[kMcActive], n_an = A.counts[kMcAnalytic];
+  if (!cubes_ok(A) || n_an + A.counts[kMcMidpoint] > A.cap_vert) return;
+  const unsigned ticket = take_ticket(A.lb_tris, &s_ticket);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int64_t base = ((int64_t)blockIdx.x * kTrisWarps + w) * 32; base < A.n_active;
-       base += (int64_t)gridDim.x * kTrisThreads) {
-    const int64_t a = base + lane;
-    const bool valid = a < A.n_active;
+  if ((int64_t)ticket * (kTrisThreads * kItems) >= n_act) return;
+  const int64_t a0 = (int64_t)ticket * (kTrisThreads * kItems) + w * (32 * kItems) + lane;
+  // the 4 KB case table: one 16-byte load per thread
+  reinterpret_cast<int4*>(&s_tri[0][0])[threadIdx.x] = reinterpret_cast<const int4*>(&d_mc.tri[0][0])[threadIdx.x];
+  if (threadIdx.x < 16)
+    reinterpret_cast<int4*>(s_ntri)[threadIdx.x] = reinterpret_cast<const int4*>(d_mc.ntri)[threadIdx.x];
+  int sum = 0;
+#pragma unroll
+  for (int x = 0; x < kItems; x++) sum += a0 + 32 * x < n_act ? A.tri_cnt[a0 + 32 * x] : 0;
+  int64_t tbase = warp_offset<kTrisThreads>(A.lb_tris, ticket, warp_total(sum));  // synchronises the block
+  if (tbase < 0) return;
+#pragma unroll 1
+  for (int x = 0; x < kItems; x++) {
+    const int64_t a = a0 + 32 * x;
+    const bool valid = a < n_act;
+    if (!__any_sync(0xffffffffu, valid)) break;
     const int cw = valid ? A.act_rec[a].w : 0;
+    const int cnt = valid ? A.tri_cnt[a] : 0;
     if (valid) {
       const int4* cv = reinterpret_cast<const int4*>(A.cube_vl + 12 * a);
       const int4 v0 = cv[0], v1 = cv[1], v2 = cv[2];
@@ -389,15 +610,9 @@ __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) 
       s_vid[w][4][lane] = v1.x; s_vid[w][5][lane] = v1.y; s_vid[w][6][lane] = v1.z; s_vid[w][7][lane] = v1.w;
       s_vid[w][8][lane] = v2.x; s_vid[w][9][lane] = v2.y; s_vid[w][10][lane] = v2.z; s_vid[w][11][lane] = v2.w;
     }
-    const int cnt = valid ? A.tri_cnt[a] : 0;
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += x;
-    }
+    const int incl = warp_incl(cnt);
     const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int64_t tbase = A.tri_off[base];
+    if (a == n_act - 1) A.counts[kMcTriangle] = tbase + incl;
     __syncwarp();
     for (int t0 = 0; t0 < total; t0 += 32) {
       const int t = t0 + lane;
@@ -431,9 +646,11 @@ __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) 
         }
       }
       const int32_t v0 = lv[32 * e0], v1 = lv[32 * e1], v2 = lv[32 * e2];
-      A.tris[3 * (tbase + t) + 0] = v2;
-      A.tris[3 * (tbase + t) + 1] = v1;
-      A.tris[3 * (tbase + t) + 2] = v0;
+      if (tbase + t < A.cap_tri) {
+        A.tris[3 * (tbase + t) + 0] = v2;
+        A.tris[3 * (tbase + t) + 1] = v1;
+        A.tris[3 * (tbase + t) + 2] = v0;
+      }
       const double* P0 = A.vpos + 3 * (int64_t)v0;
       const double* P1 = A.vpos + 3 * (int64_t)v1;
       const double* P2 = A.vpos + 3 * (int64_t)v2;
@@ -453,7 +670,7 @@ __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) 
         nn[1] *= h;
         nn[2] *= h;
         const auto add = [&](int32_t vv, int ev, double dx, double dy, double dz) {
-          if (vv >= A.n_analytic) return;
+          if (vv >= n_an) return;
           double comp;
           if (ev >= 8) comp = dx * nn[1] - dy * nn[0];        // z
           else if (ev & 1) comp = dz * nn[0] - dx * nn[2];    // y
@@ -472,6 +689,7 @@ __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) 
       A.cube_area[a] = area;
     }
     __syncwarp();
+    tbase += total;
   }
 }
 
@@ -479,12 +697,14 @@ __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) 
 // Consecutive vertices (along a ray, and of neighbouring rays) mostly lie on the same patch, so the
 // per-patch sums go through warp_add_grad.
 __global__ void k_grad_vert(MCArgs A) {
+  const int64_t n_an = A.counts[kMcAnalytic];
+  if (!cubes_ok(A) || n_an + A.counts[kMcMidpoint] > A.cap_vert) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < A.n_analytic; base += stride) {
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n_an; base += stride) {
     const int64_t v = base + (threadIdx.x & 31);
     double g[NS_GRAD_PER_PATCH];
     int32_t pid = -1;
-    const double gv = v < A.n_analytic ? A.vgrad[v] : 0.0;
+    const double gv = v < n_an ? A.vgrad[v] : 0.0;
     if (gv != 0.0) {
       const double x[3] = {A.vpos[3 * v], A.vpos[3 * v + 1], A.vpos[3 * v + 2]};
       const int32_t vp = A.vpid[v];
@@ -554,60 +774,62 @@ int grid_for(int64_t n, int threads) {
 
 }  // namespace
 
-cudaError_t mc_init_tables() {
-  int8_t tri[256][16];
-  uint16_t em[256];
-  uint8_t nt[256];
-  static const int ec[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6}, {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
-  for (int c = 0; c < 256; c++) {
-    int m = 0;
-    for (int e = 0; e < 12; e++)
-      if (((c >> ec[e][0]) & 1) != ((c >> ec[e][1]) & 1)) m |= 1 << e;
-    em[c] = (uint16_t)m;
-    const char* s = kNsMcCases[c];
-    int q = 0;
-    for (; s[q] && q < 16; q++) tri[c][q] = (int8_t)(s[q] <= '9' ? s[q] - '0' : s[q] - 'a' + 10);
-    nt[c] = (uint8_t)(q / 3);
-    for (; q < 16; q++) tri[c][q] = -1;
-  }
-  cudaError_t err = cudaMemcpyToSymbol(c_tri, tri, sizeof tri);
-  if (err == cudaSuccess) err = cudaMemcpyToSymbol(c_ntri, nt, sizeof nt);
-  if (err != cudaSuccess) return err;
-  return cudaMemcpyToSymbol(c_emask, em, sizeof em);
+static unsigned tickets(int64_t items, int most) {
+  const int64_t per = (int64_t)kPassThreads * pass_items(items, most);
+  return (unsigned)((items + per - 1) / per);
 }
 
-cudaError_t launch_vert(const VertArgs& A, int emit, cudaStream_t s) {
+McTickets mc_tickets(int64_t rays, int64_t words, int64_t cubes) {
+  return McTickets{tickets(rays, kVertItems), tickets(words, kRowsItems), tickets(cubes, kMidItems),
+                   tickets(cubes, kTrisItems)};
+}
+
+cudaError_t launch_vert(const VertArgs& A, cudaStream_t s) {
   if (A.nrays == 0) return cudaSuccess;
-  if (emit) k_vert<true><<<grid_for(A.nrays, 256), 256, 0, s>>>(A);
-  else k_vert<false><<<grid_for(A.nrays, 256), 256, 0, s>>>(A);
+  const unsigned b = tickets(A.nrays, kVertItems);
+  if (pass_items(A.nrays, kVertItems) == 4) k_vert<4><<<b, kPassThreads, 0, s>>>(A);
+  else k_vert<1><<<b, kPassThreads, 0, s>>>(A);
   return cudaGetLastError();
 }
 
-cudaError_t launch_mc_rows(const MCArgs& A, int emit, cudaStream_t s) {
-  if (A.nchunks <= 0) return cudaSuccess;
-  if (emit) k_mc_rows<true><<<grid_for(A.nchunks * 32, 256), 256, 0, s>>>(A);
-  else k_mc_rows<false><<<grid_for(A.nchunks * 32, 256), 256, 0, s>>>(A);
+cudaError_t launch_mc_rows(const MCArgs& A, cudaStream_t s) {
+  if (A.nwords_map <= 0) return cudaSuccess;
+  const unsigned b = tickets(A.nwords_map, kRowsItems);
+  const int items = pass_items(A.nwords_map, kRowsItems);
+  if (items == 8) k_mc_rows<8><<<b, kPassThreads, 0, s>>>(A);
+  else if (items == 4) k_mc_rows<4><<<b, kPassThreads, 0, s>>>(A);
+  else k_mc_rows<1><<<b, kPassThreads, 0, s>>>(A);
   return cudaGetLastError();
 }
 
-cudaError_t launch_mc_mid(const MCArgs& A, int emit, cudaStream_t s) {
-  if (A.n_active <= 0) return cudaSuccess;
-  if (emit) k_mc_mid<true><<<grid_for(A.n_active, 256), 256, 0, s>>>(A);
-  else k_mc_mid<false><<<grid_for(A.n_active, 256), 256, 0, s>>>(A);
+cudaError_t launch_mc_clear(const MCArgs& A, int b0, int b1, int64_t cubes, cudaStream_t s) {
+  k_mc_clear<<<grid_for(3 * cubes, 256), 256, 0, s>>>(A, b0, b1);
+  return cudaGetLastError();
+}
+
+// The midpoint and triangle passes take tickets for the capacity; those past the active cubes return
+// at once.
+cudaError_t launch_mc_mid(const MCArgs& A, cudaStream_t s) {
+  const unsigned b = tickets(A.cap_active, kMidItems);
+  if (pass_items(A.cap_active, kMidItems) == 4) k_mc_mid<4><<<b, kPassThreads, 0, s>>>(A);
+  else k_mc_mid<1><<<b, kPassThreads, 0, s>>>(A);
   return cudaGetLastError();
 }
 
 template <int kMinBlocks>
-cudaError_t launch_tris(const MCArgs& A, cudaStream_t s) {
-  int64_t b = (A.n_active + kTrisThreads - 1) / kTrisThreads;
-  const int64_t cap = (int64_t)sm_count() * kMinBlocks * 8;
-  k_mc_tris<kMinBlocks><<<(unsigned)(b < cap ? b : cap), kTrisThreads, 0, s>>>(A);
-  return cudaGetLastError();
+void launch_tris(const MCArgs& A, cudaStream_t s) {
+  const unsigned b = tickets(A.cap_active, kTrisItems);
+  const int items = pass_items(A.cap_active, kTrisItems);
+  if (items == 8) k_mc_tris<kMinBlocks, 8><<<b, kTrisThreads, 0, s>>>(A);
+  else if (items == 4) k_mc_tris<kMinBlocks, 4><<<b, kTrisThreads, 0, s>>>(A);
+  else k_mc_tris<kMinBlocks, 1><<<b, kTrisThreads, 0, s>>>(A);
 }
 
 cudaError_t launch_mc_tris(const MCArgs& A, int blocks_per_sm, cudaStream_t s) {
-  if (A.n_active <= 0) return cudaSuccess;
-  return blocks_per_sm >= 4 ? launch_tris<4>(A, s) : launch_tris<3>(A, s);
+  static_assert(kTrisThreads == kPassThreads, "one ticket count for both passes");
+  if (blocks_per_sm >= 4) launch_tris<4>(A, s);
+  else launch_tris<3>(A, s);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_vertex_normals(const double* vpos, const int32_t* vpid, int64_t n_analytic, const double* f64,
@@ -617,27 +839,19 @@ cudaError_t launch_vertex_normals(const double* vpos, const int32_t* vpid, int64
   return cudaGetLastError();
 }
 
-cudaError_t launch_gather_i64(const int64_t* src, const int64_t* idx, int64_t n, int64_t* dst, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  k_gather_i64<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, idx, n, dst);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_mc_push(const MCArgs& A, int64_t v0, int64_t v1, cudaStream_t s) {
-  if (v1 <= v0) return cudaSuccess;
-  k_mc_push<<<grid_for(v1 - v0, 256), 256, 0, s>>>(A, v0, v1);
+cudaError_t launch_mc_push(const MCArgs& A, int b0, int b1, int64_t vertices, cudaStream_t s) {
+  k_mc_push<<<grid_for(vertices, 256), 256, 0, s>>>(A, b0, b1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_mc_tris_bnd(const MCArgs& A, cudaStream_t s) {
-  if (A.n_active <= 0) return cudaSuccess;
-  k_mc_tris_bnd<<<sm_count() * 4, 256, 0, s>>>(A);
+  k_mc_tris_bnd<<<sm_count(), 256, 0, s>>>(A);
   return cudaGetLastError();
 }
 
-cudaError_t launch_grad_vert(const MCArgs& A, cudaStream_t s) {
-  if (A.n_analytic <= 0 || !A.vgrad) return cudaSuccess;
-  k_grad_vert<<<grid_for(A.n_analytic, 256), 256, 0, s>>>(A);
+cudaError_t launch_grad_vert(const MCArgs& A, int64_t vertices, cudaStream_t s) {
+  if (!A.vgrad) return cudaSuccess;
+  k_grad_vert<<<grid_for(vertices, 256), 256, 0, s>>>(A);
   return cudaGetLastError();
 }
 

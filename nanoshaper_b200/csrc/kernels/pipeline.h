@@ -50,7 +50,6 @@ struct StructDev {
   int64_t tile_base[3];  // first tile of each panel in the panel's tile arrays
   int64_t ray_base[kRaySets];  // first ray of each ray set in the set's ray arrays
   int64_t mc_base;       // first accurate-triangulation ray ordinal (its 3 panels are contiguous)
-  int64_t row_base;      // first marching-cubes row ((NY-2)*(NZ-2) rows per structure)
   int64_t aword_base;    // first entry of its active-cube map (ceil((NX-2)/32) per cube row)
   double A;              // side^2: the area of one pixel, volume weight of an interval length
   double ray_dir[3];     // ray length along each axis: coordinate of the last node minus the first
@@ -64,10 +63,10 @@ struct BatchDev {
   int32_t n;
   const StructDev* s;
   const int32_t* patch_struct;    // structure of every patch
-  const int32_t* tile_struct[3];  // structure of every tile of each panel
+  const int64_t* tile_base[3];    // n+1 per panel
   const int64_t* ray_base[kRaySets];  // n+1 per ray set
   const int64_t* mc_base;         // n+1
-  const int64_t* row_base;        // n+1
+  const int64_t* aword_base;      // n+1: entries of the active-cube map
 };
 
 // Largest b with base[b] <= x (base ascending, base[0] = 0).
@@ -212,15 +211,15 @@ struct TuneParams {
 
 // trace.cu: every launch covers all structures of the batch; `set` is the ray set (0..3) and
 // tile and ray indices are batch-wide.
-cudaError_t launch_windows(const PatchDev& P, int32_t* win, const BatchDev& B, cudaStream_t s);
+// Patch windows; out (4 words, zeroed by the caller) receives the window-area sum of each panel (the
+// bound of its candidate count) and the bit mask of the patch kinds present.
+cudaError_t launch_windows(const PatchDev& P, int32_t* win, const BatchDev& B, unsigned long long* out,
+                           cudaStream_t s);
 // Patch-local FP32 copy of the pool: planes (n, d + n.c), clipping spheres (s - c, r^2); with
 // quad32, the skin cells' quadrics about their local origin (see k_pool32).
 cudaError_t launch_pool32(const PatchDev& P, float4* pool32, float4* quad32, double4* quadl, cudaStream_t s);
-// Bit mask of the patch kinds present (atomicOr into *mask, which the caller zeroes).
-cudaError_t launch_kind_mask(const PatchDev& P, int* mask, cudaStream_t s);
-// tile_cnt null: only the window-area sum (the candidate bound of the panel).
-cudaError_t launch_bin_count(const PatchDev& P, const BatchDev& B, int set, int32_t* tile_cnt,
-                             unsigned long long* area, cudaStream_t s);
+// Patch counts of a panel's ray tiles (overflow path).
+cudaError_t launch_bin_count(const PatchDev& P, const BatchDev& B, int set, int32_t* tile_cnt, cudaStream_t s);
 cudaError_t launch_bin_fill(const PatchDev& P, const BatchDev& B, int set, const int64_t* tile_off,
                             int32_t* tile_cursor, int32_t* tile_list, cudaStream_t s);
 // ev (optional, profiling): 4 events recorded before the candidate kernel and after the candidate,
@@ -233,12 +232,20 @@ cudaError_t launch_trace_overflow(const PatchDev& P, const BatchDev& B, int set,
                                   const int32_t* tile_list, const TraceOut& out, int n_ovf, double* scratch,
                                   int32_t* pscratch, int precision, cudaStream_t s);
 
-// reduce.cu: out[b] (+)= sum of v over structure b's segment [base[i(b)], base[i(b+1)]) with
-// i(b) = idx[b] (idx given) or b, in a summation order fixed by the segment alone; part is scratch
-// for n * kSegParts doubles.
+// reduce.cu: out[b] = sum, over the arrays in order, of array q's segment [base[q][b],
+// base[q][b+1]) below index `limit`, each in a summation order fixed by the segment alone; part is scratch for
+// arrays * n * kSegParts doubles.
 constexpr int kSegParts = 64;
-cudaError_t launch_segment_sums(const double* v, const int64_t* base, const int64_t* idx, int n, double* out,
-                                double* part, bool accumulate, cudaStream_t s);
+constexpr int kMaxSegArrays = kRaySets;
+struct SegArrays {
+  const double* v[kMaxSegArrays];
+  const int64_t* base[kMaxSegArrays];
+};
+cudaError_t launch_segment_sums(const SegArrays& S, int arrays, int n, int64_t limit, double* out, double* part,
+                                cudaStream_t s);
+
+// reduce.cu: out[n] = the total of n counts, from their exclusive offsets out[0..n-1].
+cudaError_t launch_scan_total(const int32_t* in, int64_t n, int64_t* out, cudaStream_t s);
 
 // reduce.cu, batch uploads: per-patch structure and batch-wide pool index (err set on a pool
 // range outside the structure's pool); batch-wide patch atom indices (err on an index outside

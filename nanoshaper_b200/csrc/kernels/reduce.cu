@@ -11,14 +11,14 @@ namespace {
 
 constexpr int kSumThreads = 256;
 
-// part[b * kSegParts + k] = sum over the elements of segment b whose index i within the segment
-// has (i / kSumThreads) % kSegParts == k; lo = base[idx ? idx[b] : b], hi = base[idx ? idx[b+1] : b+1].
-__global__ void __launch_bounds__(kSumThreads) k_segment_parts(const double* __restrict__ v,
-                                                                const int64_t* __restrict__ base,
-                                                                const int64_t* __restrict__ idx, double* part) {
+// part[(q * n + b) * kSegParts + k] = sum over the elements of segment b of array q whose index i
+// within the segment has (i / kSumThreads) % kSegParts == k.
+__global__ void __launch_bounds__(kSumThreads) k_segment_parts(SegArrays S, int n, int64_t limit,
+                                                                double* part) {
   __shared__ double red[kSumThreads];
-  const int b = blockIdx.x / kSegParts, k = blockIdx.x % kSegParts;
-  const int64_t lo = base[idx ? idx[b] : b], hi = base[idx ? idx[b + 1] : b + 1];
+  const int k = blockIdx.x % kSegParts, b = (blockIdx.x / kSegParts) % n, q = blockIdx.x / (kSegParts * n);
+  const double* __restrict__ v = S.v[q];
+  const int64_t lo = S.base[q][b], end = S.base[q][b + 1], hi = end < limit ? end : limit;
   double s = 0.0;
   for (int64_t i = lo + (int64_t)k * kSumThreads + threadIdx.x; i < hi; i += (int64_t)kSegParts * kSumThreads)
     s += v[i];
@@ -31,22 +31,36 @@ __global__ void __launch_bounds__(kSumThreads) k_segment_parts(const double* __r
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// out[b] (+)= the partial sums of segment b in CTA order.
-__global__ void k_segment_total(const double* __restrict__ part, int n, double* out, int accumulate) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  double s = 0.0;
-  for (int k = 0; k < kSegParts; k++) s += part[(int64_t)b * kSegParts + k];
-  out[b] = accumulate ? out[b] + s : s;
+// out[b] = the arrays' sums of segment b in array order, each the partial sums in CTA order: one CTA
+// per segment loads the partial sums, a thread per array adds them up.
+__global__ void __launch_bounds__(kSegParts) k_segment_total(const double* __restrict__ part, int n, int arrays,
+                                                             double* out) {
+  __shared__ double s_part[kMaxSegArrays][kSegParts + 1];
+  __shared__ double s_sum[kMaxSegArrays];
+  const int b = blockIdx.x;
+  for (int q = 0; q < arrays; q++)
+    s_part[q][threadIdx.x] = part[((int64_t)q * n + b) * kSegParts + threadIdx.x];
+  __syncthreads();
+  if ((int)threadIdx.x < arrays) {
+    double s = 0.0;
+    for (int k = 0; k < kSegParts; k++) s += s_part[threadIdx.x][k];
+    s_sum[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = s_sum[0];
+    for (int q = 1; q < arrays; q++) s = s + s_sum[q];
+    out[b] = s;
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_segment_sums(const double* v, const int64_t* base, const int64_t* idx, int n, double* out,
-                                double* part, bool accumulate, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  k_segment_parts<<<(unsigned)(n * kSegParts), kSumThreads, 0, s>>>(v, base, idx, part);
-  k_segment_total<<<(n + 127) / 128, 128, 0, s>>>(part, n, out, accumulate ? 1 : 0);
+cudaError_t launch_segment_sums(const SegArrays& S, int arrays, int n, int64_t limit, double* out, double* part,
+                                cudaStream_t s) {
+  if (n <= 0 || arrays <= 0) return cudaSuccess;
+  k_segment_parts<<<(unsigned)(arrays * n * kSegParts), kSumThreads, 0, s>>>(S, n, limit, part);
+  k_segment_total<<<(unsigned)n, kSegParts, 0, s>>>(part, n, arrays, out);
   return cudaGetLastError();
 }
 
@@ -55,6 +69,11 @@ cudaError_t launch_segment_sums(const double* v, const int64_t* base, const int6
 namespace nsg {
 
 namespace {
+
+template <class In>
+__global__ void k_scan_total(const In* __restrict__ in, int64_t n, int64_t* out) {
+  out[n] = n > 0 ? out[n - 1] + (int64_t)in[n - 1] : 0;
+}
 
 // Batch upload fix-ups, one thread per patch: the structure of the patch (binary search in the
 // patch offsets), its pool index made batch-wide, and the range checked against its structure's
@@ -92,6 +111,11 @@ int grid_of(int64_t n) {
 }
 
 }  // namespace
+
+cudaError_t launch_scan_total(const int32_t* in, int64_t n, int64_t* out, cudaStream_t s) {
+  k_scan_total<<<1, 1, 0, s>>>(in, n, out);
+  return cudaGetLastError();
+}
 
 int sm_count() {
   static int cache[64] = {0};

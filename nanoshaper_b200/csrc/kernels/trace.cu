@@ -11,13 +11,12 @@
 // writes the status rows / insideness bits of its 32 rays cooperatively (coalesced rows, ballot
 // masks + atomicAnd on the 32x-packed bit grid).  The candidate set of a ray is the reference's:
 // pixel inside the patch window, inside the bounding box, inside the equatorial disc.
-#include <cub/cub.cuh>
-
 #include "pipeline.h"
 #include "ray_math.cuh"
 #include "ray_math_mixed.cuh"
 #include "grad.cuh"
 #include "isect.cuh"
+#include "lookback.cuh"
 
 namespace nsg {
 
@@ -25,36 +24,58 @@ namespace {
 
 
 
-__global__ void k_windows(PatchDev P, int32_t* win, BatchDev B) {
-  int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  const GridDev& g = B.s[B.patch_struct[p]].g;
-  const double* f = P.f64 + (int64_t)NS_PATCH_F64 * p;
-  double r = f[3];
-  double down[3], up[3];
-  bool cull = false;
-  const bool skin = ns_has_box(P.i32[NS_PATCH_I32 * p]);
-  for (int d = 0; d < 3; d++) {
-    // SES: the bounding sphere's box; skin cells and mesh triangles: their stored box
-    // (src/SkinSurface.cpp:3470-3500, src/MeshSurface.cpp:447-472)
-    down[d] = skin ? f[NS_SKIN_LO + d] : f[d] - r;
-    up[d] = skin ? f[NS_SKIN_HI + d] : f[d] + r;
-    if (down[d] > g.mx[d] + NS_EPS_INT) cull = true;
+// Pixel window of every patch (start, end per axis; -1 when culled), with the panels' window-area
+// sums (out[0..2]) and the patch kinds present (out[3]) of the same pass.
+__global__ void k_windows(PatchDev P, int32_t* win, BatchDev B, unsigned long long* out) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  unsigned kind_bit = 0, size[3] = {0, 0, 0};
+  if (p < P.n) {
+    const GridDev& g = B.s[B.patch_struct[p]].g;
+    const double* f = P.f64 + (int64_t)NS_PATCH_F64 * p;
+    const double r = f[3];
+    double down[3], up[3];
+    bool cull = false;
+    const int kind = P.i32[NS_PATCH_I32 * p];
+    kind_bit = 1u << kind;
+    const bool skin = ns_has_box(kind);
+    for (int d = 0; d < 3; d++) {
+      // SES: the bounding sphere's box; skin cells and mesh triangles: their stored box
+      // (src/SkinSurface.cpp:3470-3500, src/MeshSurface.cpp:447-472)
+      down[d] = skin ? f[NS_SKIN_LO + d] : f[d] - r;
+      up[d] = skin ? f[NS_SKIN_HI + d] : f[d] + r;
+      if (down[d] > g.mx[d] + NS_EPS_INT) cull = true;
+    }
+    for (int d = 0; d < 3; d++)
+      if (up[d] < g.mn[d] - (g.hside - NS_DELTA + NS_EPS_INT)) cull = true;
+    int32_t* w = win + 6 * p;
+    for (int d = 0; d < 3; d++) {
+      int64_t s = -1, e = -1;
+      if (!cull) {
+        s = (int64_t)rintp(fmax(0., down[d] - g.mn[d]) * g.scale);
+        e = (int64_t)rintp(fmax(0., up[d] - g.mn[d]) * g.scale);
+        if (e >= g.n[d]) e = g.n[d] - 1;
+        if (e >= s) size[d] = (unsigned)(e - s + 1);
+      }
+      w[d] = (int32_t)s;
+      w[3 + d] = (int32_t)e;
+    }
   }
-  for (int d = 0; d < 3; d++)
-    if (up[d] < g.mn[d] - (g.hside - NS_DELTA + NS_EPS_INT)) cull = true;
-  int32_t* w = win + 6 * p;
-  if (cull) {
-    for (int d = 0; d < 6; d++) w[d] = -1;
-    return;
+  // panel areas (y z, x y, x z); a window's area is below 2^31, and so is a warp's sum unless a
+  // window is exceptionally large
+  const int lane = threadIdx.x & 31;
+  const unsigned area[3] = {size[1] * size[2], size[0] * size[1], size[0] * size[2]};
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    if (__any_sync(0xffffffffu, area[q] >> 26)) {
+      if (area[q]) atomicAdd(out + q, (unsigned long long)area[q]);
+    } else {
+      const unsigned sum = __reduce_add_sync(0xffffffffu, area[q]);
+      if (lane == 0 && sum) atomicAdd(out + q, (unsigned long long)sum);
+    }
   }
-  for (int d = 0; d < 3; d++) {
-    int64_t s = (int64_t)rintp(fmax(0., down[d] - g.mn[d]) * g.scale);
-    int64_t e = (int64_t)rintp(fmax(0., up[d] - g.mn[d]) * g.scale);
-    if (e >= g.n[d]) e = g.n[d] - 1;
-    w[d] = (int32_t)s;
-    w[3 + d] = (int32_t)e;
-  }
+  kind_bit = __reduce_or_sync(0xffffffffu, kind_bit);
+  if (lane == 0 && kind_bit && (~*(volatile unsigned long long*)(out + 3) & kind_bit))
+    atomicOr(out + 3, (unsigned long long)kind_bit);
 }
 
 __global__ void k_pool32(PatchDev P, float4* out, float4* quad32, double4* quadl) {
@@ -91,28 +112,14 @@ __global__ void k_pool32(PatchDev P, float4* out, float4* quad32, double4* quadl
   }
 }
 
-__global__ void k_kind_mask(PatchDev P, int* mask) {
-  int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int bit = p < P.n ? (1 << P.i32[NS_PATCH_I32 * p]) : 0;
-  bit = __reduce_or_sync(0xffffffffu, bit);
-  if ((threadIdx.x & 31) == 0 && bit) atomicOr(mask, bit);
-}
-
 __global__ void k_bin(PatchDev P, BatchDev B, int set, int32_t* tile_cnt, const int64_t* tile_off,
-                      int32_t* tile_cursor, int32_t* tile_list, unsigned long long* area) {
+                      int32_t* tile_cursor, int32_t* tile_list) {
   int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int32_t* w = P.win + 6 * (p < P.n ? p : 0);
-  bool live = p < P.n && w[0] >= 0;
-  const StructDev& S = B.s[p < P.n ? B.patch_struct[p] : 0];
+  if (p >= P.n) return;
+  const int32_t* w = P.win + 6 * p;
+  if (w[0] < 0) return;
+  const StructDev& S = B.s[B.patch_struct[p]];
   const RaySet rs = make_ray_set(set, S.g);
-  if (area) {
-    // pixel-window area: an upper bound of the patch's candidate rays in this panel
-    const int ww = w[3 + rs.fd] - w[rs.fd] + 1, wh = w[3 + rs.ld] - w[rs.ld] + 1;
-    unsigned a = (live && ww > 0 && wh > 0) ? (unsigned)(ww * wh) : 0u;
-    unsigned sum = __reduce_add_sync(0xffffffffu, a);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(area, (unsigned long long)sum);
-  }
-  if (!live || (tile_cnt == nullptr && tile_list == nullptr)) return;
   int64_t ntm = (rs.nb + kTileM - 1) / kTileM;
   int m0 = w[rs.fd] / kTileM, m1 = w[3 + rs.fd] / kTileM;
   int n0 = w[rs.ld] / kTileN, n1 = w[3 + rs.ld] / kTileN;
@@ -416,17 +423,6 @@ __device__ __forceinline__ int cand_row(const CandBatch& q, int p, int row, int*
   return hi - lo;
 }
 
-// Smallest lane whose inclusive prefix v exceeds k (k below the warp total).
-__device__ __forceinline__ int owner_lane(int v, int k) {
-  int rr = 0;
-#pragma unroll
-  for (int step = 16; step; step >>= 1) {
-    const int x = __shfl_sync(0xffffffffu, v, rr + step - 1);
-    if (x <= k) rr += step;
-  }
-  return rr;
-}
-
 // Rows of a batch whose interval stays in shared memory between the counting and the writing pass
 // (first pixel relative to the window and count, 16 bits each); the others are found again.
 constexpr int kCandRows = 320;
@@ -727,7 +723,7 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
   constexpr int kThreads = kTraceThreads;
   const int panel = ray_set_panel(C.set);
   const int64_t tile = blockIdx.x;
-  const StructDev& S = C.B.s[C.B.tile_struct[panel][tile]];
+  const StructDev& S = C.B.s[find_struct(C.B.tile_base[panel], C.B.n, tile)];
   const GridDev g = S.g;
   const RaySet rs = make_ray_set(C.set, g);
   uint32_t* const bits = C.out.bits + S.word_base;
@@ -1147,9 +1143,10 @@ __global__ void k_trace_overflow(TraceCtx C, const int64_t* __restrict__ tile_of
 
 }  // namespace
 
-cudaError_t launch_windows(const PatchDev& P, int32_t* win, const BatchDev& B, cudaStream_t s) {
+cudaError_t launch_windows(const PatchDev& P, int32_t* win, const BatchDev& B, unsigned long long* out,
+                           cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  k_windows<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, win, B);
+  k_windows<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, win, B, out);
   return cudaGetLastError();
 }
 
@@ -1159,23 +1156,16 @@ cudaError_t launch_pool32(const PatchDev& P, float4* pool32, float4* quad32, dou
   return cudaGetLastError();
 }
 
-cudaError_t launch_kind_mask(const PatchDev& P, int* mask, cudaStream_t s) {
+cudaError_t launch_bin_count(const PatchDev& P, const BatchDev& B, int set, int32_t* tile_cnt, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  k_kind_mask<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, mask);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_bin_count(const PatchDev& P, const BatchDev& B, int set, int32_t* tile_cnt,
-                             unsigned long long* area, cudaStream_t s) {
-  if (P.n == 0) return cudaSuccess;
-  k_bin<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, B, set, tile_cnt, nullptr, nullptr, nullptr, area);
+  k_bin<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, B, set, tile_cnt, nullptr, nullptr, nullptr);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bin_fill(const PatchDev& P, const BatchDev& B, int set, const int64_t* tile_off,
                             int32_t* tile_cursor, int32_t* tile_list, cudaStream_t s) {
   if (P.n == 0) return cudaSuccess;
-  k_bin<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, B, set, nullptr, tile_off, tile_cursor, tile_list, nullptr);
+  k_bin<<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(P, B, set, nullptr, tile_off, tile_cursor, tile_list);
   return cudaGetLastError();
 }
 
