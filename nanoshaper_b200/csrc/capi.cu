@@ -264,7 +264,7 @@ struct nsg_ctx {
   int64_t cand_cap = 0, def_cap = 0;
   // trace outputs
   DevBuf status, bits, vol_ray[nsg::kRaySets], epsmap;
-  DevBuf pairs, ray_pair_off, ray_pair_cnt, cursors, ovf_rays[nsg::kRaySets], ovf_scratch, err;
+  DevBuf pairs, ray_pair_off, ray_pair_cnt, cursors, ovf_rays[nsg::kRaySets], ovf_scratch;
   DevBuf hits, ray_hit_off[nsg::kRaySets], ray_hit_cnt[nsg::kRaySets];
   int64_t pair_cap = 0, hit_cap = 0, n_pairs = 0;
   int flags = 0;
@@ -300,7 +300,7 @@ struct nsg_ctx {
   bool shape_filtered = false;
   bool ideb_ready = false;                     // ideb holds the map (after a shape filter)
   std::vector<int32_t> cav_atom_off, cav_atom_list;
-  DevBuf ca_atoms, ca_cell_off, ca_cell_atoms, ca_pairs, ca_alt, ca_count;
+  DevBuf ca_atoms, ca_pairs, ca_alt, ca_count;
   // mesh
   DevBuf amap, cube_vl, vstruct, mc_block;
   // capacities of a triangulation per vertex of the cast's pairs, raised when one did not suffice
@@ -625,9 +625,9 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield, &c->b_gatoms, &c->counters, &c->win_sums,
                     &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_node, &c->bgp_ibgp, &c->bgp_type,
                     &c->bgp_pos, &c->bgp_nor, &c->bgp_flag, &c->bgp_n, &c->aux_cnt, &c->aux_off, &c->aux_list, &c->pairs,
-                    &c->ray_pair_off, &c->ray_pair_cnt, &c->cursors, &c->ovf_scratch, &c->err, &c->hits,
+                    &c->ray_pair_off, &c->ray_pair_cnt, &c->cursors, &c->ovf_scratch, &c->hits,
                     &c->pair_pid, &c->ovf_pscratch, &c->gvol, &c->garea, &c->vpid, &c->vgrad,
-                    &c->d_atoms, &c->d_patch_atoms, &c->d_gatoms_vol, &c->d_gatoms_area, &c->d_bad, &c->amap, &c->cube_vl, &c->vstruct, &c->mc_block, &c->ca_atoms, &c->ca_cell_off, &c->ca_cell_atoms, &c->ca_pairs, &c->ca_alt, &c->ca_count,
+                    &c->d_atoms, &c->d_patch_atoms, &c->d_gatoms_vol, &c->d_gatoms_area, &c->d_bad, &c->amap, &c->cube_vl, &c->vstruct, &c->mc_block, &c->ca_atoms, &c->ca_pairs, &c->ca_alt, &c->ca_count,
                     &c->d_patch_off, &c->d_pool_off, &c->d_atom_off,
                     &c->labels, &c->is_root, &c->sruns, &c->srun_off, &c->srun_cnt, &c->fr_cnt, &c->fr_off,
                     &c->fruns, &c->frow, &c->roots, &c->cc_block, &c->cc_label_of,
@@ -2008,10 +2008,6 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
     return fail(NSG_ERR_STATE, "cavity atoms need nsg_cavities after the cast");
   if (!c->have_cav_atoms) {
     CK(cudaSetDevice(c->device));
-    {
-      int rc = ensure_dense_status(c);
-      if (rc) return rc;
-    }
     const NsGrid& g = c->grid;
     c->cav_atom_off.assign(c->ncav + 1, 0);
     c->cav_atom_list.clear();
@@ -2037,7 +2033,16 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
       const int64_t gn = ggrid, ncell = gn * gn * gn;
       double gmn[3];
       for (int d = 0; d < 3; d++) gmn[d] = g.baricenter[d] - (ggrid - 1) * 0.5 * gside;
-      std::vector<int32_t> cell_of(n_atoms), cell_off(ncell + 1, 0), cell_atoms(n_atoms);
+      // atoms, cell offsets and cell atoms, filled in one pinned block and sent in one copy
+      const size_t atom_bytes = (size_t)n_atoms * 4 * sizeof(double);
+      const size_t in_bytes = atom_bytes + ((size_t)ncell + 1 + n_atoms) * sizeof(int32_t);
+      CK(cudaStreamSynchronize(c->stream));
+      CK(c->h_layout.ensure(in_bytes));
+      memcpy(c->h_layout.p, atoms_xyzr, atom_bytes);
+      int32_t* cell_off = (int32_t*)(c->h_layout.as<char>() + atom_bytes);
+      int32_t* cell_atoms = cell_off + ncell + 1;
+      std::fill(cell_off, cell_off + ncell + 1, 0);
+      std::vector<int32_t> cell_of(n_atoms);
       for (int64_t a = 0; a < n_atoms; a++) {
         int64_t ix[3];
         for (int d = 0; d < 3; d++) ix[d] = (int64_t)floor((atoms_xyzr[4 * a + d] - gmn[d]) * gscale + 0.5);
@@ -2047,30 +2052,27 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
         cell_off[cell_of[a] + 1]++;
       }
       for (int64_t q = 0; q < ncell; q++) cell_off[q + 1] += cell_off[q];
-      {
-        std::vector<int32_t> cur(cell_off.begin(), cell_off.end() - 1);
-        for (int64_t a = 0; a < n_atoms; a++) cell_atoms[cur[cell_of[a]]++] = (int32_t)a;
-      }
+      // the offsets move up by one atom as the cells are filled, and back by one cell afterwards
+      for (int64_t a = 0; a < n_atoms; a++) cell_atoms[cell_off[cell_of[a]]++] = (int32_t)a;
+      for (int64_t q = ncell; q > 0; q--) cell_off[q] = cell_off[q - 1];
+      cell_off[0] = 0;
       const int64_t cap = c->cav_nodes;
-      CK(c->ca_atoms.ensure(std::max<int64_t>(n_atoms, 1) * 4 * sizeof(double)));
-      CK(c->ca_cell_off.ensure((ncell + 1) * sizeof(int32_t)));
-      CK(c->ca_cell_atoms.ensure(std::max<int64_t>(n_atoms, 1) * sizeof(int32_t)));
+      CK(c->ca_atoms.ensure(in_bytes));
       CK(c->ca_pairs.ensure(cap * sizeof(unsigned long long)));
       CK(c->ca_alt.ensure(cap * sizeof(unsigned long long)));
       CK(c->ca_count.ensure(2 * sizeof(unsigned long long)));
-      if (n_atoms)
-        CK(cudaMemcpyAsync(c->ca_atoms.p, atoms_xyzr, n_atoms * 4 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-      CK(cudaMemcpyAsync(c->ca_cell_off.p, cell_off.data(), (ncell + 1) * sizeof(int32_t), cudaMemcpyHostToDevice,
-                         c->stream));
-      if (n_atoms)
-        CK(cudaMemcpyAsync(c->ca_cell_atoms.p, cell_atoms.data(), n_atoms * sizeof(int32_t), cudaMemcpyHostToDevice,
-                           c->stream));
+      CK(cudaMemcpyAsync(c->ca_atoms.p, c->h_layout.p, in_bytes, cudaMemcpyHostToDevice, c->stream));
+      // pair count and error flag, read together
       CK(cudaMemsetAsync(c->ca_count.p, 0, 2 * sizeof(unsigned long long), c->stream));
-      CK(c->err.ensure(sizeof(int32_t)));
-      CK(cudaMemsetAsync(c->err.p, 0, sizeof(int32_t), c->stream));
+      int atom_bits = 1, cav_bits = 1;
+      while (((int64_t)1 << atom_bits) <= n_atoms) atom_bits++;
+      while (((int64_t)1 << cav_bits) < c->ncav) cav_bits++;
       nsg::CavAtomArgs A{};
-      A.status = c->status.as<int32_t>();
-      A.label = c->shape_filtered ? c->cav_label.as<int32_t>() : nullptr;
+      if (c->shape_filtered) {
+        A.status = c->status.as<int32_t>();
+        A.label = c->cav_label.as<int32_t>();
+      }
+      A.atom_bits = atom_bits;
       A.nx = g.nx;
       A.ny = g.ny;
       A.nz = g.nz;
@@ -2081,45 +2083,53 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
       A.gn = gn;
       for (int d = 0; d < 3; d++) A.gmn[d] = gmn[d];
       A.gscale = gscale;
-      A.cell_off = c->ca_cell_off.as<int32_t>();
-      A.cell_atoms = c->ca_cell_atoms.as<int32_t>();
       A.atoms = c->ca_atoms.as<double>();
+      A.cell_off = (const int32_t*)(c->ca_atoms.as<char>() + atom_bytes);
+      A.cell_atoms = A.cell_off + ncell + 1;
       A.pairs = c->ca_pairs.as<unsigned long long>();
       A.count = c->ca_count.as<unsigned long long>();
       A.cap = cap;
-      A.err = c->err.as<int32_t>();
-      LAUNCH(nsg::cavity_atom_pairs(A, c->stream));
-      unsigned long long npairs = 0;
-      int32_t errflag = 0;
-      CK(cudaMemcpyAsync(&npairs, c->ca_count.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-      CK(cudaMemcpyAsync(&errflag, c->err.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+      A.err = (int32_t*)(A.count + 1);
+      LAUNCH(nsg::cavity_nodes(run_args(c), c->cc_label_of.as<int32_t>(), A, c->stream));
+      LAUNCH(nsg::cavity_nearest(A, c->stream));
+      // the count of unique keys and the first keys come back in one read
+      constexpr int64_t kFirstKeys = 8191;
+      CK(c->h_read.ensure((1 + kFirstKeys) * sizeof(unsigned long long)));
+      unsigned long long* read = c->h_read.as<unsigned long long>();
+      CK(cudaMemcpyAsync(read, A.count, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
-      if (errflag) return fail(NSG_ERR_CAPACITY, "cavity boundary nodes exceed the cavity node count");
+      const int64_t npairs = (int64_t)read[0];
+      if ((int32_t)read[1]) return fail(NSG_ERR_CAPACITY, "cavity boundary nodes exceed the cavity node count");
       int64_t nu = 0;
+      std::vector<unsigned long long> more;
+      const unsigned long long* keys = read + 1;
       if (npairs > 0) {
         size_t tb = 0;
-        int64_t* d_nu = reinterpret_cast<int64_t*>(c->ca_count.as<unsigned long long>() + 1);
-        CK(nsg::sort_unique_u64(A.pairs, c->ca_alt.as<unsigned long long>(), (int64_t)npairs, d_nu, nullptr, &tb,
-                                c->stream));
+        int64_t* d_nu = (int64_t*)A.count;
+        const int bits = atom_bits + cav_bits;
+        CK(nsg::sort_unique_u64(A.pairs, c->ca_alt.as<unsigned long long>(), npairs, bits, d_nu, nullptr, &tb, c->stream));
         CK(c->temp.ensure(tb));
         tb = c->temp.cap;
         c->launches += 2;
-        CK(nsg::sort_unique_u64(A.pairs, c->ca_alt.as<unsigned long long>(), (int64_t)npairs, d_nu, c->temp.p, &tb,
+        CK(nsg::sort_unique_u64(A.pairs, c->ca_alt.as<unsigned long long>(), npairs, bits, d_nu, c->temp.p, &tb,
                                 c->stream));
-        CK(cudaMemcpyAsync(&nu, d_nu, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(read, d_nu, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(read + 1, A.pairs, std::min(npairs, kFirstKeys) * sizeof(unsigned long long),
+                           cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
-      }
-      std::vector<unsigned long long> keys(nu);
-      if (nu) {
-        CK(cudaMemcpyAsync(keys.data(), c->ca_pairs.p, nu * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                           c->stream));
-        CK(cudaStreamSynchronize(c->stream));
+        nu = (int64_t)read[0];
+        if (nu > kFirstKeys) {
+          more.resize(nu);
+          CK(cudaMemcpyAsync(more.data(), A.pairs, nu * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+          CK(cudaStreamSynchronize(c->stream));
+          keys = more.data();
+        }
       }
       c->cav_atom_list.resize(nu);
       for (int64_t q = 0; q < nu; q++) {
-        const int64_t cav = (int64_t)(keys[q] >> 32);
+        const int64_t cav = (int64_t)(keys[q] >> atom_bits);
         if (cav < 0 || cav >= c->ncav) return fail(NSG_ERR_STATE, "cavity index out of range");
-        c->cav_atom_list[q] = (int32_t)(uint32_t)(keys[q] & 0xffffffffu) - 1;
+        c->cav_atom_list[q] = (int32_t)(keys[q] & (((unsigned long long)1 << atom_bits) - 1)) - 1;
         c->cav_atom_off[cav + 1]++;
       }
       for (int q = 0; q < c->ncav; q++) c->cav_atom_off[q + 1] += c->cav_atom_off[q];

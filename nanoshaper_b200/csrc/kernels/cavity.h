@@ -38,13 +38,13 @@ cudaError_t run_fill(const RunArgs& A, const uint8_t* fill_of, uint32_t* bits, i
 // Dense status map from the runs; label_of == nullptr writes TEMPORARY_OUT for free nodes.
 cudaError_t status_write(const RunArgs& A, const int32_t* label_of, int32_t* status, cudaStream_t s);
 
-// Atoms lining the cavities (getCavitiesAtomsWithBilevelStatusMap, src/Surface.cpp:2249-2346), on
-// the dense status map after cavity detection and the reference's atom grid (buildAtomsMap,
+// Atoms lining the cavities (getCavitiesAtomsWithBilevelStatusMap, src/Surface.cpp:2249-2346), after
+// cavity detection, with the reference's atom grid (buildAtomsMap,
 // src/Surface.cpp:1695-1749): gn^3 cells of side 1/gscale from gmn, cell (x, y, z) at
 // (z*gn + y)*gn + x, its atoms in ascending index order at cell_off.
 struct CavAtomArgs {
-  const int32_t* status;
-  const int32_t* label;       // cavity membership (the labels before a shape filter); nullptr: status
+  const int32_t* status;      // filtered map and the labels before the filter; null without a filter
+  const int32_t* label;
   int64_t nx, ny, nz;
   double mn[3], side;
   int64_t gn;
@@ -52,16 +52,20 @@ struct CavAtomArgs {
   const int32_t* cell_off;    // gn^3 + 1
   const int32_t* cell_atoms;
   const double* atoms;        // x, y, z, r per atom
-  unsigned long long* pairs;  // (cavity << 32) | (atom + 1), one per cavity boundary node
+  unsigned long long* pairs;  // one per cavity boundary node: (cavity << 32) | node, then
+                              // (cavity << atom_bits) | (atom + 1)
+  int atom_bits;
   unsigned long long* count;
   int64_t cap;
   int32_t* err;               // set to 1 when the pairs overflow cap
 };
 // One pair per node of cavity c (status FIRST_CAV + c) that has a 6-neighbour of another status
-// (TEMPORARY_OUT outside the grid): c and the atom of least |a - x|^2 - r^2 over the 27 cells
-// around the node, in the reference's cell order, the first of equal ones; atom -1 when the cells
-// hold no atom.
-cudaError_t cavity_atom_pairs(const CavAtomArgs& A, cudaStream_t s);
+// (TEMPORARY_OUT outside the grid), from the labelled free runs, or from the dense map after a shape
+// filter (A.label set).
+cudaError_t cavity_nodes(const RunArgs& R, const int32_t* label_of, const CavAtomArgs& A, cudaStream_t s);
+// The pairs' nodes become atoms: the atom of least |a - x|^2 - r^2 over the 27 cells around the
+// node, in the reference's cell order, the first of equal ones; atom -1 when the cells hold no atom.
+cudaError_t cavity_nearest(const CavAtomArgs& A, cudaStream_t s);
 
 // Water-shape filter of the cavities that filling kept (filterCavitiesWithBilevelStatusMap,
 // src/Surface.cpp:3011-3290), on the dense status map after cavity detection.  A node of cavity c
@@ -105,8 +109,9 @@ cudaError_t pocket_cav2out(int32_t* status, const int32_t* label, int64_t n, cud
 // Free runs (TEMPORARY_OUT runs per x-row) of a dense status map; count pass then emit pass.
 cudaError_t dense_free_runs(const RunArgs& A, const int32_t* status, int emit, cudaStream_t s);
 
-// Sorts the n pairs and keeps one of each; pass temp == nullptr to query temp_bytes.
-cudaError_t sort_unique_u64(unsigned long long* keys, unsigned long long* keys_alt, int64_t n, int64_t* n_unique,
-                            void* temp, size_t* temp_bytes, cudaStream_t s);
+// Sorts the n keys by their low `bits` bits and keeps one of each; pass temp == nullptr to query
+// temp_bytes.
+cudaError_t sort_unique_u64(unsigned long long* keys, unsigned long long* keys_alt, int64_t n, int bits,
+                            int64_t* n_unique, void* temp, size_t* temp_bytes, cudaStream_t s);
 
 }  // namespace nsg
