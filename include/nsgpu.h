@@ -155,6 +155,10 @@ int nsg_version(void);
 const char* nsg_last_error(void);
 int nsg_ctx_create(int device, nsg_ctx** out);
 int nsg_ctx_destroy(nsg_ctx* ctx);
+/* Memory, pinned host blocks and streams of destroyed contexts serve the next ones: per device at most
+ * 4 GiB of device memory, in the process at most 32 MiB of pinned blocks, 64 streams, and 16 MiB of
+ * pinned blocks of the copy threads.  This call gives back what no context uses. */
+int nsg_release_kept(void);
 int nsg_set_stream(nsg_ctx* ctx, void* cuda_stream);
 void* nsg_get_stream(nsg_ctx* ctx);
 /* Grid of the surface (the DelPhiShared* the reference Surface holds, src/Surface.h:572). */
@@ -180,6 +184,11 @@ int nsg_set_batch(nsg_ctx* ctx, int32_t n, const NsGrid* grids);
  * structure (as nsg_patchset_export writes them). */
 int nsg_upload_batch(nsg_ctx* ctx, const int64_t* patch_off, const double* f64, const int32_t* i32,
                      const int64_t* pool_off, const double* pool, const int8_t* pool_flag, double probe_radius);
+/* The same from one array per structure (arrays of n pointers, entries of empty structures unused),
+ * for callers that hold the sets one by one. */
+int nsg_upload_batch_list(nsg_ctx* ctx, const int64_t* patch_off, const double* const* f64, const int32_t* const* i32,
+                          const int64_t* pool_off, const double* const* pool, const int8_t* const* pool_flag,
+                          double probe);
 /* Per-structure volume (last nsg_raycast) and area (last nsg_triangulate); either may be NULL. */
 int nsg_batch_results(nsg_ctx* ctx, double* volumes, double* areas);
 
@@ -206,6 +215,9 @@ int nsg_patch_grads(nsg_ctx* ctx, double* d_volume, double* d_area);
 /* The atoms behind the uploaded patches (after jitter; structure b owns [atom_off[b],
  * atom_off[b+1])) and the 3 structure-local atoms of every patch (nsg_patchset_atoms). */
 int nsg_upload_atoms(nsg_ctx* ctx, const int64_t* atom_off, const double* atoms_xyzr, const int32_t* patch_atoms);
+/* The same from one array per structure. */
+int nsg_upload_atoms_list(nsg_ctx* ctx, const int64_t* atom_off, const double* const* atoms_xyzr,
+                          const int32_t* const* patch_atoms);
 /* d volume and d area of every structure with respect to its atoms' x, y, z, r (n_atoms x 4 each),
  * chained from the patch derivatives on the device; either pointer may be NULL. */
 int nsg_atom_grads(nsg_ctx* ctx, double* d_volume, double* d_area);

@@ -66,6 +66,9 @@ _SIGNATURES = {
     "nsg_raycast": ([_P, _INT, _INT, ctypes.POINTER(_D)], _INT),
     "nsg_set_batch": ([_P, ctypes.c_int32, _P], _INT),
     "nsg_upload_batch": ([_P, _P, _P, _P, _P, _P, _P, _D], _INT),
+    "nsg_upload_batch_list": ([_P, _P, _P, _P, _P, _P, _P, _D], _INT),
+    "nsg_upload_atoms_list": ([_P, _P, _P, _P], _INT),
+    "nsg_release_kept": ([], _INT),
     "nsg_batch_results": ([_P, _P, _P], _INT),
     "nsg_set_tuning": ([_P, _P, _INT], _INT),
     "nsg_get_tuning": ([_P, _P, _INT], _INT),
@@ -160,3 +163,9 @@ def ptr(a: np.ndarray | None) -> int | None:
 
 def exported_symbols() -> list[str]:
     return list(_SIGNATURES)
+
+
+def release_kept() -> None:
+    """Gives back the device memory, pinned blocks and streams that the library keeps from destroyed
+    contexts for the next ones."""
+    check(lib().nsg_release_kept(), "release")

@@ -24,6 +24,7 @@
 #include "kernels/epsmap.h"
 #include "kernels/mc.h"
 #include "kernels/pipeline.h"
+#include "transfer.h"
 
 namespace {
 
@@ -57,8 +58,12 @@ struct DevPool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
 };
-DevPool* dev_pool(cudaError_t* err) {
+DevPool* dev_pools() {
   static DevPool* pools = new DevPool[64];  // live to the process's end, like the contexts' memory
+  return pools;
+}
+DevPool* dev_pool(cudaError_t* err) {
+  DevPool* pools = dev_pools();
   int dev = 0;
   if ((*err = cudaGetDevice(&dev)) != cudaSuccess) return nullptr;
   if (dev < 0 || dev >= 64) {
@@ -90,6 +95,16 @@ DevPool* dev_pool(cudaError_t* err) {
   return d;
 }
 
+void trim_dev_pools() {
+  for (int dev = 0; dev < 64; dev++) {
+    DevPool& d = dev_pools()[dev];
+    std::lock_guard<std::mutex> g(d.mu);
+    if (!d.stream) continue;
+    cudaStreamSynchronize(d.stream);
+    cudaMemPoolTrimTo(d.pool, 0);
+  }
+}
+
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
@@ -101,6 +116,13 @@ struct DevBuf {
     DevPool* d = dev_pool(&e);
     if (!d) return e;
     e = cudaMallocAsync(&p, want, d->pool, d->stream);
+    if (e == cudaErrorMemoryAllocation) {
+      // free pool memory in blocks of other sizes goes back first
+      cudaGetLastError();
+      cudaStreamSynchronize(d->stream);
+      cudaMemPoolTrimTo(d->pool, 0);
+      e = cudaMallocAsync(&p, want, d->pool, d->stream);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
     if (e == cudaSuccess) cap = want;
     else p = nullptr;
@@ -494,6 +516,19 @@ void stage_end(nsg_ctx* c, int id, bool count = true) {
   if (count) c->stage_calls[id]++;
 }
 
+// One contiguous host array to or from device memory (transfer.h).
+nsg::TeamCopy whole(void* dev, const void* host, size_t bytes) {
+  nsg::TeamCopy t{(char*)dev, bytes, {}};
+  if (bytes) t.pieces.push_back(nsg::HostPiece{(char*)host, 0});
+  return t;
+}
+cudaError_t upload(nsg_ctx* c, const std::vector<nsg::TeamCopy>& copies) {
+  return nsg::team_copy(copies, true, c->device, c->stream);
+}
+cudaError_t download(nsg_ctx* c, const std::vector<nsg::TeamCopy>& copies) {
+  return nsg::team_copy(copies, false, c->device, c->stream);
+}
+
 #define LAUNCH(call)  \
   do {                \
     c->launches++;    \
@@ -707,23 +742,41 @@ int nsg_upload_patches(nsg_ctx* c, int64_t n, const double* f64, const int32_t* 
   CK(c->i32.ensure(std::max<int64_t>(n, 1) * NS_PATCH_I32 * sizeof(int32_t)));
   CK(c->pool.ensure(std::max<int64_t>(npool, 1) * 4 * sizeof(double)));
   CK(c->flag.ensure(std::max<int64_t>(npool, 1)));
-  if (n) {
-    CK(cudaMemcpyAsync(c->f64.p, f64, n * NS_PATCH_F64 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->i32.p, i32, n * NS_PATCH_I32 * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-  }
-  if (npool) {
-    CK(cudaMemcpyAsync(c->pool.p, pool, npool * 4 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->flag.p, pool_flag, npool, cudaMemcpyHostToDevice, c->stream));
-  }
+  CK(upload(c, {whole(c->f64.p, f64, n * NS_PATCH_F64 * sizeof(double)),
+                whole(c->i32.p, i32, n * NS_PATCH_I32 * sizeof(int32_t)),
+                whole(c->pool.p, pool, npool * 4 * sizeof(double)), whole(c->flag.p, pool_flag, npool)}));
   c->ext_f64 = nullptr; c->ext_i32 = nullptr; c->ext_pool = nullptr; c->ext_flag = nullptr;
   return upload_common(c, n, npool, probe);
 }
 
-// Patch sets of the structures of a batch, concatenated: structure b owns patches
-// [patch_off[b], patch_off[b+1]) and pool entries [pool_off[b], pool_off[b+1]); the pool indices in
-// each patch record are local to its structure's pool.
-int nsg_upload_batch(nsg_ctx* c, const int64_t* patch_off, const double* f64, const int32_t* i32,
-                     const int64_t* pool_off, const double* pool, const int8_t* pool_flag, double probe) {
+}  // extern "C"
+
+namespace {
+
+// Host side of one array of a batch: contiguous, or one pointer per structure.
+struct BatchArray {
+  const void* all;
+  const void* const* list;
+  // the copy of items [off[0], off[n]) of `size` bytes each
+  nsg::TeamCopy to(void* dev, const int64_t* off, int32_t n, size_t size) const {
+    const size_t bytes = (size_t)off[n] * size;
+    if (!list) return whole(dev, all, bytes);
+    nsg::TeamCopy t{(char*)dev, bytes, {}};
+    for (int32_t b = 0; b < n; b++)
+      if (off[b + 1] > off[b]) t.pieces.push_back(nsg::HostPiece{(char*)list[b], (size_t)off[b] * size});
+    return t;
+  }
+  bool missing(const int64_t* off, int32_t n) const {
+    if (off[n] == 0) return false;
+    if (!list) return !all;
+    for (int32_t b = 0; b < n; b++)
+      if (off[b + 1] > off[b] && !list[b]) return true;
+    return false;
+  }
+};
+
+int upload_batch(nsg_ctx* c, const int64_t* patch_off, const BatchArray& f64, const BatchArray& i32,
+                 const int64_t* pool_off, const BatchArray& pool, const BatchArray& flag, double probe) {
   if (!c || !patch_off || !pool_off) return NSG_ERR_ARG;
   if (c->nstruct < 1) return fail(NSG_ERR_STATE, "nsg_set_batch must come first");
   const int32_t nb = c->nstruct;
@@ -732,7 +785,9 @@ int nsg_upload_batch(nsg_ctx* c, const int64_t* patch_off, const double* f64, co
     if (patch_off[b + 1] < patch_off[b] || pool_off[b + 1] < pool_off[b])
       return fail(NSG_ERR_ARG, "offsets must be non-decreasing");
   const int64_t n = patch_off[nb], npool = pool_off[nb];
-  if ((n > 0 && (!f64 || !i32)) || (npool > 0 && (!pool || !pool_flag))) return NSG_ERR_ARG;
+  if (f64.missing(patch_off, nb) || i32.missing(patch_off, nb) || pool.missing(pool_off, nb) ||
+      flag.missing(pool_off, nb))
+    return NSG_ERR_ARG;
   if (n >= (int64_t)1 << 31 || npool >= (int64_t)1 << 31) return fail(NSG_ERR_CAPACITY, "more than 2^31 patches");
   CK(cudaSetDevice(c->device));
   CK(c->f64.ensure(std::max<int64_t>(n, 1) * NS_PATCH_F64 * sizeof(double)));
@@ -742,26 +797,21 @@ int nsg_upload_batch(nsg_ctx* c, const int64_t* patch_off, const double* f64, co
   CK(c->d_patch_struct.ensure(std::max<int64_t>(n, 1) * sizeof(int32_t)));
   // straight copies of the caller's arrays (pinned buffers copy at full link speed); the pool
   // indices are made batch-wide and the patch -> structure map is built on the device
-  if (n) {
-    CK(cudaMemcpyAsync(c->f64.p, f64, n * NS_PATCH_F64 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->i32.p, i32, n * NS_PATCH_I32 * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-  }
-  if (npool) {
-    CK(cudaMemcpyAsync(c->pool.p, pool, npool * 4 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->flag.p, pool_flag, npool, cudaMemcpyHostToDevice, c->stream));
-  }
+  CK(upload(c, {f64.to(c->f64.p, patch_off, nb, NS_PATCH_F64 * sizeof(double)),
+                i32.to(c->i32.p, patch_off, nb, NS_PATCH_I32 * sizeof(int32_t)),
+                pool.to(c->pool.p, pool_off, nb, 4 * sizeof(double)), flag.to(c->flag.p, pool_off, nb, 1)}));
   std::vector<int64_t> po(patch_off, patch_off + nb + 1), qo(pool_off, pool_off + nb + 1);
   CK(upload_vec(c->d_patch_off, po, c->stream));
   CK(upload_vec(c->d_pool_off, qo, c->stream));
   CK(c->d_bad.ensure(sizeof(int32_t)));
+  CK(c->h_read.ensure(sizeof(int32_t)));
   CK(cudaMemsetAsync(c->d_bad.p, 0, sizeof(int32_t), c->stream));
   LAUNCH(nsg::launch_batch_patches(n, c->d_patch_off.as<int64_t>(), nb, c->d_pool_off.as<int64_t>(),
                                    c->i32.as<int32_t>(), c->d_patch_struct.as<int32_t>(), c->d_bad.as<int32_t>(),
                                    c->stream));
-  int32_t bad = 0;
-  CK(cudaMemcpyAsync(&bad, c->d_bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->h_read.p, c->d_bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (bad) {
+  if (*c->h_read.as<int32_t>()) {
     c->has_patches = false;
     return fail(NSG_ERR_ARG, "patch pool range outside its structure's pool");
   }
@@ -774,11 +824,7 @@ int nsg_upload_batch(nsg_ctx* c, const int64_t* patch_off, const double* f64, co
   return NSG_OK;
 }
 
-// The atoms the uploaded patches were built from (after jitter), concatenated over the batch
-// (structure b owns atoms [atom_off[b], atom_off[b+1])), and the 3 atoms of every patch with
-// indices local to its structure (nsg_patchset_atoms); needed by nsg_atom_grads.
-int nsg_upload_atoms(nsg_ctx* c, const int64_t* atom_off, const double* atoms_xyzr, const int32_t* patch_atoms) {
-  if (!c || !atom_off || !atoms_xyzr || !patch_atoms) return NSG_ERR_ARG;
+int upload_atoms(nsg_ctx* c, const int64_t* atom_off, const BatchArray& atoms, const BatchArray& patch_atoms) {
   if (!c->has_patches || c->patch_nstruct != c->nstruct || (int32_t)c->patch_off.size() != c->nstruct + 1)
     return fail(NSG_ERR_STATE, "patches of the current batch must be uploaded first");
   const int32_t nb = c->nstruct;
@@ -787,27 +833,89 @@ int nsg_upload_atoms(nsg_ctx* c, const int64_t* atom_off, const double* atoms_xy
     if (atom_off[b + 1] < atom_off[b]) return fail(NSG_ERR_ARG, "atom offsets must be non-decreasing");
   const int64_t n = atom_off[nb];
   if (n >= ((int64_t)1 << 31)) return fail(NSG_ERR_CAPACITY, "more than 2^31 atoms");
+  if (atoms.missing(atom_off, nb) || patch_atoms.missing(c->patch_off.data(), nb)) return NSG_ERR_ARG;
   CK(cudaSetDevice(c->device));
   int rc = ensure_patch_struct(c);
   if (rc) return rc;
   CK(c->d_atoms.ensure(std::max<int64_t>(n, 1) * 4 * sizeof(double)));
   CK(c->d_patch_atoms.ensure(std::max<int64_t>(3 * c->np, 1) * sizeof(int32_t)));
-  if (n) CK(cudaMemcpyAsync(c->d_atoms.p, atoms_xyzr, n * 4 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  if (c->np)
-    CK(cudaMemcpyAsync(c->d_patch_atoms.p, patch_atoms, 3 * c->np * sizeof(int32_t), cudaMemcpyHostToDevice,
-                       c->stream));
+  CK(upload(c, {atoms.to(c->d_atoms.p, atom_off, nb, 4 * sizeof(double)),
+                patch_atoms.to(c->d_patch_atoms.p, c->patch_off.data(), nb, 3 * sizeof(int32_t))}));
   std::vector<int64_t> ao(atom_off, atom_off + nb + 1);
   CK(upload_vec(c->d_atom_off, ao, c->stream));
   CK(c->d_bad.ensure(sizeof(int32_t)));
+  CK(c->h_read.ensure(sizeof(int32_t)));
   CK(cudaMemsetAsync(c->d_bad.p, 0, sizeof(int32_t), c->stream));
   LAUNCH(nsg::launch_batch_atoms(c->np, c->d_patch_struct.as<int32_t>(), c->d_atom_off.as<int64_t>(),
                                  c->d_patch_atoms.as<int32_t>(), c->d_bad.as<int32_t>(), c->stream));
-  int32_t bad = 0;
-  CK(cudaMemcpyAsync(&bad, c->d_bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->h_read.p, c->d_bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (bad) return fail(NSG_ERR_ARG, "patch atom index outside its structure");
+  if (*c->h_read.as<int32_t>()) return fail(NSG_ERR_ARG, "patch atom index outside its structure");
   c->n_atoms = n;
   c->have_atoms = true;
+  return NSG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+// Patch sets of the structures of a batch, concatenated: structure b owns patches
+// [patch_off[b], patch_off[b+1]) and pool entries [pool_off[b], pool_off[b+1]); the pool indices in
+// each patch record are local to its structure's pool.
+int nsg_upload_batch(nsg_ctx* c, const int64_t* patch_off, const double* f64, const int32_t* i32,
+                     const int64_t* pool_off, const double* pool, const int8_t* pool_flag, double probe) {
+  return upload_batch(c, patch_off, {f64, nullptr}, {i32, nullptr}, pool_off, {pool, nullptr}, {pool_flag, nullptr},
+                      probe);
+}
+
+// The same from one array per structure (arrays of n pointers, as nsg_ses_build leaves the sets), so
+// that the caller need not concatenate them.
+int nsg_upload_batch_list(nsg_ctx* c, const int64_t* patch_off, const double* const* f64, const int32_t* const* i32,
+                          const int64_t* pool_off, const double* const* pool, const int8_t* const* pool_flag,
+                          double probe) {
+  if (!f64 || !i32 || !pool || !pool_flag) return NSG_ERR_ARG;
+  return upload_batch(c, patch_off, {nullptr, (const void* const*)f64}, {nullptr, (const void* const*)i32}, pool_off,
+                      {nullptr, (const void* const*)pool}, {nullptr, (const void* const*)pool_flag}, probe);
+}
+
+// The atoms the uploaded patches were built from (after jitter), concatenated over the batch
+// (structure b owns atoms [atom_off[b], atom_off[b+1])), and the 3 atoms of every patch with
+// indices local to its structure (nsg_patchset_atoms); needed by nsg_atom_grads.
+int nsg_upload_atoms(nsg_ctx* c, const int64_t* atom_off, const double* atoms_xyzr, const int32_t* patch_atoms) {
+  if (!c || !atom_off || !atoms_xyzr || !patch_atoms) return NSG_ERR_ARG;
+  return upload_atoms(c, atom_off, {atoms_xyzr, nullptr}, {patch_atoms, nullptr});
+}
+
+// The same from one array per structure.
+int nsg_upload_atoms_list(nsg_ctx* c, const int64_t* atom_off, const double* const* atoms_xyzr,
+                          const int32_t* const* patch_atoms) {
+  if (!c || !atom_off || !atoms_xyzr || !patch_atoms) return NSG_ERR_ARG;
+  return upload_atoms(c, atom_off, {nullptr, (const void* const*)atoms_xyzr},
+                      {nullptr, (const void* const*)patch_atoms});
+}
+
+// Gives back what the library keeps from one context to the next: the devices' free pool memory,
+// pinned host blocks and streams.
+int nsg_release_kept(void) {
+  int dev = 0;
+  const bool have = cudaGetDevice(&dev) == cudaSuccess;
+  nsg::team_release();
+  {
+    PinPool& pool = pin_pool();
+    std::lock_guard<std::mutex> g(pool.mu);
+    for (auto& b : pool.kept) cudaFreeHost(b.first);
+    pool.kept.clear();
+    pool.bytes = 0;
+  }
+  {
+    StreamPool& pool = stream_pool();
+    std::lock_guard<std::mutex> g(pool.mu);
+    for (auto& s : pool.kept) cudaStreamDestroy(s.second);
+    pool.kept.clear();
+  }
+  trim_dev_pools();
+  if (have) cudaSetDevice(dev);
   return NSG_OK;
 }
 
@@ -830,13 +938,12 @@ int nsg_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
                            c->gvol.as<double>(), c->have_garea ? c->garea.as<double>() : nullptr,
                            c->d_gatoms_vol.as<double>(), c->d_gatoms_area.as<double>(), c->d_bad.as<int32_t>(),
                            c->stream));
-  int32_t bad = 0;
-  CK(cudaMemcpyAsync(&bad, c->d_bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  if (d_volume && c->n_atoms)
-    CK(cudaMemcpyAsync(d_volume, c->d_gatoms_vol.p, c->n_atoms * 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (d_area && c->n_atoms)
-    CK(cudaMemcpyAsync(d_area, c->d_gatoms_area.p, c->n_atoms * 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(c->h_read.ensure(sizeof(int32_t)));
+  CK(cudaMemcpyAsync(c->h_read.p, c->d_bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  const size_t bytes = (size_t)c->n_atoms * 4 * sizeof(double);
+  CK(download(c, {whole(c->d_gatoms_vol.p, d_volume, d_volume ? bytes : 0),
+                  whole(c->d_gatoms_area.p, d_area, d_area ? bytes : 0)}));
+  const int32_t bad = *c->h_read.as<int32_t>();
   if (bad) return fail(NSG_ERR_GEOMETRY, "a probe patch with a singular placement system was skipped");
   return NSG_OK;
 }
@@ -850,9 +957,7 @@ int nsg_patch_grads(nsg_ctx* c, double* gvol, double* garea) {
     return fail(NSG_ERR_STATE, "no gradient-mode ray cast / triangulation to read");
   CK(cudaSetDevice(c->device));
   const size_t bytes = (size_t)c->np * NS_GRAD_PER_PATCH * sizeof(double);
-  if (gvol && c->np) CK(cudaMemcpyAsync(gvol, c->gvol.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-  if (garea && c->np) CK(cudaMemcpyAsync(garea, c->garea.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(download(c, {whole(c->gvol.p, gvol, gvol ? bytes : 0), whole(c->garea.p, garea, garea ? bytes : 0)}));
   return NSG_OK;
 }
 
@@ -1073,11 +1178,8 @@ int nsg_blobby_mesh(nsg_ctx* c, int64_t* n_vertices, int64_t* n_triangles, doubl
   if (!c->b_valid) return fail(NSG_ERR_STATE, "no blobby mesh built");
   if (n_vertices) *n_vertices = c->b_nv_n;
   if (n_triangles) *n_triangles = c->b_nt_n;
-  if (vertices && c->b_nv_n)
-    CK(cudaMemcpyAsync(vertices, c->b_verts.p, c->b_nv_n * 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (triangles && c->b_nt_n)
-    CK(cudaMemcpyAsync(triangles, c->b_tris.p, c->b_nt_n * 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(download(c, {whole(c->b_verts.p, vertices, vertices ? c->b_nv_n * 3 * sizeof(double) : 0),
+                  whole(c->b_tris.p, triangles, triangles ? c->b_nt_n * 3 * sizeof(int32_t) : 0)}));
   return NSG_OK;
 }
 
@@ -1970,27 +2072,23 @@ int nsg_download_status(nsg_ctx* c, int32_t* dst) {
   int rc = ensure_dense_status(c);
   if (rc) return rc;
   const NsGrid& g = c->grid;
-  CK(cudaMemcpyAsync(dst, c->status.p, g.nx * g.ny * g.nz * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(download(c, {whole(c->status.p, dst, g.nx * g.ny * g.nz * sizeof(int32_t))}));
   return NSG_OK;
 }
 
 int nsg_download_insideness(nsg_ctx* c, uint32_t* dst) {
   if (!c || !dst || !c->have_bits) return NSG_ERR_STATE;
-  CK(cudaMemcpyAsync(dst, c->bits.p, c->words_tot * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(cudaSetDevice(c->device));
+  CK(download(c, {whole(c->bits.p, dst, c->words_tot * sizeof(uint32_t))}));
   return NSG_OK;
 }
 
 int nsg_download_mesh(nsg_ctx* c, double* verts, int32_t* vkeys, int32_t* tris) {
   if (!c) return NSG_ERR_ARG;
-  if (verts && c->n_vert)
-    CK(cudaMemcpyAsync(verts, c->vpos.p, c->n_vert * 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (vkeys && c->n_vert)
-    CK(cudaMemcpyAsync(vkeys, c->vkey.p, c->n_vert * sizeof(int4), cudaMemcpyDeviceToHost, c->stream));
-  if (tris && c->n_tri)
-    CK(cudaMemcpyAsync(tris, c->tris.p, c->n_tri * 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(cudaSetDevice(c->device));
+  CK(download(c, {whole(c->vpos.p, verts, verts ? c->n_vert * 3 * sizeof(double) : 0),
+                  whole(c->vkey.p, vkeys, vkeys ? c->n_vert * sizeof(int4) : 0),
+                  whole(c->tris.p, tris, tris ? c->n_tri * 3 * sizeof(int32_t) : 0)}));
   return NSG_OK;
 }
 
@@ -2152,9 +2250,7 @@ int nsg_download_epsmap(nsg_ctx* c, int32_t* dst) {
   if (!c->have_eps) return fail(NSG_ERR_STATE, "no epsilon maps: ray cast with NSG_RAYCAST_EPSMAP");
   CK(cudaSetDevice(c->device));
   const NsGrid& g = c->grid;
-  CK(cudaMemcpyAsync(dst, c->epsmap.p, (size_t)g.nx * g.ny * g.nz * 3 * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                     c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(download(c, {whole(c->epsmap.p, dst, (size_t)g.nx * g.ny * g.nz * 3 * sizeof(int32_t))}));
   return NSG_OK;
 }
 
@@ -2173,8 +2269,7 @@ int nsg_download_idebmap(nsg_ctx* c, uint8_t* dst) {
     LAUNCH(nsg::ideb_write(A, c->eps_filled ? c->cc_fill_of.as<uint8_t>() : nullptr, c->ideb.as<uint8_t>(),
                            c->stream));
   }
-  CK(cudaMemcpyAsync(dst, c->ideb.p, nn, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(download(c, {whole(c->ideb.p, dst, nn)}));
   return NSG_OK;
 }
 
@@ -2298,14 +2393,11 @@ int nsg_download_bgp(nsg_ctx* c, int32_t* ibgp, int32_t* type, double* scspos, d
   if ((scspos || scsnor || flag) && !c->bgp_projected) return fail(NSG_ERR_STATE, "boundary grid points not projected");
   CK(cudaSetDevice(c->device));
   const size_t n = (size_t)c->n_bgp;
-  if (n) {
-    if (ibgp) CK(cudaMemcpyAsync(ibgp, c->bgp_ibgp.p, 3 * n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    if (type) CK(cudaMemcpyAsync(type, c->bgp_type.p, n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    if (scspos) CK(cudaMemcpyAsync(scspos, c->bgp_pos.p, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (scsnor) CK(cudaMemcpyAsync(scsnor, c->bgp_nor.p, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (flag) CK(cudaMemcpyAsync(flag, c->bgp_flag.p, n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  }
-  CK(cudaStreamSynchronize(c->stream));
+  CK(download(c, {whole(c->bgp_ibgp.p, ibgp, ibgp ? 3 * n * sizeof(int32_t) : 0),
+                  whole(c->bgp_type.p, type, type ? n * sizeof(int32_t) : 0),
+                  whole(c->bgp_pos.p, scspos, scspos ? 3 * n * sizeof(double) : 0),
+                  whole(c->bgp_nor.p, scsnor, scsnor ? 3 * n * sizeof(double) : 0),
+                  whole(c->bgp_flag.p, flag, flag ? n * sizeof(int32_t) : 0)}));
   return NSG_OK;
 }
 

@@ -518,7 +518,7 @@ class Surface:
                 self.delphi.epsmap = eps.reshape(g.nz, g.ny, g.nx, 3)
                 ideb = np.empty(g.nx * g.ny * g.nz, np.uint8)
                 N.check(N.lib().nsg_download_idebmap(c, N.ptr(ideb)), "download ideb map")
-                self.delphi.idebmap = ideb.reshape(g.nz, g.ny, g.nx).astype(bool)
+                self.delphi.idebmap = ideb.reshape(g.nz, g.ny, g.nx).view(np.bool_)  # 0 or 1
         if self.projBGP:
             self.projectBoundaryGridPoints()
         return self.volume
@@ -819,6 +819,15 @@ class BlobbySurface(Surface):
         return dvol * gv if ga is None else dvol * gv + darea * ga
 
 
+class _pointers:
+    """Addresses of a list of arrays, for the calls that take one array per structure; keeps the
+    arrays (contiguous, of the wanted type) alive."""
+
+    def __init__(self, arrays: list, dtype):
+        self.arrays = [np.ascontiguousarray(a, dtype) for a in arrays]
+        self.list = (ctypes.c_void_p * len(arrays))(*[a.ctypes.data for a in self.arrays])
+
+
 class SurfaceBatch:
     """Many built surfaces, each with its own grid and patch set, ray cast and triangulated in the
     same kernel launches: one ``getSurf`` + ``triangulateSurface`` per structure, batched.
@@ -851,13 +860,18 @@ class SurfaceBatch:
             self.ctx = Context(self.device)
         return self.ctx
 
-    def packed(self) -> tuple:
-        """Concatenated patch arrays and their per-structure offsets (host)."""
-        ps = [s.patches for s in self.surfaces]
+    @staticmethod
+    def _offsets(ps: list) -> tuple[np.ndarray, np.ndarray]:
         patch_off = np.zeros(len(ps) + 1, np.int64)
         pool_off = np.zeros(len(ps) + 1, np.int64)
         patch_off[1:] = np.cumsum([p.n for p in ps])
         pool_off[1:] = np.cumsum([len(p.pool) for p in ps])
+        return patch_off, pool_off
+
+    def packed(self) -> tuple:
+        """Concatenated patch arrays and their per-structure offsets (host)."""
+        ps = [s.patches for s in self.surfaces]
+        patch_off, pool_off = self._offsets(ps)
         f64 = np.ascontiguousarray(np.concatenate([p.f64 for p in ps]))
         i32 = np.ascontiguousarray(np.concatenate([p.i32 for p in ps]))
         pool = np.ascontiguousarray(np.concatenate([p.pool for p in ps])) if pool_off[-1] else np.zeros((1, 4))
@@ -869,10 +883,13 @@ class SurfaceBatch:
         n = len(self.surfaces)
         grids = (N.NsGrid * n)(*[s.delphi.grid for s in self.surfaces])
         N.check(N.lib().nsg_set_batch(c, n, grids), "set_batch")
-        patch_off, pool_off, f64, i32, pool, flag = self.packed()
-        probe = self.surfaces[0].patches.probe
-        N.check(N.lib().nsg_upload_batch(c, N.ptr(patch_off), N.ptr(f64), N.ptr(i32), N.ptr(pool_off), N.ptr(pool),
-                                         N.ptr(flag), probe), "upload_batch")
+        # straight from every structure's arrays: the library's copy threads gather them
+        ps = [s.patches for s in self.surfaces]
+        patch_off, pool_off = self._offsets(ps)
+        f64, i32 = _pointers([p.f64 for p in ps], np.float64), _pointers([p.i32 for p in ps], np.int32)
+        pool, flag = _pointers([p.pool for p in ps], np.float64), _pointers([p.pool_flag for p in ps], np.int8)
+        N.check(N.lib().nsg_upload_batch_list(c, N.ptr(patch_off), f64.list, i32.list, N.ptr(pool_off), pool.list,
+                                              flag.list, ps[0].probe), "upload_batch")
 
     def getSurf(self, download: bool = False, grad: bool = False) -> np.ndarray:
         """Ray casts every structure's grid; returns the per-structure volumes.  With ``grad`` the
@@ -948,10 +965,14 @@ class SurfaceBatch:
         """Per structure: (d volume / d atoms, d area / d atoms), each (n_atoms, 4) for x, y, z, r,
         after a gradient-mode getSurf and triangulateSurface (chained on the device)."""
         c = self._context().handle
-        atom_off, atoms, patch_atoms = self.packed_atoms()
-        N.check(N.lib().nsg_upload_atoms(c, N.ptr(atom_off), N.ptr(atoms), N.ptr(patch_atoms)), "upload atoms")
-        gv = np.zeros((len(atoms), 4))
-        ga = np.zeros((len(atoms), 4))
+        ps = [s.patches for s in self.surfaces]
+        atom_off = np.zeros(len(ps) + 1, np.int64)
+        atom_off[1:] = np.cumsum([len(p.built_from) for p in ps])
+        atoms = _pointers([p.built_from for p in ps], np.float64)
+        patch_atoms = _pointers([p.atoms_of for p in ps], np.int32)
+        N.check(N.lib().nsg_upload_atoms_list(c, N.ptr(atom_off), atoms.list, patch_atoms.list), "upload atoms")
+        gv = np.empty((int(atom_off[-1]), 4))
+        ga = np.empty((int(atom_off[-1]), 4))
         rc = N.lib().nsg_atom_grads(c, N.ptr(gv), N.ptr(ga))
         if rc not in (N.NSG_OK, -8):
             N.check(rc, "atom gradients")
