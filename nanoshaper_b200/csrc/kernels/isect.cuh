@@ -199,9 +199,9 @@ __device__ __forceinline__ void isect_body(const TraceCtx& C, const CandOut& co,
     const double delta = ray_set_shifted(C.set) ? NS_DELTA - g.hside : 0.0;
     const double ray_dir = S.ray_dir[vc];
     const double inv_dir = S.inv_dir[vc];
-    const int64_t nb = g.n[fd];
-    const int64_t lr = rid - S.ray_base[C.set];
-    const int64_t m = lr % nb, n = lr / nb;
+    // a set has fewer than 2^31 rays
+    const unsigned nb = (unsigned)g.n[fd], lr = (unsigned)(rid - S.ray_base[C.set]);
+    const unsigned n = lr / nb, m = lr - n * nb;
     double pa[3];
     pa[fd] = gcoord(g, fd, m) + delta;
     pa[ld] = gcoord(g, ld, n) + delta;
@@ -400,9 +400,9 @@ __device__ __forceinline__ void isect_quadric_body(const TraceCtx& C, const Cand
     const StructDev& S = C.B.s[C.B.patch_struct[pid]];
     const GridDev& g = S.g;
     const double delta = ray_set_shifted(C.set) ? NS_DELTA - g.hside : 0.0;
-    const int64_t nb = g.n[fd];
-    const int64_t lr = rid - S.ray_base[C.set];
-    const int64_t m = lr % nb, n = lr / nb;
+    // a set has fewer than 2^31 rays
+    const unsigned nb = (unsigned)g.n[fd], lr = (unsigned)(rid - S.ray_base[C.set]);
+    const unsigned n = lr / nb, m = lr - n * nb;
     double pa[3];
     pa[fd] = gcoord(g, fd, m) + delta;
     pa[ld] = gcoord(g, ld, n) + delta;

@@ -160,6 +160,11 @@ struct CandOut {
   int2* dtor;
   int64_t dcap;
   unsigned long long* dcount;  // 2 counters
+  // torus candidates that pass the single-precision screen (torus_screen.h), of capacity scr_cap;
+  // their count at scr_count[1]
+  int2* scr;
+  int64_t scr_cap;
+  unsigned long long* scr_count;
   // torus candidates split by the branch their resolvent cubic takes (null: no split): the
   // cube-root branch (and the rare approximate ones) in tsa, the arccos branch in tsb, each of
   // capacity cap; counts at tscount[1] and tscount[3]
@@ -188,6 +193,7 @@ struct PatchDev {
   const int32_t* win;  // 6 per patch: start x,y,z, end x,y,z; start = -1 when culled
   int kind_mask;       // bit k set when some patch has kind k (host copy)
   const float4* quad32;  // skin cells in patch-local FP32 form, 3 per patch (mixed precision)
+  const float4* screen;  // torus patches: screen records, 5 per patch (torus_screen.h)
   const double4* quadl;  // skin cells: (A c + b, f(c)) about the local origin c, FP64 (mixed precision)
 };
 
@@ -211,10 +217,12 @@ struct TuneParams {
 
 // trace.cu: every launch covers all structures of the batch; `set` is the ray set (0..3) and
 // tile and ray indices are batch-wide.
-// Patch windows; out (4 words, zeroed by the caller) receives the window-area sum of each panel (the
-// bound of its candidate count) and the bit mask of the patch kinds present.
-cudaError_t launch_windows(const PatchDev& P, int32_t* win, const BatchDev& B, unsigned long long* out,
-                           cudaStream_t s);
+// Patch windows and the torus patches' screen records; out (kWindowSums words, zeroed by the caller)
+// receives the window-area sum of each panel (the bound of its candidate count), the same of the
+// torus patches alone, and the bit mask of the patch kinds present.
+constexpr int kWindowSums = 7;
+cudaError_t launch_windows(const PatchDev& P, int32_t* win, float4* screen, const BatchDev& B,
+                           unsigned long long* out, cudaStream_t s);
 // Patch-local FP32 copy of the pool: planes (n, d + n.c), clipping spheres (s - c, r^2); with
 // quad32, the skin cells' quadrics about their local origin (see k_pool32).
 cudaError_t launch_pool32(const PatchDev& P, float4* pool32, float4* quad32, double4* quadl, cudaStream_t s);
