@@ -83,8 +83,7 @@ class BlobbyVolumeArea(torch.autograd.Function):
             surf.build()
             vol = surf.getSurf(True, False, 0.0, download=False, grad=True)
             area = surf.triangulateSurface(download=False)
-            gv = surf.gradients(1.0, 0.0)
-            ga = surf.gradients(0.0, 1.0)
+            gv, ga = surf.atom_gradients()
         finally:
             surf.ctx.close()
         ctx.gv, ctx.ga = gv, ga

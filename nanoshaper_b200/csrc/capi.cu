@@ -335,7 +335,7 @@ struct nsg_ctx {
   DevBuf temp;  // cub temporary storage
   // blobby surface: atoms, field, the field's marching-cubes mesh and its patches, adjoint scratch
   DevBuf b_atoms, b_field, b_mask, b_nv, b_nt, b_voff, b_toff, b_vraw, b_verts, b_vkey, b_tris, b_inc_cnt, b_inc_off,
-      b_inc_cur, b_inc, b_patch_atoms, b_gpost, b_gpre, b_gfield, b_gatoms;
+      b_inc_cur, b_inc, b_patch_atoms, b_gpost, b_gpre, b_gfield[2], b_gatoms, b_win;
   int64_t b_natoms = 0, b_nv_n = 0, b_nt_n = 0;
   double b_B = -2.5;
   int b_ng = 0;
@@ -659,7 +659,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (int i = 0; i < nsg::kRaySets; i++)
     if (c->set_stream[i]) cudaStreamSynchronize(c->set_stream[i]);
-  DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield, &c->b_gatoms, &c->counters, &c->win_sums, &c->screen,
+  DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield[0], &c->b_gfield[1], &c->b_gatoms, &c->b_win, &c->counters, &c->win_sums, &c->screen,
                     &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_node, &c->bgp_ibgp, &c->bgp_type,
                     &c->bgp_pos, &c->bgp_nor, &c->bgp_flag, &c->bgp_n, &c->aux_cnt, &c->aux_off, &c->aux_list, &c->pairs,
                     &c->ray_pair_off, &c->ray_pair_cnt, &c->cursors, &c->ovf_scratch, &c->hits,
@@ -1099,7 +1099,6 @@ int nsg_blobby_build(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, doub
     return NSG_ERR_ARG;
   if (!c->has_grid || c->nstruct != 1) return fail(NSG_ERR_STATE, "a single-structure grid must be set first");
   CK(cudaSetDevice(c->device));
-  CK(nsg::blobby_init_tables());
   const NsGrid& G = c->grid;
   const nsg::GridDev g = grid_dev(G);
   const int64_t nodes = G.nx * G.ny * G.nz;
@@ -1110,7 +1109,10 @@ int nsg_blobby_build(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, doub
   // cut-off of 6 A in whole grid steps (DEFAULT_CUTOFF, src/BlobbySurface.h)
   const int ng = (int)(6.0 / G.side + 0.5);
   CK(c->b_field.ensure(nodes * sizeof(double)));
-  LAUNCH(nsg::launch_blobby_field(g, c->b_atoms.as<double>(), (int)n_atoms, blobbyness, ng, c->b_field.as<double>(), s));
+  CK(c->b_win.ensure(n_atoms * 2 * sizeof(int4)));
+  c->launches++;
+  LAUNCH(nsg::launch_blobby_field(g, c->b_atoms.as<double>(), (int)n_atoms, blobbyness, ng, c->b_win.as<int4>(),
+                                  c->b_field.as<double>(), s));
   const double iso = 1.0;
   CK(c->b_mask.ensure(std::max<int64_t>(ncubes, 1)));
   CK(c->b_nv.ensure(std::max<int64_t>(ncubes, 1) * sizeof(int32_t)));
@@ -1202,22 +1204,32 @@ int nsg_blobby_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
   const nsg::GridDev g = grid_dev(G);
   CK(c->b_gpost.ensure(std::max<int64_t>(c->b_nv_n, 1) * 3 * sizeof(double)));
   CK(c->b_gpre.ensure(std::max<int64_t>(c->b_nv_n, 1) * 3 * sizeof(double)));
-  CK(c->b_gfield.ensure(G.nx * G.ny * G.nz * sizeof(double)));
-  CK(c->b_gatoms.ensure(c->b_natoms * 4 * sizeof(double)));
+  CK(c->b_gatoms.ensure(2 * c->b_natoms * 4 * sizeof(double)));
   nsg::BlobbyMeshDev M{c->b_nv_n, c->b_nt_n, c->b_verts.as<double>(), c->b_vkey.as<int4>(), c->b_tris.as<int32_t>(),
                        c->f64.as<double>(), c->b_patch_atoms.as<int32_t>(), c->b_inc_cnt.as<int32_t>()};
+  // the mesh part of the chain for each of the two, then the field part for both at once
+  double* const dst[2] = {d_volume, d_area};
+  const size_t bytes = c->b_natoms * 4 * sizeof(double);
+  double* gatoms[2] = {nullptr, nullptr};
+  const double* gfield[2] = {nullptr, nullptr};
+  double* host[2] = {nullptr, nullptr};
+  int n = 0;
+  CK(cudaMemsetAsync(c->b_gatoms.p, 0, 2 * bytes, c->stream));
   for (int which = 0; which < 2; which++) {
-    double* dst = which == 0 ? d_volume : d_area;
-    if (!dst) continue;
-    CK(cudaMemsetAsync(c->b_gatoms.p, 0, c->b_natoms * 4 * sizeof(double), c->stream));
-    LAUNCH(nsg::launch_blobby_adjoint(g, c->b_atoms.as<double>(), (int)c->b_natoms, c->b_B, c->b_ng,
-                                      c->b_field.as<double>(), 1.0, M,
-                                      which == 0 ? c->gvol.as<double>() : c->garea.as<double>(), c->b_gpost.as<double>(),
-                                      c->b_gpre.as<double>(), c->b_gfield.as<double>(), c->b_gatoms.as<double>(),
-                                      c->stream));
-    CK(cudaMemcpyAsync(dst, c->b_gatoms.p, c->b_natoms * 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if (!dst[which]) continue;
+    CK(c->b_gfield[n].ensure(G.nx * G.ny * G.nz * sizeof(double)));
+    c->launches += 3;
+    LAUNCH(nsg::launch_mesh_adjoint(g, c->b_field.as<double>(), 1.0, M,
+                                    which == 0 ? c->gvol.as<double>() : c->garea.as<double>(), c->b_gpost.as<double>(),
+                                    c->b_gpre.as<double>(), c->b_gfield[n].as<double>(), c->stream));
+    gfield[n] = c->b_gfield[n].as<double>();
+    gatoms[n] = c->b_gatoms.as<double>() + (size_t)n * c->b_natoms * 4;
+    host[n++] = dst[which];
   }
+  if (n == 0) return NSG_OK;
+  LAUNCH(nsg::launch_field_adjoint(g, c->b_atoms.as<double>(), (int)c->b_natoms, c->b_B, c->b_ng, gfield[0], gfield[1],
+                                   gatoms[0], gatoms[1], c->stream));
+  CK(download(c, {whole(gatoms[0], host[0], bytes), whole(gatoms[1], host[1], n > 1 ? bytes : 0)}));
   return NSG_OK;
 }
 
@@ -2163,13 +2175,11 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
         if (ix[0] < 0 || ix[1] < 0 || ix[2] < 0 || ix[0] >= gn || ix[1] >= gn || ix[2] >= gn)
           return fail(NSG_ERR_ARG, "an atom lies outside the atom grid (atoms of another structure?)");
         cell_of[a] = (int32_t)((ix[2] * gn + ix[1]) * gn + ix[0]);
-        cell_off[cell_of[a] + 1]++;
+        cell_off[cell_of[a]]++;
       }
       for (int64_t q = 0; q < ncell; q++) cell_off[q + 1] += cell_off[q];
-      // the offsets move up by one atom as the cells are filled, and back by one cell afterwards
-      for (int64_t a = 0; a < n_atoms; a++) cell_atoms[cell_off[cell_of[a]]++] = (int32_t)a;
-      for (int64_t q = ncell; q > 0; q--) cell_off[q] = cell_off[q - 1];
-      cell_off[0] = 0;
+      // filled from the cells' ends, last atom first: the offsets end at the cells' starts
+      for (int64_t a = n_atoms - 1; a >= 0; a--) cell_atoms[--cell_off[cell_of[a]]] = (int32_t)a;
       const int64_t cap = c->cav_nodes;
       CK(c->ca_atoms.ensure(in_bytes));
       CK(c->ca_pairs.ensure(cap * sizeof(unsigned long long)));

@@ -25,7 +25,7 @@
 
 #include "blobby.h"
 #include "pipeline.h"
-#include "../mc_cases.h"
+#include "mc_tables.cuh"
 
 namespace nsg {
 
@@ -44,9 +44,25 @@ __device__ __forceinline__ void atom_window(const GridDev& g, const double* a, i
   }
 }
 
-__global__ void __launch_bounds__(kFieldThreads) k_blobby_field(GridDev g, const double* __restrict__ atoms, int na,
-                                                               double B, int ng, double* __restrict__ field) {
-  __shared__ int s_list[kFieldThreads];
+// Node window [lo, hi) of every atom, once per field (the tiles test it as integers).
+__global__ void k_atom_windows(GridDev g, const double* __restrict__ atoms, int na, int ng, int4* win) {
+  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
+    int lo[3], hi[3];
+    atom_window(g, atoms + 4 * (int64_t)a, ng, lo, hi);
+    win[2 * a] = make_int4(lo[0], hi[0], lo[1], hi[1]);
+    win[2 * a + 1] = make_int4(lo[2], hi[2], 0, 0);
+  }
+}
+
+// One node per thread.  Bound by the double-precision exponential and division of every (node, atom)
+// pair; the tile's atoms, their r^2 and their windows are kept in shared memory so that nothing
+// else of the pair is computed twice.  2,000 atoms at scale 3 (93 M pairs): windows formed per pair
+// 858 us -> 690 us.
+__global__ void __launch_bounds__(kFieldThreads) k_blobby_field(GridDev g, const double* __restrict__ atoms,
+                                                               const int4* __restrict__ win, int na, double B,
+                                                               double* __restrict__ field) {
+  __shared__ double4 s_atom[kFieldThreads];  // x, y, z, r^2
+  __shared__ int4 s_win[2 * kFieldThreads];
   __shared__ int s_warp[kFieldThreads / 32];
   const int tid = threadIdx.x;
   const int tx = tid % kTX, ty = (tid / kTX) % kTY, tz = tid / (kTX * kTY);
@@ -64,10 +80,11 @@ __global__ void __launch_bounds__(kFieldThreads) k_blobby_field(GridDev g, const
   for (int base = 0; base < na; base += kFieldThreads) {
     const int a = base + tid;
     bool take = false;
+    int4 w0, w1;
     if (a < na) {
-      int lo[3], hi[3];
-      atom_window(g, atoms + 4 * (int64_t)a, ng, lo, hi);
-      take = lo[0] < i0 + kTX && hi[0] > i0 && lo[1] < j0 + kTY && hi[1] > j0 && lo[2] < k0 + kTZ && hi[2] > k0;
+      w0 = win[2 * a];
+      w1 = win[2 * a + 1];
+      take = w0.x < i0 + kTX && w0.y > i0 && w0.z < j0 + kTY && w0.w > j0 && w1.x < k0 + kTZ && w1.y > k0;
     }
     // order-preserving compaction of the chunk's atoms that reach the tile
     const unsigned m = __ballot_sync(0xffffffffu, take);
@@ -78,27 +95,26 @@ __global__ void __launch_bounds__(kFieldThreads) k_blobby_field(GridDev g, const
       if (w < warp) before += s_warp[w];
       total += s_warp[w];
     }
-    if (take) s_list[before + __popc(m & ((1u << lane) - 1u))] = a;
+    if (take) {
+      const int slot = before + __popc(m & ((1u << lane) - 1u));
+      const double* at = atoms + 4 * (int64_t)a;
+      s_atom[slot] = make_double4(at[0], at[1], at[2], at[3] * at[3]);
+      s_win[2 * slot] = w0;
+      s_win[2 * slot + 1] = w1;
+    }
     __syncthreads();
     if (valid)
       for (int q = 0; q < total; q++) {
-        const double* at = atoms + 4 * (int64_t)s_list[q];
-        int lo[3], hi[3];
-        atom_window(g, at, ng, lo, hi);
-        if (i < lo[0] || i >= hi[0] || j < lo[1] || j >= hi[1] || k < lo[2] || k >= hi[2]) continue;
-        const double r = at[3];
-        const double r2 = r * r;
-        const double dist2 = (p[0] - at[0]) * (p[0] - at[0]) + (p[1] - at[1]) * (p[1] - at[1]) +
-                             (p[2] - at[2]) * (p[2] - at[2]);
-        acc += exp(B * (dist2 / r2 - 1));
+        const int4 u = s_win[2 * q], v = s_win[2 * q + 1];
+        if (i < u.x || i >= u.y || j < u.z || j >= u.w || k < v.x || k >= v.y) continue;
+        const double4 at = s_atom[q];
+        const double dist2 = (p[0] - at.x) * (p[0] - at.x) + (p[1] - at.y) * (p[1] - at.y) + (p[2] - at.z) * (p[2] - at.z);
+        acc += exp(B * (dist2 / at.w - 1));
       }
     __syncthreads();
   }
   if (valid) field[((int64_t)k * g.n[1] + j) * g.n[0] + i] = acc;
 }
-
-__constant__ int8_t c_tri[256][16];
-__constant__ int c_edge_mask[256];
 
 __device__ __forceinline__ int64_t nidx(const GridDev& g, int64_t i, int64_t j, int64_t k) {
   return (k * g.n[1] + j) * g.n[0] + i;
@@ -173,7 +189,7 @@ __global__ void k_field_cubes(GridDev g, const double* __restrict__ f, double is
     cube_of(g, c, &i, &j, &k);
     double vals[8];
     const int ci = classify(g, f, i, j, k, iso, vals);
-    const int em = c_edge_mask[ci];
+    const int em = d_mc.emask[ci];
     uint8_t m = 0;
     if (em & 32) m |= 1;
     if (em & 64) m |= 2;
@@ -182,12 +198,12 @@ __global__ void k_field_cubes(GridDev g, const double* __restrict__ f, double is
     nvert[c] = __popc(m);
     int nt = 0;
     if (em)
-      for (int q = 0; q < 16 && c_tri[ci][q] >= 0; q += 3) {
+      for (int q = 0; q < 16 && d_mc.tri[ci][q] >= 0; q += 3) {
         bool ok = true;
         for (int r = 0; r < 3; r++) {
           int64_t oi, oj, ok2;
           int slot;
-          edge_owner(edge_key(i, j, k, c_tri[ci][q + r]), &oi, &oj, &ok2, &slot);
+          edge_owner(edge_key(i, j, k, d_mc.tri[ci][q + r]), &oi, &oj, &ok2, &slot);
           if (!cube_in_range(g, oi, oj, ok2)) ok = false;
         }
         nt += ok;
@@ -244,13 +260,13 @@ __global__ void k_field_tris(GridDev g, const double* __restrict__ f, double iso
     double vals[8];
     const int ci = classify(g, f, i, j, k, iso, vals);
     int64_t t = tbase[c];
-    for (int q = 0; q < 16 && c_tri[ci][q] >= 0; q += 3) {
+    for (int q = 0; q < 16 && d_mc.tri[ci][q] >= 0; q += 3) {
       int32_t vid[3];
       bool ok = true;
       for (int r = 0; r < 3; r++) {
         int64_t oi, oj, ok2;
         int slot;
-        edge_owner(edge_key(i, j, k, c_tri[ci][q + r]), &oi, &oj, &ok2, &slot);
+        edge_owner(edge_key(i, j, k, d_mc.tri[ci][q + r]), &oi, &oj, &ok2, &slot);
         if (!cube_in_range(g, oi, oj, ok2)) {
           ok = false;
           break;
@@ -421,46 +437,67 @@ __global__ void k_mc_adjoint(GridDev g, const double* __restrict__ f, double iso
   }
 }
 
-// Transpose of the field: one warp per atom over its cube of nodes.
-__global__ void k_field_adjoint(GridDev g, const double* __restrict__ atoms, int na, double B, int ng,
-                                const double* __restrict__ gfield, double* gatoms) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t a = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; a < na; a += warps) {
-    const double* at = atoms + 4 * a;
+// Transpose of the field for kFields node derivatives at once (of the volume, of the area, or both,
+// sharing the exponentials): one block per atom over its cube of nodes, eight lanes per row of the
+// cube (rows are some 40 nodes long), so that the index arithmetic of a node is an addition.  Bound
+// by the reads of the node derivatives, most of which are zero (the field matters next to the
+// surface only).  777 atoms at scale 2, per derivative: one warp per atom 408 us -> 59 us.
+constexpr int kAdjThreads = 256;
+template <int kFields>
+__global__ void __launch_bounds__(kAdjThreads) k_field_adjoint(GridDev g, const double* __restrict__ atoms, int na,
+                                                              double B, int ng, const double* __restrict__ gf0,
+                                                              const double* __restrict__ gf1, double* g0, double* g1) {
+  constexpr int kLanes = 8, kRows = kAdjThreads / kLanes;
+  __shared__ double s_part[kAdjThreads / 32][4 * kFields];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row0 = threadIdx.x / kLanes, in_row = threadIdx.x % kLanes;
+  for (int a = blockIdx.x; a < na; a += gridDim.x) {
+    const double* at = atoms + 4 * (int64_t)a;
     int lo[3], hi[3];
     atom_window(g, at, ng, lo, hi);
-    const int nxw = hi[0] - lo[0], nyw = hi[1] - lo[1], nzw = hi[2] - lo[2];
-    const int64_t tot = (nxw > 0 && nyw > 0 && nzw > 0) ? (int64_t)nxw * nyw * nzw : 0;
+    const int nyw = hi[1] - lo[1], nzw = hi[2] - lo[2];
+    const int rows = (nyw > 0 && nzw > 0) ? nyw * nzw : 0;
     const double r = at[3], r2 = r * r;
-    double gx = 0, gy = 0, gz = 0, gr = 0;
-    for (int64_t q = lane; q < tot; q += 32) {
-      const int i = lo[0] + (int)(q % nxw), j = lo[1] + (int)((q / nxw) % nyw), k = lo[2] + (int)(q / ((int64_t)nxw * nyw));
-      const double gf = gfield[nidx(g, i, j, k)];
-      if (gf == 0.0) continue;
-      const double px = (g.mn[0] + (double)i * g.side) - g.hside;
-      const double py = (g.mn[1] + (double)j * g.side) - g.hside;
-      const double pz = (g.mn[2] + (double)k * g.side) - g.hside;
-      const double dx = px - at[0], dy = py - at[1], dz = pz - at[2];
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      const double e = exp(B * (d2 / r2 - 1)) * B * gf;
-      gx += e * (-2.0 * dx / r2);
-      gy += e * (-2.0 * dy / r2);
-      gz += e * (-2.0 * dz / r2);
-      gr += e * (-2.0 * d2 / (r2 * r));
+    double sum[4 * kFields];
+#pragma unroll
+    for (int c = 0; c < 4 * kFields; c++) sum[c] = 0.0;
+    for (int row = row0; row < rows; row += kRows) {
+      const int kk = row / nyw;
+      const int j = lo[1] + (row - kk * nyw), k = lo[2] + kk;
+      const int64_t base = nidx(g, 0, j, k);
+      for (int i = lo[0] + in_row; i < hi[0]; i += kLanes) {
+        const double d0 = gf0[base + i], d1 = kFields > 1 ? gf1[base + i] : 0.0;
+        if (d0 == 0.0 && d1 == 0.0) continue;
+        const double px = (g.mn[0] + (double)i * g.side) - g.hside;
+        const double py = (g.mn[1] + (double)j * g.side) - g.hside;
+        const double pz = (g.mn[2] + (double)k * g.side) - g.hside;
+        const double dx = px - at[0], dy = py - at[1], dz = pz - at[2];
+        const double d2 = dx * dx + dy * dy + dz * dz;
+        const double ex = exp(B * (d2 / r2 - 1)) * B;
+        const double fx = -2.0 * dx / r2, fy = -2.0 * dy / r2, fz = -2.0 * dz / r2, fr = -2.0 * d2 / (r2 * r);
+#pragma unroll
+        for (int f = 0; f < kFields; f++) {
+          const double e = ex * (f ? d1 : d0);
+          if (e == 0.0) continue;
+          sum[4 * f] += e * fx;
+          sum[4 * f + 1] += e * fy;
+          sum[4 * f + 2] += e * fz;
+          sum[4 * f + 3] += e * fr;
+        }
+      }
     }
-    for (int o = 16; o; o >>= 1) {
-      gx += __shfl_xor_sync(0xffffffffu, gx, o);
-      gy += __shfl_xor_sync(0xffffffffu, gy, o);
-      gz += __shfl_xor_sync(0xffffffffu, gz, o);
-      gr += __shfl_xor_sync(0xffffffffu, gr, o);
+#pragma unroll
+    for (int c = 0; c < 4 * kFields; c++) {
+      for (int o = 16; o; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+      if (lane == 0) s_part[warp][c] = sum[c];
     }
-    if (lane == 0) {
-      gatoms[4 * a] += gx;
-      gatoms[4 * a + 1] += gy;
-      gatoms[4 * a + 2] += gz;
-      gatoms[4 * a + 3] += gr;
+    __syncthreads();
+    if (threadIdx.x < 4 * kFields) {
+      double t = 0.0;
+      for (int w = 0; w < kAdjThreads / 32; w++) t += s_part[w][threadIdx.x];
+      (threadIdx.x < 4 ? g0 : g1)[4 * (int64_t)a + (threadIdx.x & 3)] += t;
     }
+    __syncthreads();
   }
 }
 
@@ -472,35 +509,11 @@ int grid_for(int64_t n, int threads = 256) {
 
 }  // namespace
 
-cudaError_t blobby_init_tables() {
-  static bool done[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  int8_t tri[256][16];
-  int em[256];
-  static const int ec[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6}, {6, 7}, {7, 4},
-                                {0, 4}, {1, 5}, {2, 6}, {3, 7}};
-  for (int c = 0; c < 256; c++) {
-    const char* s = kNsMcCases[c];
-    int q = 0;
-    for (; s[q]; q++) tri[c][q] = (int8_t)(s[q] <= '9' ? s[q] - '0' : s[q] - 'a' + 10);
-    for (; q < 16; q++) tri[c][q] = -1;
-    int m = 0;
-    for (int e = 0; e < 12; e++)
-      if (((c >> ec[e][0]) & 1) != ((c >> ec[e][1]) & 1)) m |= 1 << e;
-    em[c] = m;
-  }
-  cudaError_t e = cudaMemcpyToSymbol(c_tri, tri, sizeof tri);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_edge_mask, em, sizeof em);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
-  return e;
-}
-
-cudaError_t launch_blobby_field(const GridDev& g, const double* atoms, int na, double B, int ng, double* field,
-                                cudaStream_t s) {
+cudaError_t launch_blobby_field(const GridDev& g, const double* atoms, int na, double B, int ng, int4* win,
+                                double* field, cudaStream_t s) {
+  if (na > 0) k_atom_windows<<<grid_for(na), 256, 0, s>>>(g, atoms, na, ng, win);
   const int64_t tiles = ((g.n[0] + kTX - 1) / kTX) * ((g.n[1] + kTY - 1) / kTY) * ((g.n[2] + kTZ - 1) / kTZ);
-  k_blobby_field<<<(unsigned)tiles, kFieldThreads, 0, s>>>(g, atoms, na, B, ng, field);
+  k_blobby_field<<<(unsigned)tiles, kFieldThreads, 0, s>>>(g, atoms, win, na, B, field);
   return cudaGetLastError();
 }
 
@@ -551,9 +564,9 @@ cudaError_t launch_tri_patches(const double* verts, const int32_t* tris, int64_t
   return cudaGetLastError();
 }
 
-cudaError_t launch_blobby_adjoint(const GridDev& g, const double* atoms, int na, double B, int ng, const double* field,
-                                  double iso, const BlobbyMeshDev& M, const double* gpatch, double* gvert_post,
-                                  double* gvert_pre, double* gfield, double* gatoms, cudaStream_t s) {
+cudaError_t launch_mesh_adjoint(const GridDev& g, const double* field, double iso, const BlobbyMeshDev& M,
+                                const double* gpatch, double* gvert_post, double* gvert_pre, double* gfield,
+                                cudaStream_t s) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(gvert_post, 0, 3 * std::max<int64_t>(M.nv, 1) * sizeof(double), s)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(gfield, 0, g.n[0] * g.n[1] * g.n[2] * sizeof(double), s)) != cudaSuccess) return e;
@@ -563,7 +576,15 @@ cudaError_t launch_blobby_adjoint(const GridDev& g, const double* atoms, int na,
     if (M.nt > 0) k_smooth_adjoint_tris<<<grid_for(M.nt), 256, 0, s>>>(M.tris, M.nt, M.inc_cnt, gvert_post, gvert_pre);
     k_mc_adjoint<<<grid_for(M.nv), 256, 0, s>>>(g, field, iso, M.vkey, gvert_pre, M.nv, gfield);
   }
-  if (na > 0) k_field_adjoint<<<grid_for((int64_t)na * 32), 256, 0, s>>>(g, atoms, na, B, ng, gfield, gatoms);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_field_adjoint(const GridDev& g, const double* atoms, int na, double B, int ng, const double* gf0,
+                                 const double* gf1, double* g0, double* g1, cudaStream_t s) {
+  if (na <= 0) return cudaSuccess;
+  const int blocks = grid_for((int64_t)na * kAdjThreads, kAdjThreads);
+  if (gf1) k_field_adjoint<2><<<blocks, kAdjThreads, 0, s>>>(g, atoms, na, B, ng, gf0, gf1, g0, g1);
+  else k_field_adjoint<1><<<blocks, kAdjThreads, 0, s>>>(g, atoms, na, B, ng, gf0, nullptr, g0, nullptr);
   return cudaGetLastError();
 }
 

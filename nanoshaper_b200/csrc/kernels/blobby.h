@@ -20,11 +20,10 @@ struct BlobbyMeshDev {
   const int32_t* inc_cnt;
 };
 
-cudaError_t blobby_init_tables();
 // field[(k ny + j) nx + i] = sum over atoms of exp(B (d^2 / r^2 - 1)) at (x_i, y_j, z_k) - hside,
-// each atom over its cube of +-ng nodes.
-cudaError_t launch_blobby_field(const GridDev& g, const double* atoms, int na, double B, int ng, double* field,
-                                cudaStream_t s);
+// each atom over its cube of +-ng nodes; win is scratch for 2 int4 per atom.
+cudaError_t launch_blobby_field(const GridDev& g, const double* atoms, int na, double B, int ng, int4* win,
+                                double* field, cudaStream_t s);
 // Marching cubes on the field over the cubes 1..n-2 of each axis (ncubes of them): per cube the
 // own-edge cut mask and the vertex and triangle counts; then vertices (numbered by vbase) and
 // triangles (numbered by tbase).
@@ -45,10 +44,13 @@ cudaError_t launch_smooth(const double* vin, int64_t nv, const int64_t* off, int
 cudaError_t launch_quantize(double* v, int64_t n, cudaStream_t s);
 cudaError_t launch_tri_patches(const double* verts, const int32_t* tris, int64_t nt, double* f64, int32_t* i32,
                                int32_t* patch_atoms, cudaStream_t s);
-// d L / d atoms (x, y, z, r; added to gatoms) from the per-triangle slots gpatch of a ray cast of
-// the unquantised mesh; gvert_post, gvert_pre (3 per vertex) and gfield (per node) are scratch.
-cudaError_t launch_blobby_adjoint(const GridDev& g, const double* atoms, int na, double B, int ng, const double* field,
-                                  double iso, const BlobbyMeshDev& M, const double* gpatch, double* gvert_post,
-                                  double* gvert_pre, double* gfield, double* gatoms, cudaStream_t s);
+// d L / d field (per node, written to gfield) from the per-triangle slots gpatch of a ray cast of the
+// unquantised mesh; gvert_post and gvert_pre (3 per vertex) are scratch.
+cudaError_t launch_mesh_adjoint(const GridDev& g, const double* field, double iso, const BlobbyMeshDev& M,
+                                const double* gpatch, double* gvert_post, double* gvert_pre, double* gfield,
+                                cudaStream_t s);
+// d L / d atoms (x, y, z, r; added to g0, and g1 when gf1 is given) from d L / d field.
+cudaError_t launch_field_adjoint(const GridDev& g, const double* atoms, int na, double B, int ng, const double* gf0,
+                                 const double* gf1, double* g0, double* g1, cudaStream_t s);
 
 }  // namespace nsg

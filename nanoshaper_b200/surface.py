@@ -811,12 +811,17 @@ class BlobbySurface(Surface):
         """(n_atoms, 4) derivative of dvol * volume + darea * area with respect to the atoms' x, y,
         z and radius, after a gradient-mode getSurf (and triangulateSurface when darea is nonzero)
         of a differentiable blobby surface."""
-        c = self._context().handle
+        gv, ga = self.atom_gradients(area=darea != 0.0)
+        return dvol * gv if ga is None else dvol * gv + darea * ga
+
+    def atom_gradients(self, area: bool = True) -> tuple[np.ndarray, np.ndarray | None]:
+        """(d volume / d atoms, d area / d atoms), each (n_atoms, 4), in one pass over the atoms."""
         n = len(self.built_from)
         gv = np.zeros((n, 4))
-        ga = np.zeros((n, 4)) if darea != 0.0 else None
-        N.check(N.lib().nsg_blobby_atom_grads(c, N.ptr(gv), None if ga is None else N.ptr(ga)), "blobby gradients")
-        return dvol * gv if ga is None else dvol * gv + darea * ga
+        ga = np.zeros((n, 4)) if area else None
+        N.check(N.lib().nsg_blobby_atom_grads(self._context().handle, N.ptr(gv), None if ga is None else N.ptr(ga)),
+                "blobby gradients")
+        return gv, ga
 
 
 class _pointers:
