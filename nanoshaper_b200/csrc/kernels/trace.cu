@@ -11,6 +11,8 @@
 // writes the status rows / insideness bits of its 32 rays cooperatively (coalesced rows, ballot
 // masks + atomicAnd on the 32x-packed bit grid).  The candidate set of a ray is the reference's:
 // pixel inside the patch window, inside the bounding box, inside the equatorial disc.
+#include <limits.h>
+
 #include "pipeline.h"
 #include "ray_math.cuh"
 #include "ray_math_mixed.cuh"
@@ -819,6 +821,24 @@ void launch_isect(const TraceCtx& C, const CandOut& co, const HitStore& hs, int 
   }
 }
 
+// rintp of a node position as an int (positions outside the range of int saturate, which the clamps
+// to the grid and to the bit array make the same): one conversion instead of a 64-bit one.
+__device__ __forceinline__ int node_pos(double x) { return __double2int_rd(x + 0.5); }
+
+// Transposes the 32 x 32 bits of a warp: lane l's bit b becomes lane b's bit l (five exchanges of
+// half blocks, against 32 ballots).
+__device__ __forceinline__ unsigned transpose_bits(unsigned x) {
+  const int lane = threadIdx.x & 31;
+  unsigned m = 0x0000ffffu;  // positions whose bit j is clear
+#pragma unroll
+  for (int j = 16; j; j >>= 1) {
+    const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
+    m ^= m << (j >> 1);
+  }
+  return x;
+}
+
 // One CTA per 32x4 ray tile: loads, sorts and pairs the hits of its rays and performs the
 // interval fill (status runs, insideness bits, pair store, volume).
 // kGrad: the hits carry their patches (sorted along), and every interval end adds its term of
@@ -849,6 +869,20 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
   const int64_t lrid = n * rs.nb + m;
   const int64_t rid = S.ray_base[C.set] + lrid;
   int hc = valid ? hs.cnt[rid] : 0;
+  const bool mc = ray_set_shifted(rs.set);
+  if (!__any_sync(0xffffffffu, hc > 0)) {
+    // rays beside the molecule (half of a globule's grid): empty rows
+    if (valid) {
+      C.out.vol_ray[rid] = 0.0;
+      if (mc) C.out.ray_pair_cnt[S.mc_base + rs.ordinal_base + lrid] = 0;
+      else if (rs.set == 0) C.out.srun_cnt[rid] = 0;
+      if (C.out.hits) {
+        C.out.ray_hit_off[rid] = 0;
+        C.out.ray_hit_cnt[rid] = 0;
+      }
+    }
+    return;
+  }
   bool ovf = hc > kHitCap;
   int nh = ovf ? 0 : hc;
   uint8_t* pcol = kGrad ? s_slot + tid : nullptr;
@@ -883,7 +917,6 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
     }
   }
   // interval ends
-  const bool mc = ray_set_shifted(rs.set);
   double pa_vc, dirl;
   if (rs.set == 0) {
     pa_vc = gcoord(g, 0, 0);
@@ -1005,18 +1038,28 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
     }
     return;
   }
-  // accurate-triangulation rays: pair store for the vertex assembly
+  // accurate-triangulation rays: pair store for the vertex assembly; in the ray's column the node
+  // positions a < v <= b that a pair covers take the place of its ends
+  const double vmin = g.mn[rs.vc];
+  const auto set_span = [&](int q, int a, int b) { col[(2 * q) * kThreads] = __hiloint2double(b, a); };
+  const auto span = [&](int q) {
+    const double w = col[(2 * q) * kThreads];
+    return make_int2(__double2loint(w), __double2hiint(w));
+  };
   {
     int64_t off = warp_append(C.out.pair_cursor, C.out.pair_cap, np, C.out.error_flag, 3);
     if (valid && !ovf) {
       int64_t ord = S.mc_base + rs.ordinal_base + lrid;
-      if (off >= 0) {
-        for (int q = 0; q < np; q++) {
-          C.out.pairs[2 * (off + q)] = col[(2 * q) * kThreads];
-          C.out.pairs[2 * (off + q) + 1] = col[(2 * q + 1) * kThreads];
+      for (int q = 0; q < np; q++) {
+        const double lim1 = col[(2 * q) * kThreads], lim2 = col[(2 * q + 1) * kThreads];
+        if (off >= 0) {
+          reinterpret_cast<double2*>(C.out.pairs)[off + q] = make_double2(lim1, lim2);
           if (kGrad)
             C.out.pair_pid[off + q] = make_int2(slot_pid(pcol[(2 * q) * kThreads]), slot_pid(pcol[(2 * q + 1) * kThreads]));
         }
+        set_span(q, node_pos((lim1 - vmin) * g.scale), node_pos((lim2 - vmin) * g.scale));
+      }
+      if (off >= 0) {
         C.out.ray_pair_off[ord] = off;
         C.out.ray_pair_cnt[ord] = np;
       } else {
@@ -1024,16 +1067,14 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
       }
     }
   }
-  const double vmin = g.mn[rs.vc];
   if (rs.panel == 0) {
     // row bits (i, j = m, k = n), i in (a, b]: every lane clears the runs of its own row
     if (valid && !ovf) {
       const int64_t f0 = (n * NY + m) * NX;
       const int64_t maxb = nwords * 32 - 1;
       for (int q = 0; q < np; q++) {
-        const int64_t a = (int64_t)rintp((col[(2 * q) * kThreads] - vmin) * g.scale);
-        const int64_t b = (int64_t)rintp((col[(2 * q + 1) * kThreads] - vmin) * g.scale);
-        int64_t lo = f0 + a + 1, hi = f0 + b;
+        const int2 ab = span(q);
+        int64_t lo = f0 + ab.x + 1, hi = f0 + ab.y;
         if (lo < 0) lo = 0;
         if (hi > maxb) hi = maxb;
         for (int64_t w = lo >> 5; w <= (hi >> 5) && hi >= lo; w++) {
@@ -1047,56 +1088,51 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
     }
     return;
   }
-  // panels 1 and 2: lanes are consecutive i; one ballot per position along the ray axis
-  int64_t first_a = INT64_MAX, last_b = INT64_MIN;
+  // panels 1 and 2: lanes are consecutive i; 32 positions along the ray axis at a time
+  int vlo = INT_MAX, vhi = INT_MIN;
   if (np > 0) {
-    first_a = (int64_t)rintp((col[0] - vmin) * g.scale) + 1;
-    last_b = (int64_t)rintp((col[(2 * np - 1) * kThreads] - vmin) * g.scale);
+    const int a0 = span(0).x;
+    vlo = a0 < INT_MAX ? a0 + 1 : a0;
+    vhi = span(np - 1).y;
   }
-  int64_t vlo = first_a, vhi = last_b;
-  for (int o = 16; o > 0; o >>= 1) {
-    long long ol = __shfl_xor_sync(0xffffffffu, (long long)vlo, o);
-    long long oh = __shfl_xor_sync(0xffffffffu, (long long)vhi, o);
-    vlo = ol < vlo ? ol : vlo;
-    vhi = oh > vhi ? oh : vhi;
-  }
+  vlo = __reduce_min_sync(0xffffffffu, vlo);
+  vhi = __reduce_max_sync(0xffffffffu, vhi);
+  // far outside any grid; keeps the steps below from overflowing
+  if (vlo < -(1 << 30)) vlo = -(1 << 30);
+  if (vhi > (1 << 30)) vhi = 1 << 30;
   if (vlo > vhi) return;
-  // 32 positions at a time: every lane builds the 32-bit membership word of its ray over
-  // [v0, v0 + 31] from its intervals, 32 ballots transpose the words so that lane l holds the mask
-  // of the 32 rays at position v0 + l, and the lanes clear their rows' bits in parallel
-  int q = 0;
-  int64_t qa = 0, qb = -1;
+  // every lane builds the 32-bit membership word of its ray over [v0, v0 + 31] from its intervals;
+  // transposed, lane l holds the mask of the 32 rays at position v0 + l, and the lanes clear their
+  // rows' bits in parallel
+  int q = 0, qa = 0, qb = -1;
   if (np > 0) {
-    qa = (int64_t)rintp((col[0] - vmin) * g.scale);
-    qb = (int64_t)rintp((col[kThreads] - vmin) * g.scale);
+    const int2 ab = span(0);
+    qa = ab.x;
+    qb = ab.y;
   }
   const int64_t m0 = tm * kTileM;
-  for (int64_t v0 = vlo; v0 <= vhi; v0 += 32) {
-    const int64_t v1 = v0 + 31;
+  for (int v0 = vlo; v0 <= vhi; v0 += 32) {
+    const int v1 = v0 + 31;
     unsigned mem = 0;
     while (q < np && qa < v1) {
       // positions qa < v <= qb of the current interval that fall in [v0, v1]
-      const int64_t lo = qa + 1 > v0 ? qa + 1 : v0, hi = qb < v1 ? qb : v1;
+      const int lo = qa + 1 > v0 ? qa + 1 : v0, hi = qb < v1 ? qb : v1;
       if (lo <= hi) {
-        const int s0 = (int)(lo - v0), s1 = (int)(hi - v0);
+        const int s0 = lo - v0, s1 = hi - v0;
         mem |= (s1 - s0 == 31) ? 0xffffffffu : (((1u << (s1 - s0 + 1)) - 1u) << s0);
       }
       if (qb > v1) break;  // the interval continues in the next window
       q++;
       if (q < np) {
-        qa = (int64_t)rintp((col[(2 * q) * kThreads] - vmin) * g.scale);
-        qb = (int64_t)rintp((col[(2 * q + 1) * kThreads] - vmin) * g.scale);
+        const int2 ab = span(q);
+        qa = ab.x;
+        qb = ab.y;
       }
     }
-    unsigned mask = 0;
-#pragma unroll
-    for (int b = 0; b < 32; b++) {
-      const unsigned mb = __ballot_sync(0xffffffffu, (mem >> b) & 1u);
-      if (lane == b) mask = mb;
-    }
-    const int64_t v = v0 + lane;
+    const unsigned mask = transpose_bits(mem);
+    const int v = v0 + lane;
     if (mask && v <= vhi) {
-      const int64_t f0 = (rs.panel == 1) ? ((v * NY + n) * NX + m0) : ((n * NY + v) * NX + m0);
+      const int64_t f0 = (rs.panel == 1) ? (((int64_t)v * NY + n) * NX + m0) : ((n * NY + v) * NX + m0);
       if (f0 >= 0) {
         const int64_t w = f0 >> 5;
         const int sh = (int)(f0 & 31);
