@@ -142,8 +142,8 @@ struct DevBuf {
   }
 };
 
-// Streams of destroyed contexts, kept for the next ones (seven a context, 0.9 ms to make and
-// destroy); at most kStreamsKept, waited for before they come here.
+// Streams of destroyed contexts, kept for the next ones (0.13 ms to make and destroy); at most
+// kStreamsKept, waited for before they come here.
 constexpr size_t kStreamsKept = 64;
 struct StreamPool {
   std::mutex mu;
@@ -269,13 +269,10 @@ struct nsg_ctx {
   DevBuf tile_cnt[3], tile_off[3], tile_list[3], win_sums, screen;
   int64_t win_area[3] = {0, 0, 0}, torus_area[3] = {0, 0, 0};
   // wavefront tracing: candidate lists and the slot-major hit store
-  // per ray set (slot s when the ray sets run on their own streams, slot 0 otherwise)
-  DevBuf cand_sph[nsg::kRaySets], cand_tor[nsg::kRaySets], hit_t[nsg::kRaySets], hit_cnt[nsg::kRaySets],
-      cand_scr[nsg::kRaySets], def_sph[nsg::kRaySets], def_tor[nsg::kRaySets], hit_pid[nsg::kRaySets], tsplit_a[nsg::kRaySets],
-      tsplit_b[nsg::kRaySets];
-  bool concurrent_sets = true;
-  cudaStream_t set_stream[nsg::kRaySets] = {};
-  cudaEvent_t fork_ev = nullptr, join_ev[nsg::kRaySets] = {};
+  // per ray set (slot s when the sets share their launches, slot 0 when they run one after another)
+  DevBuf cand_sph[nsg::kRaySets], cand_tor[nsg::kRaySets], hit_t[nsg::kRaySets], hit_cnt, cand_scr[nsg::kRaySets],
+      def_sph[nsg::kRaySets], def_tor[nsg::kRaySets], hit_pid[nsg::kRaySets];
+  bool concurrent_sets = true;  // the ray sets in the same launches
   // gradient mode: hit / pair / vertex patches and the per-patch derivatives of volume and area
   DevBuf pair_pid, ovf_pscratch, gvol, garea, vpid, vgrad;
   // atoms behind the patches (for the device chain rule) and the atom derivatives
@@ -284,7 +281,7 @@ struct nsg_ctx {
   int64_t n_atoms = 0;
   bool have_atoms = false;
   bool grad_mode = false, have_gvol = false, have_garea = false, have_pids = false;
-  int64_t cand_cap = 0, scr_cap = 0, def_cap = 0;
+  int64_t sph_cap = 0, tor_cap = 0, def_cap = 0;
   // trace outputs
   DevBuf status, bits, vol_ray[nsg::kRaySets], epsmap;
   DevBuf pairs, ray_pair_off, ray_pair_cnt, cursors, ovf_rays[nsg::kRaySets], ovf_scratch;
@@ -657,9 +654,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   if (!c) return NSG_ERR_ARG;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (int i = 0; i < nsg::kRaySets; i++)
-    if (c->set_stream[i]) cudaStreamSynchronize(c->set_stream[i]);
-  DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield[0], &c->b_gfield[1], &c->b_gatoms, &c->b_win, &c->counters, &c->win_sums, &c->screen,
+  DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield[0], &c->b_gfield[1], &c->b_gatoms, &c->b_win, &c->counters, &c->win_sums, &c->screen, &c->hit_cnt,
                     &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_node, &c->bgp_ibgp, &c->bgp_type,
                     &c->bgp_pos, &c->bgp_nor, &c->bgp_flag, &c->bgp_n, &c->aux_cnt, &c->aux_off, &c->aux_list, &c->pairs,
                     &c->ray_pair_off, &c->ray_pair_cnt, &c->cursors, &c->ovf_scratch, &c->hits,
@@ -678,10 +673,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   for (int i = 0; i < nsg::kRaySets; i++) {
     c->vol_ray[i].release(true); c->ovf_rays[i].release(true); c->ray_hit_off[i].release(true); c->ray_hit_cnt[i].release(true);
     c->cand_sph[i].release(true); c->cand_tor[i].release(true); c->cand_scr[i].release(true); c->def_sph[i].release(true); c->def_tor[i].release(true);
-    c->hit_t[i].release(true); c->hit_cnt[i].release(true); c->hit_pid[i].release(true);
-    c->tsplit_a[i].release(true); c->tsplit_b[i].release(true);
-    if (c->set_stream[i]) give_stream(c->device, c->set_stream[i]);
-    if (c->join_ev[i]) cudaEventDestroy(c->join_ev[i]);
+    c->hit_t[i].release(true); c->hit_pid[i].release(true);
   }
   for (int i = 0; i < 8; i++)
     if (c->user_ev[i]) cudaEventDestroy(c->user_ev[i]);
@@ -690,7 +682,6 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   for (int i = 0; i < nsg::kRaySets; i++)
     for (int q = 0; q < 4; q++)
       if (c->sub_ev[i][q]) cudaEventDestroy(c->sub_ev[i][q]);
-  if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->own_stream && c->stream) give_stream(c->device, c->stream);
   delete c;
   return NSG_OK;
@@ -1318,23 +1309,29 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   const size_t read_bytes = (64 + (size_t)nb) * sizeof(unsigned long long);
   CK(c->cursors.ensure(read_bytes));
   CK(c->h_read.ensure(read_bytes));
-  // the ray sets run on their own streams (each with its own candidate lists and hit store) so
-  // that the double-precision intersection launches of one set overlap the integer-bound candidate
-  // and fill launches of another; or, with concurrent_sets off, one after another on the context's
-  // stream through slot 0
+  // the ray sets share their launches (each with its own candidate lists and hit store), so that a
+  // small cast makes a quarter of the launches and a large one has no tails between the sets; or,
+  // with concurrent_sets off, they run one after another through slot 0
   const bool conc = c->concurrent_sets && (do_mc ? 3 : 0) + ((do_status || do_eps) ? 1 : 0) + (do_eps ? 2 : 0) > 1;
-  // torus candidates split by resolvent branch (SES patch sets)
-  const bool split = c->tune.torus_split && (c->kind_mask & nsg::kSesKinds);
   const auto slot_of = [&](int set) { return conc ? set : 0; };
   // The torus candidates of a set are screened where the windows hold 2^16 and more: below, the solve
   // of all of them takes as long as a launch does (327 atoms: 8 us either way, and 7 for the screen;
   // 2,000 atoms, 2^17: 18 us without, 15 with)
   const auto screened = [&](int set) { return c->torus_area[nsg::ray_set_panel(set)] >= (1 << 16); };
+  int64_t area_max = 0;  // candidates of a set, spheres or tori, at most
   {
-    int64_t amax = std::max(c->win_area[0], std::max(c->win_area[1], c->win_area[2]));
-    c->cand_cap = std::max<int64_t>(c->cand_cap, amax + 1024);
-    c->scr_cap = std::max<int64_t>(
-        c->scr_cap, std::max(c->torus_area[0], std::max(c->torus_area[1], c->torus_area[2])) + 1024);
+    int64_t sph = 0, tor = 0;
+    for (int panel = 0; panel < 3; panel++) {
+      sph = std::max(sph, c->win_area[panel] - c->torus_area[panel]);
+      tor = std::max(tor, c->torus_area[panel]);
+    }
+    area_max = std::max(sph, tor);
+    c->sph_cap = std::max<int64_t>(c->sph_cap, sph + 1024);
+    c->tor_cap = std::max<int64_t>(c->tor_cap, tor + 1024);
+  }
+  // hit counts of all slots in one array, cleared together
+  int64_t cnt_off[nsg::kRaySets] = {0}, cnt_tot = 0;
+  {
     int64_t nr_all = 0;
     for (int set = 0; set < nsg::kRaySets; set++)
       if (cast(set)) nr_all = std::max(nr_all, c->rays_tot[set]);
@@ -1342,19 +1339,17 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       if (!cast(set)) continue;
       const int sl = slot_of(set);
       const int64_t nr = conc ? c->rays_tot[set] : nr_all;
+      if (conc) {
+        cnt_off[set] = cnt_tot;
+        cnt_tot += nr;
+      } else {
+        cnt_tot = nr;
+      }
       CK(c->hit_t[sl].ensure((size_t)nr * nsg::kHitCap * sizeof(double)));
-      CK(c->hit_cnt[sl].ensure(nr * sizeof(int32_t)));
       if (pids) CK(c->hit_pid[sl].ensure((size_t)nr * nsg::kHitCap * sizeof(int32_t)));
     }
+    CK(c->hit_cnt.ensure(std::max<int64_t>(cnt_tot, 1) * sizeof(int32_t)));
     if (grad) CK(c->gvol.ensure(std::max<int64_t>(c->np, 1) * NS_GRAD_PER_PATCH * sizeof(double)));
-    if (conc) {
-      if (!c->fork_ev) CK(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
-      for (int set = 0; set < nsg::kRaySets; set++) {
-        if (!cast(set)) continue;
-        if (!c->set_stream[set]) CK(take_stream(c->device, &c->set_stream[set]));
-        if (!c->join_ev[set]) CK(cudaEventCreateWithFlags(&c->join_ev[set], cudaEventDisableTiming));
-      }
-    }
   }
   CK(c->seg_part.ensure((size_t)nsg::kMaxSegArrays * nb * nsg::kSegParts * sizeof(double)));
   const int ovf_cap = 1 << 16;
@@ -1366,17 +1361,14 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     if (do_mc && pids) CK(c->pair_pid.ensure(c->pair_cap * sizeof(int2)));
     if (grad)
       CK(cudaMemsetAsync(c->gvol.p, 0, std::max<int64_t>(c->np, 1) * NS_GRAD_PER_PATCH * sizeof(double), c->stream));
-    if (precision == NSG_PRECISION_MIXED) c->def_cap = std::max<int64_t>(c->def_cap, c->cand_cap / 16 + (1 << 16));
+    if (precision == NSG_PRECISION_MIXED)
+      c->def_cap = std::max<int64_t>(c->def_cap, std::max(c->sph_cap, c->tor_cap) / 16 + (1 << 16));
     for (int set = 0; set < nsg::kRaySets; set++) {
       if (!cast(set)) continue;
       const int sl = slot_of(set);
-      CK(c->cand_sph[sl].ensure(c->cand_cap * sizeof(int2)));
-      CK(c->cand_tor[sl].ensure(c->cand_cap * sizeof(int2)));
-      if (screened(set)) CK(c->cand_scr[sl].ensure(c->scr_cap * sizeof(int2)));
-      if (split) {
-        CK(c->tsplit_a[sl].ensure(c->cand_cap * sizeof(int2)));
-        CK(c->tsplit_b[sl].ensure(c->cand_cap * sizeof(int2)));
-      }
+      CK(c->cand_sph[sl].ensure(c->sph_cap * sizeof(int2)));
+      CK(c->cand_tor[sl].ensure(c->tor_cap * sizeof(int2)));
+      if (screened(set)) CK(c->cand_scr[sl].ensure(c->tor_cap * sizeof(int2)));
       if (precision == NSG_PRECISION_MIXED) {
         CK(c->def_sph[sl].ensure(c->def_cap * sizeof(int2)));
         CK(c->def_tor[sl].ensure(c->def_cap * sizeof(int2)));
@@ -1395,13 +1387,15 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     if (do_mc) CK(cudaMemsetAsync(c->bits.p, 0xff, nwords * sizeof(uint32_t), c->stream));
     // cursors: 0 pairs, 1 kept hits, 2 status runs, 4..6 the overflow counts of the six ray sets
     // (int32), 8 + 2 s the candidate counts of set s (spheres, tori), 20 + 2 s its deferred counts,
-    // 32 + 4 s its split torus counts (at +1 and +3), 56 + s its screened torus count, 63 the error flag
+    // 56 + s its screened torus count, 63 the error flag
     unsigned long long* cur = c->cursors.as<unsigned long long>();
     int32_t* ovf_count = (int32_t*)(cur + 4);
     int sets[nsg::kRaySets], nsets = 0;
     for (int set = 0; set < nsg::kRaySets; set++)
       if (cast(set)) sets[nsets++] = set;
-    nsg::TraceOut outs[nsg::kRaySets];
+    nsg::TraceSets T{};
+    T.P = P;
+    T.B = B;
     if (do_eps) {
       const size_t eb = (size_t)c->grid.nx * c->grid.ny * c->grid.nz * 3 * sizeof(int32_t);
       CK(c->epsmap.ensure(eb));
@@ -1411,17 +1405,9 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       CK(c->counters.ensure(8 * sizeof(unsigned long long)));
       CK(cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
     }
-    stage_begin(c, kStageTrace);
-    if (conc) CK(cudaEventRecord(c->fork_ev, c->stream));
     for (int si = 0; si < nsets; si++) {
-      int s = sets[si];
-      cudaStream_t st = c->stream;
-      if (conc) {
-        st = c->set_stream[s];
-        CK(cudaStreamWaitEvent(st, c->fork_ev, 0));
-      }
-      int panel = nsg::ray_set_panel(s);
-      int64_t nr = c->rays_tot[s];
+      const int s = sets[si];
+      const int64_t nr = c->rays_tot[s];
       CK(c->vol_ray[s].ensure(nr * sizeof(double)));
       CK(c->ovf_rays[s].ensure(ovf_cap * sizeof(int32_t)));
       nsg::TraceOut o{};
@@ -1454,47 +1440,57 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       if (keep_hits) {
         CK(c->ray_hit_off[s].ensure(nr * sizeof(int64_t)));
         CK(c->ray_hit_cnt[s].ensure(nr * sizeof(int32_t)));
-        CK(cudaMemsetAsync(c->ray_hit_cnt[s].p, 0, nr * sizeof(int32_t), st));
+        CK(cudaMemsetAsync(c->ray_hit_cnt[s].p, 0, nr * sizeof(int32_t), c->stream));
         o.hits = c->hits.as<double>();
         o.hit_cap = c->hit_cap;
         o.hit_cursor = cur + 1;
         o.ray_hit_off = c->ray_hit_off[s].as<int64_t>();
         o.ray_hit_cnt = c->ray_hit_cnt[s].as<int32_t>();
       }
-      outs[s] = o;
       const int sl = slot_of(s);
-      nsg::CandOut co{c->cand_sph[sl].as<int2>(), c->cand_tor[sl].as<int2>(), c->cand_cap, cur + 8 + 2 * s,
-                      c->def_sph[sl].as<int2>(), c->def_tor[sl].as<int2>(), c->def_cap, cur + 20 + 2 * s,
-                      screened(s) ? c->cand_scr[sl].as<int2>() : nullptr, c->scr_cap, cur + 55 + s,
-                      split ? c->tsplit_a[sl].as<int2>() : nullptr, split ? c->tsplit_b[sl].as<int2>() : nullptr,
-                      split ? cur + 32 + 4 * s : nullptr};
-      nsg::HitStore hs{c->hit_t[sl].as<double>(), c->hit_cnt[sl].as<int32_t>(), nr,
-                       pids ? c->hit_pid[sl].as<int32_t>() : nullptr};
-      CK(cudaMemsetAsync(c->hit_cnt[sl].p, 0, nr * sizeof(int32_t), st));
-      c->launches += precision == NSG_PRECISION_MIXED ? 6 : 4;
+      T.set[si] = s;
+      T.ntiles[si] = c->tiles_tot[nsg::ray_set_panel(s)];
+      T.out[si] = o;
+      T.co[si] = nsg::CandOut{c->cand_sph[sl].as<int2>(), c->cand_tor[sl].as<int2>(), c->sph_cap, c->tor_cap,
+                              cur + 8 + 2 * s, c->def_sph[sl].as<int2>(), c->def_tor[sl].as<int2>(), c->def_cap,
+                              cur + 20 + 2 * s, screened(s) ? c->cand_scr[sl].as<int2>() : nullptr, cur + 56 + s};
+      T.hs[si] = nsg::HitStore{c->hit_t[sl].as<double>(), c->hit_cnt.as<int32_t>() + cnt_off[s], nr,
+                               pids ? c->hit_pid[sl].as<int32_t>() : nullptr};
+    }
+    stage_begin(c, kStageTrace);
+    const auto one_set = [&](int si) {
+      nsg::TraceSets one = T;
+      one.n = 1;
+      one.set[0] = T.set[si];
+      one.ntiles[0] = T.ntiles[si];
+      one.out[0] = T.out[si];
+      one.co[0] = T.co[si];
+      one.hs[0] = T.hs[si];
+      return one;
+    };
+    const int groups = conc ? std::min(nsets, 1) : nsets;
+    for (int gi = 0; gi < groups; gi++) {
       cudaEvent_t* ev = nullptr;
       if (c->profile) {
         for (int q = 0; q < 4; q++)
-          if (!c->sub_ev[s][q]) CK(cudaEventCreate(&c->sub_ev[s][q]));
-        ev = c->sub_ev[s];
+          if (!c->sub_ev[gi][q]) CK(cudaEventCreate(&c->sub_ev[gi][q]));
+        ev = c->sub_ev[gi];
       }
-      CK(nsg::launch_trace(P, B, s, c->tiles_tot[panel], o, co, hs, precision, c->tune, st, ev));
-      if (conc) CK(cudaEventRecord(c->join_ev[s], st));
+      if (conc) T.n = nsets;
+      const nsg::TraceSets G = conc ? T : one_set(gi);
+      CK(cudaMemsetAsync(c->hit_cnt.p, 0, (conc ? cnt_tot : G.hs[0].nrays) * sizeof(int32_t), c->stream));
+      CK(nsg::launch_trace(G, precision, c->tune, area_max, c->stream, &c->launches, ev));
     }
-    if (conc)
-      for (int si = 0; si < nsets; si++) CK(cudaStreamWaitEvent(c->stream, c->join_ev[sets[si]], 0));
     stage_end(c, kStageTrace);
     if (c->profile) {
-      // candidate, intersection and fill kernels of every ray set (stage_end synchronised the stream)
-      for (int si = 0; si < nsets; si++) {
-        const int s = sets[si];
+      // candidate, intersection and fill kernels of every group (stage_end synchronised the stream)
+      for (int gi = 0; gi < groups; gi++)
         for (int q = 0; q < 3; q++) {
           float ms = 0;
-          CK(cudaEventElapsedTime(&ms, c->sub_ev[s][q], c->sub_ev[s][q + 1]));
+          CK(cudaEventElapsedTime(&ms, c->sub_ev[gi][q], c->sub_ev[gi][q + 1]));
           c->stage_ms[kStageCand + q] += ms;
           c->stage_calls[kStageCand + q]++;
         }
-      }
     }
     // volume: A * sum of interval lengths over the ray sets / number of ray sets, per structure; the
     // per-structure sums run in an order fixed by the structure alone, so a structure's volume does
@@ -1535,9 +1531,9 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
       }
       CK(c->ovf_scratch.ensure((size_t)n * nsg::kOverflowCap * sizeof(double)));
       if (pids) CK(c->ovf_pscratch.ensure((size_t)n * nsg::kOverflowCap * sizeof(int32_t)));
-      LAUNCH(nsg::launch_trace_overflow(P, B, s, c->tile_off[panel].as<int64_t>(), c->tile_list[panel].as<int32_t>(),
-                                        outs[s], n, c->ovf_scratch.as<double>(),
-                                        pids ? c->ovf_pscratch.as<int32_t>() : nullptr, precision, c->stream));
+      LAUNCH(nsg::launch_trace_overflow(one_set(si), c->tile_off[panel].as<int64_t>(), c->tile_list[panel].as<int32_t>(),
+                                        n, c->ovf_scratch.as<double>(), pids ? c->ovf_pscratch.as<int32_t>() : nullptr,
+                                        c->stream));
       CK(cudaStreamSynchronize(c->stream));
     }
     stage_end(c, kStageOverflow);
@@ -1568,7 +1564,7 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
     if (errflag == 3) { c->pair_cap = std::max<int64_t>(2 * c->pair_cap, (int64_t)used[0] + 1024); continue; }
     if (errflag == 2) { c->hit_cap = std::max<int64_t>(2 * c->hit_cap, (int64_t)used[1] + 1024); continue; }
     if (errflag == 5) { c->srun_cap = std::max<int64_t>(2 * c->srun_cap, (int64_t)used[2] + 1024); continue; }
-    if (errflag == 6) { c->cand_cap *= 2; c->scr_cap *= 2; continue; }
+    if (errflag == 6) { c->sph_cap *= 2; c->tor_cap *= 2; continue; }
     if (errflag == 7) { c->def_cap *= 2; continue; }
     return fail(NSG_ERR_CAPACITY, errflag == 1 ? "too many overflow rays" : "ray hit capacity exceeded");
   }

@@ -1,8 +1,7 @@
 // Ray-patch intersection kernels of the tracer, shared by two translation units:
 //  * trace.cu compiles them without contraction of products and sums (--fmad=false), so the
-//    double-precision path (k_isect<panel, torus, false>) rounds every operation as the host
-//    restatement does;
-//  * trace_mixed.cu compiles the mixed-precision instantiations (k_isect<panel, torus, true>)
+//    double-precision path (k_isect) rounds every operation as the host restatement does;
+//  * trace_mixed.cu compiles the mixed-precision instantiations (k_isect_mixed, k_isect_quad_mixed)
 //    with fused multiply-adds, which cut the double-precision instruction count of the torus
 //    quartic; that path is held to a tolerance, not to bit equality, and its near-degenerate
 //    decisions are deferred to the double-precision kernel by guards far wider than one rounding.
@@ -11,32 +10,48 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "pipeline.h"
 #include "ray_math.cuh"
 #include "ray_math_mixed.cuh"
 
 namespace nsg {
 
+// One ray set of a launch; the parts stay in the kernel's parameters.
 struct TraceCtx {
-  PatchDev P;
-  BatchDev B;
+  const PatchDev& P;
+  const BatchDev& B;
   int set;
-  TraceOut out;
+  const TraceOut& out;
 };
 
-// Mixed-precision intersection launches of one panel: the sphere candidate list of co
-// (trace_mixed.cu) and the torus list (trace_mixed_torus.cu, built without fused multiply-adds),
-// with the deferred candidates appended to co's deferred lists.
-template <int PN>
-void launch_isect_mixed_sphere(const TraceCtx& C, const CandOut& co, const HitStore& hs, const TuneParams& tp,
-                               cudaStream_t s);
-template <int PN>
-void launch_isect_mixed_torus(const TraceCtx& C, const CandOut& co, const HitStore& hs, const TuneParams& tp,
-                              cudaStream_t s);
-// Mixed-precision skin cell launch of one panel (trace_mixed.cu).
-template <int PN>
-void launch_isect_quad_mixed(const TraceCtx& C, const CandOut& co, const HitStore& hs, const TuneParams& tp,
-                             cudaStream_t s);
+// A candidate list of one set: the candidates of a kind, the screened tori where there are any, or
+// the deferred ones.
+struct CandList {
+  const int2* list;
+  int64_t n;
+};
+template <bool kTorus, bool kDeferred>
+__device__ __forceinline__ CandList cand_list(const CandOut& co) {
+  if (kDeferred) {
+    const int64_t n = co.dcount[kTorus ? 1 : 0];
+    return CandList{kTorus ? co.dtor : co.dsph, n < co.dcap ? n : co.dcap};
+  }
+  if (!kTorus) {
+    const int64_t n = co.count[0];
+    return CandList{co.sph, n < co.cap ? n : co.cap};
+  }
+  const int64_t n = co.scr ? *co.scr_count : co.count[1];
+  return CandList{co.scr ? co.scr : co.tor, n < co.tor_cap ? n : co.tor_cap};
+}
+
+// Mixed-precision intersection launches of all sets: the sphere candidates (trace_mixed.cu) and the
+// torus candidates (trace_mixed_torus.cu, built without fused multiply-adds), with the deferred
+// candidates appended to the deferred lists; skin cells and triangles (trace_mixed.cu).
+void launch_isect_mixed_sphere(const TraceSets& T, dim3 grid, int threads, cudaStream_t s);
+void launch_isect_mixed_torus(const TraceSets& T, dim3 grid, int threads, cudaStream_t s);
+void launch_isect_quad_mixed(const TraceSets& T, dim3 grid, int threads, cudaStream_t s);
 
 namespace {
 
@@ -202,12 +217,12 @@ __device__ __forceinline__ int intersect_mixed(const double* f, int kind, int fi
 }
 
 // One thread per candidate pair of one type: intersection, feasibility, hit filing.
-template <int PN, bool kTorus, bool kMixed>
+template <int PN, bool kTorus, bool kMixed, bool kDeferred>
 __device__ __forceinline__ void isect_body(const TraceCtx& C, const CandOut& co, const HitStore& hs) {
   constexpr int fd = Ax<PN>::fd, ld = Ax<PN>::ld, vc = Ax<PN>::vc;
-  const int64_t ncand = *(co.count + (kTorus ? 1 : 0));
-  const int2* list = kTorus ? co.tor : co.sph;
-  const int64_t nlim = ncand < co.cap ? ncand : co.cap;
+  const CandList cl = cand_list<kTorus, kDeferred>(co);
+  const int2* const list = cl.list;
+  const int64_t nlim = cl.n;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   // the next candidate of this thread is loaded one iteration ahead
@@ -406,12 +421,12 @@ __device__ __forceinline__ int intersect_tri_mixed(const double* f, const double
 
 // One thread per skin or triangle candidate (in the sphere list): intersection, feasibility, hit
 // filing.
-template <int PN, bool kMixed>
+template <int PN, bool kMixed, bool kDeferred>
 __device__ __forceinline__ void isect_quadric_body(const TraceCtx& C, const CandOut& co, const HitStore& hs) {
   constexpr int fd = Ax<PN>::fd, ld = Ax<PN>::ld, vc = Ax<PN>::vc;
-  const int64_t ncand = *co.count;
-  const int2* list = co.sph;
-  const int64_t nlim = ncand < co.cap ? ncand : co.cap;
+  const CandList cl = cand_list<false, kDeferred>(co);
+  const int2* const list = cl.list;
+  const int64_t nlim = cl.n;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nlim; c += stride) {
     const int2 e = list[c];
@@ -470,27 +485,43 @@ __device__ __forceinline__ void isect_quadric_body(const TraceCtx& C, const Cand
   }
 }
 
-template <int PN>
-__global__ void __launch_bounds__(256) k_isect_quad(TraceCtx C, CandOut co, HitStore hs) {
-  isect_quadric_body<PN, false>(C, co, hs);
+// The kernels run all ray sets of a group (grid y), each with its panel's axes compiled in.  The
+// double-precision kernels serve the FP64 path and the deferred lists of the mixed path; the
+// mixed-precision ones ask for enough blocks per SM to keep the sphere kernel, which waits on its
+// loads, and the torus kernel at full residency.
+template <class Body>
+__device__ __forceinline__ void per_panel(int set, Body body) {
+  const int panel = ray_set_panel(set);
+  if (panel == 0) body(std::integral_constant<int, 0>());
+  else if (panel == 1) body(std::integral_constant<int, 1>());
+  else body(std::integral_constant<int, 2>());
 }
 
-template <int PN>
-__global__ void __launch_bounds__(256, 4) k_isect_quad_mixed(TraceCtx C, CandOut co, HitStore hs) {
-  isect_quadric_body<PN, true>(C, co, hs);
+template <bool kDeferred>
+__global__ void __launch_bounds__(256) k_isect_quad(const __grid_constant__ TraceSets T) {
+  const int y = blockIdx.y;
+  const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
+  per_panel(C.set, [&](auto pn) { isect_quadric_body<decltype(pn)::value, false, kDeferred>(C, T.co[y], T.hs[y]); });
 }
 
-// The double-precision kernels (the FP64 path and the deferred lists of the mixed path) and the
-// mixed-precision ones; the latter ask for enough blocks per SM to keep the sphere kernel, which
-// waits on its loads, and the torus kernel at full residency.
-template <int PN, bool kTorus>
-__global__ void __launch_bounds__(256) k_isect(TraceCtx C, CandOut co, HitStore hs) {
-  isect_body<PN, kTorus, false>(C, co, hs);
+__global__ void __launch_bounds__(256, 4) k_isect_quad_mixed(const __grid_constant__ TraceSets T) {
+  const int y = blockIdx.y;
+  const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
+  per_panel(C.set, [&](auto pn) { isect_quadric_body<decltype(pn)::value, true, false>(C, T.co[y], T.hs[y]); });
 }
 
-template <int PN, bool kTorus>
-__global__ void __launch_bounds__(256, kTorus ? 3 : 6) k_isect_mixed(TraceCtx C, CandOut co, HitStore hs) {
-  isect_body<PN, kTorus, true>(C, co, hs);
+template <bool kTorus, bool kDeferred>
+__global__ void __launch_bounds__(256) k_isect(const __grid_constant__ TraceSets T) {
+  const int y = blockIdx.y;
+  const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
+  per_panel(C.set, [&](auto pn) { isect_body<decltype(pn)::value, kTorus, false, kDeferred>(C, T.co[y], T.hs[y]); });
+}
+
+template <bool kTorus>
+__global__ void __launch_bounds__(256, kTorus ? 3 : 6) k_isect_mixed(const __grid_constant__ TraceSets T) {
+  const int y = blockIdx.y;
+  const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
+  per_panel(C.set, [&](auto pn) { isect_body<decltype(pn)::value, kTorus, true, false>(C, T.co[y], T.hs[y]); });
 }
 
 }  // namespace

@@ -149,28 +149,22 @@ struct TraceOut {
 enum { kCntCandidates = 0, kCntTorus = 1, kCntFbSphere = 2, kCntFbQuartic = 3, kCntFbRoot = 4, kCntRecheck = 5,
        kCntN = 8 };
 
-// Candidate (ray, patch) pairs of one ray set, by patch type (0 spheres, 1 tori), and the
-// candidates the mixed-precision pass defers to the double-precision pass (same split).
+// Candidate (ray, patch) pairs of one ray set, by patch type (0 spheres, skin cells and triangles, 1
+// tori), and the candidates the mixed-precision pass defers to the double-precision pass (same
+// split).
 struct CandOut {
   int2* sph;
   int2* tor;
-  int64_t cap;
+  int64_t cap, tor_cap;
   unsigned long long* count;   // 2 counters
   int2* dsph;
   int2* dtor;
   int64_t dcap;
   unsigned long long* dcount;  // 2 counters
-  // torus candidates that pass the single-precision screen (torus_screen.h), of capacity scr_cap;
-  // their count at scr_count[1]
+  // torus candidates that pass the single-precision screen (torus_screen.h), of capacity tor_cap;
+  // null: not screened
   int2* scr;
-  int64_t scr_cap;
   unsigned long long* scr_count;
-  // torus candidates split by the branch their resolvent cubic takes (null: no split): the
-  // cube-root branch (and the rare approximate ones) in tsa, the arccos branch in tsb, each of
-  // capacity cap; counts at tscount[1] and tscount[3]
-  int2* tsa;
-  int2* tsb;
-  unsigned long long* tscount;
 };
 
 // Slot-major hit store of one ray set: hit i of ray r at t[i * nrays + r]; cnt[r] counts the
@@ -211,7 +205,7 @@ struct TuneParams {
   int isect_threads = 256;  // threads per block of the intersection kernels (64..256)
   int isect_bpsm = 16;      // their blocks per SM (grid = SMs * isect_bpsm, grid-stride)
   int cand_threads = 256;   // threads per block of the candidate kernel (one warp per patch)
-  int torus_split = 0;      // torus candidates solved in two launches, one per resolvent branch
+  int torus_split = 0;      // accepted and reported, without effect (candidates are screened instead)
   int mc_tris_bpsm = 3;     // blocks per SM of the marching-cubes triangle kernel (3 or 4)
 };
 
@@ -230,15 +224,25 @@ cudaError_t launch_pool32(const PatchDev& P, float4* pool32, float4* quad32, dou
 cudaError_t launch_bin_count(const PatchDev& P, const BatchDev& B, int set, int32_t* tile_cnt, cudaStream_t s);
 cudaError_t launch_bin_fill(const PatchDev& P, const BatchDev& B, int set, const int64_t* tile_off,
                             int32_t* tile_cursor, int32_t* tile_list, cudaStream_t s);
-// ev (optional, profiling): 4 events recorded before the candidate kernel and after the candidate,
-// intersection and fill kernels.
-cudaError_t launch_trace(const PatchDev& P, const BatchDev& B, int set, int64_t ntiles, const TraceOut& out,
-                         const CandOut& co, const HitStore& hs, int precision, const TuneParams& tp, cudaStream_t s,
-                         cudaEvent_t* ev = nullptr);
-// pscratch: patch column of the overflow hits (gradient mode), else null.
-cudaError_t launch_trace_overflow(const PatchDev& P, const BatchDev& B, int set, const int64_t* tile_off,
-                                  const int32_t* tile_list, const TraceOut& out, int n_ovf, double* scratch,
-                                  int32_t* pscratch, int precision, cudaStream_t s);
+// The ray sets of one group of launches: every launch covers all sets of the group (grid y).
+struct TraceSets {
+  PatchDev P;
+  BatchDev B;
+  int n;
+  int set[kRaySets];
+  int64_t ntiles[kRaySets];
+  TraceOut out[kRaySets];
+  CandOut co[kRaySets];
+  HitStore hs[kRaySets];
+};
+// area: bound of a set's candidates (sizes the grids); ev (optional, profiling): 4 events recorded
+// before the candidate kernel and after the candidate, intersection and fill kernels.  Returns the
+// launches made in *launches.
+cudaError_t launch_trace(const TraceSets& T, int precision, const TuneParams& tp, int64_t area, cudaStream_t s,
+                         int64_t* launches, cudaEvent_t* ev = nullptr);
+// pscratch: patch column of the overflow hits (gradient mode), else null.  T holds one set.
+cudaError_t launch_trace_overflow(const TraceSets& T, const int64_t* tile_off, const int32_t* tile_list, int n_ovf,
+                                  double* scratch, int32_t* pscratch, cudaStream_t s);
 
 // reduce.cu: out[b] = sum, over the arrays in order, of array q's segment [base[q][b],
 // base[q][b+1]) below index `limit`, each in a summation order fixed by the segment alone; part is scratch for

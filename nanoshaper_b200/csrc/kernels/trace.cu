@@ -460,7 +460,9 @@ constexpr uint32_t kCandRowAgain = 0xffffffffu;
 // launch, 32 patches per warp and binary searches in both passes -> as it is here: 26 -> 5.7 us
 // (327 atoms, scale 2), 46 -> 8.8 us (2,000, scale 3), 77 -> 25 us (20,000, scale 4), 194 -> 179 us
 // (64 conformers, 580,000 patches, whose warps filled the GPU before).
-__global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co, int ppw) {
+__global__ void __launch_bounds__(256) k_cand(const __grid_constant__ TraceSets T, int ppw) {
+  const TraceCtx C{T.P, T.B, T.set[blockIdx.y], T.out[blockIdx.y]};
+  const CandOut& co = T.co[blockIdx.y];
   __shared__ CandBatch s_batch[8];
   __shared__ uint32_t s_row[8][kCandRows];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co, int ppw) {
     if (lane == 0 && sum1) b1 = atomicAdd(co.count + 1, (unsigned long long)sum1);
     b0 = __shfl_sync(0xffffffffu, b0, 0);
     b1 = __shfl_sync(0xffffffffu, b1, 0);
-    if ((int64_t)(b0 + sum0) > co.cap || (int64_t)(b1 + sum1) > co.cap) {
+    if ((int64_t)(b0 + sum0) > co.cap || (int64_t)(b1 + sum1) > co.tor_cap) {
       if (lane == 0) atomicExch(C.out.error_flag, 6);
       __syncwarp();
       continue;
@@ -616,91 +618,6 @@ __global__ void __launch_bounds__(256) k_cand(TraceCtx C, CandOut co, int ppw) {
   }
 }
 
-// Branch class of a torus candidate, from the operations of the double-precision path up to the
-// resolvent cubic (ray_sphere_axis, torus_coeffs_f64, the head of quartic_f64 and of
-// real_cubic_f64, the same operations in the same order): -1 when the path returns no hit there
-// (no clipping-sphere hit, or no real quartic root), 1 for the resolvent's arccos branch, 0 for
-// the cube-root branch and the rare others.
-template <int PN>
-__device__ __forceinline__ int torus_class(const double* f, double probe, const double* pa, double ray_dir) {
-  constexpr int vc = Ax<PN>::vc;
-  double t0, t1;
-  if (!ray_sphere_axis<vc>(pa, ray_dir, f, f[kR], &t0, &t1)) return -1;
-  double orig1[3] = {pa[0], pa[1], pa[2]};
-  orig1[vc] += t0 * ray_dir;
-  double b, c, d, e;
-  torus_coeffs_f64(f, probe, vc, orig1, &b, &c, &d, &e);
-  const double b_2 = 0.5 * b;
-  const double b_4 = 0.25 * b;
-  const double p = c - 1.5 * (b_2 * b_2);
-  const double q = d + b_2 * (b_2 * b_2 - c);
-  const double r = e + b_4 * (b_4 * (c - 3.0 * b_4 * b_4) - d);
-  const double ff = p * p - 4. * r;
-  const double delta =
-      4. * ff * (4. * r * (p * p) - p * (q * q) - 16. * (r * r)) + (q * q) * (128. * p * r - 27. * (q * q));
-  if (e != 0. && (fabs(p) > 3.E+3 || fabs(r) > 3.E+3 || fabs(q) > 3.E+3 || fabs(delta) > 1.E+14)) return 0;
-  if (!(delta < 0. || (delta == 0. && (p >= 0. || ff < 0.))) && !((p < 0. && ff > 0.) || (delta == 0. && p == 0. && r == 0.)))
-    return -1;
-  // the resolvent cubic x^3 + cb x^2 + cc x + cd
-  const double cb = p, cc = 0.25 * (p * p) - r, cd = (-0.125) * (q * q);
-  if (fabs(cc) < cb * cb * 1.E-6 && fabs(cd) < fabs(cb) * 1.E-6) return 0;
-  if (fabs(cd / cc) < 4.E-4) return 0;
-  const double pc = -(1.0 / 3.0) * cb * cb + cc;
-  const double qc = (2. / 27.) * cb * cb * cb - (1. / 3.) * cb * cc + cd;
-  const double D3p = (1. / 27.) * pc * pc * pc;
-  const double D3 = D3p + 0.25 * qc * qc;
-  return D3 >= 0. ? 0 : 1;
-}
-
-// One thread per torus candidate: its branch class; candidates with no hit are dropped, the
-// others appended (warp-aggregated) to the list of their class, so that each solve launch runs
-// with the lanes of a warp on one branch of the solver.
-template <int PN>
-__global__ void __launch_bounds__(256) k_torus_split(TraceCtx C, CandOut co) {
-  constexpr int fd = Ax<PN>::fd, ld = Ax<PN>::ld, vc = Ax<PN>::vc;
-  const int64_t ncand = co.count[1];
-  const int64_t nlim = ncand < co.cap ? ncand : co.cap;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
-  const int64_t c0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31);
-  for (int64_t cb = c0; cb < nlim; cb += stride) {
-    const int64_t c = cb + lane;
-    int cls = -1;
-    int2 e = make_int2(0, 0);
-    if (c < nlim) {
-      e = co.tor[c];
-      const int64_t rid = e.x, pid = e.y;
-      const StructDev& S = C.B.s[C.B.patch_struct[pid]];
-      const GridDev& g = S.g;
-      const double delta = ray_set_shifted(C.set) ? NS_DELTA - g.hside : 0.0;
-      const int64_t nb = g.n[fd];
-      const int64_t lr = rid - S.ray_base[C.set];
-      const int64_t m = lr % nb, n = lr / nb;
-      double pa[3];
-      pa[fd] = gcoord(g, fd, m) + delta;
-      pa[ld] = gcoord(g, ld, n) + delta;
-      pa[vc] = gcoord(g, vc, 0) + delta;
-      double f[18];
-      const double* src = C.P.f64 + (int64_t)NS_PATCH_F64 * pid;
-#pragma unroll
-      for (int k = 0; k < 18; k++) f[k] = __ldg(src + k);
-      cls = torus_class<PN>(f, C.P.probe, pa, S.ray_dir[vc]);
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const unsigned m = __ballot_sync(0xffffffffu, cls == k);
-      if (!m) continue;
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(co.tscount + 1 + 2 * k, (unsigned long long)__popc(m));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (cls == k) {
-        const unsigned long long slot = base + __popc(m & ((1u << lane) - 1u));
-        (k == 0 ? co.tsa : co.tsb)[slot] = e;
-      }
-    }
-  }
-}
-
 // The torus candidates that may hit (torus_screen.h), in a list of their own, so that the quartic
 // solve runs on full warps of them.  A block takes tiles of 1,024 candidates, four per thread, keeps
 // their order within the tile (a patch's candidates stay together) and reserves their places with
@@ -709,13 +626,13 @@ __global__ void __launch_bounds__(256) k_torus_split(TraceCtx C, CandOut co) {
 // 18 -> 7 + 8 us.
 constexpr int kScreenThreads = 256, kScreenItems = 4, kScreenTile = kScreenThreads * kScreenItems;
 template <int PN>
-__global__ void __launch_bounds__(kScreenThreads) k_torus_screen(TraceCtx C, CandOut co) {
+__device__ __forceinline__ void torus_screen_body(const TraceCtx& C, const CandOut& co) {
   constexpr int fd = Ax<PN>::fd, ld = Ax<PN>::ld, vc = Ax<PN>::vc;
   __shared__ int s_cnt[kScreenItems * (kScreenThreads / 32)];
   __shared__ unsigned long long s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t ncand = co.count[1];
-  const int64_t nlim = ncand < co.cap ? ncand : co.cap;
+  const int64_t nlim = ncand < co.tor_cap ? ncand : co.tor_cap;
   for (int64_t tile = blockIdx.x * (int64_t)kScreenTile; tile < nlim; tile += (int64_t)gridDim.x * kScreenTile) {
     int2 e[kScreenItems];
     unsigned kept[kScreenItems];
@@ -759,7 +676,7 @@ __global__ void __launch_bounds__(kScreenThreads) k_torus_screen(TraceCtx C, Can
     if (warp == 0) {
       const int v = s_cnt[lane];  // 4 x 8 counts, in candidate order
       const int incl = warp_incl(v);
-      if (lane == 31) s_base = incl ? atomicAdd(co.scr_count + 1, (unsigned long long)incl) : 0;
+      if (lane == 31) s_base = incl ? atomicAdd(co.scr_count, (unsigned long long)incl) : 0;
       s_cnt[lane] = incl - v;
     }
     __syncthreads();
@@ -767,7 +684,7 @@ __global__ void __launch_bounds__(kScreenThreads) k_torus_screen(TraceCtx C, Can
     for (int q = 0; q < kScreenItems; q++)
       if ((kept[q] >> lane) & 1u) {
         const unsigned long long slot = s_base + s_cnt[q * (kScreenThreads / 32) + warp] + __popc(kept[q] & ((1u << lane) - 1u));
-        if ((int64_t)slot < co.scr_cap) co.scr[slot] = e[q];
+        if ((int64_t)slot < co.tor_cap) co.scr[slot] = e[q];
         else atomicExch(C.out.error_flag, 6);
       }
     __syncthreads();
@@ -775,49 +692,55 @@ __global__ void __launch_bounds__(kScreenThreads) k_torus_screen(TraceCtx C, Can
 }
 static_assert(kScreenItems * (kScreenThreads / 32) == 32, "one warp scans the tile's counts");
 
-template <int PN>
-void launch_isect(const TraceCtx& C, const CandOut& co, const HitStore& hs, int precision, const TuneParams& tp,
-                  cudaStream_t s) {
-  const int ig = sm_count() * tp.isect_bpsm, it = tp.isect_threads;
-  const bool ses = C.P.kind_mask & kSesKinds, skin = C.P.kind_mask & kBoxKinds;
-  // the torus candidates, split by resolvent branch into two lists solved one after the other
-  const bool split = tp.torus_split && co.tsa && co.tsb && co.tscount;
-  CandOut ca = co, cb = co;
-  if (ses && co.scr) {
-    k_torus_screen<PN><<<sm_count() * 8, kScreenThreads, 0, s>>>(C, co);
-    ca.tor = co.scr;
-    ca.cap = co.scr_cap;
-    ca.count = co.scr_count;
-  }
-  if (split) {
-    k_torus_split<PN><<<ig, 256, 0, s>>>(C, ca);
-    cb = ca;
-    ca.tor = co.tsa;
-    ca.count = co.tscount;
-    cb.tor = co.tsb;
-    cb.count = co.tscount + 2;
+__global__ void __launch_bounds__(kScreenThreads) k_torus_screen(const __grid_constant__ TraceSets T) {
+  const int y = blockIdx.y;
+  if (!T.co[y].scr) return;
+  const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
+  per_panel(C.set, [&](auto pn) { torus_screen_body<decltype(pn)::value>(C, T.co[y]); });
+}
+
+// Intersection launches of all sets of a group; the grids are sized for `area` candidates a set at
+// most, so that a small input does not launch thousands of empty blocks.
+void launch_isect(const TraceSets& T, int precision, const TuneParams& tp, int64_t area, cudaStream_t s,
+                  int64_t* launches) {
+  const bool ses = T.P.kind_mask & kSesKinds, box = T.P.kind_mask & kBoxKinds;
+  const auto blocks = [&](int64_t most, int64_t per) {
+    const int64_t b = (area + per - 1) / per;
+    return dim3((unsigned)(b < 1 ? 1 : (b < most ? b : most)), (unsigned)T.n);
+  };
+  const int it = tp.isect_threads;
+  const dim3 grid = blocks((int64_t)sm_count() * tp.isect_bpsm, it);
+  bool screen = false;
+  for (int q = 0; q < T.n; q++) screen = screen || T.co[q].scr;
+  if (ses && screen) {
+    k_torus_screen<<<blocks((int64_t)sm_count() * 8, kScreenTile), kScreenThreads, 0, s>>>(T);
+    ++*launches;
   }
   if (precision == 1) {
+    // the deferred candidates follow, in double precision (few: a small grid)
+    const dim3 few = blocks(sm_count(), 256);
     if (ses) {
-      launch_isect_mixed_sphere<PN>(C, co, hs, tp, s);
-      launch_isect_mixed_torus<PN>(C, ca, hs, tp, s);
-      if (split) launch_isect_mixed_torus<PN>(C, cb, hs, tp, s);
+      launch_isect_mixed_sphere(T, grid, it, s);
+      launch_isect_mixed_torus(T, grid, it, s);
+      k_isect<false, true><<<few, 256, 0, s>>>(T);
+      k_isect<true, true><<<few, 256, 0, s>>>(T);
+      *launches += 4;
     }
-    if (skin) launch_isect_quad_mixed<PN>(C, co, hs, tp, s);
-    // the deferred candidates, in double precision (few: a small grid)
-    const CandOut dco{co.dsph, co.dtor, co.dcap, co.dcount};
-    if (ses) {
-      k_isect<PN, false><<<sm_count(), 256, 0, s>>>(C, dco, hs);
-      k_isect<PN, true><<<sm_count(), 256, 0, s>>>(C, dco, hs);
+    if (box) {
+      launch_isect_quad_mixed(T, grid, it, s);
+      k_isect_quad<true><<<few, 256, 0, s>>>(T);
+      *launches += 2;
     }
-    if (skin) k_isect_quad<PN><<<sm_count(), 256, 0, s>>>(C, dco, hs);
   } else {
     if (ses) {
-      k_isect<PN, false><<<ig, it, 0, s>>>(C, co, hs);
-      k_isect<PN, true><<<ig, it, 0, s>>>(C, ca, hs);
-      if (split) k_isect<PN, true><<<ig, it, 0, s>>>(C, cb, hs);
+      k_isect<false, false><<<grid, it, 0, s>>>(T);
+      k_isect<true, false><<<grid, it, 0, s>>>(T);
+      *launches += 2;
     }
-    if (skin) k_isect_quad<PN><<<ig, it, 0, s>>>(C, co, hs);
+    if (box) {
+      k_isect_quad<false><<<grid, it, 0, s>>>(T);
+      ++*launches;
+    }
   }
 }
 
@@ -844,10 +767,13 @@ __device__ __forceinline__ unsigned transpose_bits(unsigned x) {
 // kGrad: the hits carry their patches (sorted along), and every interval end adds its term of
 // d volume / d patch parameters; the stored pairs keep their patches for the area adjoint.
 template <bool kGrad>
-__global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore hs) {
+__global__ void __launch_bounds__(kTraceThreads, 6) k_fill(const __grid_constant__ TraceSets T) {
   constexpr int kThreads = kTraceThreads;
-  const int panel = ray_set_panel(C.set);
   const int64_t tile = blockIdx.x;
+  if (tile >= T.ntiles[blockIdx.y]) return;
+  const TraceCtx C{T.P, T.B, T.set[blockIdx.y], T.out[blockIdx.y]};
+  const HitStore& hs = T.hs[blockIdx.y];
+  const int panel = ray_set_panel(C.set);
   const StructDev& S = C.B.s[find_struct(C.B.tile_base[panel], C.B.n, tile)];
   const GridDev g = S.g;
   const RaySet rs = make_ray_set(C.set, g);
@@ -1144,8 +1070,9 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_fill(TraceCtx C, HitStore 
 }
 
 // One thread per overflow ray: the same candidate tests with the hits kept in a global column.
-__global__ void k_trace_overflow(TraceCtx C, const int64_t* __restrict__ tile_off, const int32_t* __restrict__ tile_list,
-                                 int n_ovf, double* scratch, int32_t* pscratch) {
+__global__ void k_trace_overflow(const __grid_constant__ TraceSets T, const int64_t* __restrict__ tile_off,
+                                 const int32_t* __restrict__ tile_list, int n_ovf, double* scratch, int32_t* pscratch) {
+  const TraceCtx C{T.P, T.B, T.set[0], T.out[0]};
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_ovf) return;
   int64_t rid = C.out.ovf_rays[idx];
@@ -1312,43 +1239,43 @@ cudaError_t launch_bin_fill(const PatchDev& P, const BatchDev& B, int set, const
   return cudaGetLastError();
 }
 
-cudaError_t launch_trace(const PatchDev& P, const BatchDev& B, int set, int64_t ntiles, const TraceOut& out,
-                         const CandOut& co, const HitStore& hs, int precision, const TuneParams& tp, cudaStream_t s,
-                         cudaEvent_t* ev) {
-  if (ntiles <= 0) return cudaSuccess;
-  TraceCtx C{P, B, set, out};
-  const int panel = ray_set_panel(set);
+cudaError_t launch_trace(const TraceSets& T, int precision, const TuneParams& tp, int64_t area, cudaStream_t s,
+                         int64_t* launches, cudaEvent_t* ev) {
+  int64_t ntiles = 0;
+  bool pids = false;
+  for (int q = 0; q < T.n; q++) {
+    ntiles = T.ntiles[q] > ntiles ? T.ntiles[q] : ntiles;
+    pids = pids || T.hs[q].pid;
+  }
+  if (T.n <= 0 || ntiles <= 0) return cudaSuccess;
   if (ev) cudaEventRecord(ev[0], s);
-  if (P.n > 0) {
+  if (T.P.n > 0) {
     const int wpb = tp.cand_threads / 32;
-    // patches per warp: 32 where the set fills 16 warps per SM that way, fewer (down to 4) below
     // patches per warp: 32 where the set gives 64 warps per SM (a full SM) that way, fewer below,
     // but no fewer than 4, whose rows fill the 32 lanes (skin, 97,000 patches: 238 us with 32, 213
     // with 16 warps per SM as the line, 172 with 64)
-    const int64_t per = P.n / ((int64_t)sm_count() * 64);
+    const int64_t per = T.P.n / ((int64_t)sm_count() * 64);
     const int ppw = per < 4 ? 4 : (per > 32 ? 32 : (int)per);
-    int64_t blocks = (P.n + ppw * wpb - 1) / (ppw * wpb);
+    int64_t blocks = (T.P.n + ppw * wpb - 1) / (ppw * wpb);
     if (blocks > (int64_t)sm_count() * 64) blocks = (int64_t)sm_count() * 64;
-    k_cand<<<(unsigned)blocks, tp.cand_threads, 0, s>>>(C, co, ppw);
+    k_cand<<<dim3((unsigned)blocks, (unsigned)T.n), tp.cand_threads, 0, s>>>(T, ppw);
+    ++*launches;
   }
   if (ev) cudaEventRecord(ev[1], s);
-  if (panel == 0) launch_isect<0>(C, co, hs, precision, tp, s);
-  else if (panel == 1) launch_isect<1>(C, co, hs, precision, tp, s);
-  else launch_isect<2>(C, co, hs, precision, tp, s);
+  launch_isect(T, precision, tp, area, s, launches);
   if (ev) cudaEventRecord(ev[2], s);
-  if (hs.pid) k_fill<true><<<(unsigned)ntiles, kTraceThreads, 0, s>>>(C, hs);
-  else k_fill<false><<<(unsigned)ntiles, kTraceThreads, 0, s>>>(C, hs);
+  const dim3 grid((unsigned)ntiles, (unsigned)T.n);
+  if (pids) k_fill<true><<<grid, kTraceThreads, 0, s>>>(T);
+  else k_fill<false><<<grid, kTraceThreads, 0, s>>>(T);
+  ++*launches;
   if (ev) cudaEventRecord(ev[3], s);
   return cudaGetLastError();
 }
 
-cudaError_t launch_trace_overflow(const PatchDev& P, const BatchDev& B, int set, const int64_t* tile_off,
-                                  const int32_t* tile_list, const TraceOut& out, int n_ovf, double* scratch,
-                                  int32_t* pscratch, int precision, cudaStream_t s) {
-  (void)precision;
+cudaError_t launch_trace_overflow(const TraceSets& T, const int64_t* tile_off, const int32_t* tile_list, int n_ovf,
+                                  double* scratch, int32_t* pscratch, cudaStream_t s) {
   if (n_ovf <= 0) return cudaSuccess;
-  TraceCtx C{P, B, set, out};
-  k_trace_overflow<<<(n_ovf + 63) / 64, 64, 0, s>>>(C, tile_off, tile_list, n_ovf, scratch, pscratch);
+  k_trace_overflow<<<(n_ovf + 63) / 64, 64, 0, s>>>(T, tile_off, tile_list, n_ovf, scratch, pscratch);
   return cudaGetLastError();
 }
 

@@ -5,29 +5,12 @@
 
 namespace nsg {
 
-template <int PN>
-void launch_isect_mixed_sphere(const TraceCtx& C, const CandOut& co, const HitStore& hs, const TuneParams& tp,
-                               cudaStream_t s) {
-  k_isect_mixed<PN, false><<<sm_count() * tp.isect_bpsm, tp.isect_threads, 0, s>>>(C, co, hs);
+void launch_isect_mixed_sphere(const TraceSets& T, dim3 grid, int threads, cudaStream_t s) {
+  k_isect_mixed<false><<<grid, threads, 0, s>>>(T);
 }
 
-template <int PN>
-void launch_isect_quad_mixed(const TraceCtx& C, const CandOut& co, const HitStore& hs, const TuneParams& tp,
-                             cudaStream_t s) {
-  k_isect_quad_mixed<PN><<<sm_count() * tp.isect_bpsm, tp.isect_threads, 0, s>>>(C, co, hs);
+void launch_isect_quad_mixed(const TraceSets& T, dim3 grid, int threads, cudaStream_t s) {
+  k_isect_quad_mixed<<<grid, threads, 0, s>>>(T);
 }
-
-template void launch_isect_quad_mixed<0>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                         cudaStream_t);
-template void launch_isect_quad_mixed<1>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                         cudaStream_t);
-template void launch_isect_quad_mixed<2>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                         cudaStream_t);
-template void launch_isect_mixed_sphere<0>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                           cudaStream_t);
-template void launch_isect_mixed_sphere<1>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                           cudaStream_t);
-template void launch_isect_mixed_sphere<2>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                           cudaStream_t);
 
 }  // namespace nsg

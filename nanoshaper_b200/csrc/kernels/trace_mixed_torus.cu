@@ -6,17 +6,8 @@
 
 namespace nsg {
 
-template <int PN>
-void launch_isect_mixed_torus(const TraceCtx& C, const CandOut& co, const HitStore& hs, const TuneParams& tp,
-                              cudaStream_t s) {
-  k_isect_mixed<PN, true><<<sm_count() * tp.isect_bpsm, tp.isect_threads, 0, s>>>(C, co, hs);
+void launch_isect_mixed_torus(const TraceSets& T, dim3 grid, int threads, cudaStream_t s) {
+  k_isect_mixed<true><<<grid, threads, 0, s>>>(T);
 }
-
-template void launch_isect_mixed_torus<0>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                          cudaStream_t);
-template void launch_isect_mixed_torus<1>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                          cudaStream_t);
-template void launch_isect_mixed_torus<2>(const TraceCtx&, const CandOut&, const HitStore&, const TuneParams&,
-                                          cudaStream_t);
 
 }  // namespace nsg
