@@ -52,7 +52,7 @@ int fail(int code, const char* what, cudaError_t e = cudaSuccess) {
 // only when nothing on the device uses them: a block is freed after a device wait (as cudaFree
 // waits) or after its context's streams have been waited for, and handed out after the pool's own
 // stream, which orders frees and allocations, has been waited for.
-constexpr uint64_t kDevKept = (uint64_t)4 << 30;
+constexpr uint64_t kDevKept = (uint64_t)8 << 30;
 struct DevPool {
   std::mutex mu;
   cudaMemPool_t pool = nullptr;

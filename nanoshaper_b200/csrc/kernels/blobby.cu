@@ -352,33 +352,46 @@ __global__ void k_quantize(double* v, int64_t n) {
     v[i] = off_round_trip(v[i]);
 }
 
-__global__ void k_tri_patches(const double* __restrict__ verts, const int32_t* __restrict__ tris, int64_t nt,
-                              double* f64, int32_t* i32, int32_t* patch_atoms) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
-    double* r = f64 + (int64_t)NS_PATCH_F64 * t;
-    const double* p[3];
-    for (int q = 0; q < 3; q++) {
-      const int32_t v = tris[3 * t + q];
-      p[q] = verts + 3 * (int64_t)v;
-      patch_atoms[3 * t + q] = v;
-      for (int d = 0; d < 3; d++) r[3 * q + d] = p[q][d];
+// The triangles as patch records, one triangle per lane; the 160-byte records of a warp are put
+// together in shared memory and stored as one contiguous block (written lane by lane they are 20
+// scattered 8-byte stores each: 165 us for 340,000 triangles -> 43 us).
+constexpr int kTriThreads = 128;
+__global__ void __launch_bounds__(kTriThreads) k_tri_patches(const double* __restrict__ verts,
+                                                             const int32_t* __restrict__ tris, int64_t nt, double* f64,
+                                                             int32_t* i32, int32_t* patch_atoms) {
+  constexpr int kPad = NS_PATCH_F64 + 1;  // keeps the lanes' rows on different banks
+  __shared__ double s_rec[kTriThreads / 32][32 * kPad];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* const rec = s_rec[warp];
+  const int64_t stride = (int64_t)gridDim.x * kTriThreads;
+  for (int64_t t0 = blockIdx.x * (int64_t)kTriThreads + warp * 32; t0 < nt; t0 += stride) {
+    const int64_t t = t0 + lane;
+    const int count = nt - t0 < 32 ? (int)(nt - t0) : 32;
+    if (lane < count) {
+      double* r = rec + lane * kPad;
+      double p[3][3];
+      for (int q = 0; q < 3; q++) {
+        const int32_t v = tris[3 * t + q];
+        patch_atoms[3 * t + q] = v;
+        for (int d = 0; d < 3; d++) r[3 * q + d] = p[q][d] = verts[3 * (int64_t)v + d];
+      }
+      const double e1[3] = {p[1][0] - p[0][0], p[1][1] - p[0][1], p[1][2] - p[0][2]};
+      const double e2[3] = {p[2][0] - p[0][0], p[2][1] - p[0][1], p[2][2] - p[0][2]};
+      r[NS_TRI_N] = e1[1] * e2[2] - e1[2] * e2[1];
+      r[NS_TRI_N + 1] = e1[2] * e2[0] - e1[0] * e2[2];
+      r[NS_TRI_N + 2] = e1[0] * e2[1] - e1[1] * e2[0];
+      r[12] = 0.0;
+      r[13] = 0.0;
+      for (int d = 0; d < 3; d++) {
+        r[NS_SKIN_LO + d] = fmin(p[0][d], fmin(p[1][d], p[2][d]));
+        r[NS_SKIN_HI + d] = fmax(p[0][d], fmax(p[1][d], p[2][d]));
+      }
+      reinterpret_cast<int4*>(i32)[t] = make_int4(NS_MESH_TRI, 0, 0, 0);
     }
-    const double e1[3] = {p[1][0] - p[0][0], p[1][1] - p[0][1], p[1][2] - p[0][2]};
-    const double e2[3] = {p[2][0] - p[0][0], p[2][1] - p[0][1], p[2][2] - p[0][2]};
-    r[NS_TRI_N] = e1[1] * e2[2] - e1[2] * e2[1];
-    r[NS_TRI_N + 1] = e1[2] * e2[0] - e1[0] * e2[2];
-    r[NS_TRI_N + 2] = e1[0] * e2[1] - e1[1] * e2[0];
-    r[12] = 0.0;
-    r[13] = 0.0;
-    for (int d = 0; d < 3; d++) {
-      r[NS_SKIN_LO + d] = fmin(p[0][d], fmin(p[1][d], p[2][d]));
-      r[NS_SKIN_HI + d] = fmax(p[0][d], fmax(p[1][d], p[2][d]));
-    }
-    int32_t* ir = i32 + NS_PATCH_I32 * t;
-    ir[0] = NS_MESH_TRI;
-    ir[1] = 0;
-    ir[2] = 0;
-    ir[3] = 0;
+    __syncwarp();
+    double* dst = f64 + (int64_t)NS_PATCH_F64 * t0;
+    for (int k = lane; k < NS_PATCH_F64 * count; k += 32) dst[k] = rec[(k / NS_PATCH_F64) * kPad + k % NS_PATCH_F64];
+    __syncwarp();
   }
 }
 
@@ -560,7 +573,7 @@ cudaError_t launch_quantize(double* v, int64_t n, cudaStream_t s) {
 cudaError_t launch_tri_patches(const double* verts, const int32_t* tris, int64_t nt, double* f64, int32_t* i32,
                                int32_t* patch_atoms, cudaStream_t s) {
   if (nt <= 0) return cudaSuccess;
-  k_tri_patches<<<grid_for(nt), 256, 0, s>>>(verts, tris, nt, f64, i32, patch_atoms);
+  k_tri_patches<<<grid_for(nt, kTriThreads), kTriThreads, 0, s>>>(verts, tris, nt, f64, i32, patch_atoms);
   return cudaGetLastError();
 }
 

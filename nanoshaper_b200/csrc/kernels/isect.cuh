@@ -488,7 +488,9 @@ __device__ __forceinline__ void isect_quadric_body(const TraceCtx& C, const Cand
 // The kernels run all ray sets of a group (grid y), each with its panel's axes compiled in.  The
 // double-precision kernels serve the FP64 path and the deferred lists of the mixed path; the
 // mixed-precision ones ask for enough blocks per SM to keep the sphere kernel, which waits on its
-// loads, and the torus kernel at full residency.
+// loads, and the torus kernel at full residency.  Blocks per SM, the four sets of 20,000 atoms in
+// FP64: torus 91 us with the 96 registers it takes by itself (2 blocks), 74 with 3; spheres 132, 119
+// with 5; of 64 conformers, mixed: spheres 972 with 6, 1,505 with 8, tori 871 with 2, 660 with 3.
 template <class Body>
 __device__ __forceinline__ void per_panel(int set, Body body) {
   const int panel = ray_set_panel(set);
@@ -511,7 +513,7 @@ __global__ void __launch_bounds__(256, 4) k_isect_quad_mixed(const __grid_consta
 }
 
 template <bool kTorus, bool kDeferred>
-__global__ void __launch_bounds__(256) k_isect(const __grid_constant__ TraceSets T) {
+__global__ void __launch_bounds__(256, kTorus ? 3 : 5) k_isect(const __grid_constant__ TraceSets T) {
   const int y = blockIdx.y;
   const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
   per_panel(C.set, [&](auto pn) { isect_body<decltype(pn)::value, kTorus, false, kDeferred>(C, T.co[y], T.hs[y]); });

@@ -104,25 +104,43 @@ __global__ void __launch_bounds__(kWinThreads) k_windows(PatchDev P, int32_t* wi
   if (threadIdx.x == 6 && s_sum[6]) atomicOr(out + 6, s_sum[6]);
 }
 
+// Patch-local FP32 copies of the pool entries (and of the skin quadrics).  A warp takes 32 patches and
+// spreads their entries over its lanes, in pool order: consecutive patches' entries are neighbours,
+// so loads and stores are coalesced (a patch per lane: 110 us for 2.9 M entries -> 64 us).
 __global__ void k_pool32(PatchDev P, float4* out, float4* quad32, double4* quadl) {
-  int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= P.n) return;
-  const double* f = P.f64 + (int64_t)NS_PATCH_F64 * p;
-  const int32_t* ir = P.i32 + NS_PATCH_I32 * p;
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const bool valid = p < P.n;
+  const double* f = P.f64 + (int64_t)NS_PATCH_F64 * (valid ? p : 0);
+  const int32_t* ir = P.i32 + NS_PATCH_I32 * (valid ? p : 0);
   const int kind = ir[0];
   const bool skin = ns_is_skin(kind);
-  for (int q = ir[1]; q < ir[1] + ir[2]; q++) {
-    double4 w = P.pool[q];
-    if (kind == NS_POINT) {
-      out[q] = make_float4((float)(w.x - f[0]), (float)(w.y - f[1]), (float)(w.z - f[2]), (float)w.w);
-    } else {
-      // planes about the local origin; the skin's (partly unnormalised) planes are scaled to unit
-      // normals so that the FP32 value is a distance (the scale does not change a sign)
-      const double inv = skin ? 1.0 / sqrt(w.x * w.x + w.y * w.y + w.z * w.z) : 1.0;
-      out[q] = make_float4((float)(w.x * inv), (float)(w.y * inv), (float)(w.z * inv),
-                           (float)((w.w + (w.x * f[0] + w.y * f[1] + w.z * f[2])) * inv));
+  {
+    const int lane = threadIdx.x & 31;
+    const int cnt = valid ? ir[2] : 0, first = ir[1];
+    const double c0 = f[0], c1 = f[1], c2 = f[2];
+    const int incl = warp_incl(cnt);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int e0 = 0; e0 < total; e0 += 32) {
+      const int e = e0 + lane;
+      const int l = owner_lane(incl, e < total ? e : total - 1);
+      const int q = __shfl_sync(0xffffffffu, first, l) + (e - __shfl_sync(0xffffffffu, incl - cnt, l));
+      const int k = __shfl_sync(0xffffffffu, kind, l);
+      const double o0 = __shfl_sync(0xffffffffu, c0, l), o1 = __shfl_sync(0xffffffffu, c1, l),
+                   o2 = __shfl_sync(0xffffffffu, c2, l);
+      if (e >= total) continue;
+      const double4 w = P.pool[q];
+      if (k == NS_POINT) {
+        out[q] = make_float4((float)(w.x - o0), (float)(w.y - o1), (float)(w.z - o2), (float)w.w);
+      } else {
+        // planes about the local origin; the skin's (partly unnormalised) planes are scaled to unit
+        // normals so that the FP32 value is a distance (the scale does not change a sign)
+        const double inv = ns_is_skin(k) ? 1.0 / sqrt(w.x * w.x + w.y * w.y + w.z * w.z) : 1.0;
+        out[q] = make_float4((float)(w.x * inv), (float)(w.y * inv), (float)(w.z * inv),
+                             (float)((w.w + (w.x * o0 + w.y * o1 + w.z * o2)) * inv));
+      }
     }
   }
+  if (!valid) return;
   if (skin && quad32) {
     // the quadric about the local origin c: A, bl = A c + b, cl = f(c)
     const double* Q = f + NS_SKIN_Q;
@@ -622,8 +640,9 @@ __global__ void __launch_bounds__(256) k_cand(const __grid_constant__ TraceSets 
 // solve runs on full warps of them.  A block takes tiles of 1,024 candidates, four per thread, keeps
 // their order within the tile (a patch's candidates stay together) and reserves their places with
 // one atomic.  Torus stage of a ray set, all candidates -> screen + solve: 64 conformers (11 M
-// candidates, mixed) 1,170 -> 190 + 260 us, 20,000 atoms (FP64) 106 -> 21 + 27 us, 2,000 atoms
-// 18 -> 7 + 8 us.
+// candidates, mixed) 1,170 -> 135 + 165 us, 20,000 atoms (FP64) 106 -> 15 + 18 us, 2,000 atoms
+// 18 -> 4 + 5 us.  Six blocks per SM (40 registers): 540 us for the conformers' four sets, 661 with
+// the 64 registers it takes by itself.
 constexpr int kScreenThreads = 256, kScreenItems = 4, kScreenTile = kScreenThreads * kScreenItems;
 template <int PN>
 __device__ __forceinline__ void torus_screen_body(const TraceCtx& C, const CandOut& co) {
@@ -692,7 +711,7 @@ __device__ __forceinline__ void torus_screen_body(const TraceCtx& C, const CandO
 }
 static_assert(kScreenItems * (kScreenThreads / 32) == 32, "one warp scans the tile's counts");
 
-__global__ void __launch_bounds__(kScreenThreads) k_torus_screen(const __grid_constant__ TraceSets T) {
+__global__ void __launch_bounds__(kScreenThreads, 6) k_torus_screen(const __grid_constant__ TraceSets T) {
   const int y = blockIdx.y;
   if (!T.co[y].scr) return;
   const TraceCtx C{T.P, T.B, T.set[y], T.out[y]};
