@@ -300,9 +300,9 @@ struct nsg_ctx {
   bool cav_labels = false;     // cc_label_of holds the region labels of the last detection
   bool have_eps = false;     // the last ray cast built the epsilon maps
   bool eps_filled = false;   // cavity filling has been applied to them
-  // ideb map and boundary grid points (node index, ibgp, type, projection, projection flag), the
+  // ideb map and boundary grid points (ibgp, type, projection, projection flag), the
   // auxiliary grid of the projection
-  DevBuf ideb, bgp_node, bgp_ibgp, bgp_type, bgp_pos, bgp_nor, bgp_flag, bgp_n, aux_cnt, aux_off, aux_list;
+  DevBuf ideb, bgp_ibgp, bgp_type, bgp_pos, bgp_nor, bgp_flag, bgp_n, aux_cnt, aux_off, aux_list;
   int64_t n_bgp = 0, n_bgp_ext = 0;
   bool have_bgp = false, bgp_projected = false;
   // cavities
@@ -655,7 +655,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield[0], &c->b_gfield[1], &c->b_gatoms, &c->b_win, &c->counters, &c->win_sums, &c->screen, &c->hit_cnt,
-                    &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_node, &c->bgp_ibgp, &c->bgp_type,
+                    &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_ibgp, &c->bgp_type,
                     &c->bgp_pos, &c->bgp_nor, &c->bgp_flag, &c->bgp_n, &c->aux_cnt, &c->aux_off, &c->aux_list, &c->pairs,
                     &c->ray_pair_off, &c->ray_pair_cnt, &c->cursors, &c->ovf_scratch, &c->hits,
                     &c->pair_pid, &c->ovf_pscratch, &c->gvol, &c->garea, &c->vpid, &c->vgrad,
@@ -2337,41 +2337,35 @@ int nsg_bgp(nsg_ctx* c, int project, int32_t aux_max_dim, int64_t* n_bgp, int64_
   CK(cudaSetDevice(c->device));
   const NsGrid& g = c->grid;
   const int32_t* eps = c->epsmap.as<int32_t>();
-  CK(c->bgp_n.ensure(2 * sizeof(int64_t)));
-  int32_t* cnt_d = c->bgp_n.as<int32_t>();
-  size_t tb = 0;
-  CK(nsg::bgp_select(eps, g.nx, g.ny, g.nz, nullptr, cnt_d, nullptr, &tb, c->stream));
-  CK(c->temp.ensure(tb));
-  tb = c->temp.cap;
-  c->launches++;
-  CK(nsg::bgp_select(eps, g.nx, g.ny, g.nz, nullptr, cnt_d, c->temp.p, &tb, c->stream));
+  const int64_t nodes = g.nx * g.ny * g.nz;
+  const int64_t tickets = nsg::bgp_tickets(nodes);
+  // points, external points, error flag, ticket, look-back words; a sixteenth of the nodes are points
+  // at most on all but the smallest grids (2 % of a molecule's), and the pass runs again otherwise
+  const size_t bytes = (4 + (size_t)tickets) * sizeof(int64_t);
+  CK(c->bgp_n.ensure(bytes));
+  CK(c->h_read.ensure(4 * sizeof(int64_t)));
+  int64_t* blk = c->bgp_n.as<int64_t>();
+  int64_t cap = nodes / 16 + 4096;
   int32_t n = 0;
-  CK(cudaMemcpyAsync(&n, cnt_d, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  const size_t ncap = std::max<int32_t>(n, 1);
-  CK(c->bgp_node.ensure(ncap * sizeof(int32_t)));
-  CK(c->bgp_ibgp.ensure(3 * ncap * sizeof(int32_t)));
-  CK(c->bgp_type.ensure(ncap * sizeof(int32_t)));
-  tb = 0;
-  CK(nsg::bgp_select(eps, g.nx, g.ny, g.nz, c->bgp_node.as<int32_t>(), cnt_d, nullptr, &tb, c->stream));
-  CK(c->temp.ensure(tb));
-  tb = c->temp.cap;
-  c->launches++;
-  CK(nsg::bgp_select(eps, g.nx, g.ny, g.nz, c->bgp_node.as<int32_t>(), cnt_d, c->temp.p, &tb, c->stream));
-  LAUNCH(nsg::bgp_expand(eps, g.nx, g.ny, g.nz, c->bgp_node.as<int32_t>(), n, c->bgp_ibgp.as<int32_t>(),
-                         c->bgp_type.as<int32_t>(), c->stream));
   int64_t n_ext = 0;
-  if (n > 0) {
-    int64_t* ext_d = c->bgp_n.as<int64_t>() + 1;
-    tb = 0;
-    CK(nsg::sum_i32(c->bgp_type.as<int32_t>(), n, ext_d, nullptr, &tb, c->stream));
-    CK(c->temp.ensure(tb));
-    tb = c->temp.cap;
-    c->launches++;
-    CK(nsg::sum_i32(c->bgp_type.as<int32_t>(), n, ext_d, c->temp.p, &tb, c->stream));
-    CK(cudaMemcpyAsync(&n_ext, ext_d, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  for (int attempt = 0;; attempt++) {
+    CK(c->bgp_ibgp.ensure(3 * cap * sizeof(int32_t)));
+    CK(c->bgp_type.ensure(cap * sizeof(int32_t)));
+    CK(cudaMemsetAsync(blk, 0, bytes, c->stream));
+    const nsg::LookBack lb{(unsigned long long*)(blk + 4), (unsigned int*)(blk + 3), (int32_t*)(blk + 2)};
+    LAUNCH(nsg::bgp_points(eps, g.nx, g.ny, g.nz, c->bgp_ibgp.as<int32_t>(), c->bgp_type.as<int32_t>(), cap, blk, lb,
+                           c->stream));
+    CK(cudaMemcpyAsync(c->h_read.p, blk, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    const int64_t* got = c->h_read.as<int64_t>();
+    if ((int32_t)got[2]) return fail(NSG_ERR_TIMEOUT, "a look-back wait of the boundary grid points ran out");
+    n = (int32_t)got[0];
+    n_ext = got[1];
+    if (got[0] <= cap) break;
+    if (attempt) return fail(NSG_ERR_CAPACITY, "boundary grid point capacity did not settle");
+    cap = got[0];
   }
-  CK(cudaStreamSynchronize(c->stream));
+  const size_t ncap = std::max<int32_t>(n, 1);
   c->n_bgp = n;
   c->n_bgp_ext = n_ext;
   c->have_bgp = true;

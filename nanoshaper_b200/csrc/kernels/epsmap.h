@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "cavity.h"
+#include "lookback.cuh"
 #include "pipeline.h"
 
 namespace nsg {
@@ -18,17 +19,12 @@ cudaError_t eps_fill_cavities(const RunArgs& A, const uint8_t* fill_of, int32_t*
 // src/DelphiShared.cpp:990-997).
 cudaError_t ideb_write(const RunArgs& A, const uint8_t* fill_of, uint8_t* ideb, cudaStream_t s);
 
-// Boundary grid points (src/Surface.cpp:1488-1546): nodes with ix, iy, iz >= 1 whose six edge
-// codes are not all equal, in the reference's scan order (z outer, x inner), as linear node
-// indices (nodes == nullptr only counts them); pass temp == nullptr to query temp_bytes.
-cudaError_t bgp_select(const int32_t* eps, int64_t nx, int64_t ny, int64_t nz, int32_t* nodes, int32_t* count,
-                       void* temp, size_t* temp_bytes, cudaStream_t s);
-// Sum of n int32 (the external points: EXTERNAL_BGP is 1); pass temp == nullptr to query temp_bytes.
-cudaError_t sum_i32(const int32_t* in, int32_t n, int64_t* out, void* temp, size_t* temp_bytes, cudaStream_t s);
-// ibgp (3 per point: ix, iy, iz) and the type of every selected node: EXTERNAL_BGP when one of
-// the six codes is 0, else INTERNAL_BGP.
-cudaError_t bgp_expand(const int32_t* eps, int64_t nx, int64_t ny, int64_t nz, const int32_t* nodes, int32_t n,
-                       int32_t* ibgp, int32_t* type, cudaStream_t s);
+// Boundary grid points (nodes i, j, k >= 1 whose six edge codes differ, in node order): ibgp (3 per
+// point: ix, iy, iz) and type (EXTERNAL_BGP when one of the codes is 0), the first `cap` of them.
+// counts (2, zeroed by the caller): all points and the external ones; lb: bgp_tickets(nodes) words.
+int64_t bgp_tickets(int64_t nodes);
+cudaError_t bgp_points(const int32_t* eps, int64_t nx, int64_t ny, int64_t nz, int32_t* ibgp, int32_t* type, int64_t cap,
+                       int64_t* counts, const LookBack& lb, cudaStream_t s);
 
 // The SES auxiliary grid of the projection (ConnollySurface::buildAuxiliaryGrid,
 // src/ConnollySurface.cpp:3666-3900): n^3 cells, node i of an axis at min + i*side.

@@ -9,6 +9,8 @@ the contexts.
   every copy's mesh, volume and area equal the single run's bit for bit.
 * A triangulation of pockets, whose edges carry no analytic vertex, so that the first capacities do
   not suffice: triangle and vertex counts from the downloaded bits and the case table.
+* Boundary grid points of grids below one ticket and of lattices whose points exceed the first
+  capacity, against their definition in NumPy.
 * Contexts one after another, in threads at the same time, and after nsg_release_kept give the
   same results.
 """
@@ -73,6 +75,26 @@ def test_ticket_edges(nx, ny, nz, native_lib, oracle_mod):
         setattr(g, lo, -half)
         setattr(g, hi, half)
     _against_oracle(_surface(atoms, 2.0, grid=g), oracle_mod)
+
+
+@pytest.mark.parametrize("cells,scale", [(1, 2.0), (2, 2.0), (4, 1.0), (20, 1.0)])
+def test_boundary_points(cells, scale, native_lib):
+    """Spheres of 1.5 on a lattice of 3.6: most nodes have codes that differ, so that the largest
+    grid has more points than a sixteenth of its nodes and the pass runs a second time."""
+    c = 3.6 * np.stack(np.meshgrid(*[np.arange(cells)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    surf = _surface(np.concatenate([c, np.full((len(c), 1), 1.5)], 1), scale, 85.0, probe=0.3)
+    ds = surf.delphi
+    ds.buildEpsMap = True
+    surf.projBGP = True
+    surf.getSurf(True, False, 0.0)
+    e = ds.epsmap
+    codes = np.stack([e[1:, 1:, 1:, 0], e[1:, 1:, 1:, 1], e[1:, 1:, 1:, 2], e[1:, 1:, :-1, 0], e[1:, :-1, 1:, 1],
+                      e[:-1, 1:, 1:, 2]])
+    differ = (codes != codes[0]).any(0)
+    kji = np.argwhere(differ) + 1
+    assert np.array_equal(ds.ibgp, kji[:, ::-1])
+    assert np.array_equal(ds.bgp_type == 1, (codes == 0).any(0)[differ])
+    assert ds.nbgp > 0 and (ds.nbgp > e[..., 0].size / 16 + 4096) == (cells == 20)
 
 
 @pytest.mark.parametrize("copies,precision", [(1, "fp64"), (9, "mixed"), (70, "fp64")])
