@@ -1810,7 +1810,8 @@ int nsg_filter_cavities(nsg_ctx* c, double probe_radius, int modify_status, int6
   const int64_t nn = g.nx * g.ny * g.nz;
   const int ncav = c->ncav;
   CK(c->cav_label.ensure(nn * sizeof(int32_t)));
-  CK(c->sh_support.ensure(nn));
+  const size_t support_bytes = (((size_t)nn + 31) / 32 + 1) * sizeof(uint32_t);
+  CK(c->sh_support.ensure(support_bytes));
   CK(c->sh_removed[0].ensure(nn));
   CK(c->sh_removed[1].ensure(nn));
   CK(c->sh_later.ensure(nn));
@@ -1822,9 +1823,9 @@ int nsg_filter_cavities(nsg_ctx* c, double probe_radius, int modify_status, int6
   CK(cudaMemcpyAsync(c->cav_label.p, c->status.p, nn * sizeof(int32_t), cudaMemcpyDeviceToDevice, c->stream));
   CK(cudaMemcpyAsync(c->sh_filled.p, filled.data(), ncav, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemsetAsync(c->sh_nrem.p, 0, ncav * sizeof(unsigned long long), c->stream));
+  CK(cudaMemsetAsync(c->sh_support.p, 0, support_bytes, c->stream));
   // the passes write the flags of kept cavities' nodes only
-  for (DevBuf* f : {&c->sh_support, &c->sh_removed[0], &c->sh_removed[1], &c->sh_later})
-    CK(cudaMemsetAsync(f->p, 0, nn, c->stream));
+  for (DevBuf* f : {&c->sh_removed[0], &c->sh_removed[1], &c->sh_later}) CK(cudaMemsetAsync(f->p, 0, nn, c->stream));
   if (c->have_eps && !c->ideb_ready) {
     CK(c->ideb.ensure(nn));
     nsg::RunArgs R = run_args(c);
@@ -1845,7 +1846,7 @@ int nsg_filter_cavities(nsg_ctx* c, double probe_radius, int modify_status, int6
   A.r = probe_radius;
   A.filled = c->sh_filled.as<uint8_t>();
   A.mod_status = modify_status ? 1 : 0;
-  A.support = c->sh_support.as<uint8_t>();
+  A.support = c->sh_support.as<uint32_t>();
   A.later = c->sh_later.as<uint8_t>();
   A.changed = c->sh_changed.as<int32_t>();
   A.bits = c->have_bits ? c->bits.as<uint32_t>() : nullptr;

@@ -80,7 +80,7 @@ struct ShapeArgs {
   double mn[3], side, scale, r;
   const uint8_t* filled;        // per cavity: filled by the volume threshold (skipped)
   int mod_status;               // removed nodes become STATUS_POINT_INSIDE
-  uint8_t* support;             // per node
+  uint32_t* support;            // one bit per node, and a word more (read, not used)
   uint8_t* removed;             // per node, this pass
   const uint8_t* removed_prev;  // per node, the pass before; nullptr on the first pass
   uint8_t* later;               // per node: inside a support sphere of a later cavity

@@ -84,3 +84,32 @@ def test_shape_filter_modify_status(atoms_2000, native_lib, oracle_mod):
     np.testing.assert_array_equal(fl, fl_o)
     assert not np.isin(st, [-3, -2]).any()
     print(f"ses 2000 shape filter (status modified): {nrem.value} nodes removed")
+
+
+@pytest.mark.parametrize("scale,probe", [(2.0, 0.2), (3.0, 1.4), (3.0, 4.9), (4.0, 4.0), (4.1, 4.3)])
+def test_shape_filter_wide_probes(scale, probe, native_lib, oracle_mod):
+    """A hollow ball: search boxes of 3 to 39 nodes along a row, so below, at and above the 32
+    nodes that the cover pass reads at a time."""
+    k = np.arange(240)
+    z = 1.0 - (2.0 * k + 1.0) / len(k)
+    phi = np.pi * (3.0 - np.sqrt(5.0)) * k
+    rho = np.sqrt(1.0 - z * z)
+    atoms = np.column_stack([7.0 * rho * np.cos(phi), 7.0 * rho * np.sin(phi), 7.0 * z, np.full(len(k), 1.8)])
+    nb.reset_seed()
+    ds = nb.DelPhiShared(atoms, scale, 80.0)
+    surf = nb.surfaceFactory().create(nb.ConfigFile(text="Surface = ses\nProbe_Radius = 1.4\n"
+                                                         "Accurate_Triangulation = true\n"), ds)
+    surf.build()
+    surf.getSurf(True, True, 1.0, download=False)
+    c = surf._context().handle
+    nrem = ctypes.c_int64()
+    N.check(N.lib().nsg_filter_cavities(c, probe, 0, ctypes.byref(nrem)), "shape filter")
+    g = ds.grid
+    st = np.empty(g.nx * g.ny * g.nz, np.int32)
+    N.check(N.lib().nsg_download_status(c, N.ptr(st)), "status")
+    ref = oracle_mod.run(g, surf.patches, cav_vol=1.0, threads=8,
+                         flags=oracle_mod.STATUS | oracle_mod.ACCURATE_TRIANGULATION | oracle_mod.CAVITIES)
+    st_o, _fl, _bits, _eps, _ideb, nrem_o = oracle_mod.shape_filter(g, ref.status, ref.ncav, ref.cav_filled,
+                                                                    bits=ref.bits, probe=probe, mod_status=False)
+    assert ref.ncav >= 1 and nrem.value == nrem_o
+    np.testing.assert_array_equal(st, st_o.reshape(-1))
