@@ -59,11 +59,11 @@ WORKLOADS = {
 
 STAGES = ("bin", "trace", "overflow", "cavity", "vertex", "mc", "cand", "isect", "fill")
 
-# Floating-point operations per candidate of the mixed-precision intersection kernels (adds, muls
-# and 2 per fused multiply-add, predicated-on thread instructions), measured with ncu
-# (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma,fadd,fmul,ffma}_pred_on.sum) on the
-# 64-structure conformer ensemble and divided by its candidate counts.
-FLOPS_PER_CANDIDATE = {"torus": {"fp64": 312.0, "fp32": 35.0}, "sphere": {"fp64": 26.0, "fp32": 74.0}}
+# Floating-point operations per candidate of the mixed-precision intersection kernels, the FP32 torus
+# screen included (adds, muls and 2 per fused multiply-add, predicated-on thread instructions),
+# measured with ncu (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma,fadd,fmul,ffma}_pred_on.sum)
+# on the 64-structure conformer ensemble and divided by its candidate counts.
+FLOPS_PER_CANDIDATE = {"torus": {"fp64": 72.2, "fp32": 69.2}, "sphere": {"fp64": 25.2, "fp32": 85.7}}
 # Algorithmic operations per candidate: the oracle's operation model (oracle/oracle.py OP_MODEL:
 # adds and multiplies of doubles, FMA = 2; square roots, divisions and the resolvent's cube roots,
 # arccos and cos apart) summed over the branches the double-precision path takes, per candidate of
@@ -72,9 +72,9 @@ FLOPS_PER_CANDIDATE = {"torus": {"fp64": 312.0, "fp32": 35.0}, "sphere": {"fp64"
 OPS_PER_CANDIDATE = {"torus": {"flops": 180.0, "sqrt": 5.10, "div": 4.81, "cbrt": 1.37, "acos": 0.20, "cos": 0.20},
                      "sphere": {"flops": 73.8, "sqrt": 1.0, "div": 2.0}}
 # DRAM bytes (read + written) of the mixed intersection launches per candidate, from an ncu capture
-# of the 64-structure ensemble (the ray set of panel 1: 283 MB for the sphere launch, 224 MB for the
-# torus launch, 5 MB for the deferred ones, over its 19.9 M candidates)
-ISECT_DRAM_BYTES_PER_CANDIDATE = 25.7
+# of the 64-structure ensemble (four ray sets: 656 MB for the torus screen, 1,114 MB for the sphere
+# launch, 602 MB for the torus launch, 10 MB for the deferred ones, over 79.7 M candidates)
+ISECT_DRAM_BYTES_PER_CANDIDATE = 29.9
 
 
 def load_peaks() -> dict:
@@ -612,7 +612,8 @@ def run_ensemble(args, world: int, rank: int, local: int) -> None:
     fill_bytes = 3 * 2 * 4 * nwords + 8 * rays + 16 * nv
     roofline = {"bound": "fp64", "kernel": "k_isect (ray-patch intersection, 4 ray sets)", "achieved": ach_model,
                 "peak": pk64.value / 1e12, "unit": "TFLOP/s", "frac": ach_model / (pk64.value / 1e12),
-                "work": "algorithmic operation model of the oracle (OPS_PER_CANDIDATE) x the step's candidates; "
+                "work": "algorithmic operation model of the oracle (OPS_PER_CANDIDATE) x the step's candidates, "
+                        "the torus candidates that the FP32 screen rejects before the solver included; "
                         "isect time from the profiled pass with the ray sets run one after another",
                 "ops_per_step": {"flops": flops_model, **special},
                 "executed": {"note": "ncu-counted FP64/FP32 instructions per candidate (FLOPS_PER_CANDIDATE)",

@@ -13,9 +13,9 @@
 // The push pass (k_mc_push) writes each vertex that is the first of its grid edge into the slots
 // of the (up to four) cubes that share the edge: a ray's vertices are sorted along it, so the
 // vertices of an edge have consecutive ids, the first of them is the one whose predecessor has
-// another edge key, and a slot is written once, with a plain store (the slots start at -1; the
-// host clears and fills them structure chunk by structure chunk, so that a chunk's slots stay in
-// L2 between the two).  Active cubes add an edge-midpoint vertex to their own edges 5, 6, 10
+// another edge key, and a slot is written once, with a plain store (the slots start at -1: they
+// are cleared and filled structure chunk by structure chunk, so that a chunk's slots stay in L2
+// between the two, or, where all of them fit a tenth of L2, cleared by the classification).  Active cubes add an edge-midpoint vertex to their own edges 5, 6, 10
 // that carry no analytic vertex, in (k, j, i, edge) order, appended after the analytic ones
 // (getVertices :8002-8327), and write it into the slots in the same way.  The triangle pass emits
 // the case-table triangles with reversed winding and sums their areas (the reference sums Heron

@@ -1,16 +1,15 @@
-// Patch windows, tile binning and the fused ray-trace + interval-fill kernel of the SES ray caster.
+// Patch windows, candidates, torus screen, intersections and interval fill of the ray caster.
 //
 // The reference is patch-centric: every patch loops over the pixels of its bounding window,
 // tests the rays and pushes hits into per-pixel heap lists that are then sorted
 // (ConnollySurface::getPatchIntersectionData src/ConnollySurface.cpp:4319-4590,
 // Surface::countPixelIntersections/copyPatchIntersections/reorderPatchIntersections
 // src/Surface.cpp:4941-5095) and consumed by setVerticesAndGridsWithIntersectionData
-// (src/Surface.cpp:5101-6251).  Here the work is ray-centric: patches are binned into 32x4-pixel
-// tiles; a CTA owns one tile, stages its patch list through shared memory in chunks, every thread
-// traces one ray, keeps its hits sorted in a shared-memory column, pairs them and the warp then
-// writes the status rows / insideness bits of its 32 rays cooperatively (coalesced rows, ballot
-// masks + atomicAnd on the 32x-packed bit grid).  The candidate set of a ray is the reference's:
-// pixel inside the patch window, inside the bounding box, inside the equatorial disc.
+// (src/Surface.cpp:5101-6251).  Here the (ray, patch) candidates of a ray set are listed first, tested
+// one per thread, and the hits of a ray are sorted and paired by the warp that owns its tile of 32x4
+// pixels; the kernels are described at their places below.  The candidate set of a ray is the
+// reference's: pixel inside the patch window, inside the bounding box, inside the equatorial disc.
+// Only rays with more than 32 hits go through per-tile patch lists, one thread per ray.
 #include <limits.h>
 
 #include "pipeline.h"
@@ -24,8 +23,6 @@
 namespace nsg {
 
 namespace {
-
-
 
 // Pixel window of every patch (start, end per axis; -1 when culled) and the screen record of the torus
 // patches, with the panels' window-area sums (out[0..2], out[3..5] for the torus patches) and the
