@@ -653,7 +653,10 @@ int nsg_ctx_create(int device, nsg_ctx** out) {
 int nsg_ctx_destroy(nsg_ctx* c) {
   if (!c) return NSG_ERR_ARG;
   cudaSetDevice(c->device);
-  if (c->stream) cudaStreamSynchronize(c->stream);
+  // The buffers go to other contexts as idle ones below, so everything that was queued has to be done:
+  // on the own stream, or, for a caller's stream (which may be the default stream 0, or be gone by
+  // now), on the whole device.
+  if (!c->own_stream || cudaStreamSynchronize(c->stream) != cudaSuccess) cudaDeviceSynchronize();
   DevBuf* bufs[] = {&c->f64, &c->i32, &c->pool, &c->flag, &c->win, &c->pool32, &c->quad32, &c->quadl, &c->b_atoms, &c->b_field, &c->b_mask, &c->b_nv, &c->b_nt, &c->b_voff, &c->b_toff, &c->b_vraw, &c->b_verts, &c->b_vkey, &c->b_tris, &c->b_inc_cnt, &c->b_inc_off, &c->b_inc_cur, &c->b_inc, &c->b_patch_atoms, &c->b_gpost, &c->b_gpre, &c->b_gfield[0], &c->b_gfield[1], &c->b_gatoms, &c->b_win, &c->counters, &c->win_sums, &c->screen, &c->hit_cnt,
                     &c->status, &c->bits, &c->epsmap, &c->ideb, &c->bgp_ibgp, &c->bgp_type,
                     &c->bgp_pos, &c->bgp_nor, &c->bgp_flag, &c->bgp_n, &c->aux_cnt, &c->aux_off, &c->aux_list, &c->pairs,
@@ -691,7 +694,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
 int nsg_set_stream(nsg_ctx* c, void* stream) {
   if (!c) return NSG_ERR_ARG;
   CK(cudaSetDevice(c->device));
-  if (c->stream) CK(cudaStreamSynchronize(c->stream));
+  CK(cudaStreamSynchronize(c->stream));  // 0, the default stream, as well
   if (c->own_stream && c->stream) give_stream(c->device, c->stream);
   c->stream = (cudaStream_t)stream;
   c->own_stream = false;
