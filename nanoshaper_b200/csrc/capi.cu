@@ -1722,6 +1722,7 @@ int detect_cavities(nsg_ctx* c, double cav_vol, bool pockets, int* ncav_out) {
   }
   c->cav_labels = true;  // the dense map is written, with these labels, when a call reads it
   stage_end(c, kStageCavity);
+  CK(cudaStreamSynchronize(c->stream));  // the filling of the bits and of the epsilon map
   c->cav_detected = true;
   if (ncav_out) *ncav_out = c->ncav;
   c->n_vert = c->n_tri = 0;

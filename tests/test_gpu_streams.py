@@ -4,6 +4,7 @@
   to another stream, right after calls that leave work behind (an upload from pinned memory, cavity
   filling) hands its memory on only when that work is done, so that contexts made at once get their
   own results.
+* Cavity detection returns when nothing of it is left on the stream.
 """
 import ctypes
 
@@ -16,7 +17,7 @@ from nanoshaper_b200 import generator
 
 pytestmark = pytest.mark.gpu
 
-FLAGS = 1 | 2  # status map and triangulation rays
+FLAGS = 1 | 2 | 4  # status map, triangulation rays, epsilon maps
 
 
 def _surface(n_atoms, seed, scale):
@@ -96,4 +97,17 @@ def test_moved_between_streams(case):
     _same(ctx, want)
     N.check(ctx.L.nsg_set_stream(ctx.h, None), "stream")
     _same(ctx, want)
+    ctx.close()
+
+
+def test_cavity_detection_leaves_nothing_on_the_stream(native_lib):
+    import torch
+    surf = _surface(20000, 1, 4.0)
+    p = surf.patches
+    pinned = [torch.from_numpy(a).pin_memory() for a in (p.f64, p.i32, p.pool, p.pool_flag)]
+    stream = torch.cuda.Stream()
+    ctx = _Ctx(surf, pinned, stream.cuda_stream)
+    for _ in range(3):
+        ctx.cast()
+        assert stream.query()
     ctx.close()
