@@ -31,6 +31,26 @@ __device__ __forceinline__ unsigned int take_ticket(const LookBack& lb, unsigned
   return *s_ticket;
 }
 
+// The block's only ticket, and whether the block goes on: its thread 0 decides for all of its threads,
+// because another block of the same launch may set the error word at any moment, and threads that
+// read it for themselves could part before a warp-wide exchange (all threads of the block call it).
+// A block that does not go on leaves a count of 0, so that nobody waits for it.
+template <class Condition>
+__device__ __forceinline__ bool take_ticket_if(const LookBack& lb, Condition complete, unsigned int* ticket) {
+  __shared__ unsigned int s_ticket;
+  __shared__ int s_go;
+  if (threadIdx.x == 0) {
+    const unsigned int t = atomicAdd(lb.ticket, 1u);
+    const bool go = *(volatile const int32_t*)lb.err == 0 && complete();
+    if (!go) *(volatile unsigned long long*)(lb.state + t) = 1ull << 62;
+    s_ticket = t;
+    s_go = go;
+  }
+  __syncthreads();
+  *ticket = s_ticket;
+  return s_go != 0;
+}
+
 // Sum of the counts of the tickets before t, given this ticket's count; the whole block takes part
 // and every thread gets the result (-1 when the wait ran out).  A step looks at one earlier ticket
 // per thread: with a 32-ticket window the chain of sums moved 32 tickets per L2 round trip, about

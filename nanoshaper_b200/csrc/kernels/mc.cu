@@ -161,10 +161,12 @@ __device__ __forceinline__ void push_vertex(const int2* __restrict__ amap, int32
 
 constexpr int kPassThreads = 256;
 
-// Whether the passes before left complete arrays: no look-back wait ran out and their items fit.
-__device__ __forceinline__ bool cubes_ok(const MCArgs& A) {
-  return *A.lb_rows.err == 0 && A.counts[kMcActive] <= A.cap_active && A.counts[kMcAnalytic] <= A.cap_vert;
+// Whether the passes before left complete arrays: no look-back wait ran out and their items fit.  The
+// passes that look back themselves ask through take_ticket_if.
+__device__ __forceinline__ bool cubes_fit(const MCArgs& A) {
+  return A.counts[kMcActive] <= A.cap_active && A.counts[kMcAnalytic] <= A.cap_vert;
 }
+__device__ __forceinline__ bool cubes_ok(const MCArgs& A) { return *A.lb_rows.err == 0 && cubes_fit(A); }
 
 // Items (rays, map words, cubes) per thread of a one-pass kernel.  A block waits for the blocks
 // before it about as long as it counts, so a large input wants tickets with more work: 4 items per
@@ -460,10 +462,9 @@ __global__ void k_mc_clear(MCArgs A, int b0, int b1) {
 // cube's test reads a slot that another cube's midpoint is written to.  Bound by the slot reads.
 template <int kItems>
 __global__ void __launch_bounds__(kPassThreads) k_mc_mid(MCArgs A) {
-  __shared__ unsigned int s_ticket;
   const int64_t n_act = A.counts[kMcActive], n_an = A.counts[kMcAnalytic];
-  if (!cubes_ok(A)) return;
-  const unsigned t = take_ticket(A.lb_mid, &s_ticket);
+  unsigned t;
+  if (!take_ticket_if(A.lb_mid, [&] { return cubes_fit(A); }, &t)) return;
   if ((int64_t)t * (kPassThreads * kItems) >= n_act) return;
   const int lane = threadIdx.x & 31;
   const int64_t a0 = (int64_t)t * (kPassThreads * kItems) + (threadIdx.x >> 5) * (32 * kItems) + lane;
@@ -575,15 +576,15 @@ constexpr int kMaxCubeTris = 5;  // the most triangles of a case
 // every block read from the constant bank), 2,000 atoms 5 + 28 -> 22 us.
 template <int kMinBlocks, int kItems>
 __global__ void __launch_bounds__(kTrisThreads, kMinBlocks) k_mc_tris(MCArgs A) {
-  __shared__ unsigned int s_ticket;
   __shared__ alignas(16) int8_t s_tri[256][16];
   __shared__ alignas(16) uint8_t s_ntri[256];
   // per warp: each cube's vertex slots ([slot][lane]) and the areas of the warp's triangles
   __shared__ int32_t s_vid[kTrisWarps][12][32];
   __shared__ double s_area[kTrisWarps][kMaxCubeTris * 32];
   const int64_t n_act = A.counts[kMcActive], n_an = A.counts[kMcAnalytic];
-  if (!cubes_ok(A) || n_an + A.counts[kMcMidpoint] > A.cap_vert) return;
-  const unsigned ticket = take_ticket(A.lb_tris, &s_ticket);
+  unsigned ticket;
+  if (!take_ticket_if(A.lb_tris, [&] { return cubes_fit(A) && n_an + A.counts[kMcMidpoint] <= A.cap_vert; }, &ticket))
+    return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if ((int64_t)ticket * (kTrisThreads * kItems) >= n_act) return;
   const int64_t a0 = (int64_t)ticket * (kTrisThreads * kItems) + w * (32 * kItems) + lane;
