@@ -277,6 +277,7 @@ struct nsg_ctx {
   DevBuf pair_pid, ovf_pscratch, gvol, garea, vpid, vgrad;
   // atoms behind the patches (for the device chain rule) and the atom derivatives
   std::vector<int64_t> patch_off{0, 0};
+  std::vector<int64_t> cast_patch_off;  // of the last cast, whose triangulation may follow another upload
   DevBuf d_atoms, d_patch_atoms, d_gatoms_vol, d_gatoms_area, d_bad, d_patch_off, d_pool_off, d_atom_off;
   int64_t n_atoms = 0;
   bool have_atoms = false;
@@ -1587,6 +1588,7 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   c->eps_filled = false;
   c->have_bgp = c->bgp_projected = false;
   c->have_bits = do_mc;
+  c->cast_patch_off = c->patch_off;
   c->n_vert = c->n_tri = 0;
   return NSG_OK;
 }
@@ -1994,8 +1996,9 @@ int nsg_triangulate(nsg_ctx* c, double* area_out, int64_t* nverts, int64_t* ntri
     M.clear_slots = pair_verts <= kChunkCubes / 4;
     LAUNCH(nsg::launch_mc_rows(M, c->stream));
     const auto share = [&](int32_t b0, int32_t b1) -> int64_t {
-      const double np = (double)std::max<int64_t>(c->patch_off[nb], 1);
-      return (int64_t)((double)pair_verts * ((double)(c->patch_off[b1] - c->patch_off[b0]) / np)) + 1;
+      const std::vector<int64_t>& po = c->cast_patch_off;
+      const double np = (double)std::max<int64_t>(po[nb], 1);
+      return (int64_t)((double)pair_verts * ((double)(po[b1] - po[b0]) / np)) + 1;
     };
     for (int32_t b0 = 0; b0 < nb;) {
       int32_t b1 = M.clear_slots ? nb : b0 + 1;
