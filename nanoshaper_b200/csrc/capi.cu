@@ -419,9 +419,20 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
     if (G.nx < 3 || G.ny < 3 || G.nz < 3) return fail(NSG_ERR_ARG, "grid must have at least 3 nodes per axis");
     if (G.nx * G.ny * G.nz >= (int64_t)1 << 31) return fail(NSG_ERR_ARG, "grid larger than 2^31 nodes");
   }
+  // a batch that is refused leaves the one before as it is
+  for (int set = 0; set < nsg::kRaySets; set++) {
+    int64_t sum = 0;
+    for (int32_t b = 0; b < n; b++) {
+      const nsg::RaySet rs = nsg::make_ray_set(set, grid_dev(grids[b]));
+      sum += rs.nb * rs.na;
+    }
+    if (sum >= (int64_t)1 << 31) return fail(NSG_ERR_CAPACITY, "more than 2^31 rays in one ray set of a batch");
+  }
   // an earlier layout may still be on its way out of the pinned block
   CK(cudaStreamSynchronize(c->stream));
   CK(c->h_layout.ensure(layout_bytes(n)));
+  // from here on the tables of the batch before are gone, also when an allocation fails
+  c->has_grid = c->have_status = c->have_bits = false;
   CK(c->d_layout.ensure(layout_bytes(n)));
   nsg::StructDev* sd = c->h_layout.as<nsg::StructDev>();
   int64_t* base = (int64_t*)(sd + n);
@@ -459,10 +470,7 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
       S.box_dir[d] = S.g.mx[d] - S.g.mn[d];
     }
   }
-  for (int i = 0; i < nsg::kRaySets; i++) {
-    rb[i][n] = rays[i];
-    if (rays[i] >= (int64_t)1 << 31) return fail(NSG_ERR_CAPACITY, "more than 2^31 rays in one ray set of a batch");
-  }
+  for (int i = 0; i < nsg::kRaySets; i++) rb[i][n] = rays[i];
   mcb[n] = mc;
   awb[n] = awords;
   for (int i = 0; i < 3; i++) tb[i][n] = tiles[i];
@@ -477,7 +485,6 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
   c->words_tot = words;
   c->awords_tot = awords;
   c->has_grid = true;
-  c->have_status = c->have_bits = false;
   c->volumes.assign(n, 0.0);
   c->areas.assign(n, 0.0);
   return NSG_OK;

@@ -2,6 +2,7 @@
 
 * Patches uploaded or bound between a cast and its triangulation: the triangulation is that of the
   cast.
+* A batch that is refused (more than 2^31 rays) leaves the grid before in force.
 """
 import ctypes
 
@@ -48,3 +49,25 @@ def test_triangulation_after_another_upload(copies, bind, native_lib):
         N.check(_upload(h, _surface(60, 1).patches), "upload")
     assert (batch.triangulateSurface() == area).all()
     assert batch.n_triangles == copies * len(surf.triangles)
+
+
+def test_refused_batch_leaves_the_grid(native_lib):
+    surf = _surface(300, 2)
+    vol = surf.getSurf(True, False, 0.0)
+    area = surf.triangulateSurface()
+    h = surf.ctx.handle
+    g = N.NsGrid()
+    ctypes.pointer(g)[0] = surf.delphi.grid
+    g.nx = g.ny = g.nz = 1200  # 1.44 M rays per set and structure
+    n = 1500
+    grids = (N.NsGrid * n)(*[g] * n)
+    assert N.lib().nsg_set_batch(h, n, grids) == -4  # NSG_ERR_CAPACITY
+    # what the cast left is still there, and the next cast runs on the same grid
+    st = surf.delphi.status.copy()
+    now = np.empty_like(st)
+    N.check(N.lib().nsg_download_status(h, N.ptr(now)), "status")
+    assert np.array_equal(now, st)
+    v = ctypes.c_double()
+    N.check(N.lib().nsg_raycast(h, N.STATUS | N.ACCURATE_TRIANGULATION, 0, ctypes.byref(v)), "raycast")
+    assert v.value == vol
+    assert surf.triangulateSurface() == area
