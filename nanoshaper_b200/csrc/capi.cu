@@ -1283,6 +1283,12 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   }
   if (grad && (c->kind_mask & nsg::kSkinKinds))
     return fail(NSG_ERR_STATE, "gradients are provided for SES and mesh patch sets, not for skin cells");
+  // the results of the cast before are overwritten from here on, also by a cast that fails
+  c->have_status = c->have_bits = c->have_eps = c->have_pids = false;
+  c->cav_detected = c->have_cav_atoms = c->shape_filtered = c->ideb_ready = false;
+  c->have_bgp = c->bgp_projected = false;
+  c->runs_ready = c->cav_labels = c->status_dense = c->eps_filled = false;
+  c->n_vert = c->n_tri = 0;
   c->grad_mode = grad;
   c->have_gvol = c->have_garea = false;
   c->flags = flags;
@@ -1583,20 +1589,12 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   for (int32_t b = 0; b < nb; b++) c->volumes[b] = nvol ? c->grids[b].A * vsum[b] / nvol : 0.0;
   c->volume = c->volumes[0];
   if (volume) *volume = c->volume;
-  c->runs_ready = false;
-  c->cav_labels = false;
-  c->status_dense = false;
-  c->cav_detected = c->have_cav_atoms = false;
-  c->shape_filtered = c->ideb_ready = false;
   c->have_gvol = grad;
   c->have_pids = pids && do_mc;
   c->have_status = do_status || do_eps;
   c->have_eps = do_eps;
-  c->eps_filled = false;
-  c->have_bgp = c->bgp_projected = false;
   c->have_bits = do_mc;
   c->cast_patch_off = c->patch_off;
-  c->n_vert = c->n_tri = 0;
   return NSG_OK;
 }
 

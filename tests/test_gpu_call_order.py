@@ -3,6 +3,8 @@
 * Patches uploaded or bound between a cast and its triangulation: the triangulation is that of the
   cast.
 * A batch that is refused (more than 2^31 rays) leaves the grid before in force.
+* A cast that fails (a ray with more hits than the overflow path holds) leaves no results: calls on
+  the cast before it are refused, not answered from half-written arrays; the next cast is whole.
 """
 import ctypes
 
@@ -71,3 +73,27 @@ def test_refused_batch_leaves_the_grid(native_lib):
     N.check(N.lib().nsg_raycast(h, N.STATUS | N.ACCURATE_TRIANGULATION, 0, ctypes.byref(v)), "raycast")
     assert v.value == vol
     assert surf.triangulateSurface() == area
+
+
+def test_failed_cast_leaves_no_results(native_lib):
+    surf = _surface(327, 1)
+    vol = surf.getSurf(True, True, 10.0, download=False)
+    h = surf.ctx.handle
+    n = 1100  # spheres within one another: 2,200 hits on the rays through their common centre
+    f64, i32 = np.zeros((n, 20)), np.zeros((n, 4), np.int32)
+    f64[:, 3] = 1.5 + 1e-4 * np.arange(n)
+    g = surf.delphi.grid
+    status = np.empty(g.nx * g.ny * g.nz, np.int32)
+    ncav, area, v = ctypes.c_int(), ctypes.c_double(), ctypes.c_double()
+    nv, nt = ctypes.c_int64(), ctypes.c_int64()
+    flags = N.STATUS | N.ACCURATE_TRIANGULATION
+    N.check(N.lib().nsg_upload_patches(h, n, N.ptr(f64), N.ptr(i32), 0, None, None, 1.4), "upload")
+    assert N.lib().nsg_raycast(h, flags, 0, ctypes.byref(v)) == -4  # NSG_ERR_CAPACITY
+    for rc in (N.lib().nsg_cavities(h, 10.0, ctypes.byref(ncav)), N.lib().nsg_download_status(h, N.ptr(status)),
+               N.lib().nsg_triangulate(h, ctypes.byref(area), ctypes.byref(nv), ctypes.byref(nt)),
+               N.lib().nsg_filter_cavities(h, 1.4, 0, None)):
+        assert rc == -7  # NSG_ERR_STATE
+    N.check(_upload(h, surf.patches), "upload")
+    N.check(N.lib().nsg_raycast(h, flags, 0, ctypes.byref(v)), "raycast")
+    N.check(N.lib().nsg_cavities(h, 10.0, ctypes.byref(ncav)), "cavities")
+    assert v.value == vol and ncav.value > 0
