@@ -89,9 +89,13 @@ struct Member {
     return cudaSuccess;
   }
 
-  // This member's share of the job.
+  // This member's share of the job; without a stream or pinned blocks it leaves the chunks to the others.
   void work(Job& job) {
     cudaError_t e = ready(job.device);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
     int k = 0;
     Chunk prev{};
     while (e == cudaSuccess && job.err.load(std::memory_order_relaxed) == 0) {
@@ -115,11 +119,9 @@ struct Member {
       k++;
     }
     // the last block, and whatever is still on the link before the blocks are used again
-    if (stream) {
-      if (!job.to_device && e == cudaSuccess && k > 0) e = finish(job, prev, (k - 1) & 1);
-      const cudaError_t s = cudaStreamSynchronize(stream);
-      if (e == cudaSuccess) e = s;
-    }
+    if (!job.to_device && e == cudaSuccess && k > 0) e = finish(job, prev, (k - 1) & 1);
+    const cudaError_t s = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) e = s;
     if (e != cudaSuccess) {
       int none = 0;
       job.err.compare_exchange_strong(none, (int)e);
@@ -253,7 +255,12 @@ cudaError_t team_copy(const std::vector<TeamCopy>& copies, bool to_device, int d
       for (size_t off = 0; off < copies[q].bytes; off += step)
         job.chunks.push_back(Chunk{(int)q, off, std::min(step, copies[q].bytes - off)});
   t.run(job);
-  return (cudaError_t)job.err.load();
+  e = (cudaError_t)job.err.load();
+  if (e != cudaSuccess || job.next.load() >= job.chunks.size()) return e;
+  // no member could start (a limit on pinned memory, say): the runtime's copy
+  for (size_t q = 0; q < copies.size(); q++)
+    if (paged[q] && (e = plain_copy(copies[q], to_device, stream)) != cudaSuccess) return e;
+  return to_device ? cudaSuccess : cudaStreamSynchronize(stream);
 }
 
 void team_release() {

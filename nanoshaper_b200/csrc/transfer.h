@@ -28,9 +28,10 @@ struct TeamCopy {
 
 // Runs the copies (all to the device or all from it) and returns when the data has arrived.  Work
 // already queued on `stream` (which may use the device memory) is waited for first.  Copies that are
-// small or from pinned memory, and all copies while another thread uses the team, are queued on
-// `stream` itself: an upload may then still be on its way out of pinned memory when the call
-// returns, as cudaMemcpyAsync leaves it; a download has arrived in every case.
+// small or from pinned memory, and all copies while another thread uses the team or when none of its
+// threads can make its stream and pinned blocks, are queued on `stream` itself: an upload may then
+// still be on its way out of pinned memory when the call returns, as cudaMemcpyAsync leaves it; a
+// download has arrived in every case.
 cudaError_t team_copy(const std::vector<TeamCopy>& copies, bool to_device, int device, cudaStream_t stream);
 
 // Frees the team's pinned blocks (kept from one copy to the next, at most 2 MB per thread).
