@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -47,16 +48,24 @@ int fail(int code, const char* what, cudaError_t e = cudaSuccess) {
 // Device memory of the contexts comes from one memory pool per device, so that a context that lives
 // for one call (a torch program's forward and backward) does not map and unmap its hundred buffers
 // each time: 93 cudaMalloc and 93 cudaFree were 30 of the 31 ms of the gradient of a 2,000-atom
-// molecule.  The pool keeps at most kDevKept bytes of free memory (a few such contexts); what
-// exceeds it goes back to the driver at the next wait.  Blocks move between threads and contexts
-// only when nothing on the device uses them: a block is freed after a device wait (as cudaFree
-// waits) or after its context's streams have been waited for, and handed out after the pool's own
-// stream, which orders frees and allocations, has been waited for.
-constexpr uint64_t kDevKept = (uint64_t)8 << 30;
+// molecule.  What the pool keeps is bounded by bound_kept when a context ends or one of its buffers has
+// grown, and not by the pool's release threshold: that counts the memory in use as well, so beside
+// large live contexts nothing would be kept, and it unmaps at the next wait, inside another call.
+// Blocks move between threads and contexts only when nothing on the device uses them: a block is freed
+// after a device wait (as cudaFree waits) or after its context's work has been waited for, and handed
+// out after the pool's own stream, which orders frees and allocations, has been waited for.
+//
+// Kept are at most a sixteenth of what is free on the device otherwise, so that another allocator of
+// the process finds nearly all that it would find without the library, or kAlwaysKept (0.3 % of a
+// B200: two or three contexts of single molecules).  What is free (70 us to ask; a gradient call takes
+// 1,500) is looked at when the pool holds more than that and as much has come back since the last time.
+constexpr uint64_t kAlwaysKept = (uint64_t)512 << 20;
+constexpr uint64_t kKeptShare = 16;
 struct DevPool {
   std::mutex mu;
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
+  std::atomic<uint64_t> back{0};  // bytes that have come back since the bound was last looked at
 };
 DevPool* dev_pools() {
   static DevPool* pools = new DevPool[64];  // live to the process's end, like the contexts' memory
@@ -80,7 +89,7 @@ DevPool* dev_pool(cudaError_t* err) {
       props.location.id = dev;
       cudaMemPool_t pool = nullptr;
       if ((*err = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return nullptr;
-      uint64_t keep = kDevKept;
+      uint64_t keep = UINT64_MAX;
       if ((*err = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
         cudaMemPoolDestroy(pool);
         return nullptr;
@@ -93,6 +102,22 @@ DevPool* dev_pool(cudaError_t* err) {
     }
   }
   return d;
+}
+
+// Gives back what the pool holds free beyond its bound.
+void bound_kept(DevPool* d) {
+  if (d->back.load() <= kAlwaysKept) return;
+  d->back = 0;
+  uint64_t reserved = 0, used = 0;
+  size_t free_bytes = 0, total = 0;
+  if (cudaStreamSynchronize(d->stream) != cudaSuccess ||
+      cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return;
+  const uint64_t kept = reserved > used ? reserved - used : 0;
+  if (kept <= kAlwaysKept || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return;
+  const uint64_t most = std::max<uint64_t>(kAlwaysKept, ((uint64_t)free_bytes + kept) / kKeptShare);
+  if (kept > most) cudaMemPoolTrimTo(d->pool, used + most);
 }
 
 void trim_dev_pools() {
@@ -110,6 +135,7 @@ struct DevBuf {
   size_t cap = 0;
   cudaError_t ensure(size_t bytes) {
     if (bytes <= cap) return cudaSuccess;
+    const bool grows = p != nullptr;
     release();
     const size_t want = std::max<size_t>(bytes, 256);
     cudaError_t e = cudaSuccess;
@@ -126,6 +152,7 @@ struct DevBuf {
     if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
     if (e == cudaSuccess) cap = want;
     else p = nullptr;
+    if (grows) bound_kept(d);
     return e;
   }
   template <class T>
@@ -136,7 +163,7 @@ struct DevBuf {
     if (!idle) cudaDeviceSynchronize();
     cudaError_t e = cudaSuccess;
     DevPool* d = dev_pool(&e);
-    if (d) cudaFreeAsync(p, d->stream);
+    if (d && cudaFreeAsync(p, d->stream) == cudaSuccess) d->back += cap;
     p = nullptr;
     cap = 0;
   }
@@ -686,6 +713,8 @@ int nsg_ctx_destroy(nsg_ctx* c) {
     c->cand_sph[i].release(true); c->cand_tor[i].release(true); c->cand_scr[i].release(true); c->def_sph[i].release(true); c->def_tor[i].release(true);
     c->hit_t[i].release(true); c->hit_pid[i].release(true);
   }
+  cudaError_t pool_err = cudaSuccess;
+  if (DevPool* d = dev_pool(&pool_err)) bound_kept(d);
   for (int i = 0; i < 8; i++)
     if (c->user_ev[i]) cudaEventDestroy(c->user_ev[i]);
   for (int i = 0; i < 24; i++)
