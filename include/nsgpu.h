@@ -196,8 +196,8 @@ int nsg_batch_results(nsg_ctx* ctx, double* volumes, double* areas);
 /* ---- launch-shape tuning (no counterpart in the reference) ----
  * params: [intersection threads per block (64..256), intersection blocks per SM (1..64),
  * candidate-kernel threads per block (32..256), and optionally (n >= 4) the ray sets in shared
- * launches (1, default) or one after another (0), (n >= 5) a flag that is kept and reported without
- * effect, and (n >= 6) the blocks per SM of the marching-cubes triangle kernel (3, default, or 4);
+ * launches (1, default) or one after another (0), (n >= 5) the single-precision screen of the torus
+ * candidates (0, default: where there are many; 1: none; 2: always), and (n >= 6) the blocks per SM of the marching-cubes triangle kernel (3, default, or 4);
  * results do not depend on any of them].  nsg_autotune times
  * `reps` ray casts of the current batch per candidate shape and keeps the fastest in the
  * context. */

@@ -1039,7 +1039,7 @@ int nsg_set_tuning(nsg_ctx* c, const int32_t* params, int n) {
   c->tune.isect_bpsm = bpsm;
   c->tune.cand_threads = ct;
   if (n >= 4) c->concurrent_sets = params[3] != 0;
-  if (n >= 5) c->tune.torus_split = params[4] != 0;
+  if (n >= 5) c->tune.screen = params[4] == 0 || params[4] == 2 ? params[4] : 1;
   if (n >= 6) {
     if (params[5] != 3 && params[5] != 4) return fail(NSG_ERR_ARG, "tuning parameter 5 is 3 or 4");
     c->tune.mc_tris_bpsm = params[5];
@@ -1053,7 +1053,7 @@ int nsg_get_tuning(nsg_ctx* c, int32_t* params, int n) {
   params[1] = c->tune.isect_bpsm;
   params[2] = c->tune.cand_threads;
   if (n >= 4) params[3] = c->concurrent_sets ? 1 : 0;
-  if (n >= 5) params[4] = c->tune.torus_split;
+  if (n >= 5) params[4] = c->tune.screen;
   if (n >= 6) params[5] = c->tune.mc_tris_bpsm;
   return NSG_OK;
 }
@@ -1363,7 +1363,9 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   // The torus candidates of a set are screened where the windows hold 2^16 and more: below, the solve
   // of all of them takes as long as a launch does (327 atoms: 8 us either way, and 7 for the screen;
   // 2,000 atoms, 2^17: 18 us without, 15 with)
-  const auto screened = [&](int set) { return c->torus_area[nsg::ray_set_panel(set)] >= (1 << 16); };
+  const auto screened = [&](int set) {
+    return c->tune.screen == 2 || (c->tune.screen == 0 && c->torus_area[nsg::ray_set_panel(set)] >= (1 << 16));
+  };
   int64_t area_max = 0;  // candidates of a set, spheres or tori, at most
   {
     int64_t sph = 0, tor = 0;

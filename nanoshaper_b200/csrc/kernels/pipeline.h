@@ -205,7 +205,7 @@ struct TuneParams {
   int isect_threads = 256;  // threads per block of the intersection kernels (64..256)
   int isect_bpsm = 16;      // their blocks per SM (grid = SMs * isect_bpsm, grid-stride)
   int cand_threads = 256;   // threads per block of the candidate kernel (one warp per patch)
-  int torus_split = 0;      // accepted and reported, without effect (candidates are screened instead)
+  int screen = 0;           // torus candidates: 0 screened where there are many, 1 all solved, 2 all screened
   int mc_tris_bpsm = 3;     // blocks per SM of the marching-cubes triangle kernel (3 or 4)
 };
 
