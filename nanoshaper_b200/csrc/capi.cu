@@ -25,6 +25,7 @@
 #include "kernels/epsmap.h"
 #include "kernels/mc.h"
 #include "kernels/pipeline.h"
+#include "kept_blocks.h"
 #include "transfer.h"
 
 namespace {
@@ -211,8 +212,7 @@ void give_stream(int device, cudaStream_t s) {
 constexpr size_t kPinKept = (size_t)32 << 20;
 struct PinPool {
   std::mutex mu;
-  std::vector<std::pair<void*, size_t>> kept;
-  size_t bytes = 0;
+  nsg::KeptBlocks kept;
 };
 PinPool& pin_pool() {
   static PinPool* pool = new PinPool;  // lives to the process's end: contexts may outlive static objects
@@ -228,14 +228,7 @@ struct PinBuf {
     PinPool& pool = pin_pool();
     {
       std::lock_guard<std::mutex> g(pool.mu);
-      for (size_t q = 0; q < pool.kept.size(); q++)
-        if (pool.kept[q].second >= bytes) {
-          p = pool.kept[q].first;
-          cap = pool.kept[q].second;
-          pool.bytes -= cap;
-          pool.kept.erase(pool.kept.begin() + q);
-          return cudaSuccess;
-        }
+      if (pool.kept.take(bytes, &p, &cap)) return cudaSuccess;
     }
     const size_t want = std::max<size_t>((bytes + 4095) & ~(size_t)4095, 16384);
     cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocPortable);
@@ -249,12 +242,7 @@ struct PinBuf {
     if (!p) return;
     PinPool& pool = pin_pool();
     std::lock_guard<std::mutex> g(pool.mu);
-    if (pool.bytes + cap <= kPinKept) {
-      pool.kept.emplace_back(p, cap);
-      pool.bytes += cap;
-    } else {
-      cudaFreeHost(p);
-    }
+    if (!pool.kept.give(p, cap, kPinKept)) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
   }
@@ -938,9 +926,8 @@ int nsg_release_kept(void) {
   {
     PinPool& pool = pin_pool();
     std::lock_guard<std::mutex> g(pool.mu);
-    for (auto& b : pool.kept) cudaFreeHost(b.first);
-    pool.kept.clear();
-    pool.bytes = 0;
+    for (auto& b : pool.kept.blocks) cudaFreeHost(b.first);
+    pool.kept = nsg::KeptBlocks();
   }
   {
     StreamPool& pool = stream_pool();
