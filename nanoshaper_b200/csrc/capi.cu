@@ -557,9 +557,8 @@ cudaError_t download(nsg_ctx* c, const std::vector<nsg::TeamCopy>& copies) {
     CK(call);         \
   } while (0)
 
-// Exclusive scan of n int32 (or int64) counts into n+1 int64 offsets; returns the total.
-template <class In>
-int scan_counts(nsg_ctx* c, const In* in, int64_t n, int64_t* out, int64_t* total) {
+// Exclusive scan of n int32 counts into n+1 int64 offsets; returns the total.
+int scan_counts(nsg_ctx* c, const int32_t* in, int64_t n, int64_t* out, int64_t* total) {
   size_t tb = 0;
   CK(cub::DeviceScan::ExclusiveScan(nullptr, tb, in, out, cub::Sum(), (int64_t)0, n, c->stream));
   CK(c->temp.ensure(tb));

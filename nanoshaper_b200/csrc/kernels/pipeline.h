@@ -204,13 +204,12 @@ int sm_count();
 struct TuneParams {
   int isect_threads = 256;  // threads per block of the intersection kernels (64..256)
   int isect_bpsm = 16;      // their blocks per SM (grid = SMs * isect_bpsm, grid-stride)
-  int cand_threads = 256;   // threads per block of the candidate kernel (one warp per patch)
+  int cand_threads = 256;   // threads per block of the candidate kernel (a warp per 4 to 32 patches)
   int screen = 0;           // torus candidates: 0 screened where there are many, 1 all solved, 2 all screened
   int mc_tris_bpsm = 3;     // blocks per SM of the marching-cubes triangle kernel (3 or 4)
 };
 
-// trace.cu: every launch covers all structures of the batch; `set` is the ray set (0..3) and
-// tile and ray indices are batch-wide.
+// trace.cu: every launch covers all structures of the batch, tile and ray indices are batch-wide.
 // Patch windows and the torus patches' screen records; out (kWindowSums words, zeroed by the caller)
 // receives the window-area sum of each panel (the bound of its candidate count), the same of the
 // torus patches alone, and the bit mask of the patch kinds present.
@@ -220,7 +219,7 @@ cudaError_t launch_windows(const PatchDev& P, int32_t* win, float4* screen, cons
 // Patch-local FP32 copy of the pool: planes (n, d + n.c), clipping spheres (s - c, r^2); with
 // quad32, the skin cells' quadrics about their local origin (see k_pool32).
 cudaError_t launch_pool32(const PatchDev& P, float4* pool32, float4* quad32, double4* quadl, cudaStream_t s);
-// Patch counts of a panel's ray tiles (overflow path).
+// Patch counts and lists of a panel's ray tiles (overflow path), by one of the panel's ray sets.
 cudaError_t launch_bin_count(const PatchDev& P, const BatchDev& B, int set, int32_t* tile_cnt, cudaStream_t s);
 cudaError_t launch_bin_fill(const PatchDev& P, const BatchDev& B, int set, const int64_t* tile_off,
                             int32_t* tile_cursor, int32_t* tile_list, cudaStream_t s);

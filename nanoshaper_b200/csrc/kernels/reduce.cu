@@ -70,8 +70,7 @@ namespace nsg {
 
 namespace {
 
-template <class In>
-__global__ void k_scan_total(const In* __restrict__ in, int64_t n, int64_t* out) {
+__global__ void k_scan_total(const int32_t* __restrict__ in, int64_t n, int64_t* out) {
   out[n] = n > 0 ? out[n - 1] + (int64_t)in[n - 1] : 0;
 }
 
