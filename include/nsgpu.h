@@ -156,9 +156,9 @@ const char* nsg_last_error(void);
 int nsg_ctx_create(int device, nsg_ctx** out);
 int nsg_ctx_destroy(nsg_ctx* ctx);
 /* Memory, pinned host blocks and streams of destroyed contexts serve the next ones: per device at most
- * a sixteenth of the memory that is free otherwise (or 512 MiB; and at most 512 MiB more until the bound
- * is looked at again), in the process at most 32 MiB of pinned blocks, 64 streams, and 16 MiB of pinned
- * blocks of the copy threads.  This call gives back what no context uses. */
+ * a sixteenth of the memory that is free otherwise (or 512 MiB), looked at when more is kept than before
+ * or a context of more than 2 GiB ends; in the process at most 32 MiB of pinned blocks, 64 streams, and
+ * 16 MiB of pinned blocks of the copy threads.  This call gives back what no context uses. */
 int nsg_release_kept(void);
 int nsg_set_stream(nsg_ctx* ctx, void* cuda_stream);
 void* nsg_get_stream(nsg_ctx* ctx);

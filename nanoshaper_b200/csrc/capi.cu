@@ -58,15 +58,19 @@ int fail(int code, const char* what, cudaError_t e = cudaSuccess) {
 //
 // Kept are at most a sixteenth of what is free on the device otherwise, so that another allocator of
 // the process finds nearly all that it would find without the library, or kAlwaysKept (0.3 % of a
-// B200: two or three contexts of single molecules).  What is free (70 us to ask; a gradient call takes
-// 1,500) is looked at when the pool holds more than that and as much has come back since the last time.
+// B200: two or three contexts of single molecules).  What is free is a question to the kernel driver,
+// 70 us and at times tens of milliseconds while other processes map memory, where a gradient call takes
+// 1.5 ms: it is asked when more is kept than the last answer allowed (the pool has grown since, which
+// asks that driver too) or a context has given back more than kLargeContext.
 constexpr uint64_t kAlwaysKept = (uint64_t)512 << 20;
+constexpr uint64_t kLargeContext = (uint64_t)2 << 30;
 constexpr uint64_t kKeptShare = 16;
 struct DevPool {
   std::mutex mu;
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
-  std::atomic<uint64_t> back{0};  // bytes that have come back since the bound was last looked at
+  std::atomic<uint64_t> back{0};  // bytes that have come back since bound_kept was last called
+  uint64_t allowed = 0;           // free bytes that were kept when the bound was last looked at
 };
 DevPool* dev_pools() {
   static DevPool* pools = new DevPool[64];  // live to the process's end, like the contexts' memory
@@ -107,8 +111,8 @@ DevPool* dev_pool(cudaError_t* err) {
 
 // Gives back what the pool holds free beyond its bound.
 void bound_kept(DevPool* d) {
-  if (d->back.load() <= kAlwaysKept) return;
-  d->back = 0;
+  const uint64_t back = d->back.exchange(0);
+  std::lock_guard<std::mutex> g(d->mu);
   uint64_t reserved = 0, used = 0;
   size_t free_bytes = 0, total = 0;
   if (cudaStreamSynchronize(d->stream) != cudaSuccess ||
@@ -116,9 +120,16 @@ void bound_kept(DevPool* d) {
       cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
     return;
   const uint64_t kept = reserved > used ? reserved - used : 0;
-  if (kept <= kAlwaysKept || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return;
+  if (kept <= kAlwaysKept || (kept <= d->allowed && back <= kLargeContext) ||
+      cudaMemGetInfo(&free_bytes, &total) != cudaSuccess)
+    return;
   const uint64_t most = std::max<uint64_t>(kAlwaysKept, ((uint64_t)free_bytes + kept) / kKeptShare);
-  if (kept > most) cudaMemPoolTrimTo(d->pool, used + most);
+  d->allowed = kept;
+  if (kept <= most) return;
+  cudaMemPoolTrimTo(d->pool, used + most);
+  // the pool gives back whole chunks that nothing uses: what is left may exceed the bound by parts of some
+  if (cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess)
+    d->allowed = reserved > used ? reserved - used : 0;
 }
 
 void trim_dev_pools() {
@@ -128,6 +139,7 @@ void trim_dev_pools() {
     if (!d.stream) continue;
     cudaStreamSynchronize(d.stream);
     cudaMemPoolTrimTo(d.pool, 0);
+    d.allowed = 0;
   }
 }
 
