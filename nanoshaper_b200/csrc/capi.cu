@@ -60,17 +60,23 @@ int fail(int code, const char* what, cudaError_t e = cudaSuccess) {
 // the process finds nearly all that it would find without the library, or kAlwaysKept (0.3 % of a
 // B200: two or three contexts of single molecules).  What is free is a question to the kernel driver,
 // 70 us and at times tens of milliseconds while other processes map memory, where a gradient call takes
-// 1.5 ms: it is asked when more is kept than the last answer allowed (the pool has grown since, which
-// asks that driver too) or a context has given back more than kLargeContext.
+// 1.5 ms.  It is asked when more is kept than the last answer allowed, or a context has given back more
+// than kLargeContext.  The pool itself is looked at (3 us) when the sizes of the buffers say that more
+// may be kept, and at every kLookEvery-th end of a context or growth of a buffer for what they cannot say.
 constexpr uint64_t kAlwaysKept = (uint64_t)512 << 20;
 constexpr uint64_t kLargeContext = (uint64_t)2 << 30;
 constexpr uint64_t kKeptShare = 16;
+constexpr int kLookEvery = 64;
 struct DevPool {
   std::mutex mu;
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;
-  std::atomic<uint64_t> back{0};  // bytes that have come back since bound_kept was last called
-  uint64_t allowed = 0;           // free bytes that were kept when the bound was last looked at
+  std::atomic<uint64_t> in_use{0};       // bytes of all contexts' buffers
+  std::atomic<uint64_t> most_in_use{0};  // the most of them since the last look
+  std::atomic<uint64_t> back{0};         // bytes that have come back since bound_kept was last called
+  std::atomic<uint64_t> reserved{0};     // the pool's size at the last look
+  std::atomic<uint64_t> allowed{0};      // free bytes that it kept then
+  std::atomic<int> calls{0};             // of bound_kept since the last look
 };
 DevPool* dev_pools() {
   static DevPool* pools = new DevPool[64];  // live to the process's end, like the contexts' memory
@@ -111,7 +117,11 @@ DevPool* dev_pool(cudaError_t* err) {
 
 // Gives back what the pool holds free beyond its bound.
 void bound_kept(DevPool* d) {
-  const uint64_t back = d->back.exchange(0);
+  const uint64_t back = d->back.exchange(0), in_use = d->in_use;
+  const uint64_t size = std::max<uint64_t>(d->reserved, d->most_in_use);  // at least
+  // (the pool rounds the buffers' sizes up)
+  const uint64_t expected = std::max<uint64_t>(kAlwaysKept, d->allowed + kAlwaysKept / 8);
+  if (back <= kLargeContext && size <= in_use + expected && ++d->calls < kLookEvery) return;
   std::lock_guard<std::mutex> g(d->mu);
   uint64_t reserved = 0, used = 0;
   size_t free_bytes = 0, total = 0;
@@ -119,17 +129,19 @@ void bound_kept(DevPool* d) {
       cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
       cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
     return;
-  const uint64_t kept = reserved > used ? reserved - used : 0;
-  if (kept <= kAlwaysKept || (kept <= d->allowed && back <= kLargeContext) ||
-      cudaMemGetInfo(&free_bytes, &total) != cudaSuccess)
-    return;
-  const uint64_t most = std::max<uint64_t>(kAlwaysKept, ((uint64_t)free_bytes + kept) / kKeptShare);
-  d->allowed = kept;
-  if (kept <= most) return;
-  cudaMemPoolTrimTo(d->pool, used + most);
-  // the pool gives back whole chunks that nothing uses: what is left may exceed the bound by parts of some
-  if (cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess)
-    d->allowed = reserved > used ? reserved - used : 0;
+  uint64_t kept = reserved > used ? reserved - used : 0;
+  if (kept > kAlwaysKept && (kept > d->allowed || back > kLargeContext) &&
+      cudaMemGetInfo(&free_bytes, &total) == cudaSuccess) {
+    const uint64_t most = std::max<uint64_t>(kAlwaysKept, ((uint64_t)free_bytes + kept) / kKeptShare);
+    if (kept > most) cudaMemPoolTrimTo(d->pool, used + most);
+    // the pool gives back whole chunks that nothing uses: what is left may exceed the bound by parts of some
+    if (cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) return;
+    kept = reserved > used ? reserved - used : 0;
+    d->allowed = kept;
+  }
+  d->reserved = reserved;
+  d->most_in_use = in_use;
+  d->calls = 0;
 }
 
 void trim_dev_pools() {
@@ -139,7 +151,8 @@ void trim_dev_pools() {
     if (!d.stream) continue;
     cudaStreamSynchronize(d.stream);
     cudaMemPoolTrimTo(d.pool, 0);
-    d.allowed = 0;
+    d.reserved = d.allowed = 0;
+    d.most_in_use = d.in_use.load();
   }
 }
 
@@ -165,6 +178,10 @@ struct DevBuf {
     if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
     if (e == cudaSuccess) cap = want;
     else p = nullptr;
+    const uint64_t in_use = d->in_use += cap;
+    uint64_t most = d->most_in_use.load();
+    while (most < in_use && !d->most_in_use.compare_exchange_weak(most, in_use)) {
+    }
     if (grows) bound_kept(d);
     return e;
   }
@@ -176,7 +193,11 @@ struct DevBuf {
     if (!idle) cudaDeviceSynchronize();
     cudaError_t e = cudaSuccess;
     DevPool* d = dev_pool(&e);
-    if (d && cudaFreeAsync(p, d->stream) == cudaSuccess) d->back += cap;
+    if (d) {
+      cudaFreeAsync(p, d->stream);
+      d->in_use -= cap;
+      d->back += cap;
+    }
     p = nullptr;
     cap = 0;
   }
