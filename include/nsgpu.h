@@ -244,7 +244,8 @@ int nsg_blobby_atom_grads(nsg_ctx* ctx, double* d_volume, double* d_area);
 /* ---- the hot path ---- */
 /* Ray casting of Surface::getSurf: getPatchIntersectionData (src/ConnollySurface.cpp:4319-4590),
  * pixel binning and sort (src/Surface.cpp:4766-5095), setVerticesAndGridsWithIntersectionData
- * (src/Surface.cpp:5101-6251) and the volume (src/Surface.cpp:1680-1684). */
+ * (src/Surface.cpp:5101-6251) and the volume (src/Surface.cpp:1680-1684).  A cast that fails leaves no
+ * results: calls on those of the cast before return NSG_ERR_STATE. */
 int nsg_raycast(nsg_ctx* ctx, int flags, int precision, double* volume);
 /* getCavitiesWithBilevelStatusMap + fillCavities (src/Surface.cpp:1994-2126, 2355-2484). */
 int nsg_cavities(nsg_ctx* ctx, double cavity_volume, int* n_cavities);
