@@ -5,6 +5,8 @@
 * What is kept stays within a sixteenth of the memory that is free otherwise (or 512 MiB), so that other
   allocators of the process find the rest; nsg_release_kept gives back all of it.
 """
+import gc
+
 import numpy as np
 import pytest
 
@@ -45,6 +47,7 @@ def _run(surf):
 def test_kept_beside_large_contexts(native_lib):
     import torch
     torch.zeros(1, device="cuda")
+    gc.collect()  # contexts that other tests left
     N.release_kept()
     before = _free()
     live = [_large()]
@@ -72,6 +75,7 @@ def test_kept_beside_large_contexts(native_lib):
 def test_kept_is_a_share_of_what_is_free(left_gib, native_lib):
     import torch
     torch.zeros(1, device="cuda")
+    gc.collect()
     N.release_kept()
     others = torch.empty(_free() - (left_gib << 30), dtype=torch.uint8, device="cuda")
     before = _free()

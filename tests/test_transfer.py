@@ -22,7 +22,8 @@ MANY = 1 << 20
 def check(tmp_path_factory):
     out = tmp_path_factory.mktemp("transfer") / "transfer.so"
     cuda = Path(build._nvcc()).resolve().parents[1]
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I", str(build.CSRC), "-I",
+    # -Bsymbolic: the stand-in's calls, also where another library has loaded the real runtime
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-I", str(build.CSRC), "-I",
                     str(cuda / "include"), str(ROOT / "tests" / "cxx" / "transfer_check.cpp"), "-o", str(out)], check=True)
     fn = ctypes.CDLL(str(out)).transfer_check
     fn.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
