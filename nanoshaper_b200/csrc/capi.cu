@@ -325,7 +325,12 @@ struct nsg_ctx {
   DevBuf pair_pid, ovf_pscratch, gvol, garea, vpid, vgrad;
   // atoms behind the patches (for the device chain rule) and the atom derivatives
   std::vector<int64_t> patch_off{0, 0};
-  std::vector<int64_t> cast_patch_off;  // of the last cast, whose triangulation may follow another upload
+  // Of the last cast, whose results may be read after another upload or another grid: patches of another
+  // number, or nodes of a grid of another size, do not go with its arrays.
+  std::vector<int64_t> cast_patch_off;
+  int64_t cast_np = 0;
+  bool grid_moved = false;
+  NsGrid b_grid{};  // of the blobby field
   DevBuf d_atoms, d_patch_atoms, d_gatoms_vol, d_gatoms_area, d_bad, d_patch_off, d_pool_off, d_atom_off;
   int64_t n_atoms = 0;
   bool have_atoms = false;
@@ -459,6 +464,8 @@ cudaError_t upload_vec(DevBuf& d, const std::vector<T>& h, cudaStream_t s) {
   return cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
+bool same_nodes(const NsGrid& a, const NsGrid& b) { return a.nx == b.nx && a.ny == b.ny && a.nz == b.nz; }
+
 // Host and device layout of the batch: per-structure bases of tiles, rays, MC ray ordinals, map
 // words and bit words, filled in one pinned block and sent in one copy.
 int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
@@ -481,6 +488,7 @@ int batch_layout(nsg_ctx* c, const NsGrid* grids, int32_t n) {
   CK(c->h_layout.ensure(layout_bytes(n)));
   // from here on the tables of the batch before are gone, also when an allocation fails
   c->has_grid = c->have_status = c->have_bits = false;
+  if (n != 1 || c->nstruct != 1 || !same_nodes(grids[0], c->grid)) c->grid_moved = true;
   CK(c->d_layout.ensure(layout_bytes(n)));
   nsg::StructDev* sd = c->h_layout.as<nsg::StructDev>();
   int64_t* base = (int64_t*)(sd + n);
@@ -977,7 +985,8 @@ int nsg_release_kept(void) {
 // chained on the device; either host pointer may be NULL.
 int nsg_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
   if (!c) return NSG_ERR_ARG;
-  if (!c->have_gvol || !c->have_atoms) return fail(NSG_ERR_STATE, "needs a gradient-mode ray cast and the atoms");
+  if (!c->have_gvol || !c->have_atoms || c->np != c->cast_np)
+    return fail(NSG_ERR_STATE, "needs a gradient-mode ray cast and the atoms");
   CK(cudaSetDevice(c->device));
   const int64_t n = std::max<int64_t>(c->n_atoms, 1) * 4;
   CK(c->d_gatoms_vol.ensure(n * sizeof(double)));
@@ -1006,7 +1015,7 @@ int nsg_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
 // NS_GRAD_PER_PATCH doubles per patch in upload order; either pointer may be NULL.
 int nsg_patch_grads(nsg_ctx* c, double* gvol, double* garea) {
   if (!c) return NSG_ERR_ARG;
-  if ((gvol && !c->have_gvol) || (garea && !c->have_garea))
+  if ((gvol && !c->have_gvol) || (garea && !c->have_garea) || ((gvol || garea) && c->np != c->cast_np))
     return fail(NSG_ERR_STATE, "no gradient-mode ray cast / triangulation to read");
   CK(cudaSetDevice(c->device));
   const size_t bytes = (size_t)c->np * NS_GRAD_PER_PATCH * sizeof(double);
@@ -1217,6 +1226,7 @@ int nsg_blobby_build(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, doub
   rc = upload_common(c, nt, 0, 0.0);
   if (rc) return rc;
   c->b_natoms = n_atoms;
+  c->b_grid = G;
   c->b_nv_n = nv;
   c->b_nt_n = nt;
   c->b_B = blobbyness;
@@ -1247,7 +1257,8 @@ int nsg_blobby_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
   if (!c->b_valid) return fail(NSG_ERR_STATE, "no blobby mesh built");
   if (c->b_quantized)
     return fail(NSG_ERR_STATE, "the OFF round trip is piecewise constant: build with NSG_BLOBBY_DIFFERENTIABLE");
-  if ((d_volume && !c->have_gvol) || (d_area && !c->have_garea))
+  if ((d_volume && !c->have_gvol) || (d_area && !c->have_garea) ||
+      ((d_volume || d_area) && (c->np != c->cast_np || !same_nodes(c->grid, c->b_grid))))
     return fail(NSG_ERR_STATE, "no gradient-mode ray cast / triangulation to read");
   CK(cudaSetDevice(c->device));
   const NsGrid& G = c->grid;
@@ -1645,6 +1656,8 @@ int nsg_raycast(nsg_ctx* c, int flags, int precision, double* volume) {
   c->have_eps = do_eps;
   c->have_bits = do_mc;
   c->cast_patch_off = c->patch_off;
+  c->cast_np = c->np;
+  c->grid_moved = false;
   return NSG_OK;
 }
 
@@ -1862,6 +1875,7 @@ int nsg_filter_cavities(nsg_ctx* c, double probe_radius, int modify_status, int6
   if (c->shape_filtered) return fail(NSG_ERR_STATE, "the shape filter runs once per cavity detection");
   if (n_removed) *n_removed = 0;
   if (c->ncav == 0) return NSG_OK;
+  if (c->grid_moved) return fail(NSG_ERR_STATE, "the grid is not that of the cast");
   CK(cudaSetDevice(c->device));
   {
     int rc = ensure_dense_status(c);
@@ -1956,7 +1970,7 @@ int nsg_triangulate(nsg_ctx* c, double* area_out, int64_t* nverts, int64_t* ntri
   CK(cudaSetDevice(c->device));
   const nsg::BatchDev B = batch_dev(c);
   const int32_t nb = c->nstruct;
-  const bool grad = c->grad_mode && c->have_gvol;
+  const bool grad = c->grad_mode && c->have_gvol && c->np == c->cast_np;
   // Every pass places its items by look-back and leaves its count on the device, where the next
   // passes read it: the host reads the counts and the areas once, at the end.  The capacities come
   // from the pairs of the cast (two vertices each, and about as many active cubes); a pass that
@@ -2135,6 +2149,7 @@ int nsg_vertex_normals(nsg_ctx* c, double* normals) {
   if (!c->have_pids) return fail(NSG_ERR_STATE, "ray cast with NSG_RAYCAST_NORMALS (or NSG_RAYCAST_GRAD) first");
   const int64_t nv = c->n_vert, nt = c->n_tri;
   if (nv == 0) return NSG_OK;
+  if (c->np != c->cast_np) return fail(NSG_ERR_STATE, "the patches are not those of the cast");
   CK(cudaSetDevice(c->device));
   DevBuf dn;
   CK(dn.ensure(nv * 3 * sizeof(double)));
@@ -2189,7 +2204,7 @@ int nsg_download_cavities(nsg_ctx* c, double* sizes, int32_t* filled) {
 int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int32_t* offsets, int32_t* atoms,
                      int64_t* n_total) {
   if (!c || (n_atoms > 0 && !atoms_xyzr) || n_atoms < 0 || (atoms && !offsets)) return NSG_ERR_ARG;
-  if (!c->cav_detected || c->nstruct != 1)
+  if (!c->cav_detected || c->nstruct != 1 || (c->grid_moved && !c->have_cav_atoms))
     return fail(NSG_ERR_STATE, "cavity atoms need nsg_cavities after the cast");
   if (!c->have_cav_atoms) {
     CK(cudaSetDevice(c->device));
@@ -2332,7 +2347,7 @@ int nsg_cavity_atoms(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, int3
 // cavity filling when nsg_cavities ran on this ray cast.
 int nsg_download_epsmap(nsg_ctx* c, int32_t* dst) {
   if (!c || !dst) return NSG_ERR_ARG;
-  if (!c->have_eps) return fail(NSG_ERR_STATE, "no epsilon maps: ray cast with NSG_RAYCAST_EPSMAP");
+  if (!c->have_eps || c->grid_moved) return fail(NSG_ERR_STATE, "no epsilon maps: ray cast with NSG_RAYCAST_EPSMAP");
   CK(cudaSetDevice(c->device));
   const NsGrid& g = c->grid;
   CK(download(c, {whole(c->epsmap.p, dst, (size_t)g.nx * g.ny * g.nz * 3 * sizeof(int32_t))}));
@@ -2342,7 +2357,7 @@ int nsg_download_epsmap(nsg_ctx* c, int32_t* dst) {
 // ideb map (DelPhiShared::idebmap), 1 byte per node, (k*ny + j)*nx + i.
 int nsg_download_idebmap(nsg_ctx* c, uint8_t* dst) {
   if (!c || !dst) return NSG_ERR_ARG;
-  if (!c->have_eps) return fail(NSG_ERR_STATE, "no ideb map: ray cast with NSG_RAYCAST_EPSMAP");
+  if (!c->have_eps || c->grid_moved) return fail(NSG_ERR_STATE, "no ideb map: ray cast with NSG_RAYCAST_EPSMAP");
   CK(cudaSetDevice(c->device));
   const NsGrid& g = c->grid;
   const size_t nn = (size_t)g.nx * g.ny * g.nz;
@@ -2393,7 +2408,7 @@ nsg::AuxGrid aux_grid_of(const NsGrid& g, int64_t max_dim) {
 // ConnollySurface::getProjection); aux_max_dim is Max_ses_patches_auxiliary_grid_size (50).
 int nsg_bgp(nsg_ctx* c, int project, int32_t aux_max_dim, int64_t* n_bgp, int64_t* n_external) {
   if (!c) return NSG_ERR_ARG;
-  if (!c->have_eps) return fail(NSG_ERR_STATE, "boundary grid points need the epsilon maps (NSG_RAYCAST_EPSMAP)");
+  if (!c->have_eps || c->grid_moved) return fail(NSG_ERR_STATE, "boundary grid points need the epsilon maps (NSG_RAYCAST_EPSMAP)");
   if (project && (c->kind_mask & ~nsg::kSesKinds) && c->kind_mask != (1 << NS_MESH_TRI))
     return fail(NSG_ERR_STATE, "boundary grid point projection is provided for SES and mesh patch sets");
   if (project && aux_max_dim < 1) return fail(NSG_ERR_ARG, "auxiliary grid size must be positive");

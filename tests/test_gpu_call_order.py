@@ -5,6 +5,8 @@
 * A batch that is refused (more than 2^31 rays) leaves the grid before in force.
 * A cast that fails (a ray with more hits than the overflow path holds) leaves no results: calls on
   the cast before it are refused, not answered from half-written arrays; the next cast is whole.
+* Derivatives, normals and node maps of a cast are not read with patches of another number or a grid of
+  another size: refused; with as many patches, or a grid of the same size, they are answered as before.
 """
 import ctypes
 
@@ -97,3 +99,64 @@ def test_failed_cast_leaves_no_results(native_lib):
     N.check(N.lib().nsg_raycast(h, flags, 0, ctypes.byref(v)), "raycast")
     N.check(N.lib().nsg_cavities(h, 10.0, ctypes.byref(ncav)), "cavities")
     assert v.value == vol and ncav.value > 0
+
+
+def _read_all(h, n_patches, n_nodes, n_vertices):
+    """Result codes of the calls that read a cast's arrays by patch or by node."""
+    L = N.lib()
+    eps, ideb = np.empty(3 * n_nodes, np.int32), np.empty(n_nodes, np.uint8)
+    gv, normals = np.empty((n_patches, 8)), np.empty((n_vertices, 3))  # NSG_GRAD_PER_PATCH is 8
+    n = ctypes.c_int64()
+    by_patch = [L.nsg_patch_grads(h, N.ptr(gv), None), L.nsg_vertex_normals(h, N.ptr(normals))]
+    by_node = [L.nsg_download_epsmap(h, N.ptr(eps)), L.nsg_download_idebmap(h, N.ptr(ideb)),
+               L.nsg_bgp(h, 0, 50, ctypes.byref(n), None), L.nsg_filter_cavities(h, 1.4, 0, None)]
+    return by_patch, by_node
+
+
+def test_results_and_sizes_that_do_not_go_together(native_lib):
+    L = N.lib()
+    surf, other = _surface(327, 1), _surface(60, 1)
+    surf.getSurf(True, False, 0.0)
+    area = surf.triangulateSurface()
+    h, g, p = surf.ctx.handle, surf.delphi.grid, surf.patches
+    nodes = g.nx * g.ny * g.nz
+    v, ncav, a = ctypes.c_double(), ctypes.c_int(), ctypes.c_double()
+    nv, nt = ctypes.c_int64(), ctypes.c_int64()
+
+    def cast():
+        N.check(L.nsg_set_grid(h, ctypes.byref(g)), "grid")
+        N.check(_upload(h, p), "upload")
+        N.check(L.nsg_raycast(h, N.STATUS | N.ACCURATE_TRIANGULATION | N.EPSMAP | N.GRAD, 0, ctypes.byref(v)), "raycast")
+        N.check(L.nsg_cavities(h, 10.0, ctypes.byref(ncav)), "cavities")
+
+    def triangulate():
+        N.check(L.nsg_triangulate(h, ctypes.byref(a), ctypes.byref(nv), ctypes.byref(nt)), "triangulate")
+
+    cast()
+    triangulate()
+    assert _read_all(h, p.n, nodes, nv.value) == ([0, 0], [0, 0, 0, 0])
+    # as many patches, the same grid
+    cast()
+    triangulate()
+    N.check(_upload(h, p), "upload")
+    N.check(L.nsg_set_grid(h, ctypes.byref(g)), "grid")
+    assert _read_all(h, p.n, nodes, nv.value) == ([0, 0], [0, 0, 0, 0])
+    # fewer patches: the cast's triangulation without its derivatives
+    cast()
+    N.check(_upload(h, other.patches), "upload")
+    assert other.patches.n < p.n
+    triangulate()
+    assert nt.value > 0 and nv.value > 0
+    assert _read_all(h, p.n, nodes, nv.value) == ([-7, -7], [0, 0, 0, 0])
+    # a larger grid
+    cast()
+    triangulate()
+    larger = _surface(900, 1).delphi.grid
+    assert larger.nx > g.nx
+    N.check(L.nsg_set_grid(h, ctypes.byref(larger)), "grid")
+    assert _read_all(h, p.n, larger.nx * larger.ny * larger.nz, nv.value) == ([0, 0], [-7, -7, -7, -7])
+    # and whole again
+    cast()
+    triangulate()
+    assert _read_all(h, p.n, nodes, nv.value) == ([0, 0], [0, 0, 0, 0])
+    assert area > 0
