@@ -176,8 +176,12 @@ struct DevBuf {
       e = cudaMallocAsync(&p, want, d->pool, d->stream);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
-    if (e == cudaSuccess) cap = want;
-    else p = nullptr;
+    if (e == cudaSuccess) {
+      cap = want;
+    } else {
+      cudaGetLastError();  // reported here, not by the next launch
+      p = nullptr;
+    }
     const uint64_t in_use = d->in_use += cap;
     uint64_t most = d->most_in_use.load();
     while (most < in_use && !d->most_in_use.compare_exchange_weak(most, in_use)) {
@@ -265,8 +269,12 @@ struct PinBuf {
     }
     const size_t want = std::max<size_t>((bytes + 4095) & ~(size_t)4095, 16384);
     cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocPortable);
-    if (e == cudaSuccess) cap = want;
-    else p = nullptr;
+    if (e == cudaSuccess) {
+      cap = want;
+    } else {
+      cudaGetLastError();
+      p = nullptr;
+    }
     return e;
   }
   template <class T>
@@ -464,6 +472,8 @@ cudaError_t upload_vec(DevBuf& d, const std::vector<T>& h, cudaStream_t s) {
   return cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
+// Whether the context's patches can be those of the last cast (as far as their number says).
+bool cast_patches(const nsg_ctx* c) { return c->has_patches && c->np == c->cast_np; }
 bool same_nodes(const NsGrid& a, const NsGrid& b) { return a.nx == b.nx && a.ny == b.ny && a.nz == b.nz; }
 
 // Host and device layout of the batch: per-structure bases of tiles, rays, MC ray ordinals, map
@@ -800,6 +810,7 @@ int nsg_upload_patches(nsg_ctx* c, int64_t n, const double* f64, const int32_t* 
   if (!c || n < 0 || npool < 0 || (n > 0 && (!f64 || !i32)) || (npool > 0 && (!pool || !pool_flag)))
     return NSG_ERR_ARG;
   CK(cudaSetDevice(c->device));
+  c->has_patches = false;  // the set before is overwritten, also by an upload that fails
   CK(c->f64.ensure(std::max<int64_t>(n, 1) * NS_PATCH_F64 * sizeof(double)));
   CK(c->i32.ensure(std::max<int64_t>(n, 1) * NS_PATCH_I32 * sizeof(int32_t)));
   CK(c->pool.ensure(std::max<int64_t>(npool, 1) * 4 * sizeof(double)));
@@ -852,6 +863,7 @@ int upload_batch(nsg_ctx* c, const int64_t* patch_off, const BatchArray& f64, co
     return NSG_ERR_ARG;
   if (n >= (int64_t)1 << 31 || npool >= (int64_t)1 << 31) return fail(NSG_ERR_CAPACITY, "more than 2^31 patches");
   CK(cudaSetDevice(c->device));
+  c->has_patches = false;
   CK(c->f64.ensure(std::max<int64_t>(n, 1) * NS_PATCH_F64 * sizeof(double)));
   CK(c->i32.ensure(std::max<int64_t>(n, 1) * NS_PATCH_I32 * sizeof(int32_t)));
   CK(c->pool.ensure(std::max<int64_t>(npool, 1) * 4 * sizeof(double)));
@@ -985,7 +997,7 @@ int nsg_release_kept(void) {
 // chained on the device; either host pointer may be NULL.
 int nsg_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
   if (!c) return NSG_ERR_ARG;
-  if (!c->have_gvol || !c->have_atoms || c->np != c->cast_np)
+  if (!c->have_gvol || !c->have_atoms || !cast_patches(c))
     return fail(NSG_ERR_STATE, "needs a gradient-mode ray cast and the atoms");
   CK(cudaSetDevice(c->device));
   const int64_t n = std::max<int64_t>(c->n_atoms, 1) * 4;
@@ -1015,7 +1027,7 @@ int nsg_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
 // NS_GRAD_PER_PATCH doubles per patch in upload order; either pointer may be NULL.
 int nsg_patch_grads(nsg_ctx* c, double* gvol, double* garea) {
   if (!c) return NSG_ERR_ARG;
-  if ((gvol && !c->have_gvol) || (garea && !c->have_garea) || ((gvol || garea) && c->np != c->cast_np))
+  if ((gvol && !c->have_gvol) || (garea && !c->have_garea) || ((gvol || garea) && !cast_patches(c)))
     return fail(NSG_ERR_STATE, "no gradient-mode ray cast / triangulation to read");
   CK(cudaSetDevice(c->device));
   const size_t bytes = (size_t)c->np * NS_GRAD_PER_PATCH * sizeof(double);
@@ -1214,6 +1226,7 @@ int nsg_blobby_build(nsg_ctx* c, const double* atoms_xyzr, int64_t n_atoms, doub
   const bool quantize = !(flags & 1);
   if (quantize) LAUNCH(nsg::launch_quantize(c->b_verts.as<double>(), 3 * nv, s));
   // the triangles as the context's patch set
+  c->has_patches = false;
   CK(c->f64.ensure(std::max<int64_t>(nt, 1) * NS_PATCH_F64 * sizeof(double)));
   CK(c->i32.ensure(std::max<int64_t>(nt, 1) * NS_PATCH_I32 * sizeof(int32_t)));
   CK(c->pool.ensure(4 * sizeof(double)));
@@ -1258,7 +1271,7 @@ int nsg_blobby_atom_grads(nsg_ctx* c, double* d_volume, double* d_area) {
   if (c->b_quantized)
     return fail(NSG_ERR_STATE, "the OFF round trip is piecewise constant: build with NSG_BLOBBY_DIFFERENTIABLE");
   if ((d_volume && !c->have_gvol) || (d_area && !c->have_garea) ||
-      ((d_volume || d_area) && (c->np != c->cast_np || !same_nodes(c->grid, c->b_grid))))
+      ((d_volume || d_area) && (!cast_patches(c) || !same_nodes(c->grid, c->b_grid))))
     return fail(NSG_ERR_STATE, "no gradient-mode ray cast / triangulation to read");
   CK(cudaSetDevice(c->device));
   const NsGrid& G = c->grid;
@@ -1970,7 +1983,7 @@ int nsg_triangulate(nsg_ctx* c, double* area_out, int64_t* nverts, int64_t* ntri
   CK(cudaSetDevice(c->device));
   const nsg::BatchDev B = batch_dev(c);
   const int32_t nb = c->nstruct;
-  const bool grad = c->grad_mode && c->have_gvol && c->np == c->cast_np;
+  const bool grad = c->grad_mode && c->have_gvol && cast_patches(c);
   // Every pass places its items by look-back and leaves its count on the device, where the next
   // passes read it: the host reads the counts and the areas once, at the end.  The capacities come
   // from the pairs of the cast (two vertices each, and about as many active cubes); a pass that
@@ -2149,7 +2162,7 @@ int nsg_vertex_normals(nsg_ctx* c, double* normals) {
   if (!c->have_pids) return fail(NSG_ERR_STATE, "ray cast with NSG_RAYCAST_NORMALS (or NSG_RAYCAST_GRAD) first");
   const int64_t nv = c->n_vert, nt = c->n_tri;
   if (nv == 0) return NSG_OK;
-  if (c->np != c->cast_np) return fail(NSG_ERR_STATE, "the patches are not those of the cast");
+  if (!cast_patches(c)) return fail(NSG_ERR_STATE, "the patches are not those of the cast");
   CK(cudaSetDevice(c->device));
   DevBuf dn;
   CK(dn.ensure(nv * 3 * sizeof(double)));
@@ -2412,6 +2425,7 @@ int nsg_bgp(nsg_ctx* c, int project, int32_t aux_max_dim, int64_t* n_bgp, int64_
   if (project && (c->kind_mask & ~nsg::kSesKinds) && c->kind_mask != (1 << NS_MESH_TRI))
     return fail(NSG_ERR_STATE, "boundary grid point projection is provided for SES and mesh patch sets");
   if (project && aux_max_dim < 1) return fail(NSG_ERR_ARG, "auxiliary grid size must be positive");
+  if (project && !c->has_patches) return fail(NSG_ERR_STATE, "no patches to project on");
   CK(cudaSetDevice(c->device));
   const NsGrid& g = c->grid;
   const int32_t* eps = c->epsmap.as<int32_t>();

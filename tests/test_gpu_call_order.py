@@ -7,6 +7,8 @@
   the cast before it are refused, not answered from half-written arrays; the next cast is whole.
 * Derivatives, normals and node maps of a cast are not read with patches of another number or a grid of
   another size: refused; with as many patches, or a grid of the same size, they are answered as before.
+* An upload that fails for want of memory leaves no patches, and its error does not come back with the
+  next call.
 """
 import ctypes
 
@@ -160,3 +162,25 @@ def test_results_and_sizes_that_do_not_go_together(native_lib):
     triangulate()
     assert _read_all(h, p.n, nodes, nv.value) == ([0, 0], [0, 0, 0, 0])
     assert area > 0
+
+
+def test_failed_upload_leaves_no_patches(native_lib):
+    L = N.lib()
+    surf = _surface(327, 1)
+    vol = surf.getSurf(True, False, 0.0)
+    area = surf.triangulateSurface()
+    h, p = surf.ctx.handle, surf.patches
+    v, a = ctypes.c_double(), ctypes.c_double()
+    nv, nt = ctypes.c_int64(), ctypes.c_int64()
+    flags = N.STATUS | N.ACCURATE_TRIANGULATION | N.GRAD
+    N.check(L.nsg_raycast(h, flags, 0, ctypes.byref(v)), "raycast")
+    n = 1500 * 10**6  # 240 GB of records, refused before the host arrays are read
+    assert L.nsg_upload_patches(h, n, N.ptr(p.f64), N.ptr(p.i32), 0, None, None, p.probe) < 0
+    assert L.nsg_raycast(h, flags, 0, ctypes.byref(v)) == -7
+    N.check(L.nsg_triangulate(h, ctypes.byref(a), ctypes.byref(nv), ctypes.byref(nt)), "triangulate")
+    assert a.value == area  # the cast's, without derivatives
+    gv = np.empty((p.n, 8))
+    assert L.nsg_patch_grads(h, N.ptr(gv), None) == -7
+    N.check(_upload(h, p), "upload")
+    N.check(L.nsg_raycast(h, flags, 0, ctypes.byref(v)), "raycast")
+    assert v.value == vol
