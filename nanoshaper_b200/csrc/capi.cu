@@ -1805,7 +1805,9 @@ int detect_cavities(nsg_ctx* c, double cav_vol, bool pockets, int* ncav_out) {
   }
   c->cav_labels = true;  // the dense map is written, with these labels, when a call reads it
   stage_end(c, kStageCavity);
-  CK(cudaStreamSynchronize(c->stream));  // the filling of the bits and of the epsilon map
+  // a caller's stream is left idle: the filling of the bits and of the epsilon map is done.  On the own
+  // stream only calls that come after it read them (the wait is 15 us of 970 for 327 atoms).
+  if (!c->own_stream) CK(cudaStreamSynchronize(c->stream));
   c->cav_detected = true;
   if (ncav_out) *ncav_out = c->ncav;
   c->n_vert = c->n_tri = 0;
